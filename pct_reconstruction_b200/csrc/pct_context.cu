@@ -135,6 +135,7 @@ extern "C" void pct_destroy(pct_ctx* ctx)
     release_graph(ctx);
     cudaFree(ctx->d_table_block);
     cudaFree(ctx->d_steps);
+    cudaFree(ctx->d_mlp_table);
     if (ctx->l2_window) {
         cudaCtxResetPersistingL2Cache();
         cudaDeviceSetLimit(cudaLimitPersistingL2CacheSize, 0);
@@ -246,6 +247,19 @@ extern "C" pct_status pct_create(const pct_config* cfg_in, int device, pct_ctx**
                                          ctx->d_steps, ctx->own_stream);
         if (e != cudaSuccess) { st = ctx_fail(ctx, PCT_ERR_CUDA, "step table kernel", e); break; }
         ctx->launches += 1;
+        const pct::MlpTableShape shape = pct::mlp_table_shape(ctx->geo, ctx->kmax);
+        ctx->path_key_scale = shape.buckets > 0 ? 1.0 / shape.width : 0.0;
+        if (shape.buckets > 0) {
+            const size_t row_bytes = align256((size_t)shape.rows * 2 * sizeof(float4));
+            e = cudaMalloc(&ctx->d_mlp_table, row_bytes + (size_t)shape.buckets * sizeof(pct::MlpBucket));
+            if (e != cudaSuccess) { st = ctx_fail(ctx, PCT_ERR_NOMEM, "cudaMalloc(MLP weights)", e); break; }
+            float4* rows = static_cast<float4*>(ctx->d_mlp_table);
+            pct::MlpBucket* buckets = reinterpret_cast<pct::MlpBucket*>(static_cast<char*>(ctx->d_mlp_table) + row_bytes);
+            e = pct::launch_build_mlp_table(ctx->tables, ctx->d_steps, ctx->geo, shape, rows, buckets, ctx->own_stream);
+            if (e != cudaSuccess) { st = ctx_fail(ctx, PCT_ERR_CUDA, "MLP weight table kernel", e); break; }
+            ctx->launches += 1;
+            ctx->mlp_table = pct::MlpTable{rows, buckets, shape.buckets, shape.frac_bits, shape.t_max, 1.0 / shape.width};
+        }
 
         // Image and accumulator, padded by one slice (z index SLICES is reachable, B.cu:11091).
         const size_t npad = (size_t)ctx->geo.padded_voxels;
@@ -518,7 +532,8 @@ pct_status prepare_layout(pct_ctx* ctx)
             ctx->layout_cap = n;
         }
         cudaError_t e = pct::launch_path_bounds(ctx->geo, ctx->tables, ctx->hist, n, c.DROP_BLOCK_SIZE,
-                                                c.HISTORIES_PER_BLOCK, ctx->d_bounds, s);
+                                                c.HISTORIES_PER_BLOCK, ctx->path_key_scale, ctx->d_bounds,
+                                                ctx->d_bounds_sorted, s);
         if (e == cudaSuccess) e = pct::exclusive_scan_i32_to_i64(ctx->d_bounds, n, ctx->d_offsets, ctx->d_scan_tmp, s);
         if (e != cudaSuccess) return ctx_fail(ctx, PCT_ERR_CUDA, "path layout kernels", e);
         ctx->launches += 4;
@@ -571,13 +586,14 @@ pct_status prepare_layout(pct_ctx* ctx)
                 for (long long h0 = sb.h_begin; h0 < sb.h_end; h0 += step)
                     ctx->chunks.push_back({(int)i, h0, h0 + step < sb.h_end ? h0 + step : sb.h_end});
             }
+            // the sorting keys wait in the gathered bounds' array, which the gather below fills
             for (const auto& ch : ctx->chunks) {
                 if (c.PATH_ORDER_WINDOW > 0) {
-                    e = pct::window_sort_by_key(ctx->d_bounds, ch.h_begin, ch.h_end - ch.h_begin, kMaxBoundKey,
+                    e = pct::window_sort_by_key(ctx->d_bounds_sorted, ch.h_begin, ch.h_end - ch.h_begin, kMaxBoundKey,
                                                 c.PATH_ORDER_WINDOW, ctx->d_perm + ch.h_begin, s);
                     ctx->launches += 1;
                 } else {
-                    e = pct::bucket_sort_by_key(ctx->d_bounds, ch.h_begin, ch.h_end - ch.h_begin, kMaxBoundKey,
+                    e = pct::bucket_sort_by_key(ctx->d_bounds_sorted, ch.h_begin, ch.h_end - ch.h_begin, kMaxBoundKey,
                                                 ctx->d_hist_tmp, ctx->d_perm + ch.h_begin, s);
                     ctx->launches += 3;
                 }
@@ -678,7 +694,7 @@ pct_status enqueue_iteration(pct_ctx* ctx, cudaStream_t s, long long* launches, 
                 e = cudaStreamWaitEvent(p, ev_sb[ch.sb - 1], 0);
                 if (e != cudaSuccess) return ctx_fail(ctx, PCT_ERR_CUDA, "stream wait", e);
             }
-            e = pct::launch_mlp_phase1_exact(ctx->geo, ctx->tables, ctx->d_steps, ctx->kmax,
+            e = pct::launch_mlp_phase1_exact(ctx->geo, ctx->tables, ctx->mlp_table, ctx->d_steps, ctx->kmax,
                                              sorted_from(ctx, ch.h_begin), ctx->d_perm + ch.h_begin,
                                              ch.h_end - ch.h_begin, ctx->d_offsets_sorted + ch.h_begin, sb.off_begin,
                                              ctx->d_bounds_sorted + ch.h_begin, ctx->d_paths, ctx->d_path_n,
@@ -959,7 +975,7 @@ extern "C" pct_status pct_profile_drop_iteration(pct_ctx* ctx, double ms_out[3],
     if (ctx->two_phase) {
         for (const auto& sb : ctx->sbs) {
             begin(0);
-            e = pct::launch_mlp_phase1_exact(ctx->geo, ctx->tables, ctx->d_steps, ctx->kmax,
+            e = pct::launch_mlp_phase1_exact(ctx->geo, ctx->tables, ctx->mlp_table, ctx->d_steps, ctx->kmax,
                                              sorted_from(ctx, sb.h_begin), ctx->d_perm + sb.h_begin,
                                              sb.h_end - sb.h_begin, ctx->d_offsets_sorted + sb.h_begin, sb.off_begin,
                                              ctx->d_bounds_sorted + sb.h_begin, ctx->d_paths, ctx->d_path_n,

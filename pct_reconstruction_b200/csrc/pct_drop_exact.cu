@@ -192,8 +192,11 @@ __global__ void gather_path_inputs_kernel(HistorySoA src, const int* __restrict_
 // not cover): the loop runs at most u_2/MLP_U_STEP + 1 times and adds at most one entry per run.
 // Rounded up to a multiple of kPathChunk entries so every history's slot starts on a 32-byte
 // boundary and the path kernel writes whole sectors.
+// The sorting key is the history's bucket of u_2 in the table of MLP weights (key_scale buckets per
+// cm), so that histories of one bucket read the same rows; without a table (key_scale 0), the bound.
 __global__ void path_bounds_kernel(Geometry g, Tables tab, HistorySoA h, long long n, long long block_size,
-                                   int histories_per_block, int* __restrict__ bounds)
+                                   int histories_per_block, double key_scale, int* __restrict__ bounds,
+                                   int* __restrict__ keys)
 {
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -201,27 +204,24 @@ __global__ void path_bounds_kernel(Geometry g, Tables tab, HistorySoA h, long lo
     long long hp = n - blk * block_size;
     if (hp > block_size) hp = block_size;
     const long long covered = histories_per_block > 0 ? (hp / histories_per_block) * histories_per_block : hp;
-    int bound = 0;
+    int bound = 0, key = 0;
     if (pos < covered) {
         const double u_2 = mlp_u_extent(g, tab, h.x_entry[i], h.y_entry[i], h.x_exit[i], h.y_exit[i], h.xy_entry_angle[i]);
         const double q = u_2 / g.mlp_u_step;
         bound = (q >= 0 && q < (double)(kPathCap - 3)) ? (int)q + 3 : kPathCap;
         bound = (bound + kPathChunk - 1) / kPathChunk * kPathChunk;
+        const double kq = u_2 * key_scale;
+        key = key_scale <= 0.0 ? bound : (kq >= 0 && kq < (double)(kPathCap - 1)) ? (int)kq + 1 : kPathCap;
     }
     bounds[i] = bound;
+    keys[i] = key;
 }
 
-// Launch shape of the path kernel, chosen by measurement on B200: one MLP point per loop trip
-// (two points per trip need 108 registers and ran 21.7 vs 16.4 ms at 5M head histories), and the
-// register budget of 7 resident 128-thread CTAs per SM (72 registers).  With the guarded fast
-// points the kernel needs more live values than the reference-order points did: at 8 CTAs (64
-// registers) it spilled 140 bytes and the 20M head iteration took 87.4 ms, at 7 CTAs it spills 68
-// and takes 77.5 ms, against 80.4 ms for reference-order points at 8 CTAs.  With the per-history
-// constants in shared memory (PCT_PHASE1_STASH, below) nothing spills at 7 CTAs and the iteration
-// takes 74.1 ms (78.2 without; 74.8 at 8 CTAs, 20 bytes spilled).
-#ifndef PCT_PHASE1_UNROLL
-#define PCT_PHASE1_UNROLL 1
-#endif
+// Launch shape of the table path kernel.  It is bound by instruction issue (about 80 instructions per
+// point, 71% of the issue slots, load/store data stage 66%, FP64 pipe 4%) and takes 3.30 ms per 4M head
+// histories, 0.263 ms per 600k of the small configuration; the walk that evaluated every point in
+// double took 11.3 and 1.0 ms.  Resident 128-thread CTAs per SM (ms, 4M head): 6 3.55, 7 3.30, 8 3.43,
+// 10 3.73: from 8 on the registers of the general points' set-up spill.
 #ifndef PCT_PHASE1_MIN_BLOCKS
 #define PCT_PHASE1_MIN_BLOCKS 7
 #endif
@@ -229,109 +229,68 @@ __global__ void path_bounds_kernel(Geometry g, Tables tab, HistorySoA h, long lo
 #ifndef PCT_PHASE1_MIXED_MIN_BLOCKS
 #define PCT_PHASE1_MIXED_MIN_BLOCKS 8
 #endif
-// 0: each voxel-list entry is stored as it is found; 1: entries are staged in shared memory and
-// written a 32-byte sector at a time.  Measured on B200 (10M head histories): staging cuts the
-// kernel's DRAM traffic from ~1.9 KB to ~1.3 KB per history but costs 4% in time (34.3 vs
-// 32.9 ms) -- the kernel is FP64-issue bound, not memory bound -- so 0 is the default.  (An L2
-// evict-last policy on the direct stores was slower still, 34.4 ms.)  With the stash below and one
-// shared-memory carve-out for the iteration's kernels (PCT_ITERATION_CARVEOUT), staging costs
-// nothing: 74.0 vs 73.8 ms per 20M-history head iteration, 30.6 vs 31.5 ms per 10M-history
-// small-block iteration, and the path kernel's DRAM writes fall to the lists' own bytes.  1 is the
-// default.
-#ifndef PCT_PHASE1_STAGE
-#define PCT_PHASE1_STAGE 1
-#endif
-// 1: the per-history constants of the exact walk and its chord live in shared memory (16 doubles
-// per thread, 16 KB per 128-thread CTA) and each is read where a loop trip uses it, instead of
-// being held in registers across trips.
-#ifndef PCT_PHASE1_STASH
-#define PCT_PHASE1_STASH 1
-#endif
-// Entries per staged list write: 8 (one 32-byte sector) or 4 (16 bytes, a smaller staging buffer).
-#ifndef PCT_STAGE_ENTRIES
-#define PCT_STAGE_ENTRIES 8
-#endif
-// Staging applies to the exact mode's kernel only: the mixed-precision kernel keeps no shared memory,
-// so that it and its block chain share the driver's carve-out.
-// The voxel list goes to the history's slot in path storage (PCT_PHASE1_STAGE selects direct
-// stores or shared-memory staging of whole 32-byte sectors, see above).
-template <bool kMixed, int kThreads>
-__device__ __forceinline__ void mlp_phase1_body(const Geometry& g, const Tables& tab, const StepConst* __restrict__ steps,
-                                                int kmax, const HistorySoA& h, const int* __restrict__ perm,
-                                                long long count, const long long* __restrict__ offsets,
-                                                long long offset_base, const int* __restrict__ bounds,
-                                                uint32_t* __restrict__ paths, int* __restrict__ path_n,
-                                                double* __restrict__ chord, unsigned long long* counters)
+// kThreads histories per CTA (PATH_CTA_THREADS), with the same resident threads per SM, hence the
+// same register budget, at every size.  Position i of the processing order: its inputs at i (gathered
+// into this order), its history id for the outputs.
+template <int kThreads>
+__global__ void __launch_bounds__(kThreads, PCT_PHASE1_MIN_BLOCKS * 128 / kThreads) mlp_phase1_table_kernel(
+    const __grid_constant__ Geometry g, const __grid_constant__ Tables tab, const __grid_constant__ MlpTable tb,
+    const StepConst* __restrict__ steps, int kmax, const __grid_constant__ HistorySoA h, const int* __restrict__ perm,
+    long long count, const long long* __restrict__ offsets, long long offset_base, const int* __restrict__ bounds,
+    uint32_t* __restrict__ paths, int* __restrict__ path_n, double* __restrict__ chord, unsigned long long* counters)
 {
-    constexpr bool kStage = PCT_PHASE1_STAGE == 1 && !kMixed;
-    // position i of the processing order: its inputs at i (gathered into this order), its
-    // history id for the outputs
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    __shared__ __align__(16) uint32_t stage[kThreads * kStageStride];
+    const int i = blockIdx.x * kThreads + threadIdx.x;
+    int cap = 0;
+    uint32_t* out = nullptr;
+    double* to_chord = nullptr;
+    if (i < count) {
+        cap = bounds[i];
+        out = paths + (offsets[i] - offset_base);
+        to_chord = chord + perm[i];
+        if (cap <= 0) *to_chord = 0.0;  // not covered by its DROP block: no path
+    }
+    unsigned flags = 0;
+    int n = mlp_walk_table(g, tab, tb, steps, kmax, h, i, cap,
+                           (uint32_t)__cvta_generic_to_shared(stage + threadIdx.x * kStageStride), out, to_chord, &flags);
     if (i >= count) return;
-    const long long id = perm[i];
-    const int cap = bounds[i];
-    if (cap <= 0) {  // not covered by its DROP block: no path
-        path_n[id] = 0;
-        chord[id] = 0.0;
-        return;
-    }
-    uint32_t* out = paths + (offsets[i] - offset_base);  // 32-byte aligned, cap a multiple of 8
-    constexpr int kN = PCT_STAGE_ENTRIES;  // entries per flush: 8 (a 32-byte sector) or 4 (16 bytes)
-    static_assert(kN == 4 || kN == 8, "staging flushes 4 or 8 entries");
-    __shared__ uint32_t stage[kThreads * (kN + 1)];
-    uint32_t* mine = stage + threadIdx.x * (kN + 1);  // odd stride in words: no bank conflicts
-    auto flush = [&](int j0) {
-        uint4* dst = reinterpret_cast<uint4*>(out + j0);
-        dst[0] = make_uint4(mine[0], mine[1], mine[2], mine[3]);
-        if (kN == 8) dst[1] = make_uint4(mine[4], mine[5], mine[6], mine[7]);
-    };
-    auto emit = [&](int j, uint32_t v) {
-        if (j >= cap) return;
-        if (!kStage) {
-            out[j] = v;
-            return;
-        }
-        mine[j & (kN - 1)] = v;
-        if ((j & (kN - 1)) == kN - 1) flush(j - (kN - 1));
-    };
-    WalkResult r;
-    if constexpr (kMixed)
-        r = mlp_walk_mixed<false>(g, tab, steps, kmax, nullptr, __ldg(h.first_MLP_voxel + i), __ldg(h.x_entry + i),
-                                  __ldg(h.y_entry + i), __ldg(h.z_entry + i), __ldg(h.x_exit + i),
-                                  __ldg(h.y_exit + i), __ldg(h.z_exit + i), __ldg(h.xy_entry_angle + i),
-                                  __ldg(h.xz_entry_angle + i), __ldg(h.xy_exit_angle + i),
-                                  __ldg(h.xz_exit_angle + i), emit);
-    else {
-        __shared__ double stash[PCT_PHASE1_STASH ? (kHistoryFields + PCT_STASH_CHORD) * kThreads : 1];
-        r = mlp_walk_exact<false, PCT_PHASE1_UNROLL>(
-            g, tab, steps, kmax, nullptr, __ldg(h.first_MLP_voxel + i), __ldg(h.x_entry + i), __ldg(h.y_entry + i),
-            __ldg(h.z_entry + i), __ldg(h.x_exit + i), __ldg(h.y_exit + i), __ldg(h.z_exit + i),
-            __ldg(h.xy_entry_angle + i), __ldg(h.xz_entry_angle + i), __ldg(h.xy_exit_angle + i),
-            __ldg(h.xz_exit_angle + i), emit, (uint32_t)__cvta_generic_to_shared(stash + threadIdx.x),
-            PCT_PHASE1_STASH ? kThreads * (uint32_t)sizeof(double) : 0u);
-    }
-    unsigned flags = r.flags;
-    int n = r.n;
-    if (n > cap) {  // cannot happen: cap bounds the loop count
-        flags |= kFlagPathOverflow;
-        n = cap;
-    }
-    if (kStage && (n & (kN - 1))) flush(n & ~(kN - 1));  // the last partial flush, padded (cap is a multiple of 8)
     if (flags) count_flags(flags, counters);
-    path_n[id] = n;
-    chord[id] = r.chord;
+    path_n[perm[i]] = n;
 }
 
-// kThreads histories per CTA (PATH_CTA_THREADS), with the same resident threads per SM, hence the
-// same register budget (72 for the exact kernel, 64 for the mixed one), at every size.
+// Without a table (reference-order points, or a grid too large for the fixed-point positions).
 template <int kThreads>
-__global__ void __launch_bounds__(kThreads, PCT_PHASE1_MIN_BLOCKS * 128 / kThreads) mlp_phase1_exact_kernel(
+__global__ void __launch_bounds__(kThreads, 7 * 128 / kThreads) mlp_phase1_exact_kernel(
     Geometry g, Tables tab, const StepConst* __restrict__ steps, int kmax, HistorySoA h, const int* __restrict__ perm,
     long long count, const long long* __restrict__ offsets, long long offset_base, const int* __restrict__ bounds,
     uint32_t* __restrict__ paths, int* __restrict__ path_n, double* __restrict__ chord, unsigned long long* counters)
 {
-    mlp_phase1_body<false, kThreads>(g, tab, steps, kmax, h, perm, count, offsets, offset_base, bounds, paths, path_n,
-                                     chord, counters);
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= count) return;
+    const long long id = perm[i];
+    const int cap = bounds[i];
+    if (cap <= 0) {
+        path_n[id] = 0;
+        chord[id] = 0.0;
+        return;
+    }
+    uint32_t* out = paths + (offsets[i] - offset_base);
+    const WalkResult r = mlp_walk_exact<false>(
+        g, tab, steps, kmax, nullptr, __ldg(h.first_MLP_voxel + i), __ldg(h.x_entry + i), __ldg(h.y_entry + i),
+        __ldg(h.z_entry + i), __ldg(h.x_exit + i), __ldg(h.y_exit + i), __ldg(h.z_exit + i),
+        __ldg(h.xy_entry_angle + i), __ldg(h.xz_entry_angle + i), __ldg(h.xy_exit_angle + i),
+        __ldg(h.xz_exit_angle + i), [&](int j, uint32_t v) {
+            if (j < cap) out[j] = v;
+        });
+    unsigned flags = r.flags;
+    int n = r.n;
+    if (n > cap) {
+        flags |= kFlagPathOverflow;
+        n = cap;
+    }
+    if (flags) count_flags(flags, counters);
+    path_n[id] = n;
+    chord[id] = r.chord;
 }
 
 template <int kThreads>
@@ -340,8 +299,32 @@ __global__ void __launch_bounds__(kThreads, PCT_PHASE1_MIXED_MIN_BLOCKS * 128 / 
     long long count, const long long* __restrict__ offsets, long long offset_base, const int* __restrict__ bounds,
     uint32_t* __restrict__ paths, int* __restrict__ path_n, double* __restrict__ chord, unsigned long long* counters)
 {
-    mlp_phase1_body<true, kThreads>(g, tab, steps, kmax, h, perm, count, offsets, offset_base, bounds, paths, path_n,
-                                    chord, counters);
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= count) return;
+    const long long id = perm[i];
+    const int cap = bounds[i];
+    if (cap <= 0) {
+        path_n[id] = 0;
+        chord[id] = 0.0;
+        return;
+    }
+    uint32_t* out = paths + (offsets[i] - offset_base);
+    const WalkResult r = mlp_walk_mixed<false>(
+        g, tab, steps, kmax, nullptr, __ldg(h.first_MLP_voxel + i), __ldg(h.x_entry + i), __ldg(h.y_entry + i),
+        __ldg(h.z_entry + i), __ldg(h.x_exit + i), __ldg(h.y_exit + i), __ldg(h.z_exit + i),
+        __ldg(h.xy_entry_angle + i), __ldg(h.xz_entry_angle + i), __ldg(h.xy_exit_angle + i),
+        __ldg(h.xz_exit_angle + i), [&](int j, uint32_t v) {
+            if (j < cap) out[j] = v;
+        });
+    unsigned flags = r.flags;
+    int n = r.n;
+    if (n > cap) {
+        flags |= kFlagPathOverflow;
+        n = cap;
+    }
+    if (flags) count_flags(flags, counters);
+    path_n[id] = n;
+    chord[id] = r.chord;
 }
 
 // One warp per history.  Lane l holds entries l, l+32, ..., l+224 of the stored voxel list in
@@ -565,7 +548,181 @@ __global__ void build_step_table_kernel(Tables tab, unsigned sstep, unsigned pst
     steps[k] = e;
 }
 
+// ---- the table of MLP weights (pct_mlp.cuh, "Tabulated points") --------------------------------
+
+// Rows of bucket b (m buckets per MLP step): the steps k of a walk with u_2 inside the bucket, those with
+// u_2 - k s > s; and the rows of the buckets before it.
+__host__ __device__ inline int table_row_count(int b, int m) { return b / m > 1 ? b / m - 1 : 0; }
+__host__ __device__ inline long long table_first_row(int b, int m)
+{
+    const long long f = b / m;  // whole groups of m buckets before it; group i has max(0, i - 1) rows each
+    return (f > 2 ? (f - 2) * (f - 1) / 2 : 0) * m + (long long)(b % m) * table_row_count(b, m);
+}
+
+// The weights B and C of step k for u_2 = grid point idx + delta and u_2^2 + epsilon, with Sigma_2's
+// determinant scaled by 1 + eta: the formulas of mlp_point_rest solved for the weights, in double.
+struct WeightNode {
+    double B, C;
+    double mag_num, mag_det;  // M(num) / |det| per unit of scale and M(det) / |det| (mlp_point_fast)
+    double ratio;             // sigma_t2_theta2^2 / |determinant of the moments|
+};
+__device__ WeightNode weight_node(const Tables& tab, const StepConst& st, double s, int k, unsigned sstep, long long idx,
+                                  double delta, double epsilon, double eta)
+{
+    const double u_2 = idx * kPolyTableStep + delta, d = u_2 - k * s;
+    const double t2 = tab.poly_3_12[idx] - (u_2 * u_2 + epsilon) * st.p12 + 2.0 * u_2 * st.p23 - st.p34;
+    const double tt = tab.poly_2_6[idx] - u_2 * st.p12 + st.p23;
+    const double th = tab.poly_1_2[idx] - st.p12;
+    const double mdet = t2 * th - tt * tt;
+    // the walk's index: of its first depth u_2 - s, then sstep less a step (an entry off is in eta)
+    long long is = llrint((u_2 - s) / kCoeffTableStep) - (long long)(k - 1) * sstep;
+    if (is < 0) is = 0;  // log of 0: the row comes out unusable
+    const double det2 = tab.scattering_table[is] * mdet * (1.0 + eta);
+    const double S0 = th / det2, S1 = tt / det2, S2 = t2 / det2;
+    const double c = S0 * d - S1, m0 = st.s1i0 + S0, m1 = c - st.s1i1, m3 = st.s1i2 + S2 + d * (c - S1);
+    const double det = m0 * m3 - m1 * m1;
+    const double aS0 = fabs(S0), aS1 = fabs(S1), aS2 = fabs(S2), Mc = aS0 * d + aS1, M0 = fabs(st.s1i0) + aS0,
+                 M1 = Mc + fabs(st.s1i1), M3 = fabs(st.s1i2) + aS2 + d * (Mc + aS1);
+    WeightNode w;
+    w.B = (m3 * S0 - m1 * c) / det;
+    w.C = -(m3 * S1 + m1 * (S2 - d * S1)) / det;
+    w.mag_num = (M3 * (M0 + aS1) + M1 * (M1 + d * aS1 + aS2)) / fabs(det);
+    w.mag_det = (M0 * M3 + M1 * M1) / fabs(det);
+    w.ratio = tt * tt / fabs(mdet);
+    return w;
+}
+
+// Quadratic through (z0, f0), (zp, fp), (zm, fm) as coefficients of 1, z, z^2.
+__device__ void quadratic(double z0, double f0, double zp, double fp, double zm, double fm, double (&c)[3])
+{
+    const double p = (fp - f0) / (zp - z0), q = (fm - f0) / (zm - z0);
+    c[2] = (p - q) / (zp - zm);
+    c[1] = p - c[2] * (z0 + zp);
+    c[0] = f0 - p * z0 + c[2] * z0 * zp;
+}
+
+// One CTA per bucket, one thread per step.  A row is kept while its bound is useful (kMaxErrB,
+// kMaxErrC: a few thousandths of a voxel face's neighbourhood at head-scan deflections); the first
+// row that is not ends the bucket's table.
+constexpr float kMaxErrB = 2.0e-5f, kMaxErrC = 1.0e-4f, kMaxErrR = 1.0e-7f;
+__global__ void __launch_bounds__(128) build_mlp_table_kernel(Tables tab, const StepConst* __restrict__ steps, double s,
+                                                              unsigned sstep, int m, double width, float4* __restrict__ rows,
+                                                              MlpBucket* __restrict__ bucket)
+{
+    const int b = blockIdx.x, count = table_row_count(b, m);
+    const long long first = table_first_row(b, m);
+    __shared__ float e_b[kPathCap], e_c[kPathCap];
+    __shared__ int bad, max_r, max_b, max_c, all_b, all_c;
+    if (threadIdx.x == 0) {
+        bad = count + 1;
+        max_r = max_b = max_c = all_b = all_c = 0;
+    }
+    __syncthreads();
+    const double center = (b + 0.5) * width;
+    const long long ic = llrint(center / kPolyTableStep);
+    const double kappa = count > 0 ? steps[count].p12 / (2.0 * tab.poly_2_6[ic] * count) : 0.0;
+    const double eps_max = 3.0e-7 * (b + 1) * width * (b + 1) * width;  // powf of the float u_2
+    for (int k = 1 + threadIdx.x; k <= count; k += blockDim.x) {
+        const StepConst st = steps[k];
+        auto node = [&](double z, double delta, double eps, double eta, double& zeta) {
+            const long long idx = llrint((center + 0.5 * z * width - delta) / kPolyTableStep);
+            zeta = ((idx * kPolyTableStep + delta) / width - b) * 2.0 - 1.0;
+            return weight_node(tab, st, s, k, sstep, idx, delta, eps, eta);
+        };
+        double z0, zp, zm, za, zb, qb[3], qc[3];
+        const WeightNode n0 = node(0.0, 0.0, 0.0, 0.0, z0), np = node(0.8660254, 0.0, 0.0, 0.0, zp),
+                         nm = node(-0.8660254, 0.0, 0.0, 0.0, zm), na = node(0.0, kSigmaUnit, 0.0, 0.0, za),
+                         nb = node(0.0, -kSigmaUnit, 0.0, 0.0, zb);
+        quadratic(z0, n0.B, zp, np.B, zm, nm.B, qb);
+        quadratic(z0, n0.C, zp, np.C, zm, nm.C, qc);
+        auto at = [](const double (&c)[3], double z) { return c[0] + z * (c[1] + z * c[2]); };
+        const float4 rb = make_float4((float)qb[0], (float)qb[1], (float)qb[2],
+                                      (float)(0.5 * ((na.B - at(qb, za)) - (nb.B - at(qb, zb)))));
+        const float4 rc = make_float4((float)qc[0], (float)qc[1], (float)qc[2],
+                                      (float)(0.5 * ((na.C - at(qc, za)) - (nb.C - at(qc, zb)))));
+        rows[2 * (first + k - 1)] = rb;
+        rows[2 * (first + k - 1) + 1] = rc;
+        double err_b = 0.0, err_c = 0.0;
+        for (int i = 0; i < 81; i++) {
+            const double delta = (i / 9 % 3 - 1) * kSigmaUnit, eps = (i / 27 - 1) * eps_max;
+            double zeta;
+            const WeightNode w = node((i % 9 - 4) * 0.25, delta, eps, 0.0, zeta);
+            const float z = (float)zeta, sigma = (float)((delta + k * kappa * eps) * kInvSigmaUnit);
+            err_b = fmax(err_b, fabs((double)table_weight(rb, z, sigma) - w.B));
+            err_c = fmax(err_c, fabs((double)table_weight(rc, z, sigma) - w.C));
+        }
+        double ze;
+        const double eta = 4.0e-7 * n0.ratio + 6.0e-6 / (center - k * s);
+        const WeightNode ne = node(0.0, 0.0, 0.0, eta, ze);
+        const float eb = (float)(2.0 * err_b + 2.0 * fabs(ne.B - n0.B)), ec = (float)(2.0 * err_c + 2.0 * fabs(ne.C - n0.C));
+        const float er = (float)(kBoundK * (n0.mag_num + 2.0 * n0.mag_det) * 2.0);
+        e_b[k - 1] = eb;
+        e_c[k - 1] = ec;
+        if (!(eb < kMaxErrB && ec < kMaxErrC && er < kMaxErrR)) atomicMin(&bad, k);
+        else {
+            atomicMax(&max_r, __float_as_int(er));  // non-negative floats compare as integers
+            atomicMax(&max_b, __float_as_int(fabsf(rb.x) + fabsf(rb.y) + fabsf(rb.z)));
+            atomicMax(&max_c, __float_as_int(fabsf(rc.x) + fabsf(rc.y) + fabsf(rc.z)));
+        }
+    }
+    __syncthreads();
+    for (int k = 1 + threadIdx.x; k < bad; k += blockDim.x) {
+        atomicMax(&all_b, __float_as_int(e_b[k - 1]));
+        atomicMax(&all_c, __float_as_int(e_c[k - 1]));
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        MlpBucket o;
+        o.row = (int)first;
+        o.klast = bad - 1;
+        o.err_b = __int_as_float(all_b);
+        o.err_c = __int_as_float(all_c);
+        o.err_r = __int_as_float(max_r);
+        o.max_b = __int_as_float(max_b);
+        o.max_c = __int_as_float(max_c);
+        o.steps = count;
+        o.kappa = kappa;
+        bucket[b] = o;
+    }
+}
+
 }  // namespace
+
+MlpTableShape mlp_table_shape(const Geometry& g, int kmax)
+{
+    MlpTableShape t{};
+    const double s = g.mlp_u_step;
+    if (!g.exact_fast_points || g.mixed_precision) return t;
+    // positions: frac_bits fraction bits, the rest for the grid and its surroundings
+    int extent = g.columns > g.rows ? g.columns : g.rows;
+    if (g.slices > extent) extent = g.slices;
+    int bits = 22;
+    while (bits > 18 && (1LL << (31 - bits)) < extent + 24) bits--;
+    const long long top = 1LL << (31 - bits);
+    if (top < extent + 24 || top * (1 + g.columns + (long long)g.columns * g.rows) > 0x7fffffffLL) return t;
+    t.frac_bits = bits;
+    t.per_step = (int)ceil(s / 0.05 - 1e-9);
+    if (t.per_step < 1) t.per_step = 1;
+    t.width = s / t.per_step;
+    // u_2 of a history inside the grid's cylinder, inside the tables
+    double u_max = 1.5 * extent * fmax(g.voxel_width, g.voxel_height) + 0.5;
+    if (u_max > kPolyTableRange - 0.5) u_max = kPolyTableRange - 0.5;
+    t.buckets = (int)(u_max / t.width);
+    if (t.buckets > kPathCap) t.buckets = kPathCap;
+    while (t.buckets > 0 && table_row_count(t.buckets - 1, t.per_step) > kmax) t.buckets--;
+    t.rows = table_first_row(t.buckets, t.per_step);
+    t.t_max = (float)(kMaxOffset / ((double)(1u << (bits - kOffsetShift)) * g.inv_voxel_max));
+    return t;
+}
+
+cudaError_t launch_build_mlp_table(const Tables& tab, const StepConst* steps, const Geometry& g, const MlpTableShape& shape,
+                                   float4* rows, MlpBucket* bucket, cudaStream_t stream)
+{
+    if (shape.buckets <= 0) return cudaSuccess;
+    build_mlp_table_kernel<<<shape.buckets, 128, 0, stream>>>(tab, steps, g.mlp_u_step, g.sigma_index_step,
+                                                              shape.per_step, shape.width, rows, bucket);
+    return cudaGetLastError();
+}
 
 cudaError_t launch_build_step_table(const Tables& tab, unsigned sstep, unsigned pstep, int kmax, StepConst* steps,
                                     cudaStream_t stream)
@@ -576,12 +733,13 @@ cudaError_t launch_build_step_table(const Tables& tab, unsigned sstep, unsigned 
 }
 
 cudaError_t launch_path_bounds(const Geometry& g, const Tables& tab, const HistorySoA& h, long long n,
-                               long long block_size, int histories_per_block, int* bounds, cudaStream_t stream)
+                               long long block_size, int histories_per_block, double key_scale, int* bounds, int* keys,
+                               cudaStream_t stream)
 {
     if (n <= 0) return cudaSuccess;
     const int threads = 256;
-    path_bounds_kernel<<<(unsigned)((n + threads - 1) / threads), threads, 0, stream>>>(g, tab, h, n, block_size,
-                                                                                        histories_per_block, bounds);
+    path_bounds_kernel<<<(unsigned)((n + threads - 1) / threads), threads, 0, stream>>>(
+        g, tab, h, n, block_size, histories_per_block, key_scale, bounds, keys);
     return cudaGetLastError();
 }
 
@@ -596,7 +754,8 @@ cudaError_t launch_gather_path_inputs(const HistorySoA& src, const int* perm, co
     return cudaGetLastError();
 }
 
-cudaError_t launch_mlp_phase1_exact(const Geometry& g, const Tables& tab, const StepConst* steps, int kmax,
+cudaError_t launch_mlp_phase1_exact(const Geometry& g, const Tables& tab, const MlpTable& tb, const StepConst* steps,
+                                    int kmax,
                                     const HistorySoA& h, const int* perm, long long count, const long long* offsets,
                                     long long offset_base, const int* bounds, uint32_t* paths, int* path_n,
                                     double* chord, unsigned long long* counters, cudaStream_t stream)
@@ -607,6 +766,9 @@ cudaError_t launch_mlp_phase1_exact(const Geometry& g, const Tables& tab, const 
         const unsigned blocks = (unsigned)((count + (T) - 1) / (T));                                              \
         if (g.mixed_precision)                                                                                    \
             mlp_phase1_mixed_kernel<T><<<blocks, T, 0, stream>>>(g, tab, steps, kmax, h, perm, count, offsets,    \
+                                                                 offset_base, bounds, paths, path_n, chord, counters); \
+        else if (tb.buckets > 0)                                                                                  \
+            mlp_phase1_table_kernel<T><<<blocks, T, 0, stream>>>(g, tab, tb, steps, kmax, h, perm, count, offsets, \
                                                                  offset_base, bounds, paths, path_n, chord, counters); \
         else                                                                                                      \
             mlp_phase1_exact_kernel<T><<<blocks, T, 0, stream>>>(g, tab, steps, kmax, h, perm, count, offsets,    \
@@ -671,7 +833,8 @@ cudaError_t set_iteration_carveout()
     // and its block kernels run best with the driver's choice (its L1 holds the table gathers)
     const void* kernels[] = {
         (const void*)mlp_phase1_exact_kernel<64>, (const void*)mlp_phase1_exact_kernel<128>,
-        (const void*)mlp_phase1_exact_kernel<256>,
+        (const void*)mlp_phase1_exact_kernel<256>, (const void*)mlp_phase1_table_kernel<64>,
+        (const void*)mlp_phase1_table_kernel<128>, (const void*)mlp_phase1_table_kernel<256>,
         (const void*)drop_phase2_kernel<PCT_DROP, false, 0>, (const void*)drop_phase2_kernel<PCT_DROP, true, 0>,
         (const void*)drop_phase2_kernel<PCT_ROBUSTA, false, 0>, (const void*)drop_phase2_kernel<PCT_ROBUSTA, true, 0>,
         (const void*)drop_phase2_kernel<PCT_ROBUSTB, false, 0>,

@@ -23,6 +23,17 @@ cudaError_t launch_s_curve_table(const pct_config& c, float* out, cudaStream_t s
 cudaError_t launch_build_step_table(const Tables& tab, unsigned sstep, unsigned pstep, int kmax, StepConst* steps,
                                     cudaStream_t stream);
 
+// Size of the table of MLP weights for a configuration (buckets = 0: it has none) and its build.
+struct MlpTableShape {
+    int buckets, per_step, frac_bits;  // buckets of u_2, buckets per MLP step, fraction bits of positions
+    long long rows;                    // two float4 each
+    double width;                      // bucket width, cm
+    float t_max;                       // MlpTable::t_max
+};
+MlpTableShape mlp_table_shape(const Geometry& g, int kmax);
+cudaError_t launch_build_mlp_table(const Tables& tab, const StepConst* steps, const Geometry& g, const MlpTableShape& shape,
+                                   float4* rows, MlpBucket* bucket, cudaStream_t stream);
+
 // MLP + DROP scatter for histories [begin, begin+count) (exact mode).
 cudaError_t launch_drop_block_exact(const Geometry& g, const Tables& tab, const StepConst* steps, int kmax,
                                     const float* x, float2* acc, const HistorySoA& h, long long begin,
@@ -40,7 +51,8 @@ cudaError_t launch_mlp_steps(const Geometry& g, const Tables& tab, int kmax, con
 
 // Two-phase DROP iteration (see pct_drop_exact.cu).
 cudaError_t launch_path_bounds(const Geometry& g, const Tables& tab, const HistorySoA& h, long long n,
-                               long long block_size, int histories_per_block, int* bounds, cudaStream_t stream);
+                               long long block_size, int histories_per_block, double key_scale, int* bounds, int* keys,
+                               cudaStream_t stream);
 // dst[p] = src[perm[p]] for the path kernel's inputs (the ten geometry fields and the first voxel),
 // the path bounds and the path-storage offsets, p in [0, n).
 cudaError_t launch_gather_path_inputs(const HistorySoA& src, const int* perm, const int* bounds,
@@ -49,7 +61,8 @@ cudaError_t launch_gather_path_inputs(const HistorySoA& src, const int* perm, co
 // The path kernel over `count` histories in processing order: h, bounds and offsets hold its
 // inputs in that order (from launch_gather_path_inputs, offset to the chunk), perm the history
 // each position stands for (its path length and chord are written there).
-cudaError_t launch_mlp_phase1_exact(const Geometry& g, const Tables& tab, const StepConst* steps, int kmax,
+cudaError_t launch_mlp_phase1_exact(const Geometry& g, const Tables& tab, const MlpTable& tb, const StepConst* steps,
+                                    int kmax,
                                     const HistorySoA& h, const int* perm, long long count, const long long* offsets,
                                     long long offset_base, const int* bounds, uint32_t* paths, int* path_n,
                                     double* chord, unsigned long long* counters, cudaStream_t stream);

@@ -145,59 +145,6 @@ struct MlpHistory {
     double u_2_poly_3_12, u_2_poly_2_6, u_2_poly_1_2;
     double mag_tv;  // max(|t_in| + |t_out| + |T_2_1|, |z_in| + |z_out| + |V_2_1|): the guarded fast point's bound
 };
-constexpr int kHistoryFields = 15;
-// 1: the walk parks its chord in the stash slot after the history's constants while it loops; 0 keeps
-// it in registers.
-#ifndef PCT_STASH_CHORD
-#define PCT_STASH_CHORD 1
-#endif
-static_assert(sizeof(MlpHistory) == kHistoryFields * sizeof(double), "MlpHistory is 15 doubles");
-
-// The constants of a history parked in shared memory: field f of this thread at byte address
-// addr + f * stride.  The loads are volatile, so they stay inside the loop trip that uses them and
-// the constants are not held in registers across trips.
-__device__ __forceinline__ void history_stash_store(uint32_t addr, uint32_t stride, const MlpHistory& h)
-{
-    const double* f = reinterpret_cast<const double*>(&h);
-#pragma unroll
-    for (int i = 0; i < kHistoryFields; i++)
-        asm volatile("st.shared.f64 [%0], %1;" ::"r"(addr + i * stride), "d"(f[i]) : "memory");
-}
-
-__device__ __forceinline__ MlpHistory history_stash_load(uint32_t addr, uint32_t stride)
-{
-    MlpHistory h;
-    double* f = reinterpret_cast<double*>(&h);
-#pragma unroll
-    for (int i = 0; i < kHistoryFields; i++) asm volatile("ld.shared.f64 %0, [%1];" : "=d"(f[i]) : "r"(addr + i * stride));
-    return h;
-}
-
-// Field numbers of MlpHistory (declaration order) and two ways of reading a field: from the
-// struct (registers) or from the shared-memory stash, loaded where it is used.
-enum HistoryField { kHSin, kHCos, kHTin, kHTout, kHZin, kHZout, kHT21, kHV21, kHU2, kHU2sq, kHTwoU2, kHP312, kHP26, kHP12, kHMag };
-
-struct HistoryInRegisters {
-    const MlpHistory& h;
-    template <int F>
-    __device__ __forceinline__ double get() const
-    {
-        static_assert(F >= 0 && F < kHistoryFields, "field");
-        return reinterpret_cast<const double*>(&h)[F];
-    }
-};
-
-struct HistoryInShared {
-    uint32_t addr, stride;
-    template <int F>
-    __device__ __forceinline__ double get() const
-    {
-        static_assert(F >= 0 && F < kHistoryFields, "field");
-        double v;
-        asm volatile("ld.shared.f64 %0, [%1];" : "=d"(v) : "r"(addr + F * stride));
-        return v;
-    }
-};
 
 // MLP point (t_1, v_1) of one loop iteration (B.cu:9180-9226): Sigma_2 from the tables, its
 // inverse, the 2x2 solve for t and v.  Same operations, same order as the reference.
@@ -207,22 +154,15 @@ struct Sigma2 {
 
 // The Sigma_2 moments of one point and their determinant (B.cu:9180-9186), in the reference's
 // operations and order.
-template <class HA>
-__device__ __forceinline__ Sigma2 sigma2_moments(const HA& h, const StepConst& st, const double* __restrict__ scattering,
-                                                 unsigned sigma_2_index)
-{
-    Sigma2 m;
-    m.sigma_t2 = h.template get<kHP312>() - h.template get<kHU2sq>() * st.p12 + h.template get<kHTwoU2>() * st.p23 - st.p34;
-    m.sigma_t2_theta2 = h.template get<kHP26>() - h.template get<kHU2>() * st.p12 + st.p23;
-    m.sigma_theta2 = h.template get<kHP12>() - st.p12;
-    m.determinant = __ldg(scattering + sigma_2_index) * (m.sigma_t2 * m.sigma_theta2 - powf_square(m.sigma_t2_theta2));
-    return m;
-}
-
 __device__ __forceinline__ Sigma2 sigma2_moments(const MlpHistory& h, const StepConst& st,
                                                  const double* __restrict__ scattering, unsigned sigma_2_index)
 {
-    return sigma2_moments(HistoryInRegisters{h}, st, scattering, sigma_2_index);
+    Sigma2 m;
+    m.sigma_t2 = h.u_2_poly_3_12 - h.u_2_sq * st.p12 + h.two_u_2 * st.p23 - st.p34;
+    m.sigma_t2_theta2 = h.u_2_poly_2_6 - h.u_2 * st.p12 + st.p23;
+    m.sigma_theta2 = h.u_2_poly_1_2 - st.p12;
+    m.determinant = __ldg(scattering + sigma_2_index) * (m.sigma_t2 * m.sigma_theta2 - powf_square(m.sigma_t2_theta2));
+    return m;
 }
 
 __device__ __forceinline__ void mlp_point_rest(const MlpHistory& h, const StepConst& st, const Sigma2& m,
@@ -277,9 +217,6 @@ __device__ __forceinline__ void mlp_point(const MlpHistory& h, const StepConst& 
 // well-conditioned, returns false and is recomputed in the reference's order, so the voxel list
 // is the reference's either way.
 constexpr double kBoundK = 9.094947017729282e-13;  // 2^-40
-#ifndef PCT_FAST_POINTS
-#define PCT_FAST_POINTS 1  // 0 compiles the guarded fast points out (every point in the reference's order)
-#endif
 
 // rcp.approx.ftz.f64 (a coarse hardware reciprocal of the high word) refined by two Newton steps:
 // within a few units in the last place of 1/b for the normal values it sees here.
@@ -318,10 +255,8 @@ __device__ __forceinline__ bool guarded_indices(const Geometry& g, double x, dou
 }
 
 // The fast point and its voxel (see above); false when the bound cannot prove the voxel.
-// h gives the history's constants (HistoryInRegisters or HistoryInShared); its mag_tv is
-// |t_in| + |t_out| + |T_2_1| and the same for v, the larger of the two.
-template <class HA>
-__device__ __forceinline__ bool mlp_point_fast(const Geometry& g, const HA& h, const StepConst& st, double sigma_t2,
+// h.mag_tv is |t_in| + |t_out| + |T_2_1| and the same for v, the larger of the two.
+__device__ __forceinline__ bool mlp_point_fast(const Geometry& g, const MlpHistory& h, const StepConst& st, double sigma_t2,
                                                double sigma_t2_theta2, double sigma_theta2, double det2, double d,
                                                double u_shifted, uint32_t& voxel)
 {
@@ -343,25 +278,25 @@ __device__ __forceinline__ bool mlp_point_fast(const Geometry& g, const HA& h, c
     if (!(__dmul_rn(4.0 * kBoundK, Mdet) < adet)) return false;
     const double rdet = rcp_refined(det);
     // the right-hand sides and the solves for t and v
-    double c3 = __fma_rn(S0, h.template get<kHTout>(), -__dmul_rn(S1, h.template get<kHT21>()));
-    double r0 = __fma_rn(st.s1i0, h.template get<kHTin>(), c3);
-    double r1 = __fma_rn(d, c3, __fma_rn(S2, h.template get<kHT21>(), -__fma_rn(S1, h.template get<kHTout>(), __dmul_rn(st.s1i1, h.template get<kHTin>()))));
+    double c3 = __fma_rn(S0, h.t_out, -__dmul_rn(S1, h.T_2_1));
+    double r0 = __fma_rn(st.s1i0, h.t_in, c3);
+    double r1 = __fma_rn(d, c3, __fma_rn(S2, h.T_2_1, -__fma_rn(S1, h.t_out, __dmul_rn(st.s1i1, h.t_in))));
     const double t_1 = __dmul_rn(__fma_rn(m3, r0, -__dmul_rn(m1, r1)), rdet);
-    c3 = __fma_rn(S0, h.template get<kHZout>(), -__dmul_rn(S1, h.template get<kHV21>()));
-    r0 = __fma_rn(st.s1i0, h.template get<kHZin>(), c3);
-    r1 = __fma_rn(d, c3, __fma_rn(S2, h.template get<kHV21>(), -__fma_rn(S1, h.template get<kHZout>(), __dmul_rn(st.s1i1, h.template get<kHZin>()))));
+    c3 = __fma_rn(S0, h.z_out, -__dmul_rn(S1, h.V_2_1));
+    r0 = __fma_rn(st.s1i0, h.z_in, c3);
+    r1 = __fma_rn(d, c3, __fma_rn(S2, h.V_2_1, -__fma_rn(S1, h.z_out, __dmul_rn(st.s1i1, h.z_in))));
     const double v_1 = __dmul_rn(__fma_rn(m3, r0, -__dmul_rn(m1, r1)), rdet);
     // one bound for both solves: each right-hand-side input is at most mag_tv in magnitude
     // M(r0) = mag (|s1i0| + |S0| + |S1|) = mag (M(m0) + |S1|) and
     // M(r1) = mag (d (|S0| + |S1|) + |S2| + |S1| + |s1i1|) = mag (M(m1) + d |S1| + |S2|), so
     // M(num) = M(m3) M(r0) + M(m1) M(r1) = mag (M(m3) (M(m0) + |S1|) + M(m1) (M(m1) + d |S1| + |S2|))
-    const double mag_tv = h.template get<kHMag>();
+    const double mag_tv = h.mag_tv;
     const double Mnum = __dmul_rn(mag_tv, __fma_rn(Mm3, __dadd_rn(Mm0, aS1), __dmul_rn(Mm1, __dadd_rn(Mm1, __fma_rn(d, aS1, aS2)))));
     const double err = __dmul_rn(kBoundK, __dmul_rn(__fma_rn(fmax(fabs(t_1), fabs(v_1)), Mdet, Mnum), fabs(rdet)));
     // rotation back to x/y (B.cu:9229-9232) and the voxel indices (calculate_voxel_GPU B.cu:11091)
-    const double x_1 = __fma_rn(h.template get<kHCos>(), u_shifted, -__dmul_rn(h.template get<kHSin>(), t_1));
-    const double y_1 = __fma_rn(h.template get<kHSin>(), u_shifted, __dmul_rn(h.template get<kHCos>(), t_1));
-    const double Mrot = __fma_rn(fabs(h.template get<kHCos>()) + fabs(h.template get<kHSin>()), fabs(u_shifted) + fabs(t_1), 0.0);
+    const double x_1 = __fma_rn(h.cos_term, u_shifted, -__dmul_rn(h.sin_term, t_1));
+    const double y_1 = __fma_rn(h.sin_term, u_shifted, __dmul_rn(h.cos_term, t_1));
+    const double Mrot = __fma_rn(fabs(h.cos_term) + fabs(h.sin_term), fabs(u_shifted) + fabs(t_1), 0.0);
     const double err_xy = __fma_rn(kBoundK, Mrot, err);
     int vx, vy, vz;
     if (!guarded_indices(g, x_1, y_1, v_1, err_xy, vx, vy, vz)) return false;  // err_xy >= err
@@ -491,29 +426,21 @@ struct PathWriter {
 
 // One history's MLP.  emit(j, voxel) is called for every path entry j in order.  With kSumX the
 // walk also sums the padded image x over the path (reads beyond it are reported and count as 0);
-// without it x is not touched (the voxel list does not depend on the image).  kUnroll = 2
-// evaluates two consecutive MLP points per loop trip so their independent FP64 chains overlap;
-// the depth and position recurrences are still carried one subtraction / addition at a time, so
-// every value is the one the reference computes.  A non-zero stash_stride parks the per-history
-// constants and the chord in shared memory at stash_addr (kHistoryFields + 1 slots, stash_stride
-// bytes apart) and reads each constant where a loop trip uses it.
-template <bool kSumX, int kUnroll = 1, class Emit>
+// without it x is not touched (the voxel list does not depend on the image).
+template <bool kSumX, class Emit>
 __device__ __forceinline__ WalkResult mlp_walk_exact(const Geometry& g, const Tables& tab,
                                                      const StepConst* __restrict__ steps, int kmax,
                                                      const float* __restrict__ x, uint32_t first_MLP_voxel,
                                                      double x_in_object, double y_in_object, double z_in_object,
                                                      double x_out_object, double y_out_object, double z_out_object,
                                                      double xy_entry_angle, double xz_entry_angle,
-                                                     double xy_exit_angle, double xz_exit_angle, Emit emit,
-                                                     uint32_t stash_addr = 0, uint32_t stash_stride = 0)
+                                                     double xy_exit_angle, double xz_exit_angle, Emit emit)
 {
-    static_assert(kUnroll == 1 || kUnroll == 2, "unroll 1 or 2");
     const double s = g.mlp_u_step;
     WalkResult r;
     r.flags = 0;
     MlpStart m = mlp_start(g, tab, x_in_object, y_in_object, z_in_object, x_out_object, y_out_object, z_out_object,
                            xy_entry_angle, xy_exit_angle, xz_entry_angle, xz_exit_angle, r.flags);
-    if (stash_stride) history_stash_store(stash_addr, stash_stride, m.h);
     double depth_2_go = m.depth_2_go, u_shifted = m.u_shifted;
     unsigned sigma_2_index = m.sigma_2_index;
 
@@ -521,8 +448,6 @@ __device__ __forceinline__ WalkResult mlp_walk_exact(const Geometry& g, const Ta
     w.first(first_MLP_voxel);
     r.chord = effective_chord_length(g, (xy_entry_angle + xy_exit_angle) / 2.0, (xz_entry_angle + xz_exit_angle) / 2.0);
     r.aia = powf_square(r.chord);
-    if (stash_stride && PCT_STASH_CHORD)  // the chord waits in the stash slot after the history's constants
-        asm volatile("st.shared.f64 [%0], %1;" ::"r"(stash_addr + kHistoryFields * stash_stride), "d"(r.chord) : "memory");
 
     int k = 1;
     while (m.tables_ok && depth_2_go > s) {
@@ -530,57 +455,359 @@ __device__ __forceinline__ WalkResult mlp_walk_exact(const Geometry& g, const Ta
             r.flags |= kFlagTableRange;
             break;
         }
-        if (kUnroll == 1) {
-            const StepConst& st = steps[k];
-            const HistoryInShared hs{stash_addr, stash_stride};
-            const Sigma2 m2 = stash_stride ? sigma2_moments(hs, st, tab.scattering_table, sigma_2_index)
-                                           : sigma2_moments(m.h, st, tab.scattering_table, sigma_2_index);
-            u_shifted += s;
-            uint32_t voxel;
-            bool fast = false;
-            if (PCT_FAST_POINTS && g.exact_fast_points)
-                fast = stash_stride ? mlp_point_fast(g, hs, st, m2.sigma_t2, m2.sigma_t2_theta2, m2.sigma_theta2,
-                                                     m2.determinant, depth_2_go, u_shifted, voxel)
-                                    : mlp_point_fast(g, HistoryInRegisters{m.h}, st, m2.sigma_t2, m2.sigma_t2_theta2,
-                                                     m2.sigma_theta2, m2.determinant, depth_2_go, u_shifted, voxel);
-            if (!fast) {
-                const MlpHistory h = stash_stride ? history_stash_load(stash_addr, stash_stride) : m.h;
-                double t_1, v_1;
-                mlp_point_rest(h, st, m2, depth_2_go, t_1, v_1);
-                voxel = mlp_voxel(g, h, u_shifted, t_1, v_1);
-            }
-            w.visit(voxel);
-            depth_2_go -= s;
-            sigma_2_index -= g.sigma_index_step;
-            k++;
-        } else {
-            const MlpHistory& h = m.h;
-            // the second point exists when the loop would run again after the first
-            const double depth_b = depth_2_go - s;
-            const bool have_b = depth_b > s && k + 1 <= kmax;
-            const unsigned sigma_b = have_b ? sigma_2_index - g.sigma_index_step : sigma_2_index;
-            double t_a, v_a, t_b, v_b;
-            mlp_point(h, steps[k], tab.scattering_table, depth_2_go, sigma_2_index, t_a, v_a);
-            mlp_point(h, steps[have_b ? k + 1 : k], tab.scattering_table, have_b ? depth_b : depth_2_go, sigma_b, t_b,
-                      v_b);
-            u_shifted += s;
-            w.visit(mlp_voxel(g, h, u_shifted, t_a, v_a));
-            depth_2_go = depth_b;
-            sigma_2_index -= g.sigma_index_step;
-            k++;
-            if (have_b) {
-                u_shifted += s;
-                w.visit(mlp_voxel(g, h, u_shifted, t_b, v_b));
-                depth_2_go -= s;
-                sigma_2_index -= g.sigma_index_step;
-                k++;
-            }
+        const StepConst& st = steps[k];
+        const Sigma2 m2 = sigma2_moments(m.h, st, tab.scattering_table, sigma_2_index);
+        u_shifted += s;
+        uint32_t voxel;
+        if (!(g.exact_fast_points &&
+              mlp_point_fast(g, m.h, st, m2.sigma_t2, m2.sigma_t2_theta2, m2.sigma_theta2,
+                             m2.determinant, depth_2_go, u_shifted, voxel))) {
+            double t_1, v_1;
+            mlp_point_rest(m.h, st, m2, depth_2_go, t_1, v_1);
+            voxel = mlp_voxel(g, m.h, u_shifted, t_1, v_1);
         }
+        w.visit(voxel);
+        depth_2_go -= s;
+        sigma_2_index -= g.sigma_index_step;
+        k++;
     }
     r.n = w.n < kPathCap ? w.n : kPathCap;
-    if (stash_stride && PCT_STASH_CHORD)
-        asm volatile("ld.shared.f64 %0, [%1];" : "=d"(r.chord) : "r"(stash_addr + kHistoryFields * stash_stride));
     return r;
+}
+
+// ---- Tabulated points (exact mode, EXACT_FAST_POINTS = 1) --------------------------------------
+// Written out, the MLP point is linear in the history: with M = Sigma_1^-1 + R_1^T Sigma_2^-1 R_1,
+//     t = t_in + B (t_out - t_in) + C T_2_1        v = z_in + B (z_out - z_in) + C V_2_1
+// (the weights of t_in and t_out add up to 1), and the weights B and C depend only on the step k and
+// on u_2.  What else enters them through the reference's arithmetic is small and per history: the
+// distance delta of u_2 from its polynomial-table grid point, the error epsilon of its squared u_2
+// (powf of a float), and the rounding of powf in the determinant of Sigma_2.  delta and epsilon act
+// through Sigma_2's first moment, as -2 poly_2_6(u_2) delta and -poly_1_2(u_1) epsilon, and
+// poly_1_2(u_1) is nearly proportional to k.  So B and C are tabulated once per context
+// (build_mlp_table_kernel): for every bucket of u_2 (MLP_U_STEP wide, at most 0.05 cm) and every step
+// k, a quadratic in u_2 plus a linear term in sigma = delta + k kappa epsilon, as 8 floats, and per
+// bucket a bound on how far the tabulated weights can be from the ones the reference's operations
+// give.  The bound adds
+//   * twice the largest difference between the float evaluation and the double-precision formula
+//     over a 9 x 3 x 3 grid of (u_2, delta, epsilon),
+//   * the change of B and C when Sigma_2 is scaled by the largest relative error of its determinant
+//     (powf's rounding and a scattering-table index one entry off), and
+//   * the forward rounding error bound of the guarded fast point (kBoundK) on the history's scale.
+// A point's voxel is accepted when its position is farther than that (plus the fixed-point and float
+// roundings below) from every voxel face, which leaves a few points in 10^5; those, and steps without
+// a usable row, are computed by the guarded fast point or in the reference's order.  The voxel list is
+// the reference's either way.
+//
+// The position is fixed point, in voxels from the grid's corner with frac_bits fraction bits: the
+// straight line u -> (u cos - t_in sin, u sin + t_in cos) advances in a 64-bit accumulator per axis,
+// and the lateral offset is added as a float whose mantissa holds it in units of 2^(4 - frac_bits)
+// voxels (adding kMagic leaves it there), so the voxel index is a shift and the face test one
+// unsigned comparison per axis.
+constexpr float kMagic = 12582912.0f;          // 1.5 * 2^23: the unit of last place is 1
+constexpr unsigned kMagicBits = 0x4B400000u;   // its bit pattern
+constexpr int kOffsetShift = 4;                // offset units of 2^(4 - frac_bits) voxels
+constexpr float kMaxOffset = 4.0e6f;           // < 2^22 units: the sum with kMagic keeps its exponent
+
+// One tabulated weight: quadratic in zeta (u_2 in [-1, 1] over its bucket), linear in sigma.
+__device__ __forceinline__ float table_weight(const float4& r, float zeta, float sigma)
+{
+    return __fmaf_rn(zeta, __fmaf_rn(zeta, r.z, r.y), __fmaf_rn(sigma, r.w, r.x));
+}
+
+// What a history's tabulated walk keeps in registers.
+struct TableWalk {
+    float zeta, sigma, dsigma;        // sigma of the next step and its increment
+    float dt, T, dz, V;               // dz and V already in offset units of the z axis
+    float sx, sy;                     // offset units of x and y per cm of t
+    long long ax, ay, dx, dy;         // line accumulators (frac_bits + 32 fraction bits) and their steps
+    unsigned pz, tol;                 // z of the line; face tolerance, left-aligned
+    int klast;                        // last step with a row; 0: no table for this history
+    bool whole;                       // klast is the walk's last step
+    const float4* row;                // row of step 1
+};
+
+// (one lane's) set-up; everything in double, the range checks included, so that nothing overflows.
+__device__ __forceinline__ TableWalk table_walk_start(const Geometry& g, const MlpTable& tb, const MlpHistory& h,
+                                                      double u_in, bool tables_ok)
+{
+    TableWalk t{};
+    const double s = g.mlp_u_step;
+    const double q = h.u_2 * tb.inv_width;
+    if (!tables_ok || !(q >= 0.0 && q < (double)tb.buckets)) return t;
+    const int b = (int)q;
+    const MlpBucket bk = tb.bucket[b];
+    if (bk.klast <= 0) return t;
+    // the walk's loop runs while u_2 - k s > s: b / per_step - 1 steps, unless u_2 / s is so near a whole
+    // number that the rounding of the depth recurrence decides; then the rows stop one step earlier
+    const double turns = h.u_2 / s, whole = rint(turns);
+    const bool regular = fabs(turns - whole) > 1.0e-6;
+    t.whole = regular && bk.klast == bk.steps;
+    const double unit = (double)(1u << tb.frac_bits);  // fraction units per voxel
+    const double limit = 2147483648.0 / unit - 20.0;   // voxels a 32-bit position can hold, offsets included
+    const double delta = h.u_2 - (double)(unsigned)(h.u_2 / kPolyTableStep + 0.5) * kPolyTableStep;
+    const double epsilon = __fma_rn(-h.u_2, h.u_2, h.u_2_sq);
+    t.zeta = (float)((q - b) * 2.0 - 1.0);
+    t.dsigma = (float)(bk.kappa * epsilon * kInvSigmaUnit);
+    t.sigma = (float)(delta * kInvSigmaUnit) + t.dsigma;
+    const double dt = h.t_out - h.t_in, dz = h.z_out - h.z_in;
+    const double px = (h.cos_term * u_in - h.sin_term * h.t_in - g.x_zero) * g.inv_voxel_width;
+    const double py = (g.y_zero - (h.sin_term * u_in + h.cos_term * h.t_in)) * g.inv_voxel_height;
+    const double pz = (g.z_zero - h.z_in) * g.inv_voxel_thickness;
+    const double sx = h.cos_term * s * g.inv_voxel_width, sy = -h.sin_term * s * g.inv_voxel_height;
+    const double reach = (double)bk.klast;
+    const double offset_unit = (double)(1u << (tb.frac_bits - kOffsetShift));
+    const double d_max = fmax(fabs(dt), fabs(dz)), a_max = fmax(fabs(h.T_2_1), fabs(h.V_2_1));
+    // face tolerance in fraction units: the table's bound, the float evaluation (four roundings of the
+    // offset's terms), and 24 units for the offset's rounding to 2^kOffsetShift units and the line's
+    const double tol = ((double)bk.err_b * d_max + (double)bk.err_c * a_max + (double)bk.err_r * h.mag_tv +
+                        2.4e-7 * (d_max * bk.max_b + (double)bk.max_c * a_max)) * g.inv_voxel_max * unit + 24.0;
+    const bool ok = (fabs(px) < limit) & (fabs(px + reach * sx) < limit) & (fabs(py) < limit) &
+                    (fabs(py + reach * sy) < limit) & (fabs(pz) < limit) & (tol < unit * 0.125);
+    if (!ok) {
+        t.whole = false;
+        return t;
+    }
+    const unsigned corner = kMagicBits << kOffsetShift;  // the offset's bits carry kMagic's
+    const double scale = unit * 4294967296.0;
+    t.ax = __double2ll_rn(px * scale) - ((long long)corner << 32);
+    t.ay = __double2ll_rn(py * scale) - ((long long)corner << 32);
+    t.dx = __double2ll_rn(sx * scale);
+    t.dy = __double2ll_rn(sy * scale);
+    t.pz = (unsigned)__double2int_rn(pz * unit) - corner;
+    t.tol = (unsigned)__double2int_ru(tol) << (32 - tb.frac_bits);
+    t.dt = (float)dt;
+    t.T = (float)h.T_2_1;
+    t.dz = (float)(-dz * g.inv_voxel_thickness * offset_unit);
+    t.V = (float)(-h.V_2_1 * g.inv_voxel_thickness * offset_unit);
+    t.sx = (float)(-h.sin_term * g.inv_voxel_width * offset_unit);
+    t.sy = (float)(-h.cos_term * g.inv_voxel_height * offset_unit);
+    t.klast = regular || bk.klast < bk.steps ? bk.klast : bk.klast - 1;
+    t.row = tb.rows + 2 * (long long)bk.row;
+    return t;
+}
+
+// The tabulated point of the step whose row is r0, r1: its voxel, and whether the bound proves it.
+__device__ __forceinline__ bool table_point(const Geometry& g, const MlpTable& tb, const TableWalk& t, const float4& r0,
+                                            const float4& r1, uint32_t& voxel)
+{
+    const float B = table_weight(r0, t.zeta, t.sigma), C = table_weight(r1, t.zeta, t.sigma);
+    const float lateral = __fmaf_rn(B, t.dt, __fmul_rn(C, t.T));
+    const float vertical = __fmaf_rn(B, t.dz, __fmul_rn(C, t.V));
+    const unsigned px = (unsigned)(t.ax >> 32) + (__float_as_uint(__fmaf_rn(lateral, t.sx, kMagic)) << kOffsetShift);
+    const unsigned py = (unsigned)(t.ay >> 32) + (__float_as_uint(__fmaf_rn(lateral, t.sy, kMagic)) << kOffsetShift);
+    const unsigned pz = t.pz + (__float_as_uint(__fadd_rn(vertical, kMagic)) << kOffsetShift);
+    const int frac_bits = tb.frac_bits, left = 32 - frac_bits;
+    const unsigned band = t.tol << 1;
+    const bool proven = ((px << left) + t.tol >= band) & ((py << left) + t.tol >= band) & ((pz << left) + t.tol >= band) &
+                        ((int)(px | py | pz) >= 0) & (fabsf(lateral) < tb.t_max) & (fabsf(vertical) < kMaxOffset);
+    voxel = (px >> frac_bits) + (py >> frac_bits) * (unsigned)g.columns +
+            (pz >> frac_bits) * (unsigned)(g.columns * g.rows);
+    return proven;
+}
+
+// A history's voxel list on its way to path storage: entries wait in a 16-slot ring in shared memory
+// and leave it 8 at a time, as one 32-byte sector.  flush() is called by all lanes of a warp at the
+// same steps, at most 8 put() apart, so it runs for most lanes at once: flushing each lane when its 8
+// entries are full ran that code for one or two lanes in most loop trips.
+constexpr int kStageSlots = 16;
+constexpr int kStageStride = kStageSlots + 4;  // words per thread: 16-byte aligned, spread over the banks
+struct ListStage {
+    uint32_t slots;  // shared-memory address of this thread's ring
+    uint32_t* out;   // 32-byte aligned; the history's path bound covers every entry, rounded up to 8
+    int n, sent;
+    uint32_t last;
+    __device__ __forceinline__ void store(int slot, uint32_t voxel)
+    {
+        asm volatile("st.shared.u32 [%0], %1;" ::"r"(slots + 4 * slot), "r"(voxel) : "memory");
+    }
+    __device__ __forceinline__ void first(uint32_t voxel)
+    {
+        last = voxel;
+        store(0, voxel);
+        n = 1;
+        sent = 0;
+    }
+    // Appends voxel unless it repeats the last entry (B.cu:9244-9251), without a branch: the slot of
+    // the last entry is written again.
+    __device__ __forceinline__ void put(uint32_t voxel)
+    {
+        n += voxel != last ? 1 : 0;
+        last = voxel;
+        store((n - 1) & (kStageSlots - 1), voxel);
+    }
+    __device__ __forceinline__ void send()
+    {
+        const uint32_t from = slots + 4 * (sent & (kStageSlots - 1));
+        uint4 a, b;
+        asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(a.x), "=r"(a.y), "=r"(a.z), "=r"(a.w) : "r"(from) : "memory");
+        asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(b.x), "=r"(b.y), "=r"(b.z), "=r"(b.w) : "r"(from + 16) : "memory");
+        uint4* to = reinterpret_cast<uint4*>(out + sent);
+        to[0] = a;
+        to[1] = b;
+        sent += 8;
+    }
+    __device__ __forceinline__ void flush()
+    {
+        if (n - sent >= 8) send();
+    }
+    __device__ __forceinline__ void finish()
+    {
+        while (sent < n) send();  // the last sector padded with stale slots
+    }
+};
+
+// The set-up of history i (position in h), from its inputs.
+__device__ __forceinline__ MlpStart mlp_start_of(const Geometry& g, const Tables& tab, const HistorySoA& h, long long i,
+                                                 unsigned& flags, double* chord)
+{
+    double xy_entry_angle = __ldg(h.xy_entry_angle + i), xy_exit_angle = __ldg(h.xy_exit_angle + i);
+    const double xz_entry_angle = __ldg(h.xz_entry_angle + i), xz_exit_angle = __ldg(h.xz_exit_angle + i);
+    const MlpStart m = mlp_start(g, tab, __ldg(h.x_entry + i), __ldg(h.y_entry + i), __ldg(h.z_entry + i),
+                                 __ldg(h.x_exit + i), __ldg(h.y_exit + i), __ldg(h.z_exit + i), xy_entry_angle,
+                                 xy_exit_angle, xz_entry_angle, xz_exit_angle, flags);
+    if (chord)
+        *chord = effective_chord_length(g, (xy_entry_angle + xy_exit_angle) / 2.0, (xz_entry_angle + xz_exit_angle) / 2.0);
+    return m;
+}
+
+// The voxel of one point (step k, u and depth as the walk carries them) by the guarded fast point or
+// in the reference's order.
+__device__ __forceinline__ uint32_t general_point(const Geometry& g, const Tables& tab,
+                                                  const StepConst* __restrict__ steps, const MlpStart& m, int k,
+                                                  double depth_2_go, double u_shifted)
+{
+    const StepConst& st = steps[k];
+    const Sigma2 m2 = sigma2_moments(m.h, st, tab.scattering_table,
+                                     m.sigma_2_index - (unsigned)(k - 1) * g.sigma_index_step);
+    uint32_t voxel;
+    if (g.exact_fast_points && mlp_point_fast(g, m.h, st, m2.sigma_t2, m2.sigma_t2_theta2, m2.sigma_theta2,
+                                              m2.determinant, depth_2_go, u_shifted, voxel))
+        return voxel;
+    double t_1, v_1;
+    mlp_point_rest(m.h, st, m2, depth_2_go, t_1, v_1);
+    return mlp_voxel(g, m.h, u_shifted, t_1, v_1);
+}
+
+// The depth and position of step k as the walk's recurrences carry them (step 1: u_2 - s and u_in + s).
+__device__ __forceinline__ void recurrences(const MlpStart& m, double s, int k, double& depth_2_go, double& u_shifted)
+{
+    depth_2_go = m.depth_2_go;
+    u_shifted = m.u_shifted + s;
+    for (int j = 1; j < k; j++) {
+        depth_2_go -= s;
+        u_shifted += s;
+    }
+}
+
+// What the table loop leaves to the general points starts again from the history's inputs, so that the
+// loop keeps nothing for it.  The voxel of step k of history i of h:
+__device__ __forceinline__ uint32_t general_point_of(const Geometry& g, const Tables& tab,
+                                                         const StepConst* __restrict__ steps, const HistorySoA& h,
+                                                         int i, int k)
+{
+    unsigned flags = 0;
+    const MlpStart m = mlp_start_of(g, tab, h, i, flags, nullptr);
+    double depth_2_go, u_shifted;
+    recurrences(m, g.mlp_u_step, k, depth_2_go, u_shifted);
+    return general_point(g, tab, steps, m, k, depth_2_go, u_shifted);
+}
+
+// The walk of history i from step k to its end (not inlined: few histories need it), its list of at most cap entries finished; returns the
+// list's length, and adds the walk's flags.
+static __device__ __noinline__ int general_walk_of(const Geometry& g, const Tables& tab,
+                                                   const StepConst* __restrict__ steps, int kmax, const HistorySoA& h,
+                                                   int i, int k, int cap, ListStage list, unsigned* flags)
+{
+    const double s = g.mlp_u_step;
+    unsigned f = 0;
+    const MlpStart m = mlp_start_of(g, tab, h, i, f, nullptr);
+    double depth_2_go, u_shifted;
+    recurrences(m, s, k, depth_2_go, u_shifted);
+    int trips = 0;
+    while (m.tables_ok && depth_2_go > s) {
+        if (k > kmax) {  // cannot happen while the u_2 index is inside the tables
+            f |= kFlagTableRange;
+            break;
+        }
+        const uint32_t voxel = general_point(g, tab, steps, m, k, depth_2_go, u_shifted);
+        if (voxel >= (uint32_t)g.padded_voxels) f |= kFlagVoxelOOB;
+        if (list.n < cap) list.put(voxel);
+        else f |= kFlagPathOverflow;  // cannot happen: cap bounds the loop count
+        depth_2_go -= s;
+        u_shifted += s;
+        k++;
+        if ((++trips & 7) == 0) list.flush();
+    }
+    list.finish();
+    *flags |= f;
+    return list.n;
+}
+
+// The exact walk of the path kernel: the same voxel list as mlp_walk_exact, without the sum over x, for
+// history i of h; all lanes of a warp call it, those without a history (cap = 0) write nothing.  The
+// warp runs its lanes' table rows in lockstep in an inner loop, and leaves that loop together when a
+// point is not proven.  With the general point inside the hot loop, called or inlined, its registers
+// were spilled in every step (7.7 ms per 4M head histories against 3.3 this way and 3.1 without any
+// general point).
+__device__ __forceinline__ int mlp_walk_table(const Geometry& g, const Tables& tab, const MlpTable& tb,
+                                              const StepConst* __restrict__ steps, int kmax, const HistorySoA& h,
+                                              int i, int cap, uint32_t slots, uint32_t* out, double* chord,
+                                              unsigned* flags)
+{
+    TableWalk t{};
+    t.whole = true;
+    uint32_t first = 0;
+    if (cap > 0) {
+        double c;
+        const MlpStart m = mlp_start_of(g, tab, h, i, *flags, &c);
+        *chord = c;
+        t = table_walk_start(g, tb, m.h, m.u_in, m.tables_ok);
+        if (t.klast >= cap) {  // cannot happen: the bound is at least the steps + 2
+            t.klast = cap - 1;
+            t.whole = false;
+        }
+        first = __ldg(h.first_MLP_voxel + i);
+    }
+    ListStage list{slots, out, 0, 0, 0u};
+    list.first(first);
+    bool outside = first >= (uint32_t)g.padded_voxels;
+    const int warp_last = __reduce_max_sync(0xffffffffu, t.klast);
+    for (int k = 1; k <= warp_last;) {
+        uint32_t voxel = 0;
+        bool proven = true;
+        for (;;) {
+            const bool on = k <= t.klast;
+            voxel = list.last;
+            if (on) {
+                const float4 r0 = __ldg(t.row), r1 = __ldg(t.row + 1);
+                t.row += 2;
+                t.ax += t.dx;
+                t.ay += t.dy;
+                proven = table_point(g, tb, t, r0, r1, voxel);
+                t.sigma += t.dsigma;
+            }
+            if (__any_sync(0xffffffffu, !proven)) break;
+            outside |= voxel >= (uint32_t)g.padded_voxels;
+            list.put(voxel);
+            if ((k & 7) == 0) list.flush();
+            if (++k > warp_last) break;
+        }
+        if (k > warp_last) break;
+        if (!proven) voxel = general_point_of(g, tab, steps, h, i, k);
+        __syncwarp();
+        outside |= voxel >= (uint32_t)g.padded_voxels;
+        list.put(voxel);
+        if ((k & 7) == 0) list.flush();
+        k++;
+    }
+    if (cap <= 0) return 0;
+    if (outside) *flags |= kFlagVoxelOOB;
+    if (t.whole) {
+        list.finish();
+        return list.n;
+    }
+    list.flush();
+    return general_walk_of(g, tab, steps, kmax, h, i, t.klast + 1, cap, list, flags);
 }
 
 // ------------------------------------------------------------------------------------------

@@ -20,6 +20,26 @@ struct StepConst {
     float s1i0f, s1i1f, s1i2f;  // float copies for the mixed-precision right-hand sides and inversions
 };
 
+// Tabulated MLP points (pct_mlp.cuh, "Tabulated points"): per bucket of u_2 its first row (2 float4
+// per row, step 1 first), last step with a row (0: none) and the bounds on its rows.
+struct MlpBucket {
+    int row, klast, steps;  // steps: those of a walk whose u_2 lies inside the bucket
+    float err_b, err_c;  // largest deviation of the weights B and C from the reference's
+    float err_r;         // rounding error of the reference's point per cm of the history's scale (mag_tv)
+    float max_b, max_c;  // largest |B| and |C|
+    double kappa;        // sigma = delta + k kappa epsilon
+};
+struct MlpTable {
+    const float4* rows;
+    const MlpBucket* bucket;
+    int buckets;     // 0: no table (every point by the guarded fast point or in the reference's order)
+    int frac_bits;   // fraction bits of the fixed-point positions
+    float t_max;       // largest lateral offset (cm) a position's offset holds
+    double inv_width;  // 1 / bucket width
+};
+constexpr double kSigmaUnit = 2.5e-5;  // half the polynomial-table step: delta in units of its range
+constexpr double kInvSigmaUnit = 40000.0;
+
 double trig_table_min();
 double trig_table_step();
 int trig_table_elements();
