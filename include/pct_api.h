@@ -98,11 +98,12 @@ typedef struct pct_config {
                                       (the reference launch arithmetic, B.cu:9558); 0: all   */
     /* engine options */
     int32_t PRECISION;             /* PCT_PRECISION_EXACT: the reference's arithmetic (voxel
-                                      lists bit-identical); PCT_PRECISION_MIXED: FP64 Sigma
-                                      algebra, FP32 solve and voxel indices in the path kernel
-                                      (path storage and pct_mlp_paths; the single-pass kernel
-                                      stays exact), and the DROP update in FP32 with a
-                                      compensated sum of x; PCT_PRECISION_MIXED_COMPENSATED:
+                                      lists bit-identical); PCT_PRECISION_MIXED: the DROP
+                                      update in FP32 with a compensated sum of x, and path
+                                      points that may be FP32 (FP64 Sigma algebra, FP32 solve
+                                      and voxel indices: used where EXACT_FAST_POINTS = 0 or
+                                      the grid is too large for the tabulated points, which
+                                      are the exact ones); PCT_PRECISION_MIXED_COMPENSATED:
                                       MIXED plus a compensated per-voxel accumulation of the
                                       updates (a second float array of rounding errors)        */
     int32_t SCATTER_MODE;          /* PCT_SCATTER_*                                            */

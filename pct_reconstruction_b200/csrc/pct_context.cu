@@ -1233,7 +1233,9 @@ extern "C" pct_status pct_mlp_paths(pct_ctx* ctx, int64_t start, int64_t n, int3
         da = a_dot_x ? (double*)p : nullptr;
     }
     cudaError_t e = pct::launch_mlp_paths_exact(ctx->geo, ctx->tables, ctx->d_steps, ctx->kmax, ctx->d_x, ctx->hist,
-                                                start, n, stride, dc, dv, dl, da, ctx->d_counters, ctx->stream);
+                                                start, n, stride, dc, dv, dl, da, ctx->d_counters,
+                                                // the lists an iteration uses: see launch_mlp_phase1_exact
+                                                ctx->geo.mixed_precision && ctx->mlp_table.buckets == 0, ctx->stream);
     if (e != cudaSuccess) {
         cudaFree(tmp);
         return ctx_fail(ctx, PCT_ERR_CUDA, "mlp_paths kernel", e);

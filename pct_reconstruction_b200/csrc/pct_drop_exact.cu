@@ -225,7 +225,7 @@ __global__ void path_bounds_kernel(Geometry g, Tables tab, HistorySoA h, long lo
 #ifndef PCT_PHASE1_MIN_BLOCKS
 #define PCT_PHASE1_MIN_BLOCKS 7
 #endif
-// The mixed-precision path kernel keeps 8 CTAs (64 registers), as measured when it was tuned.
+// The path kernel of FP32 points keeps 8 CTAs (64 registers), as measured when it was tuned.
 #ifndef PCT_PHASE1_MIXED_MIN_BLOCKS
 #define PCT_PHASE1_MIXED_MIN_BLOCKS 8
 #endif
@@ -293,6 +293,8 @@ __global__ void __launch_bounds__(kThreads, 7 * 128 / kThreads) mlp_phase1_exact
     chord[id] = r.chord;
 }
 
+// PRECISION MIXED or MIXED_COMPENSATED without a table.  With one, these modes take the table kernel
+// too: its points are the exact ones and cost less (2M head histories 3.47 against 5.04 ms an iteration).
 template <int kThreads>
 __global__ void __launch_bounds__(kThreads, PCT_PHASE1_MIXED_MIN_BLOCKS * 128 / kThreads) mlp_phase1_mixed_kernel(
     Geometry g, Tables tab, const StepConst* __restrict__ steps, int kmax, HistorySoA h, const int* __restrict__ perm,
@@ -692,7 +694,7 @@ MlpTableShape mlp_table_shape(const Geometry& g, int kmax)
 {
     MlpTableShape t{};
     const double s = g.mlp_u_step;
-    if (!g.exact_fast_points || g.mixed_precision) return t;
+    if (!g.exact_fast_points) return t;
     // positions: frac_bits fraction bits, the rest for the grid and its surroundings
     int extent = g.columns > g.rows ? g.columns : g.rows;
     if (g.slices > extent) extent = g.slices;
@@ -764,11 +766,11 @@ cudaError_t launch_mlp_phase1_exact(const Geometry& g, const Tables& tab, const 
 #define PCT_PHASE1(T)                                                                                             \
     do {                                                                                                          \
         const unsigned blocks = (unsigned)((count + (T) - 1) / (T));                                              \
-        if (g.mixed_precision)                                                                                    \
-            mlp_phase1_mixed_kernel<T><<<blocks, T, 0, stream>>>(g, tab, steps, kmax, h, perm, count, offsets,    \
-                                                                 offset_base, bounds, paths, path_n, chord, counters); \
-        else if (tb.buckets > 0)                                                                                  \
+        if (tb.buckets > 0)                                                                                       \
             mlp_phase1_table_kernel<T><<<blocks, T, 0, stream>>>(g, tab, tb, steps, kmax, h, perm, count, offsets, \
+                                                                 offset_base, bounds, paths, path_n, chord, counters); \
+        else if (g.mixed_precision)                                                                               \
+            mlp_phase1_mixed_kernel<T><<<blocks, T, 0, stream>>>(g, tab, steps, kmax, h, perm, count, offsets,    \
                                                                  offset_base, bounds, paths, path_n, chord, counters); \
         else                                                                                                      \
             mlp_phase1_exact_kernel<T><<<blocks, T, 0, stream>>>(g, tab, steps, kmax, h, perm, count, offsets,    \
@@ -813,29 +815,28 @@ cudaError_t launch_drop_phase2(const Geometry& g, const float* x, float2* acc, f
     return e;
 }
 
-// The carve-out, in percent of the largest shared memory an SM offers (228 KB on B200).  58% asks for
-// a little over 132 KB, so the driver takes the 164 KB configuration: 7 path-kernel CTAs of 20.5 KB
-// (stash and list staging) plus the per-CTA reserve fit, and registers, not shared memory, limit them.
-// 57% gives the 132 KB configuration, 6 path CTAs and room in the register file for one DROP-block
-// CTA beside them; measured 74.7 vs 72.9 ms per 20M-history head iteration, so 58% stays.  A
-// negative value leaves each kernel to the driver's choice.  Measured on B200 (exact
-// mode, ms per iteration): small configuration at 10M histories (blocks of 3200, 196 path chunks)
-// 31.5 with it, 66.0 without; 2M histories 6.33 vs 13.25; head 20M 73.6 vs 73.9.
+// The carve-out, in percent of the largest shared memory an SM offers (228 KB on B200), for every kernel
+// of an iteration: 7 path CTAs keep 10 KB of list staging each, the rest is L1 for the table rows and
+// the gathers.  Measured on B200 (ms per iteration; 4M head / 600k small / 2M head mixed): 25% 6.94 /
+// 1.467 / 3.82 (6 path CTAs), 35% 6.59 / 1.471 / 3.46, 45% 6.64 / 1.466 / 3.47, 58% 6.69 / 1.482 /
+// 3.49, 75% 6.82 / 1.509 / 3.49, each kernel's own 6.85 / 2.172 / 3.47.
 #ifndef PCT_ITERATION_CARVEOUT
-#define PCT_ITERATION_CARVEOUT 58
+#define PCT_ITERATION_CARVEOUT 40
 #endif
 
 cudaError_t set_iteration_carveout()
 {
     const int percent = PCT_ITERATION_CARVEOUT;
     if (percent < 0) return cudaSuccess;
-    // the exact mode's kernels only: the mixed-precision path kernel keeps no shared memory, and it
-    // and its block kernels run best with the driver's choice (its L1 holds the table gathers)
     const void* kernels[] = {
         (const void*)mlp_phase1_exact_kernel<64>, (const void*)mlp_phase1_exact_kernel<128>,
         (const void*)mlp_phase1_exact_kernel<256>, (const void*)mlp_phase1_table_kernel<64>,
         (const void*)mlp_phase1_table_kernel<128>, (const void*)mlp_phase1_table_kernel<256>,
+        (const void*)mlp_phase1_mixed_kernel<64>, (const void*)mlp_phase1_mixed_kernel<128>,
+        (const void*)mlp_phase1_mixed_kernel<256>,
         (const void*)drop_phase2_kernel<PCT_DROP, false, 0>, (const void*)drop_phase2_kernel<PCT_DROP, true, 0>,
+        (const void*)drop_phase2_kernel<PCT_DROP, false, 1>, (const void*)drop_phase2_kernel<PCT_DROP, true, 1>,
+        (const void*)drop_phase2_kernel<PCT_DROP, false, 2>,
         (const void*)drop_phase2_kernel<PCT_ROBUSTA, false, 0>, (const void*)drop_phase2_kernel<PCT_ROBUSTA, true, 0>,
         (const void*)drop_phase2_kernel<PCT_ROBUSTB, false, 0>,
         (const void*)drop_phase2_kernel<PCT_DROP, false, 0, true>, (const void*)drop_phase2_kernel<PCT_DROP, true, 0, true>};
@@ -861,12 +862,12 @@ cudaError_t launch_drop_block_exact(const Geometry& g, const Tables& tab, const 
 cudaError_t launch_mlp_paths_exact(const Geometry& g, const Tables& tab, const StepConst* steps, int kmax,
                                    const float* x, const HistorySoA& h, long long begin, long long count, int stride,
                                    uint32_t* counts, uint32_t* voxels, double* chord, double* a_dot_x,
-                                   unsigned long long* counters, cudaStream_t stream)
+                                   unsigned long long* counters, bool fp32_points, cudaStream_t stream)
 {
     if (count <= 0) return cudaSuccess;
     const int threads = 128;
     const long long blocks = (count + threads - 1) / threads;
-    if (g.mixed_precision)
+    if (fp32_points)
         mlp_paths_kernel<true><<<(unsigned)blocks, threads, 0, stream>>>(g, tab, steps, kmax, x, h, begin, count,
                                                                          stride, counts, voxels, chord, a_dot_x,
                                                                          counters);

@@ -12,7 +12,7 @@ int sm_count();
 // One shared-memory carve-out for every kernel a captured DROP iteration runs concurrently (path
 // kernels, DROP block kernels, image updates), set on the current device.  An SM runs CTAs of
 // kernels with different carve-outs only after it has drained and been reconfigured, so the block
-// chain's small kernels, interleaved with path-kernel chunks that keep 16 KB of shared memory per
+// chain's small kernels, interleaved with path-kernel chunks that keep 10 KB of shared memory per
 // CTA, would otherwise wait for whole SMs to empty.
 cudaError_t set_iteration_carveout();
 cudaError_t set_image_update_carveout(int percent);
@@ -39,11 +39,11 @@ cudaError_t launch_drop_block_exact(const Geometry& g, const Tables& tab, const 
                                     const float* x, float2* acc, const HistorySoA& h, long long begin,
                                     long long count, unsigned long long* counters, cudaStream_t stream);
 
-// MLP voxel lists for parity checks (exact mode).
+// MLP voxel lists for parity checks: the exact walk's, or with fp32_points the mixed walk's.
 cudaError_t launch_mlp_paths_exact(const Geometry& g, const Tables& tab, const StepConst* steps, int kmax,
                                    const float* x, const HistorySoA& h, long long begin, long long count, int stride,
                                    uint32_t* counts, uint32_t* voxels, double* chord, double* a_dot_x,
-                                   unsigned long long* counters, cudaStream_t stream);
+                                   unsigned long long* counters, bool fp32_points, cudaStream_t stream);
 
 // Loop trips (MLP points) of the exact walk of histories [begin, begin+count).
 cudaError_t launch_mlp_steps(const Geometry& g, const Tables& tab, int kmax, const HistorySoA& h, long long begin,

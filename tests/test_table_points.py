@@ -101,3 +101,21 @@ def test_blocks_and_order(per_block, order):
 @pytest.mark.parametrize("threads", [64, 128, 256])
 def test_irregular_histories(threads):
     both(dict(GRID, PATH_CTA_THREADS=threads), irregular, 40000, 5)
+
+
+@pytest.mark.gpu
+def test_mixed_mode_takes_the_exact_lists():
+    """With the table, PRECISION = MIXED walks the same points, so its lists are the exact mode's."""
+    from pct_reconstruction_b200 import Context
+    out = []
+    for precision in ("EXACT", "MIXED"):
+        cfg = Config(**GRID, PRECISION=precision)
+        with Context(cfg) as ctx:
+            ctx.set_reconstruction_histories(simulated(cfg, 20000, 6))
+            ctx.x_host_2_GPU(np.ones(cfg.NUM_VOXELS, np.float32))
+            out.append(ctx.mlp_paths())
+            ctx.DROP_full_tx_iteration(1)
+            out[-1] += (ctx.x_GPU_2_host(),)
+    for a, b in zip(out[0][:4], out[1][:4]):
+        np.testing.assert_array_equal(a, b)
+    np.testing.assert_allclose(out[1][4], out[0][4], rtol=0, atol=1e-6)  # FP32 updates of about 1e-4
