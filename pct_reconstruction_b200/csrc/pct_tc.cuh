@@ -46,42 +46,9 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint3
     return d;
 }
 
-// Shared-memory matrix descriptor of a K-major operand in a swizzled layout, as TMA writes it with
-// CU_TENSOR_MAP_SWIZZLE_{32,64,128}B when every row holds exactly `row_bytes` = 32, 64 or 128 bytes
-// of K: rows are row_bytes apart, 8-row groups 8 * row_bytes apart (SBO), LBO unused; the tile
-// base must be aligned to the swizzle atom (8 * row_bytes).  A K step inside the row advances the
-// start address by its byte offset.
-__device__ __forceinline__ uint64_t smem_desc_swizzled(uint32_t addr, uint32_t row_bytes)
+__device__ __forceinline__ void mbar_arrive(uint32_t mbar)
 {
-    const uint64_t layout = row_bytes == 128 ? 2u : row_bytes == 64 ? 4u : 6u;  // SWIZZLE_128B / 64B / 32B
-    uint64_t d = 0;
-    d |= static_cast<uint64_t>((addr >> 4) & 0x3FFFu);
-    d |= static_cast<uint64_t>(((8u * row_bytes) >> 4) & 0x3FFFu) << 32;
-    d |= static_cast<uint64_t>(1) << 46;
-    d |= layout << 61;
-    return d;
-}
-
-// mbarrier: one arrival that also announces the bytes the TMA copies will deliver
-__device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t mbar, uint32_t bytes)
-{
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" :: "r"(mbar), "r"(bytes) : "memory");
-}
-
-// TMA tiled loads of this CTA's own tile into its shared memory, completion counted on mbar.  The innermost
-// coordinate must be a multiple of 16 bytes; the others may fall outside the tensor (zero fill).
-__device__ __forceinline__ void tma_load_3d(uint32_t dst, const void* tmap, uint32_t mbar, int c0, int c1, int c2)
-{
-    asm volatile(
-        "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
-        :: "r"(dst), "l"(reinterpret_cast<uint64_t>(tmap)), "r"(mbar), "r"(c0), "r"(c1), "r"(c2) : "memory");
-}
-__device__ __forceinline__ void tma_load_4d(uint32_t dst, const void* tmap, uint32_t mbar, int c0, int c1, int c2,
-                                            int c3)
-{
-    asm volatile(
-        "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
-        :: "r"(dst), "l"(reinterpret_cast<uint64_t>(tmap)), "r"(mbar), "r"(c0), "r"(c1), "r"(c2), "r"(c3) : "memory");
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" :: "r"(mbar) : "memory");
 }
 
 // Instruction descriptor for kind::f16 with bf16 A and B, fp32 D, M = 128, dense.
@@ -104,6 +71,36 @@ __device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint64_t a, uint64_t b
         "setp.ne.b32 p, %4, 0;\n\t"
         "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n"
         :: "r"(tmem_d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate));
+}
+
+// The same for a warp that runs the issuing code with all its lanes: only the lane with leader != 0
+// issues.  Control flow and descriptors stay warp-uniform, so they live in uniform registers; issued
+// from a branch of one thread, an MMA of 128 x 48 x 16 took twice as long to issue as to execute.  A
+// descriptor is its high word and a low word whose address field counts 16 bytes.
+__device__ __forceinline__ void mma_bf16_warp(uint32_t tmem_d, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo, uint32_t b_hi,
+                                              uint32_t idesc, uint32_t accumulate, uint32_t leader)
+{
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t.reg .b64 a, b;\n\t"
+        "setp.ne.b32 p, %6, 0;\n\tsetp.ne.b32 q, %7, 0;\n\t"
+        "mov.b64 a, {%1, %2};\n\tmov.b64 b, {%3, %4};\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %5, p;\n\t}\n"
+        :: "r"(tmem_d), "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate), "r"(leader));
+}
+
+__device__ __forceinline__ void mma_commit_warp(uint32_t mbar, uint32_t leader)
+{
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t"
+                 "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}\n"
+                 :: "r"(mbar), "r"(leader) : "memory");
+}
+
+// 1 in one lane of the (converged) warp, 0 in the others.
+__device__ __forceinline__ uint32_t elect_one()
+{
+    uint32_t is;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.b32 %0, 1, 0, p;\n\t}\n" : "=r"(is));
+    return is;
 }
 
 __device__ __forceinline__ void mma_commit(uint32_t mbar)
@@ -134,15 +131,18 @@ __device__ __forceinline__ bool mbar_test(uint32_t mbar, uint32_t parity)
     return done != 0;
 }
 
-// Wait for the phase of the given parity to complete; false if kWaitNs passed first.
+// Wait for the phase of the given parity to complete; false if kWaitNs passed first (the clock is read
+// once in 64 polls).
 __device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t parity)
 {
-    if (mbar_test(mbar, parity)) return true;
+    for (int i = 0; i < 64; ++i)
+        if (mbar_test(mbar, parity)) return true;
     const unsigned long long t0 = global_ns();
-    while (!mbar_test(mbar, parity)) {
+    for (;;) {
+        for (int i = 0; i < 64; ++i)
+            if (mbar_test(mbar, parity)) return true;
         if (global_ns() - t0 > kWaitNs) return false;
     }
-    return true;
 }
 
 // TMEM allocation by one full warp; the column base is written to shared memory at slot.

@@ -17,18 +17,14 @@
 // Grids must have COLUMNS, ROWS and SLICES divisible by 8.
 //
 // Kernels:
-//  * conv3_fwd_kernel: implicit GEMM, one CTA per 128 output voxels (M = 128), N = output
-//    channels, K = 27 taps x input channels; per tap the CTA gathers the 128 shifted input rows
-//    and the tap's weights into shared memory (K-major core-matrix layout), one thread issues
-//    the tcgen05.mma instructions into the TMEM accumulator, two stages overlap the gather of
-//    tap t+1 with the MMAs of tap t.  The same kernel computes the data gradient with the
-//    flipped, transposed weights W'[ci][26-t][co] = W[co][t][ci].  Epilogue: bias, residual,
-//    ReLU, ReLU-mask (for gradients), bf16 store; or the image output.
+//  * conv3_slab_kernel: implicit GEMM over patches of 128 positions, all 27 taps read from one copy of
+//    the input slices in shared memory, accumulators of consecutive output slices side by side in TMEM.
+//    The same kernel computes the data gradient with the flipped, transposed weights
+//    W'[ci][26-t][co] = W[co][t][ci].  Epilogue: bias, residual, ReLU, ReLU-mask (for gradients), bf16
+//    store; or the image output.
 //  * conv3_wgrad_kernel: dW[co][t][ci] = sum_v dZ[v][co] X[v + t][ci]: M = 128 (tap, channel)
 //    rows, N = output channels, K = voxels (64 per stage, MN-major operands, which is how both
 //    lie in memory); the voxel range is split over CTAs, partial sums are added with atomics.
-#include <cuda.h>
-#include <cudaTypedefs.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -104,25 +100,10 @@ __device__ __forceinline__ void unpack8(const uint4& u, float* f)
 
 // ----------------------------------------------------------------------------- convolutions --
 
-// Taps gathered per pipeline stage for 16-channel inputs (half as many for 32).  Measured on B200
-// (200x200x32, forward 16->16 / 32->16 upsampled, ms): 1 tap 0.321 / 0.466, 2 taps 0.314 / 0.505,
-// 4 taps 0.395 / 0.542 -- the deeper gather per stage costs more than the barriers it saves.
 // Weight-gradient CTAs per SM: 4 -> 0.541 ms, 6 -> 0.413 ms (16->16); training step 9.06 -> 8.47 ms.
-#ifndef PCT_CONV_TAPS_16
-#define PCT_CONV_TAPS_16 1
-#endif
 #ifndef PCT_WGRAD_CTAS_PER_SM
 #define PCT_WGRAD_CTAS_PER_SM 6
 #endif
-__host__ __device__ constexpr int taps_per_stage(int cin)
-{
-    return cin >= 64 ? 1 : (cin == 32 ? (PCT_CONV_TAPS_16 > 1 ? PCT_CONV_TAPS_16 / 2 : 1) : PCT_CONV_TAPS_16);
-}
-__host__ __device__ constexpr int conv_stage_bytes(int cin, int cout)
-{
-    return (taps_per_stage(cin) * (cin * tc::kTileM * 2 + cout * cin * 2) + 127) & ~127;
-}
-
 struct ConvFwdArgs {
     const bf16* in;      // [nz>>up][ny>>up][nx>>up][cin]
     int cin, up;
@@ -138,289 +119,367 @@ struct ConvFwdArgs {
     const uint8_t* hull;
     float* image;
     int* status;           // set to 1 when a bounded wait expired
+    int overlap;           // launched as a programmatic dependent of the kernel before it in the stream
 };
 
-// Epilogue of a forward / data-gradient convolution tile: this thread's TMEM lane (row) holds
-// voxel v's accumulators; every thread of the CTA calls it (tcgen05.ld is warp-collective).
-__device__ __forceinline__ void conv_epilogue(const ConvFwdArgs& p, uint32_t trow, long long v, bool row_ok)
+// Epilogue of a forward / data-gradient convolution for 16 channels from c0 on: this thread's TMEM lane
+// (row) holds voxel v's accumulators; whole warps call it (tcgen05.ld is warp-collective).  What it
+// adds and masks with is requested before the wait for the accumulators.
+struct EpilogueInputs {
+    uint4 r[2], m[2];
+};
+__device__ __forceinline__ EpilogueInputs epilogue_request(const ConvFwdArgs& p, long long v, int c0, bool row_ok)
 {
+    EpilogueInputs e{};
+    const size_t o = static_cast<size_t>(v) * p.cout + c0;
+    if (p.residual && row_ok) {
+        e.r[0] = reinterpret_cast<const uint4*>(p.residual + o)[0];
+        e.r[1] = reinterpret_cast<const uint4*>(p.residual + o)[1];
+    }
+    if (p.mask && row_ok) {
+        e.m[0] = reinterpret_cast<const uint4*>(p.mask + o)[0];
+        e.m[1] = reinterpret_cast<const uint4*>(p.mask + o)[1];
+    }
+    return e;
+}
+__device__ __forceinline__ void conv_epilogue(const ConvFwdArgs& p, uint32_t trow, long long v, int c0, bool row_ok,
+                                              const EpilogueInputs& e, const float* bias)
+{
+    float acc[16];
+    tc::tmem_load16(trow, acc);
+    if (!row_ok) return;
     if (p.image) {
-        float acc[16];
-        tc::tmem_load16(trow, acc);
-        if (row_ok) {
-            const float o = acc[0] + (p.bias ? p.bias[0] : 0.f);
-            p.image[v] = p.base[v] + (p.hull[v] ? o : 0.f);
-        }
-    } else {
-        for (int c0 = 0; c0 < p.cout; c0 += 16) {
-            float acc[16];
-            tc::tmem_load16(trow + c0, acc);
-            if (!row_ok) continue;
-            const size_t o = static_cast<size_t>(v) * p.cout + c0;
-            if (p.bias) {
-#pragma unroll
-                for (int i = 0; i < 16; ++i) acc[i] += p.bias[c0 + i];
-            }
-            if (p.residual) {
-                float r[16];
-                unpack8(__ldg(reinterpret_cast<const uint4*>(p.residual + o)), r);
-                unpack8(__ldg(reinterpret_cast<const uint4*>(p.residual + o) + 1), r + 8);
-#pragma unroll
-                for (int i = 0; i < 16; ++i) acc[i] += r[i];
-            }
-            if (p.relu) {
-#pragma unroll
-                for (int i = 0; i < 16; ++i) acc[i] = fmaxf(acc[i], 0.f);
-            }
-            if (p.mask) {
-                float m[16];
-                unpack8(__ldg(reinterpret_cast<const uint4*>(p.mask + o)), m);
-                unpack8(__ldg(reinterpret_cast<const uint4*>(p.mask + o) + 1), m + 8);
-#pragma unroll
-                for (int i = 0; i < 16; ++i) acc[i] = m[i] > 0.f ? acc[i] : 0.f;
-            }
-            uint4 w0, w1;
-            w0.x = pack_bf16(acc[0], acc[1]);
-            w0.y = pack_bf16(acc[2], acc[3]);
-            w0.z = pack_bf16(acc[4], acc[5]);
-            w0.w = pack_bf16(acc[6], acc[7]);
-            w1.x = pack_bf16(acc[8], acc[9]);
-            w1.y = pack_bf16(acc[10], acc[11]);
-            w1.z = pack_bf16(acc[12], acc[13]);
-            w1.w = pack_bf16(acc[14], acc[15]);
-            reinterpret_cast<uint4*>(p.out + o)[0] = w0;
-            reinterpret_cast<uint4*>(p.out + o)[1] = w1;
-        }
+        const float o = acc[0] + (p.bias ? bias[0] : 0.f);
+        p.image[v] = p.base[v] + (p.hull[v] ? o : 0.f);
+        return;
     }
+    if (p.bias) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) acc[i] += bias[i];
+    }
+    if (p.residual) {
+        float r[16];
+        unpack8(e.r[0], r);
+        unpack8(e.r[1], r + 8);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) acc[i] += r[i];
+    }
+    if (p.relu) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) acc[i] = fmaxf(acc[i], 0.f);
+    }
+    if (p.mask) {
+        float m[16];
+        unpack8(e.m[0], m);
+        unpack8(e.m[1], m + 8);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) acc[i] = m[i] > 0.f ? acc[i] : 0.f;
+    }
+    uint4 w0, w1;
+    w0.x = pack_bf16(acc[0], acc[1]);
+    w0.y = pack_bf16(acc[2], acc[3]);
+    w0.z = pack_bf16(acc[4], acc[5]);
+    w0.w = pack_bf16(acc[6], acc[7]);
+    w1.x = pack_bf16(acc[8], acc[9]);
+    w1.y = pack_bf16(acc[10], acc[11]);
+    w1.z = pack_bf16(acc[12], acc[13]);
+    w1.w = pack_bf16(acc[14], acc[15]);
+    uint4* out = reinterpret_cast<uint4*>(p.out + static_cast<size_t>(v) * p.cout + c0);
+    out[0] = w0;
+    out[1] = w1;
 }
 
-__global__ void __launch_bounds__(kThreads) conv3_fwd_kernel(ConvFwdArgs p)
-{
-    extern __shared__ __align__(128) uint8_t smem[];
-    __shared__ __align__(8) uint64_t mbar[2];
-    __shared__ uint32_t tmem_slot;
-    const int tid = threadIdx.x, warp = tid >> 5;
-    const long long V = static_cast<long long>(p.nx) * p.ny * p.nz;
-    const long long v = static_cast<long long>(blockIdx.x) * tc::kTileM + tid;
-    const uint32_t ncols = tc::tmem_columns(p.cout);
-    const int tps = taps_per_stage(p.cin);
-    const int a_tap = p.cin * tc::kTileM * 2, b_tap = p.cout * p.cin * 2;
-    const int stage_bytes = conv_stage_bytes(p.cin, p.cout);
+// ---- slab convolution -------------------------------------------------------------------------
+// One CTA computes nc output channels of a patch of W x H voxels over a run of zt slices.  It keeps the
+// 27 taps' weights for its channels in shared memory and streams the run's input slices, each with its
+// one-voxel halo, through a ring; every slice is brought from L2 once per CTA instead of once per tap.
+//
+// In shared memory a slice is [channels / 8][position][8 channels], positions being the patch with its
+// halo in rows of W + 2.  In the no-swizzle K-major layout eight consecutive rows of 16 bytes are a
+// core matrix, and here every position is a row, so a tap (dy, dx) is the same matrix from a start
+// address (dy (W + 2) + dx) 16 bytes further: all nine taps of a slice read one copy.  The M = 128 rows
+// of an MMA are 128 consecutive positions from there; the rows of the halo columns come out unused.
+//
+// The three taps in z are the N side: the weights of dz = +1, 0, -1 lie one below the other, and the
+// accumulators of consecutive output slices in consecutive TMEM columns, so one MMA of N = 3 nc adds
+// an input slice to the three output slices that it reaches.  For every output the products are added
+// in the order of the taps 0 to 26 and channels ascending.
+//
+// What bounds it is shared memory: an MMA of N = 48 reads 5.5 KB for 128 x 48 x 16 products, 44 of its
+// 54 cycles.  One pass over 200x200x32 takes, in us (the kernels that brought every tap's inputs
+// apart, by TMA or by threads for an upsampled input, in brackets): 16 to 16 channels 50 (263), 32 to 16
+// upsampled with a skip 98 (466); 100x100x16, 32 to 32 27, 64 to 32 upsampled 39; 50x50x8, 64 to 64 20;
+// 25x25x4, 128 to 128 20.  The network's forward pass 0.55 ms (2.04).
+//
+// Four warps bring the slices (cp.async, zero fill outside the grid, indices halved for an upsampled
+// input), `ahead` of them in flight; one thread of the fifth issues the MMAs; four more write each
+// output slice as soon as its last input slice is done.  A CTA keeps its weights and goes on with every
+// gridDim.x-th tile (patch and run); with two accumulator stages the MMAs of a tile run while the
+// previous tile is written.
+constexpr int kSlabProducers = 128;
+constexpr int kSlabThreads = kSlabProducers + 32 + 128;  // 416 with a second group of writers: one CTA per SM fewer
+constexpr int kSlabMaxRing = 6;
+constexpr int kSlabMaxSlices = 32;
+constexpr int kSlabMaxPositions = 512;
+constexpr int kSlabSmemLimit = 224 * 1024;  // dynamic; the per-block maximum (227 KB) also holds the static part
 
-    if (warp == 0) tc::tmem_alloc(tc::smem_addr(&tmem_slot), ncols);
-    if (tid == 0) {
-        tc::mbar_init(tc::smem_addr(&mbar[0]), 1);
-        tc::mbar_init(tc::smem_addr(&mbar[1]), 1);
-        tc::mbar_init_fence();
-    }
-    tc::fence_before_sync();
-    __syncthreads();
-    tc::fence_after_sync();
-    const uint32_t tmem = tmem_slot;
-    Pipe pp{{tc::smem_addr(&mbar[0]), tc::smem_addr(&mbar[1])}, {0, 0}, {0, 0}};
-
-    const bool row_ok = v < V;
-    int x = 0, y = 0, z = 0;
-    if (row_ok) {
-        x = static_cast<int>(v % p.nx);
-        const long long r = v / p.nx;
-        y = static_cast<int>(r % p.ny);
-        z = static_cast<int>(r / p.ny);
-    }
-    const int sx = p.nx >> p.up, sy = p.ny >> p.up;
-    const uint32_t sbo = static_cast<uint32_t>(p.cin) * 16u;  // 8 rows x cin bf16
-    const int kc = p.cin >> 3;                                // 16-byte chunks per row
-    const uint32_t idesc = tc::idesc_bf16_f32(p.cout, false);
-    bool ok = true;
-    int it = 0;
-    for (int t0 = 0; t0 < 27; t0 += tps, ++it) {
-        const int b = it & 1;
-        if (!stage_free(pp, b)) {
-            ok = false;
-            break;
-        }
-        uint8_t* sa = smem + b * stage_bytes;
-        uint8_t* sb = sa + tps * a_tap;
-        const int nt = t0 + tps <= 27 ? tps : 27 - t0;
-        for (int q = 0; q < nt; ++q) {
-            const int t = t0 + q;
-            const int zz = z + t / 9 - 1, yy = y + (t / 3) % 3 - 1, xx = x + t % 3 - 1;
-            const bool inside = row_ok && zz >= 0 && zz < p.nz && yy >= 0 && yy < p.ny && xx >= 0 && xx < p.nx;
-            uint8_t* dst = sa + q * a_tap + (tid >> 3) * sbo + (tid & 7) * 16;
-            if (inside) {
-                const size_t src_voxel = (static_cast<size_t>(zz >> p.up) * sy + (yy >> p.up)) * sx + (xx >> p.up);
-                const uint4* src = reinterpret_cast<const uint4*>(p.in + src_voxel * p.cin);
-                for (int c = 0; c < kc; ++c) *reinterpret_cast<uint4*>(dst + c * 128) = __ldg(src + c);
-            } else {
-                for (int c = 0; c < kc; ++c) *reinterpret_cast<uint4*>(dst + c * 128) = make_uint4(0, 0, 0, 0);
-            }
-            uint8_t* sbq = sb + q * b_tap;
-            for (int u = tid; u < p.cout * kc; u += kThreads) {
-                const int n = u / kc, c = u - n * kc;
-                const uint4 w = __ldg(reinterpret_cast<const uint4*>(p.weight + (static_cast<size_t>(n) * 27 + t) * p.cin) + c);
-                *reinterpret_cast<uint4*>(sbq + (n >> 3) * sbo + c * 128 + (n & 7) * 16) = w;
-            }
-        }
-        tc::fence_proxy_async();
-        __syncthreads();
-        if (tid == 0) {
-            tc::fence_after_sync();
-            for (int q = 0; q < nt; ++q) {
-                const uint32_t a0 = tc::smem_addr(sa + q * a_tap), b0 = tc::smem_addr(sb + q * b_tap);
-                for (int j = 0; j < (p.cin >> 4); ++j)
-                    tc::mma_bf16(tmem, tc::smem_desc(a0 + j * 256, 128, sbo), tc::smem_desc(b0 + j * 256, 128, sbo),
-                                 idesc, (t0 | q | j) != 0);
-            }
-            tc::mma_commit(pp.mbar[b]);
-        }
-        pp.issued[b]++;
-    }
-    ok = drain(pp) && ok;
-    tc::fence_after_sync();
-    if (ok) {
-        conv_epilogue(p, tmem + (static_cast<uint32_t>(warp * 32) << 16), v, row_ok);
-    } else if (tid == 0) {
-        atomicExch(p.status, 1);
-    }
-    tc::fence_before_sync();
-    __syncthreads();
-    if (warp == 0) {
-        tc::fence_after_sync();
-        tc::tmem_dealloc(tmem, ncols);
-    }
-}
-
-// ---- TMA-fed forward convolution ------------------------------------------------------------
-// The same convolution with the operand tiles brought by TMA instead of thread gathers.  A CTA owns
-// the 128 voxels of a 32 x 4 patch of one slice (TMEM lane = y_local * 32 + x_local).  For tap t
-// the A tile is the box of the channels-last activation tensor at (x0+dx, y0+dy, z+dz) -- boxes
-// that reach outside the grid are zero-filled by TMA, which is the convolution's zero padding --
-// and the B tile is the tap's [cout][cin] weight slab.  Both arrive in the swizzled K-major layout
-// the MMA reads (rows of 32/64/128 bytes: 16/32/64 channels per box; 128 channels take two boxes).
-// One thread drives a kTmaMaxStages-deep pipeline: "full" barriers count TMA bytes, "empty"
-// barriers are armed by tcgen05.commit when the MMAs of a stage are done.  Not used for an
-// upsampled input (a box copy cannot duplicate voxels).
-constexpr int kTmaTileX = 32, kTmaTileY = 4;
-// Pipeline depth, measured on B200 (200x200x32 network, 16 -> 16 forward / training step):
-// 4 stages 0.263 / 7.01 ms, 6 stages 0.286 / 7.49 ms, 8 stages 0.385 / 8.52 ms -- deeper stages
-// cost CTAs per SM.
-#ifndef PCT_TMA_STAGES
-#define PCT_TMA_STAGES 4
-#endif
-constexpr int kTmaMaxStages = PCT_TMA_STAGES;
-constexpr int kTmaSmemLimit = 226 * 1024;  // dynamic; the per-block maximum (227 KB) also holds the static barriers
-
-struct TmaConvShape {
-    int bc, nsub;        // channels per box (row bytes / 2), boxes per row
-    int a_sub, b_sub;    // bytes of one A / B box
-    int tx;              // bytes one stage receives
-    int stage, stages;   // bytes per stage (1024-aligned), stages
+struct SlabShape {
+    int W, H, tiles_x, tiles_y;  // patch and patches
+    int tiles, ctas;             // patches x runs; CTAs that share them
+    int nc, nc_log2, zt;         // channels and slices of a tile
+    int stages;                  // accumulator stages, 1 or 2
+    int ring, ahead;             // input slices in shared memory, requested before the first is awaited
+    int positions;               // (W + 2) (H + 2)
+    int chunk_bytes;             // one 8-channel plane of a slice
+    int slice_bytes, weight_bytes, smem;
+    unsigned columns;            // TMEM
 };
 
-__host__ __device__ inline TmaConvShape tma_conv_shape(int cin, int cout)
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool fill)
 {
-    TmaConvShape s;
-    s.bc = cin < 64 ? cin : 64;
-    s.nsub = cin / s.bc;
-    s.a_sub = kTmaTileX * kTmaTileY * s.bc * 2;
-    s.b_sub = cout * s.bc * 2;
-    s.tx = s.nsub * (s.a_sub + s.b_sub);
-    s.stage = (s.tx + 1023) & ~1023;
-    const int fit = (kTmaSmemLimit - 2048) / s.stage;
-    s.stages = fit < kTmaMaxStages ? fit : kTmaMaxStages;
-    return s;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(fill ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+// A tile: its patch corner, output slices [z0, z1) and input slices [zi0, zi1).
+struct SlabTile {
+    int x0, y0, z0, z1, zi0, zi1;
+};
+__device__ __forceinline__ SlabTile slab_tile(const SlabShape& sh, int tile, int nz)
+{
+    const int patches = sh.tiles_x * sh.tiles_y;
+    const int run = tile / patches, patch = tile - run * patches;
+    const int py = patch / sh.tiles_x;
+    SlabTile t;
+    t.x0 = (patch - py * sh.tiles_x) * sh.W;
+    t.y0 = py * sh.H;
+    t.z0 = run * sh.zt;
+    t.z1 = t.z0 + sh.zt < nz ? t.z0 + sh.zt : nz;
+    t.zi0 = t.z0 > 0 ? t.z0 - 1 : 0;
+    t.zi1 = t.z1 < nz ? t.z1 + 1 : nz;
+    return t;
 }
 
-__global__ void __launch_bounds__(kThreads) conv3_fwd_tma_kernel(const __grid_constant__ CUtensorMap tm_in,
-                                                                const __grid_constant__ CUtensorMap tm_w, ConvFwdArgs p)
+template <int kCin>
+__global__ void __launch_bounds__(kSlabThreads) conv3_slab_kernel(const __grid_constant__ ConvFwdArgs p,
+                                                                  const __grid_constant__ SlabShape sh)
 {
+    constexpr int kc = kCin / 8, kcl = kc == 2 ? 1 : kc == 4 ? 2 : kc == 8 ? 3 : 4;
     extern __shared__ uint8_t smem_raw[];
-    __shared__ __align__(8) uint64_t full[kTmaMaxStages];
-    __shared__ __align__(8) uint64_t empty[kTmaMaxStages];
-    __shared__ __align__(8) uint64_t done;
+    __shared__ __align__(8) uint64_t full[kSlabMaxRing];
+    __shared__ __align__(8) uint64_t empty[kSlabMaxRing];
+    __shared__ __align__(8) uint64_t ready[2 * kSlabMaxSlices];  // output slices of a stage
+    __shared__ __align__(8) uint64_t drained[2];                 // stages written out
+    __shared__ __align__(8) uint64_t weighed;                    // weights in place
     __shared__ uint32_t tmem_slot;
-    __shared__ int issue_failed;
-    const int tid = threadIdx.x, warp = tid >> 5;
-    const TmaConvShape sh = tma_conv_shape(p.cin, p.cout);
-    const uint32_t base = (tc::smem_addr(smem_raw) + 1023u) & ~1023u;
-    const int tiles_x = (p.nx + kTmaTileX - 1) / kTmaTileX, tiles_y = (p.ny + kTmaTileY - 1) / kTmaTileY;
-    const int tx = blockIdx.x % tiles_x, ty = (blockIdx.x / tiles_x) % tiles_y, z = blockIdx.x / (tiles_x * tiles_y);
-    const int x0 = tx * kTmaTileX, y0 = ty * kTmaTileY;
-    const uint32_t ncols = tc::tmem_columns(p.cout);
+    __shared__ int failed;
+    __shared__ float bias[64];
+    __shared__ uint32_t corner[kSlabMaxPositions];  // y << 16 | x of a position within the patch and its halo
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+    const uint32_t base = (tc::smem_addr(smem_raw) + 127u) & ~127u;
+    const uint32_t weights = base + sh.ring * sh.slice_bytes;
+    const int pitch = sh.W + 2;
+    const int c_first = blockIdx.y * sh.nc;
 
-    if (warp == 0) tc::tmem_alloc(tc::smem_addr(&tmem_slot), ncols);
-    if (tid == 0) {
-        for (int i = 0; i < kTmaMaxStages; ++i) {
-            tc::mbar_init(tc::smem_addr(&full[i]), 1);
-            tc::mbar_init(tc::smem_addr(&empty[i]), 1);
-        }
-        tc::mbar_init(tc::smem_addr(&done), 1);
-        tc::mbar_init_fence();
-        issue_failed = 0;
+    if (warp == 4) tc::tmem_alloc(tc::smem_addr(&tmem_slot), sh.columns);
+    if (tid < kSlabMaxRing) {
+        tc::mbar_init(tc::smem_addr(&full[tid]), 4);
+        tc::mbar_init(tc::smem_addr(&empty[tid]), 1);
+    }
+    if (tid < 2 * kSlabMaxSlices) tc::mbar_init(tc::smem_addr(&ready[tid]), 1);
+    if (tid < 2) tc::mbar_init(tc::smem_addr(&drained[tid]), 4);
+    if (tid == 2) tc::mbar_init(tc::smem_addr(&weighed), (kSlabThreads - kSlabProducers) / 32);
+    if (tid < 2 * kSlabMaxSlices) tc::mbar_init_fence();
+    if (tid == 0) failed = 0;
+    if (p.bias && tid < sh.nc) bias[tid] = p.bias[c_first + tid];
+    for (int q = tid; q < sh.positions; q += kSlabThreads) {
+        const int yy = q / pitch;
+        corner[q] = static_cast<uint32_t>(yy) << 16 | static_cast<uint32_t>(q - yy * pitch);
     }
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
     const uint32_t tmem = tmem_slot;
+    if (tid >= kSlabProducers) {
+        // weights [cout][27][cin] -> [tap of the slice][channels / 8][dz = 2, 1, 0][nc][8 channels]
+        for (int u = tid - kSlabProducers; u < 27 * sh.nc << kcl; u += kSlabThreads - kSlabProducers) {
+            const int c = u & (kc - 1), w = u >> kcl;
+            const int co = w & (sh.nc - 1), tap = w >> sh.nc_log2;  // tap: 3 (tap of the slice) + (2 - dz)
+            const int t = tap / 3, r = tap - 3 * t;
+            cp_async16(weights + ((((t << kcl) + c) * 3 + r) * sh.nc + co) * 16,
+                       p.weight + (static_cast<size_t>(c_first + co) * 27 + (2 - r) * 9 + t) * kCin + c * 8, true);
+        }
+        cp_async_commit();
+    }
+    // What follows reads what the kernels before wrote; the weights are written by no kernel of a pass.
+    // The next kernel may start once every CTA is here: by then all earlier ones have ended.
+    grid_dependency_wait();
+    allow_dependent_launch();
+    auto weights_here = [&]() {
+        cp_async_wait<0>();
+        tc::fence_proxy_async();
+        __syncwarp();
+        if ((tid & 31) == 0) tc::mbar_arrive(tc::smem_addr(&weighed));
+    };
 
-    if (tid == 0) {
-        const uint32_t idesc = tc::idesc_bf16_f32(p.cout, false);
-        const uint32_t row_bytes = static_cast<uint32_t>(sh.bc) * 2u;
-        const int S = sh.stages;
-        bool bad = false;
-        for (int t = 0; t < 27 + S - 1 && !bad; ++t) {
-            if (t < 27) {
-                const int st = t % S, round = t / S;
-                if (round > 0 && !tc::mbar_wait(tc::smem_addr(&empty[st]), (round - 1) & 1)) {
-                    bad = true;
-                    break;
-                }
-                const uint32_t sa = base + st * sh.stage, sb = sa + sh.nsub * sh.a_sub;
-                const uint32_t bar = tc::smem_addr(&full[st]);
-                tc::mbar_arrive_expect_tx(bar, static_cast<uint32_t>(sh.tx));
-                const int dz = t / 9 - 1, dy = (t / 3) % 3 - 1, dx = t % 3 - 1;
-                for (int j = 0; j < sh.nsub; ++j) {
-                    tc::tma_load_4d(sa + j * sh.a_sub, &tm_in, bar, j * sh.bc, x0 + dx, y0 + dy, z + dz);
-                    tc::tma_load_3d(sb + j * sh.b_sub, &tm_w, bar, j * sh.bc, t, 0);
-                }
+    if (warp < 4) {
+        // One commit group per slice.  A slice is announced when `ahead` more have been requested, or at
+        // once when there is no free slot to request into: the slot may become free only by the MMAs of
+        // what is to be announced.
+        const int sx = p.nx >> p.up, sy = p.ny >> p.up;
+        const int units = sh.positions << kcl;
+        bool ok = true;
+        int slot = 0, round = 0, told = 0, pending = 0;
+        auto announce = [&](int keep) {
+            if (keep == 0) cp_async_wait<0>();
+            else if (keep == 1) cp_async_wait<1>();
+            else cp_async_wait<2>();
+            tc::fence_proxy_async();
+            __syncwarp();
+            for (; pending > keep; --pending) {
+                if ((tid & 31) == 0) tc::mbar_arrive(tc::smem_addr(&full[told]));
+                if (++told == sh.ring) told = 0;
             }
-            const int u = t - (S - 1);
-            if (u >= 0) {
-                const int su = u % S;
-                if (!tc::mbar_wait(tc::smem_addr(&full[su]), (u / S) & 1)) {
-                    bad = true;
-                    break;
+        };
+        for (int tile = blockIdx.x; tile < sh.tiles && ok; tile += sh.ctas) {
+            const SlabTile t = slab_tile(sh, tile, p.nz);
+            for (int zi = t.zi0; zi < t.zi1 && ok; ++zi) {
+                if (round > 0 && !__all_sync(0xffffffffu, tc::mbar_test(tc::smem_addr(&empty[slot]), (round - 1) & 1))) {
+                    if (pending > 0) announce(0);
+                    ok = __all_sync(0xffffffffu, tc::mbar_wait(tc::smem_addr(&empty[slot]), (round - 1) & 1));
+                    if (!ok) break;
                 }
-                tc::fence_after_sync();
-                const uint32_t sa = base + su * sh.stage, sb = sa + sh.nsub * sh.a_sub;
-                for (int j = 0; j < sh.nsub; ++j)
-                    for (int kk = 0; kk < sh.bc / 16; ++kk)
-                        tc::mma_bf16(tmem, tc::smem_desc_swizzled(sa + j * sh.a_sub + kk * 32, row_bytes),
-                                     tc::smem_desc_swizzled(sb + j * sh.b_sub + kk * 32, row_bytes), idesc,
-                                     (u | j | kk) != 0);
-                tc::mma_commit(tc::smem_addr(&empty[su]));
+                const bf16* plane = p.in + static_cast<size_t>(zi >> p.up) * sy * sx * kCin;
+                const uint32_t dst = base + slot * sh.slice_bytes;
+                for (int u = tid; u < units; u += kSlabProducers) {
+                    const int q = u >> kcl, c = u & (kc - 1);
+                    const uint32_t at = corner[q];
+                    const int y = t.y0 + static_cast<int>(at >> 16) - 1, x = t.x0 + static_cast<int>(at & 0xffffu) - 1;
+                    const bool inside = static_cast<unsigned>(x) < static_cast<unsigned>(p.nx) &&
+                                        static_cast<unsigned>(y) < static_cast<unsigned>(p.ny);
+                    const int from = inside ? (y >> p.up) * sx + (x >> p.up) : 0;
+                    cp_async16(dst + c * sh.chunk_bytes + q * 16, plane + static_cast<size_t>(from) * kCin + c * 8, inside);
+                }
+                if (++slot == sh.ring) {
+                    slot = 0;
+                    ++round;
+                }
+                cp_async_commit();
+                if (++pending > sh.ahead) announce(sh.ahead);
             }
         }
-        tc::mma_commit(tc::smem_addr(&done));  // tracks every MMA issued above
-        if (bad) issue_failed = 1;
-    }
-    int bad = 0;
-    if (tid == 0) bad = !tc::mbar_wait(tc::smem_addr(&done), 0) || issue_failed;
-    bad = __syncthreads_or(bad);
-    tc::fence_after_sync();
-    if (!bad) {
-        const int x = x0 + (tid & (kTmaTileX - 1)), y = y0 + tid / kTmaTileX;
-        const bool row_ok = x < p.nx && y < p.ny;
-        const long long v = (static_cast<long long>(z) * p.ny + y) * p.nx + x;
-        conv_epilogue(p, tmem + (static_cast<uint32_t>(warp * 32) << 16), v, row_ok);
-    } else if (tid == 0) {
-        atomicExch(p.status, 1);
+        announce(0);
+        if (!ok) failed = 1;
+    } else if (warp == 4) {
+        constexpr int ksteps = kCin / 16;
+        const uint32_t leader = tc::elect_one();
+        const uint32_t rows = 3u * sh.nc;
+        const uint32_t a_step = 2 * (sh.chunk_bytes >> 4), b_step = 2 * rows;
+        const uint64_t a_base = tc::smem_desc(base, sh.chunk_bytes, 128), b_base = tc::smem_desc(weights, rows * 16, 128);
+        const uint32_t a_hi = static_cast<uint32_t>(a_base >> 32), b_hi = static_cast<uint32_t>(b_base >> 32);
+        weights_here();
+        bool ok = __all_sync(0xffffffffu, tc::mbar_wait(tc::smem_addr(&weighed), 0));
+        int slot = 0, phase = 0, k = 0;
+        for (int tile = blockIdx.x; tile < sh.tiles && ok; tile += sh.ctas, ++k) {
+            const SlabTile t = slab_tile(sh, tile, p.nz);
+            const int stage = sh.stages == 2 ? k & 1 : 0, use = sh.stages == 2 ? k >> 1 : k;
+            if (use > 0) {
+                ok = __all_sync(0xffffffffu, tc::mbar_wait(tc::smem_addr(&drained[stage]), (use - 1) & 1));
+                tc::fence_after_sync();
+            }
+            const uint32_t acc = tmem + stage * sh.zt * sh.nc;
+            const uint32_t done = tc::smem_addr(ready + stage * kSlabMaxSlices);
+            int reached = t.z0 - 1;  // last output slice that has a product
+            for (int zi = t.zi0; zi < t.zi1 && ok; ++zi) {
+                ok = __all_sync(0xffffffffu, tc::mbar_wait(tc::smem_addr(&full[slot]), phase));
+                if (!ok) break;
+                tc::fence_after_sync();
+                const int lo = zi - 1 > t.z0 ? zi - 1 : t.z0, hi = zi + 1 < t.z1 ? zi + 1 : t.z1 - 1;  // reached by it
+                const uint32_t a0 = static_cast<uint32_t>(a_base) + slot * (sh.slice_bytes >> 4);
+                const uint32_t b0 = static_cast<uint32_t>(b_base) + (lo - (zi - 1)) * sh.nc;
+                const uint32_t d = acc + (lo - t.z0) * sh.nc;
+                const uint32_t idesc = tc::idesc_bf16_f32((hi - lo + 1) * sh.nc, false);
+                if (hi > reached) {
+                    // output slices without a product yet start here: the first MMA in two parts
+                    if (reached >= lo)
+                        tc::mma_bf16_warp(d, a0, a_hi, b0, b_hi, tc::idesc_bf16_f32((reached - lo + 1) * sh.nc, false), 1, leader);
+                    const int fresh = reached >= lo ? reached + 1 - lo : 0;
+                    tc::mma_bf16_warp(d + fresh * sh.nc, a0, a_hi, b0 + fresh * sh.nc, b_hi,
+                                      tc::idesc_bf16_f32((hi - lo + 1 - fresh) * sh.nc, false), 0, leader);
+                } else {
+                    tc::mma_bf16_warp(d, a0, a_hi, b0, b_hi, idesc, 1, leader);
+                }
+#pragma unroll
+                for (int i = 1; i < 9 * ksteps; ++i) {  // tap i / ksteps, channels 16 (i % ksteps) and on
+                    const int tap = i / ksteps;
+                    tc::mma_bf16_warp(d, a0 + (tap / 3 * pitch + tap % 3) + (i % ksteps) * a_step, a_hi, b0 + i * b_step, b_hi,
+                                      idesc, 1, leader);
+                }
+                reached = hi;
+                // an output slice is complete after the input slice above it, or the grid's last
+                tc::mma_commit_warp(tc::smem_addr(&empty[slot]), leader);
+                if (zi > t.z0) tc::mma_commit_warp(done + 8 * (zi - 1 - t.z0), leader);
+                if (zi + 1 == p.nz) tc::mma_commit_warp(done + 8 * (zi - t.z0), leader);
+                if (++slot == sh.ring) {
+                    slot = 0;
+                    phase ^= 1;
+                }
+            }
+        }
+        if (!ok) failed = 1;
+    } else {
+        // row m of the MMAs is TMEM lane m; a warp reads the lanes 32 (warp % 4) and on
+        const int m = (warp & 3) * 32 + (tid & 31);
+        const int yy = m / pitch, xx = m - yy * pitch;
+        const uint32_t lane = tmem + (static_cast<uint32_t>(warp & 3) * 32u << 16);
+        const long long plane = static_cast<long long>(p.nx) * p.ny;
+        weights_here();
+        bool ok = true;
+        int k = 0;
+        for (int tile = blockIdx.x; tile < sh.tiles && ok; tile += sh.ctas, ++k) {
+            const SlabTile t = slab_tile(sh, tile, p.nz);
+            const int stage = sh.stages == 2 ? k & 1 : 0, use = sh.stages == 2 ? k >> 1 : k;
+            const uint32_t acc = lane + stage * sh.zt * sh.nc;
+            const int x = t.x0 + xx, y = t.y0 + yy;
+            const bool row_ok = xx < sh.W && yy < sh.H && x < p.nx && y < p.ny;
+            // a piece is 16 channels of a slice; the next piece's inputs are requested before this one is written
+            int z = t.z0, c = 0;
+            long long v = (static_cast<long long>(z) * p.ny + y) * p.nx + x;
+            EpilogueInputs e = epilogue_request(p, v, c_first, row_ok && z < t.z1);
+            while (z < t.z1) {
+                if (c == 0) {
+                    ok = __all_sync(0xffffffffu, tc::mbar_wait(tc::smem_addr(&ready[stage * kSlabMaxSlices + z - t.z0]), use & 1));
+                    if (!ok) break;
+                    tc::fence_after_sync();
+                }
+                int zn = z, cn = c + 16;
+                long long vn = v;
+                if (cn == sh.nc) {
+                    cn = 0;
+                    zn += 1;
+                    vn += plane;
+                }
+                const EpilogueInputs next = epilogue_request(p, vn, c_first + cn, row_ok && zn < t.z1);
+                conv_epilogue(p, acc + (z - t.z0) * sh.nc + c, v, c_first + c, row_ok, e, bias + c);
+                e = next;
+                z = zn;
+                c = cn;
+                v = vn;
+            }
+            tc::fence_before_sync();
+            __syncwarp();
+            if ((tid & 31) == 0) tc::mbar_arrive(tc::smem_addr(&drained[stage]));
+        }
+        if (!ok) failed = 1;
     }
     tc::fence_before_sync();
     __syncthreads();
-    if (warp == 0) {
+    if (tid == 0 && failed) atomicExch(p.status, 1);
+    if (warp == 4) {
         tc::fence_after_sync();
-        tc::tmem_dealloc(tmem, ncols);
+        tc::tmem_dealloc(tmem, sh.columns);
     }
 }
 
@@ -562,8 +621,10 @@ __global__ void pack_input_kernel(const float* __restrict__ x0, const uint8_t* _
 }
 
 // 2x2x2 average; one thread per (coarse voxel, 8 channels).
-__global__ void avgpool_kernel(const bf16* __restrict__ in, int nx, int ny, int nz, int c, bf16* __restrict__ out)
+__global__ void avgpool_kernel(const bf16* in, int nx, int ny, int nz, int c, bf16* __restrict__ out)
 {
+    grid_dependency_wait();  // `in` is not read through the read-only path: its writer may have just ended
+    allow_dependent_launch();
     const int cx = nx / 2, cy = ny / 2, cz = nz / 2, g = c / 8;
     const long long n = static_cast<long long>(cx) * cy * cz * g;
     for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < n;
@@ -575,7 +636,7 @@ __global__ void avgpool_kernel(const bf16* __restrict__ in, int nx, int ny, int 
         for (int d = 0; d < 8; ++d) {
             const long long fv = (static_cast<long long>(2 * z + (d >> 2)) * ny + 2 * y + ((d >> 1) & 1)) * nx + 2 * x + (d & 1);
             float f[8];
-            unpack8(__ldg(reinterpret_cast<const uint4*>(in + fv * c) + cg), f);
+            unpack8(*(reinterpret_cast<const uint4*>(in + fv * c) + cg), f);
 #pragma unroll
             for (int k = 0; k < 8; ++k) s[k] += f[k];
         }
@@ -758,86 +819,119 @@ cudaError_t set_smem_limits()
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
     if (dev >= 0 && dev < 64 && done[dev]) return cudaSuccess;
-    e = cudaFuncSetAttribute(conv3_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    for (auto kernel : {conv3_slab_kernel<16>, conv3_slab_kernel<32>, conv3_slab_kernel<64>, conv3_slab_kernel<128>})
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSlabSmemLimit);
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(conv3_wgrad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(conv3_fwd_tma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTmaSmemLimit);
     if (e == cudaSuccess && dev >= 0 && dev < 64) done[dev] = true;
     return e;
 }
 
 bool valid_channels(int c) { return c == 16 || c == 32 || c == 64 || c == 128; }
 
-// Tensor maps of the TMA convolution: the activation [nz][ny][nx][c] as a 4-D tensor (c innermost)
-// with a (bc, 32, 4, 1) box, and the weights [cout][27][cin] as a 3-D tensor with a (bc, 1, cout)
-// box; the swizzle matches the box row (bc * 2 bytes).
-// cuTensorMapEncodeTiled through the runtime's driver entry point, so the library does not link the
-// driver library itself (it still loads on machines without a GPU); null if unavailable.
-PFN_cuTensorMapEncodeTiled tensor_map_encoder()
+// The slab kernel's shape for a convolution: the patch that covers the grid with the fewest patches
+// (rows of W + 2 positions, 128 positions in all), and the channels, slices and ring of a CTA with the
+// least estimated time.  The estimate takes per input slice the larger of its MMAs (32 + N/4 cycles each:
+// both operands are read from shared memory at 128 bytes a cycle) and its bytes at 48 a cycle, for each
+// of the CTAs that share an SM, or the latency of one request over the requests in flight; and once per
+// CTA its weights, start and end.
+SlabShape slab_shape(int cin, int cout, int nx, int ny, int nz)
 {
-    static PFN_cuTensorMapEncodeTiled fn = nullptr;
-    static bool looked = false;
-    if (!looked) {
-        looked = true;
-        void* f = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &q) == cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            fn = reinterpret_cast<PFN_cuTensorMapEncodeTiled>(f);
-        else
-            cudaGetLastError();
+    SlabShape best{};
+    long long fewest = 0;
+    for (int W = 1; W <= 126 && W <= nx; ++W) {
+        int H = (128 - W) / (W + 2) + 1;
+        if (H > ny) H = ny;
+        const int positions = (W + 2) * (H + 2);
+        if (positions > kSlabMaxPositions) continue;
+        const int tx = (nx + W - 1) / W, ty = (ny + H - 1) / H;
+        const long long cost = static_cast<long long>(tx) * ty * (256 + positions);
+        if (fewest == 0 || cost < fewest) {
+            fewest = cost;
+            best.W = W;
+            best.H = H;
+            best.tiles_x = tx;
+            best.tiles_y = ty;
+            best.positions = positions;
+        }
     }
-    return fn;
-}
-
-bool encode_conv_maps(const ConvFwdArgs& a, int bc, CUtensorMap* act, CUtensorMap* w)
-{
-    const PFN_cuTensorMapEncodeTiled cuTensorMapEncodeTiled = tensor_map_encoder();
-    if (!cuTensorMapEncodeTiled) return false;
-    const CUtensorMapSwizzle sw = bc == 16 ? CU_TENSOR_MAP_SWIZZLE_32B
-                                : bc == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B;
-    const cuuint64_t c = a.cin;
-    cuuint64_t adim[4] = {c, (cuuint64_t)a.nx, (cuuint64_t)a.ny, (cuuint64_t)a.nz};
-    cuuint64_t astr[3] = {c * 2, c * 2 * a.nx, c * 2 * a.nx * a.ny};
-    cuuint32_t abox[4] = {(cuuint32_t)bc, kTmaTileX, kTmaTileY, 1};
-    cuuint32_t one[4] = {1, 1, 1, 1};
-    if (cuTensorMapEncodeTiled(act, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<bf16*>(a.in), adim, astr, abox, one,
-                               CU_TENSOR_MAP_INTERLEAVE_NONE, sw, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-        return false;
-    cuuint64_t wdim[3] = {c, 27, (cuuint64_t)a.cout};
-    cuuint64_t wstr[2] = {c * 2, c * 2 * 27};
-    cuuint32_t wbox[3] = {(cuuint32_t)bc, 1, (cuuint32_t)a.cout};
-    return cuTensorMapEncodeTiled(w, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<bf16*>(a.weight), wdim, wstr, wbox,
-                                  one, CU_TENSOR_MAP_INTERLEAVE_NONE, sw, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    // rows of an MMA reach 2 (W + 2) + 2 + 127 positions into a plane; the last plane's excess falls in
+    // the weights or the slack behind them
+    best.chunk_bytes = best.positions * 16;
+    best.slice_bytes = best.chunk_bytes * (cin / 8);
+    double least = 0.0;
+    SlabShape chosen = best;
+    for (int nc = cout < 64 ? cout : 64; nc >= 16; nc /= 2)
+        for (int zt = 1; zt <= nz && zt <= kSlabMaxSlices && zt * nc <= kTmemColumns; zt = zt < nz && 2 * zt > nz ? nz : 2 * zt)
+            for (int ring = 2; ring <= kSlabMaxRing; ++ring) {
+                SlabShape t = best;
+                t.nc = nc;
+                t.nc_log2 = nc == 64 ? 6 : nc == 32 ? 5 : 4;
+                t.zt = zt;
+                t.ring = ring;
+                t.ahead = ring - 1 < 2 ? ring - 1 : 2;
+                t.weight_bytes = 27 * cin * nc * 2;
+                t.tiles = t.tiles_x * t.tiles_y * ((nz + zt - 1) / zt);
+                t.smem = ring * t.slice_bytes + t.weight_bytes + 4096 + 128;
+                if (t.smem > kSlabSmemLimit) continue;
+                const int groups = cout / nc;
+                for (t.stages = 1; t.stages <= 2 && t.stages * zt * nc <= kTmemColumns; ++t.stages) {
+                    SlabShape u = t;
+                    u.columns = 32;
+                    while (u.columns < static_cast<unsigned>(u.stages * zt * nc)) u.columns *= 2;
+                    int per_sm = kTmemColumns / static_cast<int>(u.columns);
+                    if (per_sm > 4) per_sm = 4;
+                    const int floor_bytes = kSmemPerSm / (per_sm + 1) + 1;  // no more CTAs than TMEM holds
+                    if (u.smem < floor_bytes) u.smem = floor_bytes;
+                    const int fit = kSmemPerSm / (u.smem + 4096);
+                    if (per_sm > fit) per_sm = fit;
+                    if (per_sm < 1) per_sm = 1;
+                    long long ctas = 148LL * per_sm / groups;
+                    if (ctas < 1) ctas = 1;
+                    u.ctas = static_cast<int>(ctas < u.tiles ? ctas : u.tiles);
+                    const double laps = ceil(static_cast<double>(u.tiles) / u.ctas);
+                    const double share = ceil(static_cast<double>(u.ctas) * groups / 148.0);
+                    const int slices = zt + 2 < nz ? zt + 2 : nz;
+                    const double mma = 9.0 * (cin / 16) * (32 + 0.75 * nc) * share, load = u.slice_bytes / 48.0 * share;
+                    const double wait = 1500.0 / u.ahead;
+                    double slice = mma > load ? mma : load;
+                    if (wait > slice) slice = wait;
+                    // the MMAs need a slice or two in hand while others are on their way
+                    slice *= ring >= 5 ? 1.0 : ring == 4 ? 1.1 : ring == 3 ? 1.25 : 1.5;
+                    // with one stage a tile's MMAs wait until the last one is written
+                    const double tile = slices * slice + (u.stages == 1 ? 1500.0 : 0.0);
+                    const double time = 6000.0 + u.weight_bytes * share / 32.0 + laps * tile;
+                    if (least == 0.0 || time < least) {
+                        least = time;
+                        chosen = u;
+                    }
+                }
+            }
+    return chosen;
 }
 
 cudaError_t launch_conv_fwd(const ConvFwdArgs& a, cudaStream_t s)
 {
     cudaError_t e = set_smem_limits();
     if (e != cudaSuccess) return e;
-    // TMA path: inputs at full resolution whose base addresses meet TMA's 16-byte rule
-    const bool aligned = (reinterpret_cast<uintptr_t>(a.in) & 15) == 0 && (reinterpret_cast<uintptr_t>(a.weight) & 15) == 0;
-    if (!a.up && aligned) {
-        const TmaConvShape sh = tma_conv_shape(a.cin, a.cout);
-        CUtensorMap act, w;
-        if (sh.stages >= 2 && encode_conv_maps(a, sh.bc, &act, &w)) {
-            const int per_sm = kTmemColumns / static_cast<int>(tc::tmem_columns(a.cout));
-            int smem = sh.stages * sh.stage + 1024;
-            const int floor_bytes = kSmemPerSm / (per_sm + 1) + 1;
-            if (smem < floor_bytes) smem = floor_bytes;
-            const long long tiles = static_cast<long long>((a.nx + kTmaTileX - 1) / kTmaTileX) *
-                                    ((a.ny + kTmaTileY - 1) / kTmaTileY) * a.nz;
-            conv3_fwd_tma_kernel<<<static_cast<unsigned>(tiles), kThreads, smem, s>>>(act, w, a);
-            return cudaGetLastError();
-        }
+    const SlabShape sh = slab_shape(a.cin, a.cout, a.nx, a.ny, a.nz);
+    if (sh.smem == 0) return cudaErrorInvalidConfiguration;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(sh.ctas, a.cout / sh.nc);
+    cfg.blockDim = dim3(kSlabThreads);
+    cfg.dynamicSmemBytes = sh.smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = a.overlap ? 1 : 0;
+    switch (a.cin) {
+        case 16: return cudaLaunchKernelEx(&cfg, conv3_slab_kernel<16>, a, sh);
+        case 32: return cudaLaunchKernelEx(&cfg, conv3_slab_kernel<32>, a, sh);
+        case 64: return cudaLaunchKernelEx(&cfg, conv3_slab_kernel<64>, a, sh);
+        default: return cudaLaunchKernelEx(&cfg, conv3_slab_kernel<128>, a, sh);
     }
-    const long long V = static_cast<long long>(a.nx) * a.ny * a.nz;
-    const int blocks = static_cast<int>((V + tc::kTileM - 1) / tc::kTileM);
-    conv3_fwd_kernel<<<blocks, kThreads, conv_smem(conv_stage_bytes(a.cin, a.cout), a.cout), s>>>(a);
-    return cudaGetLastError();
 }
 
 cudaError_t launch_conv_wgrad(ConvWgradArgs a, cudaStream_t s)
@@ -980,9 +1074,9 @@ pct_status forward(pct_unet* n, const float* x0, const uint8_t* hull, float* ima
         if (L.input == kPoolInput) {
             const int f = L.level - 1;  // pool the previous level's last encoder output
             const int src = 2 * f + 1;
-            avgpool_kernel<<<grid_for(n->nv[L.level] * (kSpec[src].cout / 8), 256), 256, 0, s>>>(
-                n->act[src], n->nx[f], n->ny[f], n->nz[f], kSpec[src].cout, n->pool[L.level]);
-            UNET_CK(cudaGetLastError(), "avgpool_kernel");
+            UNET_CK(pct::launch_kernel(true, avgpool_kernel, grid_for(n->nv[L.level] * (kSpec[src].cout / 8), 256), 256, s,
+                                       n->act[src], n->nx[f], n->ny[f], n->nz[f], kSpec[src].cout, n->pool[L.level]),
+                    "avgpool_kernel");
         }
         ConvFwdArgs a{};
         a.in = layer_input(n, l);
@@ -996,6 +1090,7 @@ pct_status forward(pct_unet* n, const float* x0, const uint8_t* hull, float* ima
         a.bias = n->params + n->b_off[l];
         a.residual = L.residual >= 0 ? n->act[L.residual] : nullptr;
         a.status = n->status;
+        a.overlap = 1;
         if (l == kLayers - 1) {
             a.base = x0;
             a.hull = hull;
@@ -1042,6 +1137,7 @@ pct_status backward(pct_unet* n, cudaStream_t s)
         d.ny = ny;
         d.nz = nz;
         d.status = n->status;
+        d.overlap = 1;
         const bool into_tmp = L.up || L.input == kPoolInput;
         if (into_tmp) {
             d.out = n->tmp;  // gradient wrt the upsampled / pooled tensor
