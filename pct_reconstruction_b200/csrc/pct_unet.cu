@@ -22,9 +22,8 @@
 //    The same kernel computes the data gradient with the flipped, transposed weights
 //    W'[ci][26-t][co] = W[co][t][ci].  Epilogue: bias, residual, ReLU, ReLU-mask (for gradients), bf16
 //    store; or the image output.
-//  * conv3_wgrad_kernel: dW[co][t][ci] = sum_v dZ[v][co] X[v + t][ci]: M = 128 (tap, channel)
-//    rows, N = output channels, K = voxels (64 per stage, MN-major operands, which is how both
-//    lie in memory); the voxel range is split over CTAs, partial sums are added with atomics.
+//  * conv3_wgrad_slab_kernel: dW[co][t][ci] = sum_v dZ[v][co] X[v + t][ci]: M = taps in y and input
+//    channels, N = taps in z and output channels, K = voxels; partial sums are added with atomics.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -43,43 +42,8 @@ namespace pct {
 namespace unet {
 
 using bf16 = __nv_bfloat16;
-constexpr int kThreads = 128;
-constexpr int kChunk = 64;          // voxels per weight-gradient stage
 constexpr int kSmemPerSm = 233472;  // shared memory per SM on sm_100
 constexpr int kTmemColumns = 512;   // TMEM columns per SM
-
-// ------------------------------------------------------------------ MMA pipeline bookkeeping --
-
-// Two shared-memory stages, each guarded by an mbarrier that the MMAs reading it commit to.
-// issued/waited count commits and completed waits per stage; every thread keeps the same counts,
-// only thread 0 polls the barrier, and the verdict is shared with __syncthreads_or.
-struct Pipe {
-    uint32_t mbar[2];
-    int issued[2];
-    int waited[2];
-};
-
-__device__ __forceinline__ bool stage_free(Pipe& pp, int b)
-{
-    int bad = 0;
-    if (pp.issued[b] > pp.waited[b]) {
-        if (threadIdx.x == 0) bad = !tc::mbar_wait(pp.mbar[b], pp.waited[b] & 1);
-        pp.waited[b]++;
-    }
-    return __syncthreads_or(bad) == 0;
-}
-
-__device__ __forceinline__ bool drain(Pipe& pp)
-{
-    int bad = 0;
-    for (int b = 0; b < 2; ++b) {
-        while (pp.issued[b] > pp.waited[b]) {
-            if (threadIdx.x == 0 && !bad) bad = !tc::mbar_wait(pp.mbar[b], pp.waited[b] & 1);
-            pp.waited[b]++;
-        }
-    }
-    return __syncthreads_or(bad) == 0;
-}
 
 __device__ __forceinline__ uint32_t pack_bf16(float a, float b)
 {
@@ -100,10 +64,6 @@ __device__ __forceinline__ void unpack8(const uint4& u, float* f)
 
 // ----------------------------------------------------------------------------- convolutions --
 
-// Weight-gradient CTAs per SM: 4 -> 0.541 ms, 6 -> 0.413 ms (16->16); training step 9.06 -> 8.47 ms.
-#ifndef PCT_WGRAD_CTAS_PER_SM
-#define PCT_WGRAD_CTAS_PER_SM 6
-#endif
 struct ConvFwdArgs {
     const bf16* in;      // [nz>>up][ny>>up][nx>>up][cin]
     int cin, up;
@@ -483,127 +443,257 @@ __global__ void __launch_bounds__(kSlabThreads) conv3_slab_kernel(const __grid_c
     }
 }
 
+// ---- slab weight gradient ---------------------------------------------------------------------
+// dW[co][t][ci] = sum_v dZ[v][co] X[v + t][ci], and db[co] = sum_v dZ[v][co].
+//
+// A GEMM whose K side is the voxels.  Both operands are kept as the convolution keeps its input, [channels
+// / 8][position][8 channels], which is the MN-major no-swizzle layout: eight positions are a core matrix,
+// so a tap's shift is again a start address.  A tile is a patch of W x 2 voxels over a run of slices; X
+// has four rows of pitch W + 2 per slice and 8-channel plane, dZ two rows with zeros in the two columns
+// between them, so that K is one run of 2 W + 2 positions (W = 7 mod 8: whole steps of 16).
+//
+// M = 128 rows are 16 groups of 8 channels, one pitch apart: group 4 c + dy is plane c read dy rows
+// further, so one MMA covers the three taps in y of 32 channels (dy = 3 is not used); with 16 input
+// channels the upper eight groups are the next slice.  N is dZ of the slices that an input slice meets
+// through the three taps in z (four for a pair of slices), times the output channels.  The taps in x are
+// three MMAs with accumulators of their own.  So every voxel of X and dZ is brought once per CTA, and 27
+// taps cost three MMAs per 16 positions.
+//
+// Eight warps bring the tiles (two stages), sum dZ for the bias and add the results to dw with atomics;
+// the ninth issues the MMAs.  The tensor core's accumulation truncates, and its error grows by about
+// 1.4e-8 of the result per K step, so the accumulators are added to dw (and start again) after at most
+// `epoch` tiles.  A CTA computes 32 (or 16) x 32 (or 16) channels of dW for its
+// share of the tiles.
+//
+// One pass, in us (the kernel that gathered each tap's rows by threads, 128 rows of dW a CTA, in
+// brackets): 200x200x32, 16 to 16 channels 80 (394), 32 to 16 upsampled 128 (643); 100x100x16, 32 to
+// 32 57 (160) with the bias sums (8) in it; 50x50x8, 64 to 64 22 (56); 25x25x4, 128 to 128 16 (18).
+// All layers of the 200x200x32 network 0.79 ms (3.23, and 0.22 for the bias sums).  The bytes brought
+// bound it: halos double X, and dZ is read with two more slices per run.
 struct ConvWgradArgs {
     const bf16* in;  // forward input, [nz>>up][ny>>up][nx>>up][cin]
-    int cin, cin_log2, up;
+    int cin, up;
     const bf16* dz;  // gradient at the conv output (before bias/ReLU), [V][cout]
     int cout;
     int nx, ny, nz;
     float* dw;       // [cout][27][cin], accumulated
-    int chunks_per_cta;
+    float* db;       // [cout], accumulated, or null
     int* status;
 };
 
-__global__ void __launch_bounds__(kThreads) conv3_wgrad_kernel(ConvWgradArgs p)
-{
-    extern __shared__ __align__(128) uint8_t smem[];
-    __shared__ __align__(8) uint64_t mbar[2];
-    __shared__ uint32_t tmem_slot;
-    const int tid = threadIdx.x, warp = tid >> 5;
-    const int R = 27 * p.cin;
-    const int m0 = blockIdx.x * tc::kTileM;
-    const long long V = static_cast<long long>(p.nx) * p.ny * p.nz;
-    const long long nchunks = (V + kChunk - 1) / kChunk;
-    const long long c_begin = static_cast<long long>(blockIdx.y) * p.chunks_per_cta;
-    const long long c_end = c_begin + p.chunks_per_cta < nchunks ? c_begin + p.chunks_per_cta : nchunks;
-    const uint32_t ncols = tc::tmem_columns(p.cout);
-    const int a_bytes = tc::kTileM * kChunk * 2;
-    const int stage_bytes = a_bytes + p.cout * kChunk * 2;
-    constexpr uint32_t kSbo = (kChunk / 8) * 128;  // next 8 rows along M (N): past all K groups
+struct WgradShape {
+    int W, positions, steps;  // patch width, positions of an X plane (4 pitch), K steps of 16
+    int tiles_x, tiles_y, zt; // patches, slices of a run
+    int tiles, ctas;          // patches x runs, CTAs per channel tile
+    int epoch;                // tiles of a CTA between two additions of the accumulators to dw
+    int ci_tiles, co_tiles, co;  // channel tiles, output channels of a tile
+    int x_plane, x_slice, z_plane, z_slice, stage, smem;  // bytes
+    unsigned columns;
+};
 
-    if (warp == 0) tc::tmem_alloc(tc::smem_addr(&tmem_slot), ncols);
-    if (tid == 0) {
-        tc::mbar_init(tc::smem_addr(&mbar[0]), 1);
-        tc::mbar_init(tc::smem_addr(&mbar[1]), 1);
-        tc::mbar_init_fence();
+constexpr int kWgradLoaders = 256;
+constexpr int kWgradThreads = kWgradLoaders + 32;
+
+template <bool kPair>
+__global__ void __launch_bounds__(kWgradThreads) conv3_wgrad_slab_kernel(const __grid_constant__ ConvWgradArgs p,
+                                                                         const __grid_constant__ WgradShape sh)
+{
+    constexpr int kXPlanes = kPair ? 2 : 4, kXLog = kPair ? 1 : 2;  // 8-channel planes of an input tile
+    constexpr int kWindow = kPair ? 4 : 3;                         // dZ slices that an MMA covers
+    extern __shared__ uint8_t smem_raw[];
+    __shared__ __align__(8) uint64_t full[2];
+    __shared__ __align__(8) uint64_t empty[2];
+    __shared__ __align__(8) uint64_t done;     // an epoch's MMAs
+    __shared__ __align__(8) uint64_t flushed;  // an epoch's accumulators read
+    __shared__ uint32_t tmem_slot;
+    __shared__ int failed;
+    __shared__ uint32_t corner[272];  // row << 16 | column of a position
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+    const uint32_t base = (tc::smem_addr(smem_raw) + 127u) & ~127u;
+    const int pitch = sh.W + 2;
+    const int ci0 = blockIdx.y % sh.ci_tiles * 32, co0 = blockIdx.y / sh.ci_tiles * sh.co;
+    const int zc = sh.co >> 3, zcl = zc == 2 ? 1 : 2;  // 8-channel planes of dZ
+    const int patches = sh.tiles_x * sh.tiles_y;
+
+    if (warp == 8) tc::tmem_alloc(tc::smem_addr(&tmem_slot), sh.columns);
+    if (tid < 2) {
+        tc::mbar_init(tc::smem_addr(&full[tid]), kWgradLoaders / 32);
+        tc::mbar_init(tc::smem_addr(&empty[tid]), 1);
+    }
+    if (tid == 2) tc::mbar_init(tc::smem_addr(&done), 1);
+    if (tid == 3) tc::mbar_init(tc::smem_addr(&flushed), kWgradLoaders / 32);
+    if (tid < 4) tc::mbar_init_fence();
+    if (tid == 0) failed = 0;
+    for (int q = tid; q < sh.positions; q += kWgradThreads) {
+        const int row = q / pitch;
+        corner[q] = static_cast<uint32_t>(row) << 16 | static_cast<uint32_t>(q - row * pitch);
     }
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
     const uint32_t tmem = tmem_slot;
-    Pipe pp{{tc::smem_addr(&mbar[0]), tc::smem_addr(&mbar[1])}, {0, 0}, {0, 0}};
-    const int sx = p.nx >> p.up, sy = p.ny >> p.up;
-    const uint32_t idesc = tc::idesc_bf16_f32(p.cout, true);
-    const int b_units = (p.cout >> 3) * kChunk;
-    bool ok = true;
-    int it = 0;
-    for (long long ch = c_begin; ch < c_end; ++ch, ++it) {
-        const int b = it & 1;
-        if (!stage_free(pp, b)) {
-            ok = false;
-            break;
-        }
-        uint8_t* sa = smem + b * stage_bytes;
-        uint8_t* sb = sa + a_bytes;
-        const long long vb = ch * kChunk;
-        // A: rows m = (tap, channel) of this tile, K = voxels; 16-byte unit = 8 channels of one voxel.
-        // Thread tid always handles voxel k = tid % 64 of the stage (units j*128 + tid), so its
-        // coordinates are computed once per stage; row groups g = 2j + tid / 64.
-        {
-            const int k = tid & (kChunk - 1);
-            const long long vv = vb + k;
-            const bool vok = vv < V;
-            const int vi = static_cast<int>(vok ? vv : 0);
-            const int x = vi % p.nx, r = vi / p.nx;
-            const int y = r % p.ny, z = r / p.ny;
-            uint8_t* dst = sa + (k >> 3) * 128 + (k & 7) * 16;
-#pragma unroll 4
-            for (int j = 0; j < (tc::kTileM / 8) * kChunk / kThreads; ++j) {
-                const int g = 2 * j + (tid >> 6);
-                const int m = m0 + g * 8;
-                uint4 val = make_uint4(0, 0, 0, 0);
-                if (vok && m < R) {
-                    const int tap = m >> p.cin_log2, ci = m & (p.cin - 1);
-                    const int zz = z + tap / 9 - 1, yy = y + (tap / 3) % 3 - 1, xx = x + tap % 3 - 1;
-                    if (zz >= 0 && zz < p.nz && yy >= 0 && yy < p.ny && xx >= 0 && xx < p.nx) {
-                        const size_t sv = (static_cast<size_t>(zz >> p.up) * sy + (yy >> p.up)) * sx + (xx >> p.up);
-                        val = __ldg(reinterpret_cast<const uint4*>(p.in + sv * p.cin + ci));
-                    }
-                }
-                *reinterpret_cast<uint4*>(dst + g * kSbo) = val;
-            }
-        }
-        // B: N = output channels, K = voxels
-        for (int u = tid; u < b_units; u += kThreads) {
-            const int k = u & (kChunk - 1), g = u / kChunk;
-            const long long vv = vb + k;
-            const uint4 val = vv < V ? __ldg(reinterpret_cast<const uint4*>(p.dz + vv * p.cout + g * 8))
-                                     : make_uint4(0, 0, 0, 0);
-            *reinterpret_cast<uint4*>(sb + g * kSbo + (k >> 3) * 128 + (k & 7) * 16) = val;
-        }
-        tc::fence_proxy_async();
-        __syncthreads();
-        if (tid == 0) {
-            tc::fence_after_sync();
-            const uint32_t a0 = tc::smem_addr(sa), b0 = tc::smem_addr(sb);
-            for (int j = 0; j < kChunk / 16; ++j)
-                tc::mma_bf16(tmem, tc::smem_desc(a0 + j * 256, 128, kSbo), tc::smem_desc(b0 + j * 256, 128, kSbo),
-                             idesc, (it | j) != 0);
-            tc::mma_commit(pp.mbar[b]);
-        }
-        pp.issued[b]++;
-    }
-    ok = drain(pp) && ok;
-    tc::fence_after_sync();
-    if (ok && it > 0) {
-        const uint32_t trow = tmem + (static_cast<uint32_t>(warp * 32) << 16);
-        const int m = m0 + tid;
-        for (int c0 = 0; c0 < p.cout; c0 += 16) {
-            float acc[16];
-            tc::tmem_load16(trow + c0, acc);
-            if (m < R) {
+
+    if (warp < 8) {
+        const int sx = p.nx >> p.up, sy = p.ny >> p.up;
+        const int x_units = sh.positions << kXLog, z_units = (sh.steps * 16) << zcl;
+        const bool sums = p.db != nullptr && ci0 == 0;
+        float bias[8] = {0, 0, 0, 0, 0, 0, 0, 0};  // of dZ plane tid % zc
+        bool ok = true;
+        int pending = 0, told = 0, requested = 0;
+        // Announces all but the newest `keep` requested tiles; this thread adds up the dZ units it brought.
+        auto announce = [&](int keep) {
+            if (keep == 0) cp_async_wait<0>();
+            else cp_async_wait<1>();
+            tc::fence_proxy_async();
+            __syncwarp();
+            for (; pending > keep; --pending) {
+                if ((tid & 31) == 0) tc::mbar_arrive(tc::smem_addr(&full[told & 1]));
+                if (sums) {
+                    const uint32_t from = base + (told & 1) * sh.stage + sh.zt * sh.x_slice + (tid & (zc - 1)) * sh.z_plane;
+                    for (int s = 1; s <= sh.zt; ++s)  // the run's own slices
+                        for (int u = tid; u < z_units; u += kWgradLoaders) {
+                            uint4 raw;
+                            asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
+                                         : "=r"(raw.x), "=r"(raw.y), "=r"(raw.z), "=r"(raw.w)
+                                         : "r"(from + s * sh.z_slice + (u >> zcl) * 16) : "memory");
+                            float f[8];
+                            unpack8(raw, f);
 #pragma unroll
-                for (int i = 0; i < 16; ++i) atomicAdd(p.dw + static_cast<size_t>(c0 + i) * R + m, acc[i]);
+                            for (int i = 0; i < 8; ++i) bias[i] += f[i];
+                        }
+                }
+                ++told;
             }
+        };
+        // TMEM lane (row) m of the M side: plane, row shift and channel; upper half: the next slice
+        const int m = (warp & 3) * 32 + (tid & 31);
+        const int half = kPair ? m >> 6 : 0, dy = (m >> 3) & 3;
+        const int ci = ci0 + (kPair ? (m & 63) >> 5 : m >> 5) * 8 + (m & 7);
+        int epochs = 0;
+        auto flush = [&]() {  // waits for the epoch's MMAs and adds its accumulators to dw
+            if (!__all_sync(0xffffffffu, tc::mbar_wait(tc::smem_addr(&done), epochs++ & 1))) return false;
+            tc::fence_after_sync();
+            const uint32_t lane = tmem + (static_cast<uint32_t>(warp & 3) * 32u << 16);
+            const int n = kWindow * sh.co;
+            for (int b = warp >> 2; b < 3 * n / 16; b += 2) {  // 16 columns: one tap in x, dZ slice, output channels
+                float acc[16];
+                tc::tmem_load16(lane + b * 16, acc);
+                const int dx = b * 16 / n, column = b * 16 - dx * n;
+                const int w = column / sh.co, co = co0 + column - w * sh.co;
+                const int dz = half + 2 - w;
+                if (dy < 3 && dz >= 0 && dz < 3) {
+                    float* to = p.dw + (static_cast<size_t>(co) * 27 + dz * 9 + dy * 3 + dx) * p.cin + ci;
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) atomicAdd(to + static_cast<size_t>(i) * 27 * p.cin, acc[i]);
+                }
+            }
+            tc::fence_before_sync();
+            __syncwarp();
+            if ((tid & 31) == 0) tc::mbar_arrive(tc::smem_addr(&flushed));
+            return true;
+        };
+        for (int tile = blockIdx.x; tile < sh.tiles && ok; tile += sh.ctas, ++requested) {
+            const int run = tile / patches, patch = tile - run * patches, py = patch / sh.tiles_x;
+            const int x0 = (patch - py * sh.tiles_x) * sh.W, y0 = py * 2, z0 = run * sh.zt;
+            const int stage = requested & 1;
+            if (requested >= 2) {
+                const uint32_t parity = (requested / 2 - 1) & 1;
+                if (!__all_sync(0xffffffffu, tc::mbar_test(tc::smem_addr(&empty[stage]), parity))) {
+                    if (pending > 0) announce(0);
+                    ok = __all_sync(0xffffffffu, tc::mbar_wait(tc::smem_addr(&empty[stage]), parity));
+                    if (!ok) break;
+                }
+            }
+            const uint32_t dst = base + stage * sh.stage, dst_z = dst + sh.zt * sh.x_slice;
+            for (int u = tid; u < x_units; u += kWgradLoaders) {
+                const int q = u >> kXLog, c = u & (kXPlanes - 1);
+                const uint32_t at = corner[q];
+                const int y = y0 + static_cast<int>(at >> 16) - 1, x = x0 + static_cast<int>(at & 0xffffu) - 1;
+                const bool inside = static_cast<unsigned>(x) < static_cast<unsigned>(p.nx) &&
+                                    static_cast<unsigned>(y) < static_cast<unsigned>(p.ny);
+                const bf16* from = p.in + static_cast<size_t>(inside ? (y >> p.up) * sx + (x >> p.up) : 0) * p.cin + ci0 + c * 8;
+                const uint32_t to = dst + c * sh.x_plane + q * 16;
+                for (int s = 0; s < sh.zt; ++s) {
+                    const bool there = inside && z0 + s < p.nz;
+                    cp_async16(to + s * sh.x_slice,
+                               from + (there ? static_cast<size_t>((z0 + s) >> p.up) * sy * sx * p.cin : 0), there);
+                }
+            }
+            for (int u = tid; u < z_units; u += kWgradLoaders) {
+                const int q = u >> zcl, c = u & (zc - 1);
+                const uint32_t at = corner[q];
+                const int row = static_cast<int>(at >> 16), column = static_cast<int>(at & 0xffffu);
+                const int y = y0 + row, x = x0 + column;
+                const bool inside = row < 2 && column < sh.W && x < p.nx && y < p.ny;
+                const bf16* from = p.dz + (inside ? static_cast<size_t>(y) * p.nx + x : 0) * p.cout + co0 + c * 8;
+                const uint32_t to = dst_z + c * sh.z_plane + q * 16;
+                for (int s = 0; s < sh.zt + 2; ++s) {
+                    const int z = z0 - 1 + s;
+                    const bool there = inside && z >= 0 && z < p.nz;
+                    cp_async16(to + s * sh.z_slice, from + (there ? static_cast<size_t>(z) * p.ny * p.nx * p.cout : 0), there);
+                }
+            }
+            cp_async_commit();
+            if (++pending > 1) announce(1);
+            if (requested > 0 && requested % sh.epoch == 0) ok = flush();
         }
-    } else if (!ok && tid == 0) {
-        atomicExch(p.status, 1);
+        announce(0);
+        if (ok) ok = flush();
+        if (sums && ok) {
+            // lanes of the same plane
+#pragma unroll
+            for (int o = 16; o >= 2; o >>= 1)
+                if (o >= zc)
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) bias[i] += __shfl_xor_sync(0xffffffffu, bias[i], o);
+            if ((tid & 31) < zc)
+#pragma unroll
+                for (int i = 0; i < 8; ++i) atomicAdd(p.db + co0 + (tid & 31) * 8 + i, bias[i]);
+        }
+        if (!ok) failed = 1;
+    } else {
+        const uint32_t leader = tc::elect_one();
+        const uint32_t n = kWindow * sh.co, idesc = tc::idesc_bf16_f32(static_cast<int>(n), true);
+        const uint64_t a_base = tc::smem_desc(base, 128, pitch * 16), b_base = tc::smem_desc(base + sh.zt * sh.x_slice, 128, sh.z_plane);
+        const uint32_t a_hi = static_cast<uint32_t>(a_base >> 32), b_hi = static_cast<uint32_t>(b_base >> 32);
+        bool ok = true;
+        uint32_t started = 0;
+        int k = 0;
+        for (int tile = blockIdx.x; tile < sh.tiles && ok; tile += sh.ctas, ++k) {
+            const int z0 = tile / patches * sh.zt, stage = k & 1;
+            if (k > 0 && k % sh.epoch == 0) {
+                tc::mma_commit_warp(tc::smem_addr(&done), leader);
+                ok = __all_sync(0xffffffffu, tc::mbar_wait(tc::smem_addr(&flushed), (k / sh.epoch - 1) & 1));
+                if (!ok) break;
+                tc::fence_after_sync();
+                started = 0;
+            }
+            ok = __all_sync(0xffffffffu, tc::mbar_wait(tc::smem_addr(&full[stage]), (k >> 1) & 1));
+            if (!ok) break;
+            tc::fence_after_sync();
+            const int slices = z0 + sh.zt < p.nz ? sh.zt : p.nz - z0;
+            for (int s = 0; s < slices; s += kPair ? 2 : 1) {
+                // the descriptors' address fields count 16 bytes: one position
+                uint32_t a = static_cast<uint32_t>(a_base) + ((stage * sh.stage + s * sh.x_slice) >> 4);
+                uint32_t b = static_cast<uint32_t>(b_base) + ((stage * sh.stage + s * sh.z_slice) >> 4);
+                for (int j = 0; j < sh.steps; ++j, a += 16, b += 16) {
+                    tc::mma_bf16_warp(tmem, a, a_hi, b, b_hi, idesc, started, leader);
+                    tc::mma_bf16_warp(tmem + n, a + 1, a_hi, b, b_hi, idesc, started, leader);
+                    tc::mma_bf16_warp(tmem + 2 * n, a + 2, a_hi, b, b_hi, idesc, started, leader);
+                    started = 1;
+                }
+            }
+            tc::mma_commit_warp(tc::smem_addr(&empty[stage]), leader);
+        }
+        tc::mma_commit_warp(tc::smem_addr(&done), leader);
+        if (!ok) failed = 1;
     }
     tc::fence_before_sync();
     __syncthreads();
-    if (warp == 0) {
+    if (tid == 0 && failed) atomicExch(p.status, 1);
+    if (warp == 8) {
         tc::fence_after_sync();
-        tc::tmem_dealloc(tmem, ncols);
+        tc::tmem_dealloc(tmem, sh.columns);
     }
 }
 
@@ -708,23 +798,6 @@ __global__ void upsum_mask_kernel(const bf16* __restrict__ du, const bf16* __res
     }
 }
 
-// db[c] += sum_v dz[v][c]; 256 threads, cout divides 256.
-__global__ void bias_grad_kernel(const bf16* __restrict__ dz, int cout, long long V, float* __restrict__ db)
-{
-    __shared__ float red[256];
-    const int c = threadIdx.x % cout, lanes = 256 / cout, off = threadIdx.x / cout;
-    float s = 0.f;
-    for (long long v = static_cast<long long>(blockIdx.x) * lanes + off; v < V; v += static_cast<long long>(gridDim.x) * lanes)
-        s += __bfloat162float(dz[v * cout + c]);
-    red[threadIdx.x] = s;
-    __syncthreads();
-    if (off == 0) {
-        float t = 0.f;
-        for (int l = 0; l < lanes; ++l) t += red[l * cout + c];
-        atomicAdd(db + c, t);
-    }
-}
-
 __global__ void count_kernel(const uint8_t* __restrict__ hull, long long V, unsigned long long* __restrict__ count)
 {
     unsigned long long n = 0;
@@ -802,16 +875,6 @@ int grid_for(long long n, int threads)
     return static_cast<int>(b < 1 ? 1 : b);
 }
 
-// Dynamic shared memory for a conv CTA: its two stages, raised when needed so that no more CTAs
-// share an SM than its TMEM columns can hold at once.
-int conv_smem(int stage_bytes, int cout)
-{
-    const int per_sm = kTmemColumns / static_cast<int>(tc::tmem_columns(cout));
-    const int floor_bytes = kSmemPerSm / (per_sm + 1) + 1;
-    const int need = 2 * stage_bytes;
-    return need > floor_bytes ? need : floor_bytes;
-}
-
 cudaError_t set_smem_limits()
 {
     static bool done[64] = {};
@@ -821,8 +884,8 @@ cudaError_t set_smem_limits()
     if (dev >= 0 && dev < 64 && done[dev]) return cudaSuccess;
     for (auto kernel : {conv3_slab_kernel<16>, conv3_slab_kernel<32>, conv3_slab_kernel<64>, conv3_slab_kernel<128>})
         if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSlabSmemLimit);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(conv3_wgrad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    for (auto kernel : {conv3_wgrad_slab_kernel<false>, conv3_wgrad_slab_kernel<true>})
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSlabSmemLimit);
     if (e == cudaSuccess && dev >= 0 && dev < 64) done[dev] = true;
     return e;
 }
@@ -934,22 +997,75 @@ cudaError_t launch_conv_fwd(const ConvFwdArgs& a, cudaStream_t s)
     }
 }
 
-cudaError_t launch_conv_wgrad(ConvWgradArgs a, cudaStream_t s)
+// The weight gradient's shape: the patch width with the fewest K steps over the grid, and the run length
+// with the least estimated time (MMAs at 32 + N/4 cycles or bytes at 40 a cycle, whichever is more, the
+// first tile's bytes, which nothing overlaps, and the additions to dw).
+WgradShape wgrad_shape(int cin, int cout, int nx, int ny, int nz)
+{
+    const bool pair = cin == 16;
+    WgradShape best{};
+    int fewest = 0;
+    for (int W = 7; W <= 63; W += 8) {
+        const int cost = (nx + W - 1) / W * (2 * W + 2 + 16);
+        if (fewest == 0 || cost <= fewest) {
+            fewest = cost;
+            best.W = W;
+        }
+    }
+    const int planes = pair ? 2 : 4;
+    best.positions = 4 * (best.W + 2);
+    best.steps = (2 * best.W + 2) / 16;
+    best.tiles_x = (nx + best.W - 1) / best.W;
+    best.tiles_y = (ny + 1) / 2;
+    best.ci_tiles = pair ? 1 : cin / 32;
+    best.co = cout == 16 ? 16 : 32;
+    best.co_tiles = cout / best.co;
+    best.x_plane = best.positions * 16;
+    best.x_slice = best.x_plane * planes;
+    best.z_plane = best.steps * 256;
+    best.z_slice = best.z_plane * (best.co / 8);
+    const int n = (pair ? 4 : 3) * best.co;
+    best.columns = 3 * n <= 256 ? 256 : 512;
+    const int groups = best.ci_tiles * best.co_tiles;
+    // K steps of an accumulator: at most 96 (an error near 1.3e-6), or on larger grids what 888 CTAs of 128
+    // rows of dW would take
+    const long long share = (static_cast<long long>(nx) * ny * nz * ((27 * cin + 127) / 128)) / (16 * 888);
+    const int chain = static_cast<int>(share > 96 ? share : 96);
+    WgradShape chosen = best;
+    double least = 0.0;
+    for (int zt = pair ? 2 : 1; zt <= (pair ? nz + 1 : nz) && zt <= 32; zt += pair ? 2 : 1) {
+        WgradShape t = best;
+        t.zt = zt;
+        t.stage = (zt * t.x_slice + (zt + 2) * t.z_slice + 127) & ~127;
+        // rows that are not used read up to a pitch and a step past the last plane
+        t.smem = 2 * t.stage + (t.W + 24) * 16 + 128;
+        const int per_tile = (pair ? (zt + 1) / 2 : zt) * t.steps;
+        if (t.smem > kSlabSmemLimit || (per_tile > chain && chosen.smem != 0)) break;
+        t.epoch = chain / per_tile > 1 ? chain / per_tile : 1;
+        t.tiles = t.tiles_x * t.tiles_y * ((nz + zt - 1) / zt);
+        const int ctas = 148 / groups > 1 ? 148 / groups : 1;
+        t.ctas = ctas < t.tiles ? ctas : t.tiles;
+        const double laps = ceil(static_cast<double>(t.tiles) / t.ctas);
+        const double mma = (pair ? (zt + 1) / 2 : zt) * t.steps * 3.0 * (32 + n / 4.0);
+        const double load = (zt * t.x_slice + (zt + 2.0) * t.z_slice) / 40.0;
+        const double time = laps * ((mma > load ? mma : load) + 300.0) + load + ceil(laps / t.epoch) * (1000.0 + 10.0 * n);
+        if (least == 0.0 || time < least) {
+            least = time;
+            chosen = t;
+        }
+    }
+    return chosen;
+}
+
+cudaError_t launch_conv_wgrad(const ConvWgradArgs& a, cudaStream_t s)
 {
     cudaError_t e = set_smem_limits();
     if (e != cudaSuccess) return e;
-    a.cin_log2 = a.cin == 16 ? 4 : a.cin == 32 ? 5 : a.cin == 64 ? 6 : 7;
-    const long long V = static_cast<long long>(a.nx) * a.ny * a.nz;
-    const int m_tiles = (27 * a.cin + tc::kTileM - 1) / tc::kTileM;
-    const long long chunks = (V + kChunk - 1) / kChunk;
-    // about six resident CTAs per SM (the two 18-34 KB stages allow six to eight)
-    long long splits = (148LL * PCT_WGRAD_CTAS_PER_SM + m_tiles - 1) / m_tiles;
-    if (splits > chunks) splits = chunks;
-    if (splits < 1) splits = 1;
-    a.chunks_per_cta = static_cast<int>((chunks + splits - 1) / splits);
-    splits = (chunks + a.chunks_per_cta - 1) / a.chunks_per_cta;
-    const int stage = tc::kTileM * kChunk * 2 + a.cout * kChunk * 2;
-    conv3_wgrad_kernel<<<dim3(m_tiles, static_cast<unsigned>(splits)), kThreads, conv_smem(stage, a.cout), s>>>(a);
+    const WgradShape sh = wgrad_shape(a.cin, a.cout, a.nx, a.ny, a.nz);
+    if (sh.smem == 0) return cudaErrorInvalidConfiguration;
+    const dim3 grid(sh.ctas, sh.ci_tiles * sh.co_tiles);
+    if (a.cin == 16) conv3_wgrad_slab_kernel<true><<<grid, kWgradThreads, sh.smem, s>>>(a, sh);
+    else conv3_wgrad_slab_kernel<false><<<grid, kWgradThreads, sh.smem, s>>>(a, sh);
     return cudaGetLastError();
 }
 
@@ -1122,10 +1238,9 @@ pct_status backward(pct_unet* n, cudaStream_t s)
         w.ny = ny;
         w.nz = nz;
         w.dw = n->grads + n->w_off[l];
+        w.db = n->grads + n->b_off[l];
         w.status = n->status;
         UNET_CK(launch_conv_wgrad(w, s), "conv3_wgrad_kernel");
-        bias_grad_kernel<<<296, 256, 0, s>>>(n->dz[l], L.cout, n->nv[L.level], n->grads + n->b_off[l]);
-        UNET_CK(cudaGetLastError(), "bias_grad_kernel");
         if (l == 0) break;
         // data gradient: conv of dz with the flipped, transposed weights
         ConvFwdArgs d{};

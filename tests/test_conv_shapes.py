@@ -35,3 +35,49 @@ def test_convolution_is_exact_on_exact_inputs(nz, ny, nx, cin, cout, up):
     out = gconv(dev(x), cin, shape, dev(w), cout, upsample=up, bias=torch.from_numpy(b).cuda(), residual=dev(r),
                 mask=dev(m), relu=True)
     np.testing.assert_array_equal(out.float().cpu().numpy().reshape(shape + (cout,)), ref)
+
+
+# the weight gradient's patches are W x 2 voxels, W = 7, 15, ..., 63; slices in pairs for 16 input channels;
+# accumulators are added to dw after at most 96 steps of 16 positions (the last two shapes: several times)
+WGRAD_SHAPES = [(1, 1, 1, 16, 16, 0), (2, 1, 8, 16, 32, 0), (3, 5, 63, 16, 16, 0), (5, 2, 64, 16, 128, 0),
+                (1, 3, 9, 32, 16, 0), (2, 2, 2, 32, 32, 1), (7, 9, 31, 64, 64, 0), (4, 6, 30, 128, 32, 1),
+                (4, 25, 25, 128, 128, 0), (33, 60, 70, 16, 16, 0), (40, 60, 58, 64, 32, 0)]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nz,ny,nx,cin,cout,up", WGRAD_SHAPES)
+def test_weight_gradient_is_exact_on_exact_inputs(nz, ny, nx, cin, cout, up):
+    import torch
+    from oracle.unet_oracle import conv3d_wgrad
+    from pct_reconstruction_b200.learned import conv3d_wgrad as gwgrad
+    rng = np.random.default_rng(nz * 1013 + ny * 37 + nx + cin + cout)
+    shape = (nz, ny, nx)
+    source = tuple(s // 2 for s in shape) if up else shape
+    x = rng.integers(-3, 4, source + (cin,)).astype(np.float32)   # |sum| <= 9 * 139,200 < 2^24
+    dz = rng.integers(-3, 4, shape + (cout,)).astype(np.float32)
+    dev = lambda a: torch.from_numpy(a).cuda().to(torch.bfloat16)
+    got = gwgrad(dev(x), cin, shape, dev(dz), cout, upsample=up).cpu().numpy()
+    np.testing.assert_array_equal(got, conv3d_wgrad(x, dz, bool(up)).astype(np.float32).reshape(-1))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape", [(8, 8, 8), (16, 40, 24)])
+def test_bias_gradients_are_the_sums_of_the_layer_gradients(shape):
+    """The bias gradient of the output layer is the sum of the loss gradient, 2 (y - t) / count over the hull
+    in bf16, which an untrained network (y = x_0) lets the test form itself."""
+    import torch
+    from oracle.unet_oracle import param_layout
+    from pct_reconstruction_b200.learned import UNet
+    rng = np.random.default_rng(3)
+    v = int(np.prod(shape))
+    x0 = rng.uniform(0.5, 1.5, v).astype(np.float32)
+    target = (x0 + rng.normal(0, 0.1, v)).astype(np.float32)
+    hull = (rng.uniform(size=v) < 0.7).astype(np.uint8)
+    T = [torch.from_numpy(a).cuda() for a in (x0, hull, target)]
+    with UNet(shape[2], shape[1], shape[0], seed=2) as net:
+        _, g = net.gradients(*T)
+    d = np.where(hull, x0 - target, 0).astype(np.float64)
+    expected = bf16((2 * d / hull.sum()).astype(np.float32)).astype(np.float64)
+    got = g[param_layout()[0][-1][1]:]
+    assert abs(got[0] - expected.sum()) <= 1e-6 * np.abs(expected).sum()
+    assert not got[1:].any()
