@@ -81,3 +81,34 @@ def test_bias_gradients_are_the_sums_of_the_layer_gradients(shape):
     got = g[param_layout()[0][-1][1]:]
     assert abs(got[0] - expected.sum()) <= 1e-6 * np.abs(expected).sum()
     assert not got[1:].any()
+
+
+@pytest.mark.gpu
+def test_convolutions_from_many_threads():
+    """More calls at once than there are status words, each on its own stream, next to one another."""
+    import threading
+
+    import torch
+    from pct_reconstruction_b200.learned import conv3d as gconv
+    rng = np.random.default_rng(8)
+    shape = (6, 20, 30)
+    x = torch.from_numpy(rng.integers(-4, 5, shape + (16,)).astype(np.float32)).cuda().to(torch.bfloat16)
+    w = torch.from_numpy((rng.integers(-4, 5, (16, 27, 16)) / 4).astype(np.float32)).cuda().to(torch.bfloat16)
+    expected = gconv(x, 16, shape, w, 16)
+    torch.cuda.synchronize()
+    wrong = []
+
+    def work():
+        stream = torch.cuda.Stream()
+        for _ in range(5):
+            with torch.cuda.stream(stream):
+                out = gconv(x, 16, shape, w, 16, stream=stream)
+                if not torch.equal(out, expected):
+                    wrong.append(1)
+
+    threads = [threading.Thread(target=work) for _ in range(80)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong
