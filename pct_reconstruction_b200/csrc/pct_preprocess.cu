@@ -50,6 +50,7 @@ struct PreGeom {
     double source_radius, rsp_air, fbp_threshold;
     double sc_lower, sc_upper, msc_lower, msc_upper, sm_lower, sm_scale;
     int msc_diff_thresh;
+    int fast_walks;  // EXACT_FAST_POINTS: voxel walks by crossing times where the order is certain
 };
 
 PreGeom make_pregeom(const pct_config& c)
@@ -84,6 +85,7 @@ PreGeom make_pregeom(const pct_config& c)
     g.sm_lower = c.SM_LOWER_THRESHOLD;
     g.sm_scale = c.SM_SCALE_THRESHOLD;
     g.msc_diff_thresh = c.MSC_DIFF_THRESH;
+    g.fast_walks = c.EXACT_FAST_POINTS ? 1 : 0;
     return g;
 }
 
@@ -142,6 +144,7 @@ struct Preproc {
     int *MSC_counts = nullptr, *SM_counts = nullptr, *SM_differences = nullptr, *SM_thresholds = nullptr;
     int* edge_tmp = nullptr;
     unsigned* walk_hist = nullptr;  // bucket-sort scratch of the walk order
+    uint32_t* hull_bits = nullptr;  // hull, one bit per voxel (for the endpoint walks)
     bool hull_ready = false;
 };
 
@@ -159,7 +162,7 @@ void preproc_release(Preproc* p)
                     p->bin_counts, p->mean_WEPL, p->mean_rel_ut_angle, p->mean_rel_uv_angle, p->stddev_WEPL,
                     p->stddev_rel_ut_angle, p->stddev_rel_uv_angle, p->sinogram, p->sinogram_filtered,
                     p->FBP_image, p->FBP_median, p->FBP_hull, p->SC_hull, p->hull, p->MSC_counts, p->SM_counts,
-                    p->SM_differences, p->SM_thresholds, p->edge_tmp, p->walk_hist};
+                    p->SM_differences, p->SM_thresholds, p->edge_tmp, p->walk_hist, p->hull_bits};
     for (void* q : ptrs) cudaFree(q);
     delete p;
 }
@@ -690,6 +693,208 @@ __device__ void take_2D_step(const PreGeom& g, int xd, int yd, double dy_dx, dou
     w.voxel = w.vx + w.vy * g.columns + w.vz * g.columns * g.rows;
 }
 
+// ---- voxel walks by crossing times --------------------------------------------------------------
+// A step of the reference's walk is about 40 double operations, three ways: it moves to the nearest
+// voxel face, computes the other two coordinates there, and their distances to the next faces.  Which
+// face is nearest depends only on the line's crossing times with the three families of planes, which
+// are arithmetic sequences.  So the walk carries the next crossing time of each axis as a 32-bit fixed
+// point number and steps on the smallest one: an addition and a voxel index increment.
+//  * A step is taken this way only when the smallest time leads the others by more than the reference's
+//    coordinates can be off: its slopes are float quotients (or powf and tanf values), so a coordinate is
+//    off by that relative error times the distance travelled.
+//  * Otherwise the state the reference has at this point is set up again from the last face crossed (every
+//    coordinate it keeps follows from that face and the line) and the reference's own step decides: one
+//    warp step in 200.
+//  * All lanes of a warp stay in one loop, which they leave together; a lane that needs the reference's
+//    step waits for that.
+// The voxels visited are the reference's either way (EXACT_FAST_POINTS = 0 takes every step by the
+// reference's code).  On the head scan the end points of 3.3M histories took 5.74 ms with the reference's
+// steps and take 3.20 ms, bound by instruction issue; a warp's walks differ in length, so 12 of its 32
+// lanes step on average.
+enum WalkAxis { kAxisX = 0, kAxisY = 1, kAxisZ = 2, kAxisNone = 3 };
+struct WalkLine {
+    double x0, y0, z0;
+    int xd, yd, zd;
+};
+struct WalkSlopes {
+    double dy_dx, dz_dx, dz_dy, dx_dy, dx_dz, dy_dz;
+};
+
+// The coordinates on the face last crossed (the assignments of take_3D_step's three cases).
+__device__ __forceinline__ void face_position(const PreGeom& g, const WalkLine& l, const WalkSlopes& m, int axis, WalkState& w)
+{
+    if (axis == kAxisX) {
+        w.x = edge_coordinate(-g.R, w.vx, g.voxel_width, 1, l.xd);
+        w.y = corresponding_coordinate(m.dy_dx, w.x, l.x0, l.y0);
+        w.z = corresponding_coordinate(m.dz_dx, w.x, l.x0, l.z0);
+    } else if (axis == kAxisY) {
+        w.y = edge_coordinate(g.R, w.vy, g.voxel_height, -1, l.yd);
+        w.x = corresponding_coordinate(m.dx_dy, w.y, l.y0, l.x0);
+        w.z = corresponding_coordinate(m.dz_dy, w.y, l.y0, l.z0);
+    } else if (axis == kAxisZ) {
+        w.z = edge_coordinate(g.H / 2, w.vz, g.voxel_thickness, -1, l.zd);
+        w.x = corresponding_coordinate(m.dx_dz, w.z, l.z0, l.x0);
+        w.y = corresponding_coordinate(m.dy_dz, w.z, l.z0, l.y0);
+    } else {
+        w.x = l.x0;
+        w.y = l.y0;
+        w.z = l.z0;
+    }
+}
+
+__device__ __forceinline__ void face_distances(const PreGeom& g, const WalkLine& l, int axis, WalkState& w)
+{
+    w.x_to_go = axis == kAxisX ? g.voxel_width : distance_remaining(-g.R, w.x, 1, l.xd, g.voxel_width, w.vx);
+    w.y_to_go = axis == kAxisY ? g.voxel_height : distance_remaining(g.R, w.y, -1, l.yd, g.voxel_height, w.vy);
+    w.z_to_go = axis == kAxisZ ? g.voxel_thickness : distance_remaining(g.H / 2, w.z, -1, l.zd, g.voxel_thickness, w.vz);
+}
+
+__device__ __forceinline__ bool walk_outside(const PreGeom& g, const WalkState& w)
+{
+    return w.vx >= g.columns || w.vy >= g.rows || w.vz >= g.slices || w.vx < 0 || w.vy < 0 || w.vz < 0;
+}
+
+struct CrossingTimes {
+    unsigned tx, ty, tz, bx, by, bz;  // next crossings and their spacing
+    int ix, iy, iz;                   // voxel index increments
+    unsigned stop;         // from here on a crossing may leave the grid
+    unsigned lead, lead_y; // by which a crossing decides (lead_y where y is involved)
+    int exit_axis;         // the crossing that leaves the grid (kAxisNone: through its top)
+};
+
+// w: the walk's initial state; |dx|, |dy|, |dz|: the line's direction.  `error` and `error_y` (where y is
+// involved): how far the reference's crossing times can be off, relative to the walk's length (its slopes'
+// relative errors); to that come the roundings of its coordinates (1e-13 cm) and of the fixed point
+// (half a unit of 2^-30 of the walk per crossing).  False where the line is too close to a coordinate
+// plane for the times to be of use.
+__device__ __forceinline__ bool crossing_times(const PreGeom& g, const WalkLine& l, const WalkState& w, double dx, double dy,
+                                               double dz, double error, double error_y, CrossingTimes& c)
+{
+    if (!g.fast_walks || l.xd == 0 || l.yd == 0 || l.zd == 0 || !(dx > 1e-9) || !(dy > 1e-9) || !(dz > 1e-9) ||
+        !(error_y < 0.05) || !(dx < 1e9 && dy < 1e9 && dz < 1e9))
+        return false;
+    // a start beyond the grid's zero corner has the mirrored index: its first planes lie behind it
+    if (w.x < -g.R || w.y > g.R || w.z > g.H / 2) return false;
+    const double rx = 1.0 / dx, ry = 1.0 / dy, rz = 1.0 / dz;
+    const double tx = w.x_to_go * rx, ty = w.y_to_go * ry, tz = w.z_to_go * rz;
+    const double bx = g.voxel_width * rx, by = g.voxel_height * ry, bz = g.voxel_thickness * rz;
+    // planes before the one that leaves the grid (columns grow with x; rows and slices fall with y and z)
+    const int nx = l.xd > 0 ? g.columns - 1 - w.vx : w.vx;
+    const int ny = l.yd > 0 ? w.vy : g.rows - 1 - w.vy;
+    const int nz = l.zd > 0 ? w.vz : g.slices - 1 - w.vz;
+    const double ex = tx + nx * bx, ey = ty + ny * by, ez = tz + nz * bz, end = fmin(fmin(ex, ey), ez);
+    if (!(end > 0.0) || !(end < 1e12)) return false;
+    const double unit = 1073741824.0 / end;  // 2^30
+    auto fixed = [&](double t) { return (unsigned)fmin(t * unit + 0.5, 1.6e9); };
+    c.tx = fixed(tx);
+    c.ty = fixed(ty);
+    c.tz = fixed(tz);
+    c.bx = fixed(bx);
+    c.by = fixed(by);
+    c.bz = fixed(bz);
+    c.ix = l.xd;
+    c.iy = -l.yd * g.columns;
+    c.iz = -l.zd * g.columns * g.rows;
+    const double roundings = 1.0e-13 * fmax(fmax(rx, ry), rz) * unit + max(max(nx, ny), nz) + 8.0;
+    c.lead = (unsigned)fmin(roundings + error * 1073741824.0, 1.0e9);
+    c.lead_y = (unsigned)fmin(roundings + error_y * 1073741824.0, 1.0e9);
+    if (c.lead_y > min(min(c.bx, c.by), c.bz) / 8) return false;  // also tells the last crossing from the one before
+    const double leave = 1073741824.0 - 2.0 * c.lead_y;
+    c.stop = leave > 0.0 ? (unsigned)leave : 0u;
+    c.exit_axis = ex == end ? kAxisX : ey == end ? kAxisY : l.zd > 0 ? kAxisNone : kAxisZ;
+    return true;
+}
+
+// Walks from w (inside the grid, `done` false) until visit(voxel), called for every voxel entered, returns
+// true, or the walk leaves the grid, or more than max_steps steps have been taken (limit is then set).
+// All lanes of the warp call it; those with done set do nothing.  Leaves the last voxel in w.vx, w.vy,
+// w.vz, w.voxel, and returns the axis last crossed, kAxisNone if w.x, w.y, w.z are those of the last
+// voxel.  `slopes` gives the line's slopes, only where a step needs them.
+// visit(voxel, step) is also called without a step (step = false), with any voxel of the grid, and returns
+// false then.
+template <class Slopes, class Visit>
+__device__ __forceinline__ int walk_3D(const PreGeom& g, const WalkLine& l, const CrossingTimes& times, bool fast, bool done,
+                                       const Slopes& slopes, const Visit& visit, int max_steps, WalkState& w, bool& limit)
+{
+    CrossingTimes c = times;
+    const int vx0 = w.vx, vy0 = w.vy, vz0 = w.vz;
+    int voxel = w.voxel, axis = kAxisNone, extra = 0;  // extra: steps that did not move one index
+    bool left = false;
+    limit = false;
+    const bool walked = !done;
+    if (done) voxel = 0;  // any index that may be looked at
+    for (;;) {
+        bool stuck = !fast && !done;
+        do {
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const unsigned t = min(min(c.tx, c.ty), c.tz);
+                const unsigned far_y = t + c.lead_y, far = c.ty == t ? far_y : t + c.lead;
+                const bool px = c.tx <= far, py = c.ty <= far_y, pz = c.tz <= far;
+                stuck = stuck || (!done && ((px && py) || (px && pz) || (py && pz) || t >= c.stop));
+                const bool go = !stuck && !done;
+                c.tx += go && px ? c.bx : 0u;
+                c.ty += go && py ? c.by : 0u;
+                c.tz += go && pz ? c.bz : 0u;
+                voxel += go ? (px ? c.ix : py ? c.iy : c.iz) : 0;
+                axis = go ? (px ? kAxisX : py ? kAxisY : kAxisZ) : axis;
+                done = visit(voxel, go) || done;
+            }
+        } while (!__any_sync(0xffffffffu, stuck) && __any_sync(0xffffffffu, !done));
+        if (stuck && fast) {
+            // a crossing that is certain and leaves the grid (not through its top) ends the walk here
+            const unsigned t = min(min(c.tx, c.ty), c.tz), far_y = t + c.lead_y, far = c.ty == t ? far_y : t + c.lead;
+            const bool px = c.tx <= far, py = c.ty <= far_y, pz = c.tz <= far;
+            if (px + py + pz == 1 && (px ? kAxisX : py ? kAxisY : kAxisZ) == c.exit_axis && t + c.lead_y >= 1073741824u) {
+                left = done = true;
+                stuck = false;
+            }
+        }
+        if (stuck) {
+            const WalkSlopes m = slopes();
+            const int slab = g.columns * g.rows;
+            w.vz = voxel / slab;
+            w.vy = (voxel - w.vz * slab) / g.columns;
+            w.vx = voxel - w.vz * slab - w.vy * g.columns;
+            face_position(g, l, m, axis, w);
+            face_distances(g, l, axis, w);
+            int moved;
+            do {
+                // near the grid's end every step is the reference's: beyond its top the slice index is
+                // clamped, and the coordinates no longer follow from the last face
+                if (min(min(c.tx, c.ty), c.tz) >= c.stop) fast = false;
+                const int vx = w.vx, vy = w.vy, vz = w.vz;
+                take_3D_step(g, l.xd, l.yd, l.zd, m.dy_dx, m.dz_dx, m.dz_dy, m.dx_dy, m.dx_dz, m.dy_dz, l.x0, l.y0, l.z0, w);
+                left = walk_outside(g, w);
+                voxel = w.voxel;
+                if (w.vx != vx) c.tx += c.bx;
+                if (w.vy != vy) c.ty += c.by;
+                if (w.vz != vz) c.tz += c.bz;
+                moved = (w.vx != vx) + (w.vy != vy) + (w.vz != vz);
+                axis = w.vx != vx ? kAxisX : w.vy != vy ? kAxisY : kAxisZ;
+                done = left || visit(voxel, true);
+                extra += 1 - moved;
+                if (!done && abs(w.vx - vx0) + abs(w.vy - vy0) + abs(w.vz - vz0) + extra > max_steps) {
+                    limit = true;
+                    done = true;
+                }
+                // a step across one face can be set up again from that face, one across an edge cannot
+            } while (!done && (moved != 1 || !fast));
+            if (done) axis = kAxisNone;
+        }
+        __syncwarp();
+        if (!__any_sync(0xffffffffu, !done)) break;
+    }
+    if (walked && !left) {
+        const int slab = g.columns * g.rows;
+        w.vz = voxel / slab;
+        w.vy = (voxel - w.vz * slab) / g.columns;
+        w.vx = voxel - w.vz * slab - w.vy * g.columns;
+        w.voxel = voxel;
+    }
+    return axis;
+}
+
 // Processing order of the voxel walks.  A history's walk lengths depend on where its line crosses
 // the grid: its distance t from the z axis and its direction (the chord for the hull walk, the gap
 // to the hull for the endpoint walks), and one thread walks one history, so neighbouring threads
@@ -728,17 +933,28 @@ __global__ void hull_walks_kernel(PreGeom g, long long n, const int* __restrict_
                                   unsigned long long* counters)
 {
     const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= n) return;
-    const long long i = order[k];
-    if (missed[i]) return;
-    const float wepl = WEPL[i];
-    const bool sc = sc_hull && (wepl <= g.sc_upper) && (wepl >= g.sc_lower);
-    const bool msc = msc_counts && (wepl <= g.msc_upper) && (wepl >= g.msc_lower);
-    const bool sm = sm_counts && (wepl >= g.sm_lower);
-    if (!(sc || msc || sm)) return;
+    bool sc = false, msc = false, sm = false;
+    float xe = 0, ye = 0, ze = 0, xo = 0, yo = 0, zo = 0;
+    if (k < n) {
+        const long long i = order[k];
+        if (!missed[i]) {
+            const float wepl = WEPL[i];
+            sc = sc_hull && (wepl <= g.sc_upper) && (wepl >= g.sc_lower);
+            msc = msc_counts && (wepl <= g.msc_upper) && (wepl >= g.msc_lower);
+            sm = sm_counts && (wepl >= g.sm_lower);
+            if (sc || msc || sm) {
+                xe = G.a[kXE][i];
+                ye = G.a[kYE][i];
+                ze = G.a[kZE][i];
+                xo = G.a[kXO][i];
+                yo = G.a[kYO][i];
+                zo = G.a[kZO][i];
+            }
+        }
+    }
+    bool done = !(sc || msc || sm);
     const double X0 = -g.R, Y0 = g.R, Z0 = g.H / 2;
-    const float xe = G.a[kXE][i], ye = G.a[kYE][i], ze = G.a[kZE][i], xo = G.a[kXO][i], yo = G.a[kYO][i], zo = G.a[kZO][i];
-    const int xd = (xe <= xo) - (xe >= xo), yd = (ye <= yo) - (ye >= yo), zd = (ze <= zo) - (ze >= zo);
+    const WalkLine l{xe, ye, ze, (xe <= xo) - (xe >= xo), (ye <= yo) - (ye >= yo), (ze <= zo) - (ze >= zo)};
     WalkState w;
     w.x = xe;
     w.y = ye;
@@ -747,38 +963,46 @@ __global__ void hull_walks_kernel(PreGeom g, long long n, const int* __restrict_
     w.vy = calculate_voxel(Y0, ye, g.voxel_height);
     w.vz = calculate_voxel(Z0, ze, g.voxel_thickness);
     w.voxel = w.vx + w.vy * g.columns + w.vz * g.columns * g.rows;
-    w.x_to_go = distance_remaining(X0, w.x, 1, xd, g.voxel_width, w.vx);
-    w.y_to_go = distance_remaining(Y0, w.y, -1, yd, g.voxel_height, w.vy);
-    w.z_to_go = distance_remaining(Z0, w.z, -1, zd, g.voxel_thickness, w.vz);
-    const double dy_dx = (double)__fdiv_rn(__fsub_rn(yo, ye), __fsub_rn(xo, xe));
-    const double dz_dx = (double)__fdiv_rn(__fsub_rn(zo, ze), __fsub_rn(xo, xe));
-    const double dz_dy = (double)__fdiv_rn(__fsub_rn(zo, ze), __fsub_rn(yo, ye));
-    const double dx_dy = (double)__fdiv_rn(__fsub_rn(xo, xe), __fsub_rn(yo, ye));
-    const double dx_dz = (double)__fdiv_rn(__fsub_rn(xo, xe), __fsub_rn(zo, ze));
-    const double dy_dz = (double)__fdiv_rn(__fsub_rn(yo, ye), __fsub_rn(zo, ze));
-    const int vx_out = calculate_voxel(X0, xo, g.voxel_width), vy_out = calculate_voxel(Y0, yo, g.voxel_height),
-              vz_out = calculate_voxel(Z0, zo, g.voxel_thickness);
-    const int voxel_out = vx_out + vy_out * g.columns + vz_out * g.columns * g.rows;
-    auto outside = [&]() { return w.vx >= g.columns || w.vy >= g.rows || w.vz >= g.slices || w.vx < 0 || w.vy < 0 || w.vz < 0; };
-    auto mark = [&]() {
-        if (sc) sc_hull[w.voxel] = 0;
-        if (msc) atomicAdd(msc_counts + w.voxel, 1);
-        if (sm) atomicAdd(sm_counts + w.voxel, 1);
+    face_distances(g, l, kAxisNone, w);
+    const float dx = __fsub_rn(xo, xe), dy = __fsub_rn(yo, ye), dz = __fsub_rn(zo, ze);
+    auto slopes = [&]() {
+        return WalkSlopes{(double)__fdiv_rn(dy, dx), (double)__fdiv_rn(dz, dx), (double)__fdiv_rn(dz, dy),
+                          (double)__fdiv_rn(dx, dy), (double)__fdiv_rn(dx, dz), (double)__fdiv_rn(dy, dz)};
     };
-    bool end_walk = (w.voxel == voxel_out) || outside();
-    if (!end_walk) mark();
+    const int voxel_out = calculate_voxel(X0, xo, g.voxel_width) + calculate_voxel(Y0, yo, g.voxel_height) * g.columns +
+                          calculate_voxel(Z0, zo, g.voxel_thickness) * g.columns * g.rows;
+    auto mark = [&](int voxel, bool step) {
+        const bool end = step && voxel == voxel_out;
+        if (step && !end) {
+            if (sc) sc_hull[voxel] = 0;
+            if (msc) atomicAdd(msc_counts + voxel, 1);
+            if (sm) atomicAdd(sm_counts + voxel, 1);
+        }
+        return end;
+    };
+    if (!done) done = walk_outside(g, w) || mark(w.voxel, true);
     const int max_steps = 4 * (g.columns + g.rows + g.slices) + 16;
-    int steps = 0;
-    while (!end_walk) {
-        if (zd != 0) take_3D_step(g, xd, yd, zd, dy_dx, dz_dx, dz_dy, dx_dy, dx_dz, dy_dz, xe, ye, ze, w);
-        else take_2D_step(g, xd, yd, dy_dx, dx_dy, xe, ye, w);
-        end_walk = (w.voxel == voxel_out) || outside();
-        if (!end_walk) mark();
-        if (++steps > max_steps) {
-            atomicAdd(counters + kCntWaitExpired, 1ull);
-            break;
+    // the slopes are float quotients of dx, dy and dz, 2^-24 off each; a comparison involves up to four
+    CrossingTimes times{};
+    const bool flat = l.zd == 0;
+    const bool fast = !done && !flat && crossing_times(g, l, w, fabs((double)dx), fabs((double)dy), fabs((double)dz), 5.0e-7,
+                                                       5.0e-7, times);
+    bool limit;
+    walk_3D(g, l, times, fast, done || flat, slopes, mark, max_steps, w, limit);
+    if (flat && !done) {
+        const WalkSlopes m = slopes();
+        int steps = 0;
+        while (!done) {
+            take_2D_step(g, l.xd, l.yd, m.dy_dx, m.dx_dy, xe, ye, w);
+            done = (w.voxel == voxel_out) || walk_outside(g, w);
+            if (!done) mark(w.voxel, true);
+            if (++steps > max_steps) {
+                limit = true;
+                break;
+            }
         }
     }
+    if (limit) atomicAdd(counters + kCntWaitExpired, 1ull);
 }
 
 // MSC_edge_detection_GPU (B.cu:6911-6956), out of place: 3x3 maximum difference over the
@@ -891,144 +1115,134 @@ __global__ void hybrid_kernel(long long n, const uint8_t* __restrict__ hull, con
     if (i < n) x[i] = hull[i] ? fbp[i] : 0.0f;
 }
 
-// find_MLP_endpoints_GPU (B.cu:7581-7773): walk from the cylinder point along the straight line
-// (angle + PI when leaving) until the first hull voxel or the image edge.
-__device__ bool find_endpoint(const PreGeom& g, const uint8_t* __restrict__ image, double x_start, double y_start,
-                              double z_start, double xy_angle, double xz_angle, double& x_object, double& y_object,
-                              double& z_object, int& voxel_x, int& voxel_y, int& voxel_z, bool entering)
+// The hull as bits: 160 KB for 1.28 million voxels, which stay in L1 where the bytes did not.
+__global__ void hull_bits_kernel(long long words, long long n, const uint8_t* __restrict__ hull, uint32_t* __restrict__ bits)
 {
-    const double X0 = -g.R, Y0 = g.R, Z0 = g.H / 2;
-    double x = x_start, y = y_start, z = z_start;
-    bool hit_hull = false;
+    const long long word = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (word >= words) return;  // whole warps: a warp writes one word
+    const long long v = word * 32 + (threadIdx.x & 31);
+    const unsigned b = __ballot_sync(0xffffffffu, v < n && hull[v] == 1);
+    if ((threadIdx.x & 31) == 0) bits[word] = b;
+}
+
+// find_MLP_endpoints_GPU (B.cu:7581-7773): walk from the cylinder point along the straight line
+// (angle + PI when leaving) until the first hull voxel or the image edge.  All lanes of a warp call it;
+// lanes without a history (have = false) walk nothing.
+__device__ __forceinline__ bool find_endpoint(const PreGeom& g, const uint32_t* __restrict__ bits, bool have, double x_start,
+                                              double y_start, double z_start, double xy_angle, double xz_angle,
+                                              double& x_object, double& y_object, double& z_object, int& voxel_x,
+                                              int& voxel_y, int& voxel_z, bool entering)
+{
     if (!entering) xy_angle += kPi;
-    int x_move_direction = (cos(xy_angle) >= 0) - (cos(xy_angle) <= 0);
-    const int y_move_direction = (sin(xy_angle) >= 0) - (sin(xy_angle) <= 0);
-    int z_move_direction = (sin(xz_angle) >= 0) - (sin(xz_angle) <= 0);
-    if (x_move_direction < 0) z_move_direction *= -1;
-    voxel_x = calculate_voxel(X0, x, g.voxel_width);
-    voxel_y = calculate_voxel(Y0, y, g.voxel_height);
-    voxel_z = calculate_voxel(Z0, z, g.voxel_thickness);
-    double x_to_go = distance_remaining(X0, x, 1, x_move_direction, g.voxel_width, voxel_x);
-    double y_to_go = distance_remaining(Y0, y, -1, y_move_direction, g.voxel_height, voxel_y);
-    double z_to_go = distance_remaining(Z0, z, -1, z_move_direction, g.voxel_thickness, voxel_z);
-    int voxel = voxel_x + (voxel_y + voxel_z * g.rows) * g.columns;
-    const double delta_yx = fabs(tan(xy_angle));
-    const double delta_zx = fabs(tan(xz_angle));
-    const double delta_zy = fabs(tan(xz_angle) / tan(xy_angle));
-    const double dy_dx = tan(xy_angle);
-    const double dz_dx = tan(xz_angle);
-    const double dz_dy = tan(xz_angle) / tan(xy_angle);
-    const double dx_dy = powf((float)tan(xy_angle), -1.0f);
-    const double dx_dz = powf((float)tan(xz_angle), -1.0f);
-    const double dy_dz = tanf((float)xy_angle) / tan(xz_angle);
-    auto outside = [&]() {
-        return (voxel_x >= g.columns) || (voxel_y >= g.rows) || (voxel_z >= g.slices) || (voxel_x < 0) || (voxel_y < 0) || (voxel_z < 0);
+    WalkLine l{x_start, y_start, z_start, 0, 0, 0};
+    l.xd = (cos(xy_angle) >= 0) - (cos(xy_angle) <= 0);
+    l.yd = (sin(xy_angle) >= 0) - (sin(xy_angle) <= 0);
+    l.zd = (sin(xz_angle) >= 0) - (sin(xz_angle) <= 0);
+    if (l.xd < 0) l.zd *= -1;
+    WalkState w;
+    w.x = x_start;
+    w.y = y_start;
+    w.z = z_start;
+    w.vx = calculate_voxel(-g.R, x_start, g.voxel_width);
+    w.vy = calculate_voxel(g.R, y_start, g.voxel_height);
+    w.vz = calculate_voxel(g.H / 2, z_start, g.voxel_thickness);
+    w.voxel = w.vx + (w.vy + w.vz * g.rows) * g.columns;
+    face_distances(g, l, kAxisNone, w);
+    const double tan_xy = tan(xy_angle), tan_xz = tan(xz_angle);
+    auto slopes = [&]() {
+        return WalkSlopes{tan_xy, tan_xz, tan_xz / tan_xy, (double)powf((float)tan_xy, -1.0f),
+                          (double)powf((float)tan_xz, -1.0f), tanf((float)xy_angle) / tan_xz};
     };
-    bool outside_image = outside();
-    if (!outside_image) hit_hull = (image[voxel] == 1);
-    bool end_walk = outside_image || hit_hull;
+    bool hit_hull = false;
+    auto visit = [&](int voxel, bool step) {
+        const bool hit = step && ((__ldg(bits + (voxel >> 5)) >> (voxel & 31)) & 1u);
+        hit_hull = hit_hull || hit;
+        return hit;
+    };
+    bool done = !have || walk_outside(g, w);
+    if (!done) done = visit(w.voxel, true);
     // every pass moves one index monotonically, so the walk leaves the grid within this bound
     const int max_steps = 2 * (g.columns + g.rows + g.slices) + 16;
-    int steps = 0;
-    if (z_move_direction != 0) {
-        while (!end_walk && steps++ < max_steps) {
-            const double x_extension = delta_zx * x_to_go;
-            const double y_extension = delta_zy * y_to_go;
-            if ((z_to_go <= x_extension) && (z_to_go <= y_extension)) {
-                voxel_z -= z_move_direction;
-                z = edge_coordinate(Z0, voxel_z, g.voxel_thickness, -1, z_move_direction);
-                x = corresponding_coordinate(dx_dz, z, z_start, x_start);
-                y = corresponding_coordinate(dy_dz, z, z_start, y_start);
-                x_to_go = distance_remaining(X0, x, 1, x_move_direction, g.voxel_width, voxel_x);
-                y_to_go = distance_remaining(Y0, y, -1, y_move_direction, g.voxel_height, voxel_y);
-                z_to_go = g.voxel_thickness;
-            } else if (x_extension <= y_extension) {
-                voxel_x += x_move_direction;
-                x = edge_coordinate(X0, voxel_x, g.voxel_width, 1, x_move_direction);
-                y = corresponding_coordinate(dy_dx, x, x_start, y_start);
-                z = corresponding_coordinate(dz_dx, x, x_start, z_start);
-                x_to_go = g.voxel_width;
-                y_to_go = distance_remaining(Y0, y, -1, y_move_direction, g.voxel_height, voxel_y);
-                z_to_go = distance_remaining(Z0, z, -1, z_move_direction, g.voxel_thickness, voxel_z);
+    // slopes: tan in double, powf of a float within 4 units in the last place (5.4e-7 with the float's own
+    // rounding), and for y after a z crossing tanf (4 units) of the angle as a float, whose rounding
+    // changes the tangent by 2 / |sin 2 angle| = tan + 1 / tan times that
+    const double a_xy = fabs(tan_xy), a_xz = fabs(tan_xz), scale = 1.0 / fmax(fmax(a_xy, a_xz), 1.0);
+    CrossingTimes times{};
+    const bool flat = l.zd == 0;
+    const double turn = 1.2e-7 * fabs(xy_angle) + 1.0e-7;
+    // an elevation beyond a right angle moves z against its own direction: left to the reference's steps
+    const bool forward = (tan_xy > 0) == (l.xd * l.yd > 0) && (tan_xz > 0) == (l.xd * l.zd > 0);
+    const bool fast = !done && !flat && forward && crossing_times(g, l, w, scale, a_xy * scale, a_xz * scale, 1.2e-6,
+                                                       2.4e-6 + turn * (a_xy + 1.0 / a_xy), times);
+    bool limit;
+    int axis = walk_3D(g, l, times, fast, done || flat, slopes, visit, max_steps - 1, w, limit);
+    if (flat && !done) {
+        // the reference's 2D loop of this walk (B.cu:7718-7752) keeps its slice index and its start height
+        const double delta_yx = fabs(tan_xy);
+        const WalkSlopes m = slopes();
+        int steps = 0;
+        while (!done && steps++ < max_steps) {
+            const double y_extension = w.y_to_go / delta_yx;
+            if (w.x_to_go <= y_extension) {
+                w.vx += l.xd;
+                w.x = edge_coordinate(-g.R, w.vx, g.voxel_width, 1, l.xd);
+                w.y = corresponding_coordinate(m.dy_dx, w.x, x_start, y_start);
+                w.x_to_go = g.voxel_width;
+                w.y_to_go = distance_remaining(g.R, w.y, -1, l.yd, g.voxel_height, w.vy);
             } else {
-                voxel_y -= y_move_direction;
-                y = edge_coordinate(Y0, voxel_y, g.voxel_height, -1, y_move_direction);
-                x = corresponding_coordinate(dx_dy, y, y_start, x_start);
-                z = corresponding_coordinate(dz_dy, y, y_start, z_start);
-                x_to_go = distance_remaining(X0, x, 1, x_move_direction, g.voxel_width, voxel_x);
-                y_to_go = g.voxel_height;
-                z_to_go = distance_remaining(Z0, z, -1, z_move_direction, g.voxel_thickness, voxel_z);
-            }
-            if (x_to_go == 0) {
-                x_to_go = g.voxel_width;
-                voxel_x += x_move_direction;
-            }
-            if (y_to_go == 0) {
-                y_to_go = g.voxel_height;
-                voxel_y -= y_move_direction;
-            }
-            if (z_to_go == 0) {
-                z_to_go = g.voxel_thickness;
-                voxel_z -= z_move_direction;
-            }
-            voxel_z = max(voxel_z, 0);
-            voxel = voxel_x + voxel_y * g.columns + voxel_z * g.columns * g.rows;
-            outside_image = outside();
-            if (!outside_image) hit_hull = (image[voxel] == 1);
-            end_walk = outside_image || hit_hull;
-        }
-    } else {
-        while (!end_walk && steps++ < max_steps) {
-            const double y_extension = y_to_go / delta_yx;
-            if (x_to_go <= y_extension) {
-                voxel_x += x_move_direction;
-                x = edge_coordinate(X0, voxel_x, g.voxel_width, 1, x_move_direction);
-                y = corresponding_coordinate(dy_dx, x, x_start, y_start);
-                x_to_go = g.voxel_width;
-                y_to_go = distance_remaining(Y0, y, -1, y_move_direction, g.voxel_height, voxel_y);
-            } else {
-                voxel_y -= y_move_direction;
+                w.vy -= l.yd;
                 // the reference passes Z_INCREASING_DIRECTION here (B.cu:7736); it equals Y's
-                y = edge_coordinate(Y0, voxel_y, g.voxel_height, -1, y_move_direction);
-                x = corresponding_coordinate(dx_dy, y, y_start, x_start);
-                x_to_go = distance_remaining(X0, x, 1, x_move_direction, g.voxel_width, voxel_x);
-                y_to_go = g.voxel_height;
+                w.y = edge_coordinate(g.R, w.vy, g.voxel_height, -1, l.yd);
+                w.x = corresponding_coordinate(m.dx_dy, w.y, y_start, x_start);
+                w.x_to_go = distance_remaining(-g.R, w.x, 1, l.xd, g.voxel_width, w.vx);
+                w.y_to_go = g.voxel_height;
             }
-            if (x_to_go == 0) {
-                x_to_go = g.voxel_width;
-                voxel_x += x_move_direction;
+            if (w.x_to_go == 0) {
+                w.x_to_go = g.voxel_width;
+                w.vx += l.xd;
             }
-            if (y_to_go == 0) {
-                y_to_go = g.voxel_height;
-                voxel_y -= y_move_direction;
+            if (w.y_to_go == 0) {
+                w.y_to_go = g.voxel_height;
+                w.vy -= l.yd;
             }
-            voxel = voxel_x + voxel_y * g.columns + voxel_z * g.columns * g.rows;
-            outside_image = outside();
-            if (!outside_image) hit_hull = (image[voxel] == 1);
-            end_walk = outside_image || hit_hull;
+            w.voxel = w.vx + w.vy * g.columns + w.vz * g.columns * g.rows;
+            done = walk_outside(g, w);
+            if (!done) done = visit(w.voxel, true);
         }
+        axis = kAxisNone;
+    } else if (hit_hull && axis != kAxisNone) {
+        face_position(g, l, slopes(), axis, w);  // where the reference's step left x, y and z
     }
+    voxel_x = w.vx;
+    voxel_y = w.vy;
+    voxel_z = w.vz;
     if (hit_hull) {
-        x_object = x;
-        y_object = y;
-        z_object = z;
+        x_object = w.x;
+        y_object = w.y;
+        z_object = w.z;
     }
     return hit_hull;
 }
 
-// collect_MLP_endpoints_GPU_nobool (B.cu:7819-7854)
-__global__ void endpoints_kernel(PreGeom g, long long n, const int* __restrict__ order, const uint8_t* __restrict__ hull,
-                                 GeomPtrs G, uint32_t* __restrict__ first_voxel, int* __restrict__ keep)
+// collect_MLP_endpoints_GPU_nobool (B.cu:7819-7854).  Six CTAs per SM: 3.20 ms for 3.3M histories against
+// 4.26 ms with the registers it would take alone (118: four CTAs) and 3.34 ms with eight (which spill).
+__global__ void __launch_bounds__(128, 6) endpoints_kernel(PreGeom g, long long n, const int* __restrict__ order,
+                                                           const uint32_t* __restrict__ hull_bits, GeomPtrs G,
+                                                           uint32_t* __restrict__ first_voxel, int* __restrict__ keep)
 {
     const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= n) return;
-    const long long i = order[k];
+    const bool have = k < n;
+    const long long i = have ? order[k] : 0;
+    float p[kNumGeom];
+#pragma unroll
+    for (int a = 0; a < kNumGeom; a++) p[a] = have ? G.a[a][i] : 0.5f;
     int vx = 0, vy = 0, vz = 0, vx2 = 0, vy2 = 0, vz2 = 0;
     double xin = 0, yin = 0, zin = 0, xout = 0, yout = 0, zout = 0;
-    const bool entered = find_endpoint(g, hull, G.a[kXE][i], G.a[kYE][i], G.a[kZE][i], G.a[kXYE][i], G.a[kXZE][i], xin,
-                                       yin, zin, vx, vy, vz, true);
-    const bool exited = find_endpoint(g, hull, G.a[kXO][i], G.a[kYO][i], G.a[kZO][i], G.a[kXYO][i], G.a[kXZO][i], xout,
-                                      yout, zout, vx2, vy2, vz2, false);
+    const bool entered =
+        find_endpoint(g, hull_bits, have, p[kXE], p[kYE], p[kZE], p[kXYE], p[kXZE], xin, yin, zin, vx, vy, vz, true);
+    const bool exited = find_endpoint(g, hull_bits, have && entered, p[kXO], p[kYO], p[kZO], p[kXYO], p[kXZO], xout, yout,
+                                      zout, vx2, vy2, vz2, false);
+    if (!have) return;
     if (entered && exited) {
         first_voxel[i] = (uint32_t)(vx + g.columns * vy + g.rows * g.columns * vz);
         G.a[kXE][i] = (float)xin;
@@ -1137,6 +1351,7 @@ pct_status ensure_fixed(pct_ctx* ctx, Preproc* p)
     if (e == cudaSuccess) e = alloc(p->SM_differences, nv);
     if (e == cudaSuccess) e = alloc(p->edge_tmp, nv);
     if (e == cudaSuccess) e = alloc(p->walk_hist, 2 * pct::kWalkKeys);
+    if (e == cudaSuccess) e = alloc(p->hull_bits, (nv + 31) / 32);
     if (e == cudaSuccess) e = alloc(p->SM_thresholds, ctx->cfg.SLICES);
     if (e != cudaSuccess) {
         cudaGetLastError();
@@ -1556,7 +1771,10 @@ extern "C" pct_status pct_reconstruction_cuts(pct_ctx* ctx)
     if (n > 0) {
         int* order = walk_order(ctx, p, n, p->vec_geom, pct::kWalkDir);
         if (!order) return fail(ctx, PCT_ERR_CUDA, "walk order", cudaGetLastError());
-        pct::endpoints_kernel<<<pct::grid_for(n, 128), 128, 0, s>>>(g, n, order, p->hull, geom_ptrs(p->vec_geom),
+        const long long words = (ctx->cfg.NUM_VOXELS + 31LL) / 32;
+        pct::hull_bits_kernel<<<pct::grid_for(words * 32, 256), 256, 0, s>>>(words, ctx->cfg.NUM_VOXELS, p->hull, p->hull_bits);
+        ctx->launches += 1;
+        pct::endpoints_kernel<<<pct::grid_for(n, 128), 128, 0, s>>>(g, n, order, p->hull_bits, geom_ptrs(p->vec_geom),
                                                                     p->vec_first_voxel, p->flags);
     }
     PRE_TRY(cudaGetLastError(), "endpoints kernel");
