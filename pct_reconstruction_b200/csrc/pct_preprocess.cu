@@ -145,6 +145,7 @@ struct Preproc {
     int *MSC_counts = nullptr, *SM_counts = nullptr, *SM_differences = nullptr, *SM_thresholds = nullptr;
     int* edge_tmp = nullptr;
     unsigned* walk_hist = nullptr;  // bucket-sort scratch of the walk order
+    int* hull_starts = nullptr;     // the hull walk's ranges of histories
     uint32_t* hull_bits = nullptr;  // hull, one bit per voxel (for the endpoint walks)
     bool hull_ready = false;
 };
@@ -163,7 +164,7 @@ void preproc_release(Preproc* p)
                     p->bin_counts, p->mean_WEPL, p->mean_rel_ut_angle, p->mean_rel_uv_angle, p->stddev_WEPL,
                     p->stddev_rel_ut_angle, p->stddev_rel_uv_angle, p->sinogram, p->sinogram_filtered,
                     p->FBP_image, p->FBP_median, p->FBP_hull, p->SC_hull, p->hull, p->MSC_counts, p->SM_counts,
-                    p->SM_differences, p->SM_thresholds, p->edge_tmp, p->walk_hist, p->hull_bits, p->fbp_tables};
+                    p->SM_differences, p->SM_thresholds, p->edge_tmp, p->walk_hist, p->hull_starts, p->hull_bits, p->fbp_tables};
     for (void* q : ptrs) cudaFree(q);
     delete p;
 }
@@ -971,13 +972,13 @@ __device__ __forceinline__ bool crossing_times(const PreGeom& g, const WalkLine&
     return true;
 }
 
-// Walks from w (inside the grid, `done` false) until visit(voxel), called for every voxel entered, returns
+// Walks from w (inside the grid, `done` false) until visit, called for every voxel entered, returns
 // true, or the walk leaves the grid, or more than max_steps steps have been taken (limit is then set).
 // All lanes of the warp call it; those with done set do nothing.  Leaves the last voxel in w.vx, w.vy,
 // w.vz, w.voxel, and returns the axis last crossed, kAxisNone if w.x, w.y, w.z are those of the last
 // voxel.  `slopes` gives the line's slopes, only where a step needs them.
-// visit(voxel, step) is also called without a step (step = false), with any voxel of the grid, and returns
-// false then.
+// visit(voxel, step, timed) is also called without a step (step = false), with any voxel of the grid, and
+// returns false then; timed tells the steps by crossing times, which never enter a voxel twice.
 template <class Slopes, class Visit>
 __device__ __forceinline__ int walk_3D(const PreGeom& g, const WalkLine& l, const CrossingTimes& times, bool fast, bool done,
                                        const Slopes& slopes, const Visit& visit, int max_steps, WalkState& w, bool& limit)
@@ -1004,7 +1005,7 @@ __device__ __forceinline__ int walk_3D(const PreGeom& g, const WalkLine& l, cons
                 c.tz += go && pz ? c.bz : 0u;
                 voxel += go ? (px ? c.ix : py ? c.iy : c.iz) : 0;
                 axis = go ? (px ? kAxisX : py ? kAxisY : kAxisZ) : axis;
-                done = visit(voxel, go) || done;
+                done = visit(voxel, go, true) || done;
             }
         } while (!__any_sync(0xffffffffu, stuck) && __any_sync(0xffffffffu, !done));
         if (stuck && fast) {
@@ -1038,7 +1039,7 @@ __device__ __forceinline__ int walk_3D(const PreGeom& g, const WalkLine& l, cons
                 if (w.vz != vz) c.tz += c.bz;
                 moved = (w.vx != vx) + (w.vy != vy) + (w.vz != vz);
                 axis = w.vx != vx ? kAxisX : w.vy != vy ? kAxisY : kAxisZ;
-                done = left || visit(voxel, true);
+                done = left || visit(voxel, true, false);
                 extra += 1 - moved;
                 if (!done && abs(w.vx - vx0) + abs(w.vy - vy0) + abs(w.vz - vz0) + extra > max_steps) {
                     limit = true;
@@ -1069,7 +1070,7 @@ __device__ __forceinline__ int walk_3D(const PreGeom& g, const WalkLine& l, cons
 // buckets shorten the endpoint walks (38.2 -> 31.2 ms; t alone 33.8) but not the hull walks, which
 // run entry to exit (23.0 -> 21.5 ms with t alone, 23.7 with 32 directions).  The order changes no
 // result (integer counts, per-history endpoints).
-constexpr int kWalkT = 32, kWalkDir = 32, kWalkKeys = kWalkT * kWalkDir;
+constexpr int kWalkT = 32, kWalkDir = 32;
 __global__ void walk_order_key_kernel(long long n, const float* __restrict__ xe, const float* __restrict__ ye,
                                       const float* __restrict__ xo, const float* __restrict__ yo, float R,
                                       int dir_buckets, int* __restrict__ key)
@@ -1093,32 +1094,43 @@ __global__ void walk_order_key_kernel(long long n, const float* __restrict__ xe,
 // what they do at each voxel: SC carves (writes 0), MSC and SM count.  Here each history walks once
 // and applies every hull whose window (and *_ON switch) it satisfies, so the voxel sequence each
 // hull sees is the one its own kernel would walk.
-__global__ void hull_walks_kernel(PreGeom g, long long n, const int* __restrict__ order, GeomPtrs G,
-                                  const float* __restrict__ WEPL, const uint8_t* __restrict__ missed,
-                                  uint8_t* __restrict__ sc_hull, int* __restrict__ msc_counts, int* __restrict__ sm_counts,
-                                  unsigned long long* counters)
+enum HullMask { kHullSC = 1, kHullMSC = 2, kHullSM = 4 };
+struct HullImages {
+    uint8_t* sc;  // null where the hull is off
+    int *msc, *sm;
+};
+
+__device__ __forceinline__ int hull_mask(const PreGeom& g, const HullImages& im, float wepl)
 {
-    const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    bool sc = false, msc = false, sm = false;
+    const bool sc = im.sc && (wepl <= g.sc_upper) && (wepl >= g.sc_lower);
+    const bool msc = im.msc && (wepl <= g.msc_upper) && (wepl >= g.msc_lower);
+    const bool sm = im.sm && (wepl >= g.sm_lower);
+    return (sc ? kHullSC : 0) | (msc ? kHullMSC : 0) | (sm ? kHullSM : 0);
+}
+
+__device__ __forceinline__ void hull_mark(const HullImages& im, int mask, int voxel, int count)
+{
+    if (mask & kHullSC) im.sc[voxel] = 0;
+    if (mask & kHullMSC) atomicAdd(im.msc + voxel, count);
+    if (mask & kHullSM) atomicAdd(im.sm + voxel, count);
+}
+
+// The walk of history i, by all lanes of a warp (have = false: without one); count(voxel, timed) is called
+// for every voxel but the last.
+template <class Count>
+__device__ __forceinline__ void hull_walk(const PreGeom& g, bool have, long long i, const GeomPtrs& G, const Count& count,
+                                          unsigned long long* counters)
+{
     float xe = 0, ye = 0, ze = 0, xo = 0, yo = 0, zo = 0;
-    if (k < n) {
-        const long long i = order[k];
-        if (!missed[i]) {
-            const float wepl = WEPL[i];
-            sc = sc_hull && (wepl <= g.sc_upper) && (wepl >= g.sc_lower);
-            msc = msc_counts && (wepl <= g.msc_upper) && (wepl >= g.msc_lower);
-            sm = sm_counts && (wepl >= g.sm_lower);
-            if (sc || msc || sm) {
-                xe = G.a[kXE][i];
-                ye = G.a[kYE][i];
-                ze = G.a[kZE][i];
-                xo = G.a[kXO][i];
-                yo = G.a[kYO][i];
-                zo = G.a[kZO][i];
-            }
-        }
+    if (have) {
+        xe = G.a[kXE][i];
+        ye = G.a[kYE][i];
+        ze = G.a[kZE][i];
+        xo = G.a[kXO][i];
+        yo = G.a[kYO][i];
+        zo = G.a[kZO][i];
     }
-    bool done = !(sc || msc || sm);
+    bool done = !have;
     const double X0 = -g.R, Y0 = g.R, Z0 = g.H / 2;
     const WalkLine l{xe, ye, ze, (xe <= xo) - (xe >= xo), (ye <= yo) - (ye >= yo), (ze <= zo) - (ze >= zo)};
     WalkState w;
@@ -1137,16 +1149,12 @@ __global__ void hull_walks_kernel(PreGeom g, long long n, const int* __restrict_
     };
     const int voxel_out = calculate_voxel(X0, xo, g.voxel_width) + calculate_voxel(Y0, yo, g.voxel_height) * g.columns +
                           calculate_voxel(Z0, zo, g.voxel_thickness) * g.columns * g.rows;
-    auto mark = [&](int voxel, bool step) {
+    auto mark = [&](int voxel, bool step, bool timed) {
         const bool end = step && voxel == voxel_out;
-        if (step && !end) {
-            if (sc) sc_hull[voxel] = 0;
-            if (msc) atomicAdd(msc_counts + voxel, 1);
-            if (sm) atomicAdd(sm_counts + voxel, 1);
-        }
+        if (step && !end) count(voxel, timed);
         return end;
     };
-    if (!done) done = walk_outside(g, w) || mark(w.voxel, true);
+    if (!done) done = walk_outside(g, w) || mark(w.voxel, true, true);
     const int max_steps = 4 * (g.columns + g.rows + g.slices) + 16;
     // the slopes are float quotients of dx, dy and dz, 2^-24 off each; a comparison involves up to four
     CrossingTimes times{};
@@ -1161,7 +1169,7 @@ __global__ void hull_walks_kernel(PreGeom g, long long n, const int* __restrict_
         while (!done) {
             take_2D_step(g, l.xd, l.yd, m.dy_dx, m.dx_dy, xe, ye, w);
             done = (w.voxel == voxel_out) || walk_outside(g, w);
-            if (!done) mark(w.voxel, true);
+            if (!done) mark(w.voxel, true, false);
             if (++steps > max_steps) {
                 limit = true;
                 break;
@@ -1169,6 +1177,165 @@ __global__ void hull_walks_kernel(PreGeom g, long long n, const int* __restrict_
         }
     }
     if (limit) atomicAdd(counters + kCntWaitExpired, 1ull);
+}
+
+// One thread per history, every mark an atomic on its image: bound by the L2's atomics, 155 G/s.
+__global__ void __launch_bounds__(128) hull_walks_kernel(PreGeom g, long long n, const int* __restrict__ order, GeomPtrs G,
+                                                         const float* __restrict__ WEPL, const uint8_t* __restrict__ missed,
+                                                         HullImages im, unsigned long long* counters)
+{
+    const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const long long i = k < n ? order[k] : 0;
+    const int mask = k < n && !missed[i] ? hull_mask(g, im, WEPL[i]) : 0;
+    hull_walk(g, mask != 0, i, G, [&](int voxel, bool) { hull_mark(im, mask, voxel, 1); }, counters);
+}
+
+// The same with the marks counted in shared memory.  All histories of one mask mark the same voxels in
+// the same images, so one 16-bit count per voxel serves them; a CTA counts those of a window of as many
+// slices as shared memory holds and adds the window to the images when the mask or the window
+// changes.  The histories are sorted by (mask, first slice they touch, distance from the axis); a CTA
+// takes a contiguous range of them, and the ranges cost the same by the chords' lengths.  Marks
+// outside the window, and those of the reference's own steps, go to the images directly.
+// On the head scan (4M histories, 650M marks, windows of two slices) 1.75 ms against 4.21 ms with every
+// mark in L2, bound by the walks' instructions; 512 threads take 1.97 ms, 1024 (which spill) 1.74 ms.  The
+// sort by more keys and the ranges take 65 us where the other walk's order takes 30, so few histories
+// stay with that (300,000 with few marks: 71 us against 45).
+constexpr long long kHullWindowMin = 1 << 19;
+constexpr int kHullKeys = 4096, kHullThreads = 768, kHullWindow = 200 * 1024;
+// histories between two additions of the window: a timed step enters a voxel once, so counts stay below 2^16
+constexpr int kHullFlush = 65000;
+
+struct HullPlan {
+    int window;     // slices of a window (0: one does not fit)
+    int first;      // window starts: 0 .. first - 1
+    int distances;  // buckets of the distance from the axis
+};
+HullPlan hull_plan(const PreGeom& g)
+{
+    HullPlan p{};
+    const long long fit = kHullWindow / (2LL * g.columns * g.rows);
+    p.window = (int)(fit < g.slices ? fit : g.slices);
+    p.first = g.slices - p.window + 1;
+    p.distances = kHullKeys / (8 * p.first);
+    if (p.distances > 32) p.distances = 32;
+    if (p.distances == 0) p.window = 0;
+    return p;
+}
+
+__global__ void hull_key_kernel(PreGeom g, HullPlan plan, long long n, GeomPtrs G, const float* __restrict__ WEPL,
+                                const uint8_t* __restrict__ missed, HullImages im, int* __restrict__ key)
+{
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const int mask = !missed[i] ? hull_mask(g, im, WEPL[i]) : 0;
+    if (mask == 0) {
+        key[i] = 0;
+        return;
+    }
+    const float xe = G.a[kXE][i], ye = G.a[kYE][i], xo = G.a[kXO][i], yo = G.a[kYO][i];
+    const float dx = xo - xe, dy = yo - ye, len = sqrtf(dx * dx + dy * dy);
+    const float t = len > 0.f ? fabsf(xe * yo - xo * ye) / len : 0.f;
+    const int kt = (int)fminf(t / (float)g.R * plan.distances, (float)(plan.distances - 1));
+    const int z = min(calculate_voxel(g.H / 2, G.a[kZE][i], g.voxel_thickness), calculate_voxel(g.H / 2, G.a[kZO][i], g.voxel_thickness));
+    key[i] = (mask * plan.first + max(0, min(z, plan.first - 1))) * plan.distances + max(kt, 0);
+}
+
+// starts[b]: where CTA b's range begins.  hist: histories of each key, in descending order of the keys.
+__global__ void __launch_bounds__(1024) hull_ranges_kernel(PreGeom g, HullPlan plan, const unsigned* __restrict__ hist, int blocks,
+                                                           int* __restrict__ starts)
+{
+    __shared__ unsigned long long cost[1024];
+    __shared__ unsigned count[1024];
+    const int keys = 8 * plan.first * plan.distances, none = plan.first * plan.distances, per = (keys + 1023) / 1024;
+    auto weight = [&](int key) {  // of a history: its setup and its steps
+        const double t = (key % plan.distances + 0.5) / plan.distances;
+        return key < none ? 0u : (unsigned)(60.0 + 2.5 * g.R * sqrt(1.0 - t * t) / g.voxel_width);
+    };
+    unsigned long long own_cost = 0;
+    unsigned own = 0;
+    for (int j = 0; j < per; j++) {
+        const int key = keys - 1 - ((int)threadIdx.x * per + j);
+        if (key < 0) break;
+        own += hist[key];
+        own_cost += (unsigned long long)hist[key] * weight(key);
+    }
+    cost[threadIdx.x] = own_cost;
+    count[threadIdx.x] = own;
+    __syncthreads();
+    for (int o = 1; o < 1024; o <<= 1) {
+        const unsigned long long c = threadIdx.x >= o ? cost[threadIdx.x - o] : 0;
+        const unsigned m = threadIdx.x >= o ? count[threadIdx.x - o] : 0;
+        __syncthreads();
+        cost[threadIdx.x] += c;
+        count[threadIdx.x] += m;
+        __syncthreads();
+    }
+    const unsigned long long total = cost[1023];
+    for (int b = threadIdx.x; b <= blocks; b += 1024) {
+        const unsigned long long target = total / blocks * b + total % blocks * b / blocks;
+        int lo = 0, hi = 1023;  // the first thread whose keys reach the target
+        while (lo < hi) {
+            const int mid = (lo + hi) / 2;
+            if (cost[mid] >= target) hi = mid;
+            else lo = mid + 1;
+        }
+        unsigned long long c = lo ? cost[lo - 1] : 0;
+        unsigned position = lo ? count[lo - 1] : 0;
+        for (int j = 0; j < per; j++) {
+            const int key = keys - 1 - (lo * per + j);
+            if (key < none) break;
+            const unsigned long long here = (unsigned long long)hist[key] * weight(key);
+            if (c + here >= target) {
+                position += (unsigned)((target - c) / weight(key));
+                break;
+            }
+            c += here;
+            position += hist[key];
+        }
+        starts[b] = (int)position;
+    }
+}
+
+__global__ void __launch_bounds__(kHullThreads, 1)
+    hull_window_kernel(PreGeom g, HullPlan plan, const int* __restrict__ order, const int* __restrict__ key,
+                       const unsigned* __restrict__ bucket_end, const int* __restrict__ starts, GeomPtrs G, HullImages im,
+                       unsigned long long* counters)
+{
+    extern __shared__ unsigned window[];
+    __shared__ int next;
+    const int lane = threadIdx.x & 31, slab = g.columns * g.rows, voxels = plan.window * slab, words = (voxels + 1) / 2;
+    for (int k = threadIdx.x; k < words; k += blockDim.x) window[k] = 0;
+    const int end = starts[blockIdx.x + 1];
+    for (int p = starts[blockIdx.x]; p < end;) {
+        const int group = key[order[p]] / plan.distances, mask = group / plan.first;
+        const int base = (group - mask * plan.first) * slab;
+        const int last = min(min(end, (int)bucket_end[group * plan.distances]), p + kHullFlush);
+        if (threadIdx.x == 0) next = p;
+        __syncthreads();
+        for (;;) {
+            int first;
+            if (lane == 0) first = atomicAdd(&next, 32);
+            first = __shfl_sync(0xffffffffu, first, 0);
+            if (first >= last) break;
+            const bool have = first + lane < last;
+            hull_walk(g, have, have ? order[first + lane] : 0, G,
+                      [&](int voxel, bool timed) {
+                          const unsigned local = (unsigned)(voxel - base);
+                          if (timed && local < (unsigned)voxels) atomicAdd(window + (local >> 1), (local & 1) ? 0x10000u : 1u);
+                          else hull_mark(im, mask, voxel, 1);
+                      },
+                      counters);
+        }
+        __syncthreads();
+        for (int k = threadIdx.x; k < words; k += blockDim.x) {
+            const unsigned both = window[k];
+            if (both == 0) continue;
+            window[k] = 0;
+            if (both & 0xffffu) hull_mark(im, mask, base + 2 * k, both & 0xffffu);
+            if (both >> 16) hull_mark(im, mask, base + 2 * k + 1, both >> 16);
+        }
+        p = last;
+    }
 }
 
 // MSC_edge_detection_GPU (B.cu:6911-6956), out of place: 3x3 maximum difference over the
@@ -1320,13 +1487,13 @@ __device__ __forceinline__ bool find_endpoint(const PreGeom& g, const uint32_t* 
                           (double)powf((float)tan_xz, -1.0f), tanf((float)xy_angle) / tan_xz};
     };
     bool hit_hull = false;
-    auto visit = [&](int voxel, bool step) {
+    auto visit = [&](int voxel, bool step, bool) {
         const bool hit = step && ((__ldg(bits + (voxel >> 5)) >> (voxel & 31)) & 1u);
         hit_hull = hit_hull || hit;
         return hit;
     };
     bool done = !have || walk_outside(g, w);
-    if (!done) done = visit(w.voxel, true);
+    if (!done) done = visit(w.voxel, true, false);
     // every pass moves one index monotonically, so the walk leaves the grid within this bound
     const int max_steps = 2 * (g.columns + g.rows + g.slices) + 16;
     // slopes: tan in double, powf of a float within 4 units in the last place (5.4e-7 with the float's own
@@ -1373,7 +1540,7 @@ __device__ __forceinline__ bool find_endpoint(const PreGeom& g, const uint32_t* 
             }
             w.voxel = w.vx + w.vy * g.columns + w.vz * g.columns * g.rows;
             done = walk_outside(g, w);
-            if (!done) done = visit(w.voxel, true);
+            if (!done) done = visit(w.voxel, true, false);
         }
         axis = kAxisNone;
     } else if (hit_hull && axis != kAxisNone) {
@@ -1516,7 +1683,8 @@ pct_status ensure_fixed(pct_ctx* ctx, Preproc* p)
     if (e == cudaSuccess) e = alloc(p->SM_counts, nv);
     if (e == cudaSuccess) e = alloc(p->SM_differences, nv);
     if (e == cudaSuccess) e = alloc(p->edge_tmp, nv);
-    if (e == cudaSuccess) e = alloc(p->walk_hist, 2 * pct::kWalkKeys);
+    if (e == cudaSuccess) e = alloc(p->walk_hist, 2 * pct::kHullKeys);
+    if (e == cudaSuccess) e = alloc(p->hull_starts, pct::sm_count() + 1);
     if (e == cudaSuccess) e = alloc(p->hull_bits, (nv + 31) / 32);
     if (e == cudaSuccess) e = alloc(p->SM_thresholds, ctx->cfg.SLICES);
     const long long bins_tv = (long long)ctx->cfg.T_BINS * ctx->cfg.V_BINS;
@@ -1748,12 +1916,28 @@ extern "C" pct_status pct_hull_detection(pct_ctx* ctx)
         if (ctx->cfg.SC_ON || ctx->cfg.MSC_ON || ctx->cfg.SM_ON) {
             st = ensure_scratch(ctx, p, n);
             if (st != PCT_OK) return st;
-            int* order = walk_order(ctx, p, n, p->raw_geom, 1);
-            if (!order) return fail(ctx, PCT_ERR_CUDA, "walk order", cudaGetLastError());
-            pct::hull_walks_kernel<<<pct::grid_for(n, 128), 128, 0, s>>>(
-                g, n, order, G, p->raw_wepl, p->missed, ctx->cfg.SC_ON ? p->SC_hull : nullptr,
-                ctx->cfg.MSC_ON ? p->MSC_counts : nullptr, ctx->cfg.SM_ON ? p->SM_counts : nullptr, ctx->d_counters);
-            ctx->launches += 1;
+            const pct::HullImages im{ctx->cfg.SC_ON ? p->SC_hull : nullptr, ctx->cfg.MSC_ON ? p->MSC_counts : nullptr,
+                                     ctx->cfg.SM_ON ? p->SM_counts : nullptr};
+            const pct::HullPlan plan = pct::hull_plan(g);
+            if (plan.window > 0 && n >= pct::kHullWindowMin) {
+                const int keys = 8 * plan.first * plan.distances, blocks = pct::sm_count();
+                const size_t shared = 4 * ((size_t)plan.window * g.columns * g.rows / 2 + 1);
+                int *key = p->tmp_bin_num, *order = reinterpret_cast<int*>(p->offsets);
+                pct::hull_key_kernel<<<pct::grid_for(n, 256), 256, 0, s>>>(g, plan, n, G, p->raw_wepl, p->missed, im, key);
+                PRE_TRY(pct::bucket_sort_by_key(key, 0, n, keys, p->walk_hist, order, s), "walk order");
+                PRE_TRY(cudaFuncSetAttribute(pct::hull_window_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, pct::kHullWindow + 4),
+                        "hull window");
+                pct::hull_ranges_kernel<<<1, 1024, 0, s>>>(g, plan, p->walk_hist, blocks, p->hull_starts);
+                pct::hull_window_kernel<<<blocks, pct::kHullThreads, shared, s>>>(g, plan, order, key, p->walk_hist + keys,
+                                                                                  p->hull_starts, G, im, ctx->d_counters);
+                ctx->launches += 6;
+            } else {
+                int* order = walk_order(ctx, p, n, p->raw_geom, 1);
+                if (!order) return fail(ctx, PCT_ERR_CUDA, "walk order", cudaGetLastError());
+                pct::hull_walks_kernel<<<pct::grid_for(n, 128), 128, 0, s>>>(g, n, order, G, p->raw_wepl, p->missed, im,
+                                                                             ctx->d_counters);
+                ctx->launches += 1;
+            }
         }
     }
     PRE_TRY(cudaGetLastError(), "hull walk kernels");

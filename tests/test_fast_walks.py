@@ -91,3 +91,26 @@ def test_endpoints_are_identical(columns, slices, n):
     assert n < 1000 or len(out[0]["x_entry_reconstruction"]) > n // 4
     for k in out[0]:
         np.testing.assert_array_equal(out[0][k].view(np.uint32), out[1][k].view(np.uint32), err_msg=k)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("columns,slices,n", [(64, 8, 530001), (200, 12, 600000), (317, 5, 524288), (330, 4, 524288)])
+def test_windowed_counts_are_identical(columns, slices, n):
+    """The hull walk's counts in shared memory (524,288 histories or more): all slices in one window, some,
+    one with an odd number of voxels, and slices too large for one; histories in one to three of the images.
+    Without fast points every mark goes to the images directly."""
+    from pct_reconstruction_b200 import Context
+    p = L.scan_config((columns, columns, slices), 60000, 12, SC_UPPER_THRESHOLD=2.0, MSC_LOWER_THRESHOLD=-10.0,
+                      MSC_UPPER_THRESHOLD=5.0, SM_LOWER_THRESHOLD=1.0)
+    td = scan(Config(**p), n, columns, False)
+    out = []
+    for fast in (1, 0):
+        with Context(Config(**p, EXACT_FAST_POINTS=fast)) as ctx:
+            ctx.load_tracker_data(td)
+            for stage in ("recon_volume_intersections", "binning", "hull_detection"):
+                ctx.stage(stage)
+            out.append({k: ctx.get_array(k) for k in ("SC_hull", "MSC_counts", "SM_counts")})
+    a, b = out
+    assert (a["SC_hull"] == 0).any() and a["MSC_counts"].max() > 1 and a["SM_counts"].max() > 1
+    for k in a:
+        np.testing.assert_array_equal(a[k], b[k], err_msg=k)
