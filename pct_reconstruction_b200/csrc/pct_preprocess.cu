@@ -876,8 +876,8 @@ __device__ void take_2D_step(const PreGeom& g, int xd, int yd, double dy_dx, dou
 //    step waits for that.
 // The voxels visited are the reference's either way (EXACT_FAST_POINTS = 0 takes every step by the
 // reference's code).  On the head scan the end points of 3.3M histories took 5.74 ms with the reference's
-// steps and take 3.20 ms, bound by instruction issue; a warp's walks differ in length, so 12 of its 32
-// lanes step on average.
+// steps and take 2.53 ms, half of it the walks' setup (trigonometry, divisions), half the steps; a warp's
+// walks differ in length, so 12 of its 32 lanes step on average.
 enum WalkAxis { kAxisX = 0, kAxisY = 1, kAxisZ = 2, kAxisNone = 3 };
 struct WalkLine {
     double x0, y0, z0;
@@ -925,21 +925,21 @@ struct CrossingTimes {
     unsigned tx, ty, tz, bx, by, bz;  // next crossings and their spacing
     int ix, iy, iz;                   // voxel index increments
     unsigned stop;         // from here on a crossing may leave the grid
-    unsigned lead, lead_y; // by which a crossing decides (lead_y where y is involved)
+    unsigned lead;         // by which a crossing decides
     int exit_axis;         // the crossing that leaves the grid (kAxisNone: through its top)
 };
 
-// w: the walk's initial state; |dx|, |dy|, |dz|: the line's direction.  `error` and `error_y` (where y is
-// involved): how far the reference's crossing times can be off, relative to the walk's length (its slopes'
-// relative errors); to that come the roundings of its coordinates (1e-13 cm) and of the fixed point
+// w: the walk's initial state; |dx|, |dy|, |dz|: the line's direction.  `error`: how far the reference's
+// crossing times can be off, relative to the walk's length (its slopes' relative errors); to that come the roundings of its coordinates (1e-13 cm) and of the fixed point
 // (half a unit of 2^-30 of the walk per crossing).  False where the line is too close to a coordinate
 // plane for the times to be of use.
 __device__ __forceinline__ bool crossing_times(const PreGeom& g, const WalkLine& l, const WalkState& w, double dx, double dy,
-                                               double dz, double error, double error_y, CrossingTimes& c)
+                                               double dz, double error, CrossingTimes& c)
 {
     if (!g.fast_walks || l.xd == 0 || l.yd == 0 || l.zd == 0 || !(dx > 1e-9) || !(dy > 1e-9) || !(dz > 1e-9) ||
-        !(error_y < 0.05) || !(dx < 1e9 && dy < 1e9 && dz < 1e9))
+        !(error < 0.05) || !(dx < 1e9 && dy < 1e9 && dz < 1e9))
         return false;
+    if (g.columns < 2 || g.rows < 2) return false;  // index increments tell the axes
     // a start beyond the grid's zero corner has the mirrored index: its first planes lie behind it
     if (w.x < -g.R || w.y > g.R || w.z > g.H / 2) return false;
     const double rx = 1.0 / dx, ry = 1.0 / dy, rz = 1.0 / dz;
@@ -964,9 +964,8 @@ __device__ __forceinline__ bool crossing_times(const PreGeom& g, const WalkLine&
     c.iz = -l.zd * g.columns * g.rows;
     const double roundings = 1.0e-13 * fmax(fmax(rx, ry), rz) * unit + max(max(nx, ny), nz) + 8.0;
     c.lead = (unsigned)fmin(roundings + error * 1073741824.0, 1.0e9);
-    c.lead_y = (unsigned)fmin(roundings + error_y * 1073741824.0, 1.0e9);
-    if (c.lead_y > min(min(c.bx, c.by), c.bz) / 8) return false;  // also tells the last crossing from the one before
-    const double leave = 1073741824.0 - 2.0 * c.lead_y;
+    if (c.lead > min(min(c.bx, c.by), c.bz) / 8) return false;  // also tells the last crossing from the one before
+    const double leave = 1073741824.0 - 2.0 * c.lead;
     c.stop = leave > 0.0 ? (unsigned)leave : 0u;
     c.exit_axis = ex == end ? kAxisX : ey == end ? kAxisY : l.zd > 0 ? kAxisNone : kAxisZ;
     return true;
@@ -985,35 +984,53 @@ __device__ __forceinline__ int walk_3D(const PreGeom& g, const WalkLine& l, cons
 {
     CrossingTimes c = times;
     const int vx0 = w.vx, vy0 = w.vy, vz0 = w.vz;
-    int voxel = w.voxel, axis = kAxisNone, extra = 0;  // extra: steps that did not move one index
+    int voxel = w.voxel, before = voxel, extra = 0;  // before: the last step; extra: steps that did not move one index
     bool left = false;
     limit = false;
     const bool walked = !done;
-    if (done) voxel = 0;  // any index that may be looked at
+    if (done) voxel = before = 0;  // any index that may be looked at
+    // a step that is not certain leaves its lane as it is, and so does every step after it, until the
+    // reference's step below has been taken; a lane that is done has stop = 0
+    if (done || !fast) c.stop = 0;
+    auto last_axis = [&]() {
+        const int d = voxel - before;
+        return d == 0 ? kAxisNone : d == c.ix ? kAxisX : d == c.iy ? kAxisY : kAxisZ;
+    };
     for (;;) {
-        bool stuck = !fast && !done;
+        bool stuck;
         do {
 #pragma unroll
             for (int k = 0; k < 4; k++) {
-                const unsigned t = min(min(c.tx, c.ty), c.tz);
-                const unsigned far_y = t + c.lead_y, far = c.ty == t ? far_y : t + c.lead;
-                const bool px = c.tx <= far, py = c.ty <= far_y, pz = c.tz <= far;
-                stuck = stuck || (!done && ((px && py) || (px && pz) || (py && pz) || t >= c.stop));
-                const bool go = !stuck && !done;
-                c.tx += go && px ? c.bx : 0u;
-                c.ty += go && py ? c.by : 0u;
-                c.tz += go && pz ? c.bz : 0u;
-                voxel += go ? (px ? c.ix : py ? c.iy : c.iz) : 0;
-                axis = go ? (px ? kAxisX : py ? kAxisY : kAxisZ) : axis;
-                done = visit(voxel, go, true) || done;
+                const unsigned t = min(min(c.tx, c.ty), c.tz), far = t + c.lead;
+                const bool px = c.tx <= far, py = c.ty <= far, pz = c.tz <= far;
+                const bool go = !((px && py) || (px && pz) || (py && pz) || t >= c.stop);
+                if (go) before = voxel;
+                if (go && px) {
+                    c.tx += c.bx;
+                    voxel += c.ix;
+                }
+                if (go && py) {
+                    c.ty += c.by;
+                    voxel += c.iy;
+                }
+                if (go && pz) {
+                    c.tz += c.bz;
+                    voxel += c.iz;
+                }
+                if (visit(voxel, go, true)) {
+                    done = true;
+                    c.stop = 0;
+                }
+                stuck = !go && !done;
             }
         } while (!__any_sync(0xffffffffu, stuck) && __any_sync(0xffffffffu, !done));
         if (stuck && fast) {
             // a crossing that is certain and leaves the grid (not through its top) ends the walk here
-            const unsigned t = min(min(c.tx, c.ty), c.tz), far_y = t + c.lead_y, far = c.ty == t ? far_y : t + c.lead;
-            const bool px = c.tx <= far, py = c.ty <= far_y, pz = c.tz <= far;
-            if (px + py + pz == 1 && (px ? kAxisX : py ? kAxisY : kAxisZ) == c.exit_axis && t + c.lead_y >= 1073741824u) {
+            const unsigned t = min(min(c.tx, c.ty), c.tz), far = t + c.lead;
+            const bool px = c.tx <= far, py = c.ty <= far, pz = c.tz <= far;
+            if (px + py + pz == 1 && (px ? kAxisX : py ? kAxisY : kAxisZ) == c.exit_axis && far >= 1073741824u) {
                 left = done = true;
+                c.stop = 0;
                 stuck = false;
             }
         }
@@ -1023,9 +1040,9 @@ __device__ __forceinline__ int walk_3D(const PreGeom& g, const WalkLine& l, cons
             w.vz = voxel / slab;
             w.vy = (voxel - w.vz * slab) / g.columns;
             w.vx = voxel - w.vz * slab - w.vy * g.columns;
+            int axis = last_axis(), moved;
             face_position(g, l, m, axis, w);
             face_distances(g, l, axis, w);
-            int moved;
             do {
                 // near the grid's end every step is the reference's: beyond its top the slice index is
                 // clamped, and the coordinates no longer follow from the last face
@@ -1047,7 +1064,8 @@ __device__ __forceinline__ int walk_3D(const PreGeom& g, const WalkLine& l, cons
                 }
                 // a step across one face can be set up again from that face, one across an edge cannot
             } while (!done && (moved != 1 || !fast));
-            if (done) axis = kAxisNone;
+            before = done ? voxel : voxel - (axis == kAxisX ? c.ix : axis == kAxisY ? c.iy : c.iz);
+            if (done || !fast) c.stop = 0;
         }
         __syncwarp();
         if (!__any_sync(0xffffffffu, !done)) break;
@@ -1059,7 +1077,7 @@ __device__ __forceinline__ int walk_3D(const PreGeom& g, const WalkLine& l, cons
         w.vx = voxel - w.vz * slab - w.vy * g.columns;
         w.voxel = voxel;
     }
-    return axis;
+    return last_axis();
 }
 
 // Processing order of the voxel walks.  A history's walk lengths depend on where its line crosses
@@ -1160,7 +1178,7 @@ __device__ __forceinline__ void hull_walk(const PreGeom& g, bool have, long long
     CrossingTimes times{};
     const bool flat = l.zd == 0;
     const bool fast = !done && !flat && crossing_times(g, l, w, fabs((double)dx), fabs((double)dy), fabs((double)dz), 5.0e-7,
-                                                       5.0e-7, times);
+                                                       times);
     bool limit;
     walk_3D(g, l, times, fast, done || flat, slopes, mark, max_steps, w, limit);
     if (flat && !done) {
@@ -1196,8 +1214,9 @@ __global__ void __launch_bounds__(128) hull_walks_kernel(PreGeom g, long long n,
 // changes.  The histories are sorted by (mask, first slice they touch, distance from the axis); a CTA
 // takes a contiguous range of them, and the ranges cost the same by the chords' lengths.  Marks
 // outside the window, and those of the reference's own steps, go to the images directly.
-// On the head scan (4M histories, 650M marks, windows of two slices) 1.75 ms against 4.21 ms with every
-// mark in L2, bound by the walks' instructions; 512 threads take 1.97 ms, 1024 (which spill) 1.74 ms.  The
+// On the head scan (4M histories, 650M marks, windows of two slices) 1.61 ms against 4.21 ms with every
+// mark in L2, bound by the walks' instructions; before the steps were shortened 768 threads took 1.75 ms,
+// 512 1.97 and 1024 (which spill) 1.74.  The
 // sort by more keys and the ranges take 65 us where the other walk's order takes 30, so few histories
 // stay with that (300,000 with few marks: 71 us against 45).
 constexpr long long kHullWindowMin = 1 << 19;
@@ -1505,7 +1524,7 @@ __device__ __forceinline__ bool find_endpoint(const PreGeom& g, const uint32_t* 
     const double turn = 1.2e-7 * fabs(xy_angle) + 1.0e-7;
     // an elevation beyond a right angle moves z against its own direction: left to the reference's steps
     const bool forward = (tan_xy > 0) == (l.xd * l.yd > 0) && (tan_xz > 0) == (l.xd * l.zd > 0);
-    const bool fast = !done && !flat && forward && crossing_times(g, l, w, scale, a_xy * scale, a_xz * scale, 1.2e-6,
+    const bool fast = !done && !flat && forward && crossing_times(g, l, w, scale, a_xy * scale, a_xz * scale,
                                                        2.4e-6 + turn * (a_xy + 1.0 / a_xy), times);
     bool limit;
     int axis = walk_3D(g, l, times, fast, done || flat, slopes, visit, max_steps - 1, w, limit);
@@ -1557,8 +1576,8 @@ __device__ __forceinline__ bool find_endpoint(const PreGeom& g, const uint32_t* 
     return hit_hull;
 }
 
-// collect_MLP_endpoints_GPU_nobool (B.cu:7819-7854).  Six CTAs per SM: 3.20 ms for 3.3M histories against
-// 4.26 ms with the registers it would take alone (118: four CTAs) and 3.34 ms with eight (which spill).
+// collect_MLP_endpoints_GPU_nobool (B.cu:7819-7854).  Six CTAs per SM: 2.53 ms for 3.3M histories, five
+// 2.63 ms (before the steps were shortened: six 3.20 ms, four 4.26, eight, which spill, 3.34).
 __global__ void __launch_bounds__(128, 6) endpoints_kernel(PreGeom g, long long n, const int* __restrict__ order,
                                                            const uint32_t* __restrict__ hull_bits, GeomPtrs G,
                                                            uint32_t* __restrict__ first_voxel, int* __restrict__ keep)
