@@ -9,11 +9,11 @@
 // Design: the image never leaves HBM.  One repetition is three kinds of launch:
 //   gradient    G (the TV subgradient, gathered per voxel instead of scattered), ||G||^2 and
 //               TV(x), reduced in fixed order by the last block to arrive (no spin waits);
-//   candidates  TV(x - beta_j * G/||G||) for 16 consecutive trial exponents L0+16q .. L0+16q+15
-//               in one pass over x and G; the last block picks the first trial the reference's
-//               loop would accept (TV_y <= TV_x, |TV_y - TV_prev|/TV_y < TV_THRESHOLD, or
-//               L > 300) and records beta and the new L.  Chunks after the accepting one exit at
-//               once, so the chain of launches is fixed and graph-capturable;
+//   candidates  TV(x - beta_j * G/||G||) for consecutive trial exponents, several in one pass over
+//               x and G; the last block picks the first trial the reference's loop would accept
+//               (TV_y <= TV_x, |TV_y - TV_prev|/TV_y < TV_THRESHOLD, or L > 300) and records beta
+//               and the new L.  Launches after the accepting one exit at once, so the chain of
+//               launches is fixed and graph-capturable;
 //   apply       x = x - beta * G/||G|| on hull voxels.
 // The L draw of NTVS (randi, B.cu:11478: uniform in [L_0 + k - 1, L]) uses a seeded
 // splitmix64 hash of (seed, k) instead of the wall clock, so runs are reproducible.
@@ -48,7 +48,7 @@ struct TvsState {
 
 struct TvsDims {
     int C, R;
-    long long nv;
+    int nv;
 };
 
 struct TvsTable {
@@ -65,7 +65,12 @@ struct TvsStep {
 
 constexpr int kTvsThreads = 256;
 constexpr int kTvsWarps = kTvsThreads / 32;
-constexpr int kTvsTrials = 16;
+// Trials per launch.  L carries over from one repetition to the next, so that all but an image's first
+// repetition accept one of the first trials: the first launches are short (4 trials take 23 us on 200x200x32
+// voxels, 16 take 80), and the last takes all that are left, 16 in a pass.
+constexpr int kTvsChain[] = {4, 4, 8, 16};
+constexpr int kTvsRest = 16;
+constexpr int kTvsLastL = 300;  // beyond it a trial is always accepted
 
 __host__ __device__ inline int tvs_randi(int lo, int hi, unsigned long long seed, int k)
 {
@@ -85,16 +90,20 @@ __device__ __forceinline__ float eta_at(const TvsTable& t, int L)
 }
 
 // Forward differences at voxel v: gx = x[v+1]-x[v], gy = x[v+C]-x[v].
-__device__ __forceinline__ void forward_diff(const float* __restrict__ x, long long v, int C, float& gx, float& gy)
+__device__ __forceinline__ void forward_diff(const float* __restrict__ x, int v, int C, float& gx, float& gy)
 {
     const float x0 = x[v];
     gx = __fsub_rn(x[v + 1], x0);
     gy = __fsub_rn(x[v + C], x0);
 }
 
+// Flat regions make exact zeros, which the library's roots and quotients take through their slow paths;
+// roots of zero and quotients of zero by a positive number are given here (3 times the time of the rest).
+
 // G_norm = sqrt(pow(G_x, 2) + pow(G_y, 2)) in double, stored as float (B.cu:10266).
 __device__ __forceinline__ float grad_norm(float gx, float gy)
 {
+    if (gx == 0.0f && gy == 0.0f) return 0.0f;
     const double a = (double)gx, b = (double)gy;
     return (float)__dsqrt_rn(__dadd_rn(__dmul_rn(a, a), __dmul_rn(b, b)));
 }
@@ -102,8 +111,12 @@ __device__ __forceinline__ float grad_norm(float gx, float gy)
 // One term of calculate_total_variation (B.cu:10175): sqrt(dy^2 + dx^2) in float.
 __device__ __forceinline__ float tv_term(float dy, float dx)
 {
-    return __fsqrt_rn(__fadd_rn(__fmul_rn(dy, dy), __fmul_rn(dx, dx)));
+    const float s = __fadd_rn(__fmul_rn(dy, dy), __fmul_rn(dx, dx));
+    return s == 0.0f ? s : __fsqrt_rn(s);
 }
+
+// a / b, b positive
+__device__ __forceinline__ float over(float a, float b) { return a == 0.0f ? a : __fdiv_rn(a, b); }
 
 // Sums N doubles over the block in a fixed order; thread 0 gets the totals.
 template <int N>
@@ -129,30 +142,49 @@ __device__ void block_sum(double (&v)[N], double* smem /* [N * kTvsWarps] */)
     __syncthreads();
 }
 
-// Writes this block's N partial sums; returns true in the last block to arrive, after which
-// `totals` holds the grid totals in thread 0 (fixed order: block b's partial at [i*nblocks+b]).
+// Writes this block's N partial sums (fixed order: block b's i-th at [(first + i) * nblocks + b]).
 template <int N>
-__device__ bool grid_sum(double (&v)[N], double* __restrict__ partials, unsigned nblocks, TvsState* st, double* smem)
+__device__ void block_partials(double (&v)[N], double* __restrict__ partials, int first, unsigned nblocks, double* smem)
+{
+    block_sum<N>(v, smem);
+    if (threadIdx.x == 0)
+        for (int i = 0; i < N; i++) partials[(size_t)(first + i) * nblocks + blockIdx.x] = v[i];
+}
+
+// True in the last block to arrive.
+__device__ bool last_block(unsigned nblocks, TvsState* st)
 {
     __shared__ bool last;
-    block_sum<N>(v, smem);
     if (threadIdx.x == 0) {
-        for (int i = 0; i < N; i++) partials[(size_t)i * nblocks + blockIdx.x] = v[i];
         __threadfence();
         last = atomicAdd(&st->arrive, 1u) == nblocks - 1;
+        if (last) st->arrive = 0;
     }
     __syncthreads();
-    if (!last) return false;
-    __threadfence();
+    if (last) __threadfence();
+    return last;
+}
+
+// The grid totals of N sums, in thread 0 of the last block.
+template <int N>
+__device__ void grid_totals(double (&v)[N], const double* __restrict__ partials, int first, unsigned nblocks, double* smem)
+{
 #pragma unroll
     for (int i = 0; i < N; i++) {
         double a = 0.0;
         for (unsigned b = threadIdx.x; b < nblocks; b += kTvsThreads)
-            a += ((volatile double*)partials)[(size_t)i * nblocks + b];
+            a += ((const volatile double*)partials)[(size_t)(first + i) * nblocks + b];
         v[i] = a;
     }
     block_sum<N>(v, smem);
-    if (threadIdx.x == 0) st->arrive = 0;
+}
+
+template <int N>
+__device__ bool grid_sum(double (&v)[N], double* __restrict__ partials, unsigned nblocks, TvsState* st, double* smem)
+{
+    block_partials<N>(v, partials, 0, nblocks, smem);
+    if (!last_block(nblocks, st)) return false;
+    grid_totals<N>(v, partials, 0, nblocks, smem);
     return true;
 }
 
@@ -163,26 +195,28 @@ __global__ void __launch_bounds__(kTvsThreads) tvs_gradient_kernel(const float* 
                                                                  TvsState* st)
 {
     __shared__ double smem[2 * kTvsWarps];
+    allow_dependent_launch();
+    grid_dependency_wait();
     double acc[2] = {0.0, 0.0};  // TV(x), ||G||^2
-    const long long stride = (long long)gridDim.x * kTvsThreads;
-    for (long long v = blockIdx.x * (long long)kTvsThreads + threadIdx.x; v < d.nv; v += stride) {
-        const int c = (int)(v % d.C), r = (int)((v / d.C) % d.R);
+    const unsigned stride = gridDim.x * kTvsThreads;
+    for (unsigned u = blockIdx.x * kTvsThreads + threadIdx.x; u < (unsigned)d.nv; u += stride) {
+        const int v = (int)u, line = v / d.C, c = v - line * d.C, r = line % d.R;
         float g = 0.0f, gx, gy, gn;
         // contributions in the reference's loop order: from v-C (row above), v-1, then v itself
         if (r > 0 && c < d.C - 1) {
             forward_diff(x, v - d.C, d.C, gx, gy);
             gn = grad_norm(gx, gy);
-            if (gn > 0.0f) g = __fadd_rn(g, __fdiv_rn(gy, gn));
+            if (gn > 0.0f) g = __fadd_rn(g, over(gy, gn));
         }
         if (c > 0 && r < d.R - 1) {
             forward_diff(x, v - 1, d.C, gx, gy);
             gn = grad_norm(gx, gy);
-            if (gn > 0.0f) g = __fadd_rn(g, __fdiv_rn(gx, gn));
+            if (gn > 0.0f) g = __fadd_rn(g, over(gx, gn));
         }
         if (c < d.C - 1 && r < d.R - 1) {
             forward_diff(x, v, d.C, gx, gy);
             gn = grad_norm(gx, gy);
-            if (gn > 0.0f) g = __fsub_rn(g, __fdiv_rn(__fadd_rn(gx, gy), gn));
+            if (gn > 0.0f) g = __fsub_rn(g, over(__fadd_rn(gx, gy), gn));
             acc[0] += (double)tv_term(gy, gx);
         }
         G[v] = g;
@@ -206,9 +240,9 @@ __global__ void __launch_bounds__(kTvsThreads) tvs_gradient_kernel(const float* 
 }
 
 // The perturbation direction v = G/||G|| (0 when ||G|| = 0), B.cu:10309-10316.
-__device__ __forceinline__ float direction(const float* __restrict__ G, long long v, float norm)
+__device__ __forceinline__ float direction(const float* __restrict__ G, int v, float norm)
 {
-    return norm != 0.0f ? __fdiv_rn(G[v], norm) : 0.0f;
+    return norm != 0.0f ? over(G[v], norm) : 0.0f;
 }
 
 __device__ __forceinline__ float perturbed(float x, bool in_hull, float beta, float w)
@@ -216,71 +250,89 @@ __device__ __forceinline__ float perturbed(float x, bool in_hull, float beta, fl
     return in_hull ? __fsub_rn(x, __fmul_rn(beta, w)) : x;
 }
 
-// TV of x - beta_j v for trials j = L0 + base .. L0 + base + 15 (the while loop of B.cu:10499).
+// TV of x - beta_j v for the trials j = L0 + base .. L0 + base + kTrials * passes - 1 (the while loop of
+// B.cu:10499).  Every launch sums in the gradient kernel's order, so that a beta that changes nothing
+// gives TV(x) itself.
+template <int kTrials>
 __global__ void __launch_bounds__(kTvsThreads) tvs_trials_kernel(const float* __restrict__ x,
                                                                const float* __restrict__ G,
                                                                const uint8_t* __restrict__ hull, TvsDims d,
-                                                               TvsTable tab, int base, double threshold,
+                                                               TvsTable tab, int base, int passes, double threshold,
                                                                double* __restrict__ partials, unsigned nblocks,
                                                                TvsState* st)
 {
-    __shared__ double smem[kTvsTrials * kTvsWarps];
+    __shared__ double smem[kTrials * kTvsWarps];
+    __shared__ bool accepted;
+    allow_dependent_launch();
+    grid_dependency_wait();
     if (st->done) return;  // uniform across the grid: written by an earlier launch
     const int L0 = st->L0;
     const float norm = st->norm;
-    float beta[kTvsTrials];
+    const unsigned stride = gridDim.x * kTvsThreads;
+    double acc[kTrials];
+    for (int pass = 0; pass < passes; pass++) {
+        float beta[kTrials];
 #pragma unroll
-    for (int j = 0; j < kTvsTrials; j++) beta[j] = eta_at(tab, L0 + base + j);
-    double acc[kTvsTrials];
-#pragma unroll
-    for (int j = 0; j < kTvsTrials; j++) acc[j] = 0.0;
-    const long long stride = (long long)gridDim.x * kTvsThreads;
-    for (long long v = blockIdx.x * (long long)kTvsThreads + threadIdx.x; v < d.nv; v += stride) {
-        const int c = (int)(v % d.C), r = (int)((v / d.C) % d.R);
-        if (c >= d.C - 1 || r >= d.R - 1) continue;
-        const float x0 = x[v], x1 = x[v + 1], x2 = x[v + d.C];
-        const bool h0 = hull[v] != 0, h1 = hull[v + 1] != 0, h2 = hull[v + d.C] != 0;
-        const float w0 = direction(G, v, norm), w1 = direction(G, v + 1, norm), w2 = direction(G, v + d.C, norm);
-#pragma unroll
-        for (int j = 0; j < kTvsTrials; j++) {
-            const float p0 = perturbed(x0, h0, beta[j], w0);
-            const float p1 = perturbed(x1, h1, beta[j], w1);
-            const float p2 = perturbed(x2, h2, beta[j], w2);
-            acc[j] += (double)tv_term(__fsub_rn(p2, p0), __fsub_rn(p1, p0));
+        for (int j = 0; j < kTrials; j++) {
+            beta[j] = eta_at(tab, L0 + base + pass * kTrials + j);
+            acc[j] = 0.0;
         }
-    }
-    if (!grid_sum<kTvsTrials>(acc, partials, nblocks, st, smem)) return;
-    if (threadIdx.x == 0) {
-        double prev = st->tv_prev;
-        for (int j = 0; j < kTvsTrials; j++) {
-            const int L_after = L0 + base + j + 1;  // L++ precedes the test
-            const double tv_y = acc[j];
-            const bool accept =
-                (tv_y <= st->tv_x) || (fabs(tv_y - prev) / tv_y < threshold) || L_after > 300;
-            if (accept) {
-                st->beta = beta[j];
-                st->L = L_after;
-                st->tv_y = tv_y;
-                st->done = 1;
-                break;
+        for (unsigned u = blockIdx.x * kTvsThreads + threadIdx.x; u < (unsigned)d.nv; u += stride) {
+            const int v = (int)u, line = v / d.C, c = v - line * d.C, r = line % d.R;
+            if (c >= d.C - 1 || r >= d.R - 1) continue;
+            const float x0 = x[v], x1 = x[v + 1], x2 = x[v + d.C];
+            const bool h0 = hull[v] != 0, h1 = hull[v + 1] != 0, h2 = hull[v + d.C] != 0;
+            const float w0 = direction(G, v, norm), w1 = direction(G, v + 1, norm), w2 = direction(G, v + d.C, norm);
+#pragma unroll
+            for (int j = 0; j < kTrials; j++) {
+                const float p0 = perturbed(x0, h0, beta[j], w0);
+                const float p1 = perturbed(x1, h1, beta[j], w1);
+                const float p2 = perturbed(x2, h2, beta[j], w2);
+                acc[j] += (double)tv_term(__fsub_rn(p2, p0), __fsub_rn(p1, p0));
             }
-            prev = tv_y;
         }
-        st->tv_prev = prev;
+        block_partials<kTrials>(acc, partials, pass * kTrials, nblocks, smem);
+    }
+    if (!last_block(nblocks, st)) return;
+    for (int pass = 0; pass < passes; pass++) {
+        grid_totals<kTrials>(acc, partials, pass * kTrials, nblocks, smem);
+        if (threadIdx.x == 0) {
+            double prev = st->tv_prev;
+            bool accept = false;
+            for (int j = 0; j < kTrials && !accept; j++) {
+                const int L_after = L0 + base + pass * kTrials + j + 1;  // L++ precedes the test
+                const double tv_y = acc[j];
+                accept = (tv_y <= st->tv_x) || (fabs(tv_y - prev) / tv_y < threshold) || L_after > kTvsLastL;
+                if (accept) {
+                    st->beta = eta_at(tab, L_after - 1);
+                    st->L = L_after;
+                    st->tv_y = tv_y;
+                    st->done = 1;
+                } else {
+                    prev = tv_y;
+                }
+            }
+            st->tv_prev = prev;
+            accepted = accept;
+        }
+        __syncthreads();
+        if (accepted) return;
     }
 }
 
 // image = x_TVS - beta v on hull voxels (apply_TVS_perturbation B.cu:10413).
 __global__ void tvs_apply_kernel(float* __restrict__ x, const float* __restrict__ G, const uint8_t* __restrict__ hull,
-                                 long long nv, const TvsState* __restrict__ st, unsigned long long* counters)
+                                 int nv, const TvsState* __restrict__ st, unsigned long long* counters)
 {
+    allow_dependent_launch();
+    grid_dependency_wait();
     if (!st->done) {  // no trial accepted (cannot happen: beta = 0 is always accepted)
         if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&counters[kCntWaitExpired], 1ull);
         return;
     }
     const float beta = st->beta, norm = st->norm;
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < nv; v += stride)
+    const unsigned stride = gridDim.x * blockDim.x;
+    for (unsigned v = blockIdx.x * blockDim.x + threadIdx.x; v < (unsigned)nv; v += stride)
         if (hull[v]) x[v] = __fsub_rn(x[v], __fmul_rn(beta, direction(G, v, norm)));
 }
 
@@ -292,9 +344,9 @@ __global__ void __launch_bounds__(kTvsThreads) tvs_total_variation_kernel(const 
 {
     __shared__ double smem[kTvsWarps];
     double acc[1] = {0.0};
-    const long long stride = (long long)gridDim.x * kTvsThreads;
-    for (long long v = blockIdx.x * (long long)kTvsThreads + threadIdx.x; v < d.nv; v += stride) {
-        const int c = (int)(v % d.C), r = (int)((v / d.C) % d.R);
+    const unsigned stride = gridDim.x * kTvsThreads;
+    for (unsigned u = blockIdx.x * kTvsThreads + threadIdx.x; u < (unsigned)d.nv; u += stride) {
+        const int v = (int)u, line = v / d.C, c = v - line * d.C, r = line % d.R;
         if (c >= d.C - 1 || r >= d.R - 1) continue;
         float gx, gy;
         forward_diff(x, v, d.C, gx, gy);
@@ -328,6 +380,7 @@ struct pct_tvs {
     double* partials = nullptr;
     double* scalar = nullptr;
     int eta_len = 0;  // TVS_ETA_SEQUENCE_LENGTH - L_0 filled entries
+    int passes = 0;   // of the launch with the rest of the trials
     unsigned blocks = 0;
 };
 
@@ -357,7 +410,7 @@ pct_status tvs_fail(pct_ctx* ctx, pct_status s, const std::string& what, cudaErr
 
 pct::TvsDims dims_of(const pct_ctx* ctx)
 {
-    return pct::TvsDims{ctx->cfg.COLUMNS, ctx->cfg.ROWS, (long long)ctx->cfg.NUM_VOXELS};
+    return pct::TvsDims{ctx->cfg.COLUMNS, ctx->cfg.ROWS, ctx->cfg.NUM_VOXELS};
 }
 
 // Lazily allocates the TVS buffers and the beta table (generate_TVS_eta_sequence B.cu:10149).
@@ -375,10 +428,18 @@ pct_status ensure_tvs(pct_ctx* ctx)
     const long long nv = c.NUM_VOXELS;
     long long b = (nv + pct::kTvsThreads - 1) / pct::kTvsThreads;
     t->blocks = (unsigned)(b < 1 ? 1 : b > 148 * 4 ? 148 * 4 : b);
+    // trials until beta = 0 (past the table), which is always accepted, or until L passes kTvsLastL
+    int trials = t->eta_len + 1 < pct::kTvsLastL + 1 ? t->eta_len + 1 : pct::kTvsLastL + 1, most = 0;
+    for (int n : pct::kTvsChain) {
+        trials -= n;
+        most = n > most ? n : most;
+    }
+    t->passes = trials > 0 ? (trials + pct::kTvsRest - 1) / pct::kTvsRest : 0;
+    if (most < t->passes * pct::kTvsRest) most = t->passes * pct::kTvsRest;
     cudaError_t e = cudaMalloc(&t->st, sizeof(pct::TvsState));
     if (e == cudaSuccess) e = cudaMalloc(&t->G, sizeof(float) * (size_t)nv);
     if (e == cudaSuccess) e = cudaMalloc(&t->eta, sizeof(float) * (eta.empty() ? 1 : eta.size()));
-    if (e == cudaSuccess) e = cudaMalloc(&t->partials, sizeof(double) * (size_t)pct::kTvsTrials * t->blocks);
+    if (e == cudaSuccess) e = cudaMalloc(&t->partials, sizeof(double) * (size_t)most * t->blocks);
     if (e == cudaSuccess) e = cudaMalloc(&t->scalar, sizeof(double));
     if (e == cudaSuccess && !eta.empty())
         e = cudaMemcpyAsync(t->eta, eta.data(), sizeof(float) * eta.size(), cudaMemcpyHostToDevice, ctx->stream);
@@ -432,26 +493,31 @@ extern "C" pct_status pct_ntvs_iteration(pct_ctx* ctx, int iteration)
     const bool ntvs = !c.TVS_OLD;                            // NTVS_ON = TVS_ON && !TVS_OLD
     const int reps = c.TVS_OLD ? 1 : c.TVS_REPETITIONS;      // TVS_OLD: TVS_REPETITIONS = 1
     const bool conditioned = c.TVS_CONDITIONED != 0;
-    // Trials until beta = 0 (past the table) is reached, which is always accepted.
-    const int trial_chunks = (t->eta_len + 1 + pct::kTvsTrials - 1) / pct::kTvsTrials + 1;
     cudaStream_t st = ctx->stream;
     long long launches = 0;
+    cudaError_t e = cudaSuccess;
+    // every kernel but the first starts while the one before it ends, and waits for it
+    auto launch = [&](auto kernel, auto... args) {
+        if (e == cudaSuccess) e = pct::launch_kernel(launches > 0, kernel, t->blocks, pct::kTvsThreads, st, args...);
+        launches++;
+    };
     for (int n = 0; n < reps; n++) {
         const pct::TvsStep step{(ntvs && n == 0) ? 1 : 0, iteration, conditioned ? 0 : 1, (long long)c.TVS_SEED};
-        pct::tvs_gradient_kernel<<<t->blocks, pct::kTvsThreads, 0, st>>>(ctx->d_x, t->G, d, tab, step, t->partials,
-                                                                          t->blocks, t->st);
-        launches++;
-        if (conditioned)
-            for (int q = 0; q < trial_chunks; q++) {
-                pct::tvs_trials_kernel<<<t->blocks, pct::kTvsThreads, 0, st>>>(
-                    ctx->d_x, t->G, hull, d, tab, q * pct::kTvsTrials, c.TV_THRESHOLD, t->partials, t->blocks, t->st);
-                launches++;
+        launch(pct::tvs_gradient_kernel, ctx->d_x, t->G, d, tab, step, t->partials, t->blocks, t->st);
+        if (conditioned) {
+            int base = 0;
+            for (int trials : pct::kTvsChain) {
+                const auto kernel = trials == 4 ? pct::tvs_trials_kernel<4> : trials == 8 ? pct::tvs_trials_kernel<8> : pct::tvs_trials_kernel<16>;
+                launch(kernel, ctx->d_x, t->G, hull, d, tab, base, 1, c.TV_THRESHOLD, t->partials, t->blocks, t->st);
+                base += trials;
             }
-        pct::tvs_apply_kernel<<<t->blocks, pct::kTvsThreads, 0, st>>>(ctx->d_x, t->G, hull, d.nv, t->st,
-                                                                       ctx->d_counters);
-        launches++;
+            if (t->passes > 0)
+                launch(pct::tvs_trials_kernel<pct::kTvsRest>, ctx->d_x, t->G, hull, d, tab, base, t->passes, c.TV_THRESHOLD,
+                       t->partials, t->blocks, t->st);
+        }
+        launch(pct::tvs_apply_kernel, ctx->d_x, t->G, hull, d.nv, t->st, ctx->d_counters);
     }
-    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) return tvs_fail(ctx, PCT_ERR_CUDA, "NTVS kernels", e);
     ctx->launches += launches;
     return PCT_OK;
