@@ -258,8 +258,10 @@ __global__ void __launch_bounds__(kThreads, PCT_PHASE1_MIN_BLOCKS * 128 / kThrea
     path_n[perm[i]] = n;
 }
 
-// Without a table (reference-order points, or a grid too large for the fixed-point positions).
-template <int kThreads>
+// Without a table: reference-order points, or (kTryFast) a grid too large for the fixed-point positions.
+// Without the certain points' code in it, reference-order points take 10.11 ms for 3M head histories (11.04
+// with it, chosen at run time; 10.46 with 6 CTAs per SM, 10.22 with 8).
+template <int kThreads, bool kTryFast>
 __global__ void __launch_bounds__(kThreads, 7 * 128 / kThreads) mlp_phase1_exact_kernel(
     Geometry g, Tables tab, const StepConst* __restrict__ steps, int kmax, HistorySoA h, const int* __restrict__ perm,
     long long count, const long long* __restrict__ offsets, long long offset_base, const int* __restrict__ bounds,
@@ -275,7 +277,7 @@ __global__ void __launch_bounds__(kThreads, 7 * 128 / kThreads) mlp_phase1_exact
         return;
     }
     uint32_t* out = paths + (offsets[i] - offset_base);
-    const WalkResult r = mlp_walk_exact<false>(
+    const WalkResult r = mlp_walk_exact<false, kTryFast>(
         g, tab, steps, kmax, nullptr, __ldg(h.first_MLP_voxel + i), __ldg(h.x_entry + i), __ldg(h.y_entry + i),
         __ldg(h.z_entry + i), __ldg(h.x_exit + i), __ldg(h.y_exit + i), __ldg(h.z_exit + i),
         __ldg(h.xy_entry_angle + i), __ldg(h.xz_entry_angle + i), __ldg(h.xy_exit_angle + i),
@@ -772,9 +774,12 @@ cudaError_t launch_mlp_phase1_exact(const Geometry& g, const Tables& tab, const 
         else if (g.mixed_precision)                                                                               \
             mlp_phase1_mixed_kernel<T><<<blocks, T, 0, stream>>>(g, tab, steps, kmax, h, perm, count, offsets,    \
                                                                  offset_base, bounds, paths, path_n, chord, counters); \
+        else if (g.exact_fast_points)                                                                             \
+            mlp_phase1_exact_kernel<T, true><<<blocks, T, 0, stream>>>(                                           \
+                g, tab, steps, kmax, h, perm, count, offsets, offset_base, bounds, paths, path_n, chord, counters); \
         else                                                                                                      \
-            mlp_phase1_exact_kernel<T><<<blocks, T, 0, stream>>>(g, tab, steps, kmax, h, perm, count, offsets,    \
-                                                                 offset_base, bounds, paths, path_n, chord, counters); \
+            mlp_phase1_exact_kernel<T, false><<<blocks, T, 0, stream>>>(                                          \
+                g, tab, steps, kmax, h, perm, count, offsets, offset_base, bounds, paths, path_n, chord, counters); \
     } while (0)
     if (g.path_cta_threads == 64) PCT_PHASE1(64);
     else if (g.path_cta_threads == 256) PCT_PHASE1(256);
@@ -829,8 +834,10 @@ cudaError_t set_iteration_carveout()
     const int percent = PCT_ITERATION_CARVEOUT;
     if (percent < 0) return cudaSuccess;
     const void* kernels[] = {
-        (const void*)mlp_phase1_exact_kernel<64>, (const void*)mlp_phase1_exact_kernel<128>,
-        (const void*)mlp_phase1_exact_kernel<256>, (const void*)mlp_phase1_table_kernel<64>,
+        (const void*)mlp_phase1_exact_kernel<64, false>, (const void*)mlp_phase1_exact_kernel<128, false>,
+        (const void*)mlp_phase1_exact_kernel<256, false>, (const void*)mlp_phase1_exact_kernel<64, true>,
+        (const void*)mlp_phase1_exact_kernel<128, true>, (const void*)mlp_phase1_exact_kernel<256, true>,
+        (const void*)mlp_phase1_table_kernel<64>,
         (const void*)mlp_phase1_table_kernel<128>, (const void*)mlp_phase1_table_kernel<256>,
         (const void*)mlp_phase1_mixed_kernel<64>, (const void*)mlp_phase1_mixed_kernel<128>,
         (const void*)mlp_phase1_mixed_kernel<256>,

@@ -426,8 +426,9 @@ struct PathWriter {
 
 // One history's MLP.  emit(j, voxel) is called for every path entry j in order.  With kSumX the
 // walk also sums the padded image x over the path (reads beyond it are reported and count as 0);
-// without it x is not touched (the voxel list does not depend on the image).
-template <bool kSumX, class Emit>
+// without it x is not touched (the voxel list does not depend on the image).  kTryFast: with
+// EXACT_FAST_POINTS, points whose voxel is certain skip the reference's order of operations.
+template <bool kSumX, bool kTryFast = true, class Emit>
 __device__ __forceinline__ WalkResult mlp_walk_exact(const Geometry& g, const Tables& tab,
                                                      const StepConst* __restrict__ steps, int kmax,
                                                      const float* __restrict__ x, uint32_t first_MLP_voxel,
@@ -459,7 +460,7 @@ __device__ __forceinline__ WalkResult mlp_walk_exact(const Geometry& g, const Ta
         const Sigma2 m2 = sigma2_moments(m.h, st, tab.scattering_table, sigma_2_index);
         u_shifted += s;
         uint32_t voxel;
-        if (!(g.exact_fast_points &&
+        if (!(kTryFast && g.exact_fast_points &&
               mlp_point_fast(g, m.h, st, m2.sigma_t2, m2.sigma_t2_theta2, m2.sigma_theta2,
                              m2.determinant, depth_2_go, u_shifted, voxel))) {
             double t_1, v_1;
