@@ -356,7 +356,15 @@ __global__ void __launch_bounds__(kThreads, PCT_PHASE1_MIXED_MIN_BLOCKS * 128 / 
 // unbounded): the kernel is bound by the latency of its L2 reductions, so it keeps the warps per
 // SM of the plain instantiations (39 registers, 6 CTAs).  A minimum of 0 leaves the others as
 // they are (a minimum of 1 moves them to 48 registers).
-constexpr int kRegEntries = 8;
+//
+// kMany: blocks of many histories, where warps that wait for the L2 are replaced by others rather than by
+// loads ahead.  Measured, ms per iteration of 4M head histories in blocks of 60000 (2M for FP32 updates;
+// 1M in blocks of 10000 / 3200 in brackets):
+//   double updates: 4 entries in registers (32, 8 CTAs) 6.39, 8 entries 6.56 (2.603, 2.595 / 3.99, 3.79)
+//   FP32 updates:   8 CTAs per SM 3.17, 6 CTAs 3.28 (2.463, 2.524 / 3.86, 3.70)
+// Small blocks keep the entries that are loaded before the wait.  The lines: double updates from 256
+// histories per SM (1M in blocks of 20000: 2.211 with 4 entries, 2.205 with 8), FP32 from 64.
+constexpr int kManyDouble = 256, kManyFloat = 64;
 
 // TwoSum (Knuth): s = RN(a + b) and the exact error e with a + b = s + e, six float operations.
 __device__ __forceinline__ float two_sum(float a, float b, float& e)
@@ -367,14 +375,15 @@ __device__ __forceinline__ float two_sum(float a, float b, float& e)
     return s;
 }
 
-template <int kAlgo, bool kDet, int kMixed, bool kSCurve = false>
-__global__ void __launch_bounds__(256, kSCurve ? 6 : 0) drop_phase2_kernel(Geometry g, const float* __restrict__ x, float2* __restrict__ acc,
+template <int kAlgo, bool kDet, int kMixed, bool kSCurve = false, bool kMany = false>
+__global__ void __launch_bounds__(256, kSCurve ? 6 : kMany && kMixed ? 8 : 0) drop_phase2_kernel(Geometry g, const float* __restrict__ x, float2* __restrict__ acc,
                                                           float* __restrict__ normA, FixedAcc fx,
                                                           const float* __restrict__ WEPL,
                                                           const long long* __restrict__ offsets, long long offset_base,
                                                           const uint32_t* __restrict__ paths, const int* __restrict__ path_n,
                                                           const double* __restrict__ chord, long long begin, long long count)
 {
+    constexpr int kRegEntries = kMany && !kMixed ? 4 : 8;
     allow_dependent_launch();
     const long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
@@ -797,24 +806,27 @@ cudaError_t launch_drop_phase2(const Geometry& g, const float* x, float2* acc, f
     const int threads = 256;
     const unsigned blocks = (unsigned)((count * 32 + threads - 1) / threads);
     cudaError_t e = cudaSuccess;
-#define PCT_PHASE2(ALGO, DET, MIXED, SC)                                                                    \
-    e = launch_kernel(pdl, drop_phase2_kernel<ALGO, DET, MIXED, SC>, blocks, threads, stream, g, x, acc, normA, \
-                      fx, WEPL, offsets, offset_base, paths, path_n, chord, begin, count)
+#define PCT_PHASE2(ALGO, DET, MIXED, SC, MANY)                                                              \
+    e = launch_kernel(pdl, drop_phase2_kernel<ALGO, DET, MIXED, SC, MANY>, blocks, threads, stream, g, x, acc,  \
+                      normA, fx, WEPL, offsets, offset_base, paths, path_n, chord, begin, count)
+    const bool many = count >= (long long)sm_count() * (g.mixed_precision ? kManyFloat : kManyDouble);
     if (g.projection_algorithm == PCT_ROBUSTA) {
-        if (g.deterministic) PCT_PHASE2(PCT_ROBUSTA, true, 0, false);
-        else PCT_PHASE2(PCT_ROBUSTA, false, 0, false);
+        if (g.deterministic) PCT_PHASE2(PCT_ROBUSTA, true, 0, false, false);
+        else PCT_PHASE2(PCT_ROBUSTA, false, 0, false, false);
     } else if (g.projection_algorithm == PCT_ROBUSTB) {
-        PCT_PHASE2(PCT_ROBUSTB, false, 0, false);
+        PCT_PHASE2(PCT_ROBUSTB, false, 0, false, false);
     } else if (g.mixed_precision) {
-        if (g.deterministic) PCT_PHASE2(PCT_DROP, true, 1, false);  // fixed-point sums need no compensation
-        else if (g.compensated) PCT_PHASE2(PCT_DROP, false, 2, false);
-        else PCT_PHASE2(PCT_DROP, false, 1, false);
+        if (g.deterministic) PCT_PHASE2(PCT_DROP, true, 1, false, false);  // fixed-point sums need no compensation
+        else if (g.compensated) PCT_PHASE2(PCT_DROP, false, 2, false, false);
+        else if (many) PCT_PHASE2(PCT_DROP, false, 1, false, true);
+        else PCT_PHASE2(PCT_DROP, false, 1, false, false);
     } else if (g.s_curve) {
-        if (g.deterministic) PCT_PHASE2(PCT_DROP, true, 0, true);
-        else PCT_PHASE2(PCT_DROP, false, 0, true);
+        if (g.deterministic) PCT_PHASE2(PCT_DROP, true, 0, true, false);
+        else PCT_PHASE2(PCT_DROP, false, 0, true, false);
     } else {
-        if (g.deterministic) PCT_PHASE2(PCT_DROP, true, 0, false);
-        else PCT_PHASE2(PCT_DROP, false, 0, false);
+        if (g.deterministic) PCT_PHASE2(PCT_DROP, true, 0, false, false);
+        else if (many) PCT_PHASE2(PCT_DROP, false, 0, false, true);
+        else PCT_PHASE2(PCT_DROP, false, 0, false, false);
     }
 #undef PCT_PHASE2
     return e;
@@ -846,7 +858,9 @@ cudaError_t set_iteration_carveout()
         (const void*)drop_phase2_kernel<PCT_DROP, false, 2>,
         (const void*)drop_phase2_kernel<PCT_ROBUSTA, false, 0>, (const void*)drop_phase2_kernel<PCT_ROBUSTA, true, 0>,
         (const void*)drop_phase2_kernel<PCT_ROBUSTB, false, 0>,
-        (const void*)drop_phase2_kernel<PCT_DROP, false, 0, true>, (const void*)drop_phase2_kernel<PCT_DROP, true, 0, true>};
+        (const void*)drop_phase2_kernel<PCT_DROP, false, 0, true>, (const void*)drop_phase2_kernel<PCT_DROP, true, 0, true>,
+        (const void*)drop_phase2_kernel<PCT_DROP, false, 0, false, true>,
+        (const void*)drop_phase2_kernel<PCT_DROP, false, 1, false, true>};
     for (const void* k : kernels) {
         const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, percent);
         if (e != cudaSuccess) return e;
