@@ -799,14 +799,28 @@ __global__ void upsum_mask_kernel(const bf16* __restrict__ du, const bf16* __res
     }
 }
 
+// The sum over a CTA of 256 threads, in its first thread: one atomic per CTA on the address that all
+// share.  With one per warp, 19,000 of them, the loss took 34 us on 200x200x32 voxels.
+template <class T>
+__device__ __forceinline__ T cta_sum(T v)
+{
+    __shared__ T part[8];
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = v;
+    __syncthreads();
+    if (threadIdx.x == 0)
+        for (int w = 1; w < 8; ++w) v += part[w];
+    return v;
+}
+
 __global__ void count_kernel(const uint8_t* __restrict__ hull, long long V, unsigned long long* __restrict__ count)
 {
     unsigned long long n = 0;
     for (long long v = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; v < V;
          v += static_cast<long long>(gridDim.x) * blockDim.x)
         n += hull[v] ? 1 : 0;
-    for (int o = 16; o > 0; o >>= 1) n += __shfl_xor_sync(0xffffffffu, n, o);
-    if ((threadIdx.x & 31) == 0 && n) atomicAdd(count, n);
+    n = cta_sum(n);
+    if (threadIdx.x == 0 && n) atomicAdd(count, n);
 }
 
 // Masked mean-squared error over the hull voxels: loss += (y - t)^2 / count, and the gradient
@@ -825,8 +839,8 @@ __global__ void loss_kernel(const float* __restrict__ y, const float* __restrict
         reinterpret_cast<uint4*>(dy + v * 16)[0] = make_uint4(pack_bf16(g, 0.f), 0, 0, 0);
         reinterpret_cast<uint4*>(dy + v * 16)[1] = make_uint4(0, 0, 0, 0);
     }
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if ((threadIdx.x & 31) == 0) atomicAdd(loss, acc * inv);
+    const double sum = cta_sum(acc);
+    if (threadIdx.x == 0) atomicAdd(loss, sum * inv);
 }
 
 __global__ void nonfinite_kernel(const float* __restrict__ y, long long V, unsigned long long* __restrict__ count)
