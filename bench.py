@@ -31,21 +31,12 @@ import sys
 import time
 from pathlib import Path
 
-import ctypes as C
-
 import numpy as np
 
 ROOT = Path(__file__).resolve().parent
 sys.path.insert(0, str(ROOT))
 
 METRIC = "MLP+DROP histories/s/iter on 1 B200"
-# FP64 operations (add, subtract, multiply, divide; each one rounding) of one MLP point of the
-# exact walk, counted from find_MLP_path_GPU_tabulated (B.cu:9180-9244): Sigma_2 moments 9, its
-# determinant 3 (plus a float powf), its inverse 3 divisions, the first term 11 and its determinant
-# 3, each of the t and v solves 16, the rotation back 6, the three voxel indices 6, and the depth
-# and position recurrences 2 -- 75 in all.  The per-history setup (about 1% of a path's work) is
-# not counted.
-FP64_OPS_PER_MLP_POINT = 75
 UNIT = "histories/s"
 PEAKS_FALLBACK = {"hbm_gbs": 6650.0}
 
@@ -187,15 +178,6 @@ def profiled_traffic_per_history(kernel_name):
         return None
     try:
         return float(json.loads(p.read_text())["dram_bytes_per_history"])
-    except Exception:
-        return None
-
-
-def profiled_fp64_pipe_pct(kernel_name):
-    """FP64-pipe utilisation (%) of `kernel_name` from the committed ncu summary, if any."""
-    p = ROOT / "profiles" / f"{kernel_name}.json"
-    try:
-        return float(json.loads(p.read_text())["fp64_pipe_pct"])
     except Exception:
         return None
 
@@ -875,44 +857,17 @@ def main():
     bytes_per_launch = groups[dom] / prof[dom]["launches"]
     peaks, peak_kind = measured_peaks()
     achieved = bytes_per_launch / (avg_ms / 1000.0) / 1e9
-    kernel_name = {"path": "mlp_phase1_exact_kernel", "block": ("drop_phase2_kernel" if two_phase
+    kernel_name = {"path": "mlp_phase1_table_kernel", "block": ("drop_phase2_kernel" if two_phase
                                                                else "drop_block_exact_kernel")}[dom]
     tph = profiled_traffic_per_history(kernel_name)
     hbm = {"achieved": achieved, "peak": peaks["hbm_gbs"], "unit": "GB/s", "frac": achieved / peaks["hbm_gbs"],
            "peak_source": f"{peak_kind} hbm_gbs (MEASURED_PEAKS.json)", "algorithmic_bytes_per_launch": bytes_per_launch}
-    if dom == "path":
-        # the path kernel is bound by FP64 issue: its algorithmic work is FP64_OPS_PER_MLP_POINT
-        # operations per MLP point (loop trip), counted by pct_mlp_steps; the peak is this GPU's FP64
-        # FMA issue rate measured now (pct_fp64_fma_rate), one operation per instruction, because
-        # the exact mode keeps every multiply and add separately rounded (no contraction)
-        trips = torch.zeros(n, dtype=torch.int32, device=dev)
-        ctx.mlp_steps_device(0, n, trips)
-        sum_trips = float(trips[covered].to(torch.int64).sum().item())
-        rate = C.c_double(0.0)
-        st = ctx.lib.pct_fp64_fma_rate(local, C.byref(rate))
-        peak_tops = rate.value / 1e12 if st == 0 else None
-        ops_per_launch = FP64_OPS_PER_MLP_POINT * sum_trips / prof[dom]["launches"]
-        achieved_tops = ops_per_launch / (avg_ms / 1000.0) / 1e12
-        roofline = {"bound": "fp64", "achieved": achieved_tops, "peak": peak_tops, "unit": "TFLOP/s",
-                    "frac": (achieved_tops / peak_tops) if peak_tops else None,
-                    "traffic": (tph * n_cov / prof[dom]["launches"] if tph else None),
-                    "kernel": kernel_name,
-                    "peak_source": "measured in this run: FP64 FMA instructions/s of all SMs (pct_fp64_fma_rate), one "
-                                   "operation per instruction; MEASURED_PEAKS.json holds no FP64 figure",
-                    "peak_fma_2flop_tflops": 2 * peak_tops if peak_tops else None,
-                    "algorithmic_fp64_ops_per_launch": ops_per_launch,
-                    "fp64_ops_per_mlp_point": FP64_OPS_PER_MLP_POINT,
-                    "mlp_points_per_history": sum_trips / max(n_cov, 1),
-                    "kernel_ms_avg": avg_ms, "launches": prof[dom]["launches"],
-                    "mean_path_voxels": sum_n / max(n_cov, 1),
-                    "iteration_breakdown_ms": {g: prof[g]["ms"] for g in prof},
-                    "fp64_pipe_pct_profiled": profiled_fp64_pipe_pct(kernel_name),
-                    "hbm": hbm}
-    else:
-        roofline = {"bound": "hbm", **hbm, "traffic": (tph * n_cov / prof[dom]["launches"] if tph else None),
-                    "kernel": kernel_name, "kernel_ms_avg": avg_ms, "launches": prof[dom]["launches"],
-                    "mean_path_voxels": sum_n / max(n_cov, 1),
-                    "iteration_breakdown_ms": {g: prof[g]["ms"] for g in prof}}
+    # The path kernel is bound by instruction issue and the block kernel by the L2's reductions (profiles/);
+    # against a measured peak both stand by their algorithmic bytes.
+    roofline = {"bound": "hbm", **hbm, "traffic": (tph * n_cov / prof[dom]["launches"] if tph else None),
+                "kernel": kernel_name, "kernel_ms_avg": avg_ms, "launches": prof[dom]["launches"],
+                "mean_path_voxels": sum_n / max(n_cov, 1),
+                "iteration_breakdown_ms": {g: prof[g]["ms"] for g in prof}}
 
     # ---- e2e: same metric through the C ABI with host buffers (H2D of the histories and D2H of
     #      the image inside the timed region) ----

@@ -1230,7 +1230,7 @@ pct_status forward(pct_unet* n, const float* x0, const uint8_t* hull, float* ima
             a.relu = 1;
             a.out = n->act[l];
         }
-        UNET_CK(launch_conv_fwd(a, s), "conv3_fwd_kernel");
+        UNET_CK(launch_conv_fwd(a, s), "conv3_slab_kernel");
     }
     return PCT_OK;
 }
@@ -1255,7 +1255,7 @@ pct_status backward(pct_unet* n, cudaStream_t s)
         w.dw = n->grads + n->w_off[l];
         w.db = n->grads + n->b_off[l];
         w.status = n->status;
-        UNET_CK(launch_conv_wgrad(w, s), "conv3_wgrad_kernel");
+        UNET_CK(launch_conv_wgrad(w, s), "conv3_wgrad_slab_kernel");
         if (l == 0) break;
         // data gradient: conv of dz with the flipped, transposed weights
         ConvFwdArgs d{};
@@ -1275,7 +1275,7 @@ pct_status backward(pct_unet* n, cudaStream_t s)
             d.out = n->dz[L.input];
             d.mask = n->act[L.input];  // ReLU of the producing layer
         }
-        UNET_CK(launch_conv_fwd(d, s), "conv3_fwd_kernel (data gradient)");
+        UNET_CK(launch_conv_fwd(d, s), "conv3_slab_kernel (data gradient)");
         if (L.up) {
             const int src = L.input, cl = L.level + 1;
             upsum_mask_kernel<<<grid_for(n->nv[cl] * (L.cin / 8), 256), 256, 0, s>>>(
