@@ -1218,7 +1218,9 @@ __global__ void __launch_bounds__(128) hull_walks_kernel(PreGeom g, long long n,
 // mark in L2, bound by the walks' instructions; before the steps were shortened 768 threads took 1.75 ms,
 // 512 1.97 and 1024 (which spill) 1.74.  The
 // sort by more keys and the ranges take 65 us where the other walk's order takes 30, so few histories
-// stay with that (300,000 with few marks: 71 us against 45).
+// stay with that (300,000 with few marks: 71 us against 45).  Above the line the whole stage of 600,000
+// histories takes 338 us on 200x200x32 voxels (697 with the reference's steps and every mark in L2), 213 with
+// few marks (571), and 573 where a window holds one slice of 316x316 (773).
 constexpr long long kHullWindowMin = 1 << 19;
 constexpr int kHullKeys = 4096, kHullThreads = 768, kHullWindow = 200 * 1024;
 // histories between two additions of the window: a timed step enters a voxel once, so counts stay below 2^16
