@@ -183,6 +183,7 @@ constexpr int kSlabMaxRing = 6;
 constexpr int kSlabMaxSlices = 32;
 constexpr int kSlabMaxPositions = 512;
 constexpr int kSlabSmemLimit = 224 * 1024;  // dynamic; the per-block maximum (227 KB) also holds the static part
+constexpr int kSlabSlack = 4096 + 128;       // what unused rows read past the last plane, and the alignment
 
 struct SlabShape {
     int W, H, tiles_x, tiles_y;  // patch and patches
@@ -908,7 +909,8 @@ cudaError_t set_smem_limits()
 bool valid_channels(int c) { return c == 16 || c == 32 || c == 64 || c == 128; }
 
 // The slab kernel's shape for a convolution: the patch that covers the grid with the fewest patches
-// (rows of W + 2 positions, 128 positions in all), and the channels, slices and ring of a CTA with the
+// (rows of W + 2 positions, 128 positions in all) among those of which two slices fit beside the weights
+// of 16 channels (with 128 input channels a patch one row high may hold 223 positions, not 384), and the channels, slices and ring of a CTA with the
 // least estimated time.  The estimate takes per input slice the larger of its MMAs (32 + N/4 cycles each:
 // both operands are read from shared memory at 128 bytes a cycle) and its bytes at 48 a cycle, for each
 // of the CTAs that share an SM, or the latency of one request over the requests in flight; and once per
@@ -921,7 +923,7 @@ SlabShape slab_shape(int cin, int cout, int nx, int ny, int nz)
         int H = (128 - W) / (W + 2) + 1;
         if (H > ny) H = ny;
         const int positions = (W + 2) * (H + 2);
-        if (positions > kSlabMaxPositions) continue;
+        if (positions > kSlabMaxPositions || 2 * positions * 16 * (cin / 8) + 27 * cin * 16 * 2 + kSlabSlack > kSlabSmemLimit) continue;
         const int tx = (nx + W - 1) / W, ty = (ny + H - 1) / H;
         const long long cost = static_cast<long long>(tx) * ty * (256 + positions);
         if (fewest == 0 || cost < fewest) {
@@ -950,7 +952,7 @@ SlabShape slab_shape(int cin, int cout, int nx, int ny, int nz)
                 t.ahead = ring - 1 < 2 ? ring - 1 : 2;
                 t.weight_bytes = 27 * cin * nc * 2;
                 t.tiles = t.tiles_x * t.tiles_y * ((nz + zt - 1) / zt);
-                t.smem = ring * t.slice_bytes + t.weight_bytes + 4096 + 128;
+                t.smem = ring * t.slice_bytes + t.weight_bytes + kSlabSlack;
                 if (t.smem > kSlabSmemLimit) continue;
                 const int groups = cout / nc;
                 for (t.stages = 1; t.stages <= 2 && t.stages * zt * nc <= kTmemColumns; ++t.stages) {
