@@ -496,8 +496,41 @@ struct WgradShape {
 constexpr int kWgradLoaders = 256;
 constexpr int kWgradThreads = kWgradLoaders + 32;
 
+// The elements `which` (bits: output channels from co on) of a CTA's tiles [from, to), summed from memory and
+// added to dw: those whose accumulator is not finite.  The zeros of dZ between a patch's rows meet
+// values of X there, and an infinity or a NaN among these would reach taps that never see it.  The
+// check for it costs 1 us of 70 a call at 100x100x16, 32 to 32 channels, and none at 200x200x32.
 template <bool kPair>
-__global__ void __launch_bounds__(kWgradThreads) conv3_wgrad_slab_kernel(const __grid_constant__ ConvWgradArgs p,
+__device__ __forceinline__ void wgrad_direct(const ConvWgradArgs& p, const WgradShape& sh, int from, int to, unsigned which,
+                                          int half, int dz, int dy, int dx, int ci, int co)
+{
+    const int patches = sh.tiles_x * sh.tiles_y, sx = p.nx >> p.up, sy = p.ny >> p.up;
+    for (; which; which &= which - 1) {
+        const int c = co + __ffs(which) - 1;
+        float sum = 0.f;
+        for (int k = from; k < to && !isnan(sum); ++k) {
+            const int tile = blockIdx.x + k * sh.ctas, run = tile / patches, patch = tile - run * patches;
+            const int py = patch / sh.tiles_x, x0 = (patch - py * sh.tiles_x) * sh.W, y0 = py * 2, z0 = run * sh.zt;
+            for (int zi = z0 + half; zi < min(z0 + sh.zt, p.nz); zi += kPair ? 2 : 1) {
+                const int z = zi + 1 - dz;
+                if (z < 0 || z >= p.nz) continue;
+                for (int y = y0; y < min(y0 + 2, p.ny); ++y)
+#pragma unroll 4
+                    for (int x = x0; x < min(x0 + sh.W, p.nx); ++x) {
+                        const int yi = y + dy - 1, xi = x + dx - 1;
+                        float in = 0.f;
+                        if (yi >= 0 && yi < p.ny && xi >= 0 && xi < p.nx)
+                            in = __bfloat162float(p.in[((static_cast<size_t>(zi >> p.up) * sy + (yi >> p.up)) * sx + (xi >> p.up)) * p.cin + ci]);
+                        sum += in * __bfloat162float(p.dz[((static_cast<size_t>(z) * p.ny + y) * p.nx + x) * p.cout + c]);
+                    }
+            }
+        }
+        atomicAdd(p.dw + (static_cast<size_t>(c) * 27 + dz * 9 + dy * 3 + dx) * p.cin + ci, sum);
+    }
+}
+
+template <bool kPair>
+__global__ void __launch_bounds__(kWgradThreads, 2) conv3_wgrad_slab_kernel(const __grid_constant__ ConvWgradArgs p,
                                                                          const __grid_constant__ WgradShape sh)
 {
     constexpr int kXPlanes = kPair ? 2 : 4, kXLog = kPair ? 1 : 2;  // 8-channel planes of an input tile
@@ -572,7 +605,7 @@ __global__ void __launch_bounds__(kWgradThreads) conv3_wgrad_slab_kernel(const _
         const int half = kPair ? m >> 6 : 0, dy = (m >> 3) & 3;
         const int ci = ci0 + (kPair ? (m & 63) >> 5 : m >> 5) * 8 + (m & 7);
         int epochs = 0;
-        auto flush = [&]() {  // waits for the epoch's MMAs and adds its accumulators to dw
+        auto flush = [&](int from, int to) {  // waits for the MMAs of tiles [from, to) and adds their accumulators to dw
             if (!__all_sync(0xffffffffu, tc::mbar_wait(tc::smem_addr(&done), epochs++ & 1))) return false;
             tc::fence_after_sync();
             const uint32_t lane = tmem + (static_cast<uint32_t>(warp & 3) * 32u << 16);
@@ -584,10 +617,23 @@ __global__ void __launch_bounds__(kWgradThreads) conv3_wgrad_slab_kernel(const _
                 const int w = column / sh.co, co = co0 + column - w * sh.co;
                 const int dz = half + 2 - w;
                 if (dy < 3 && dz >= 0 && dz < 3) {
-                    float* to = p.dw + (static_cast<size_t>(co) * 27 + dz * 9 + dy * 3 + dx) * p.cin + ci;
+                    float finite = 0.f;
 #pragma unroll
-                    for (int i = 0; i < 16; ++i) atomicAdd(to + static_cast<size_t>(i) * 27 * p.cin, acc[i]);
+                    for (int i = 0; i < 16; ++i) finite = fmaf(acc[i], 0.f, finite);
+                    float* dw = p.dw + (static_cast<size_t>(co) * 27 + dz * 9 + dy * 3 + dx) * p.cin + ci;
+                    if (finite == 0.f) {
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) atomicAdd(dw + static_cast<size_t>(i) * 27 * p.cin, acc[i]);
+                    } else {
+                        unsigned direct = 0;
+#pragma unroll
+                        for (int i = 0; i < 16; ++i)
+                            if (isfinite(acc[i])) atomicAdd(dw + static_cast<size_t>(i) * 27 * p.cin, acc[i]);
+                            else direct |= 1u << i;
+                        wgrad_direct<kPair>(p, sh, from, to, direct, half, dz, dy, dx, ci, co);
+                    }
                 }
+                __syncwarp();
             }
             tc::fence_before_sync();
             __syncwarp();
@@ -637,10 +683,10 @@ __global__ void __launch_bounds__(kWgradThreads) conv3_wgrad_slab_kernel(const _
             }
             cp_async_commit();
             if (++pending > 1) announce(1);
-            if (requested > 0 && requested % sh.epoch == 0) ok = flush();
+            if (requested > 0 && requested % sh.epoch == 0) ok = flush(requested - sh.epoch, requested);
         }
         announce(0);
-        if (ok) ok = flush();
+        if (ok) ok = flush(requested > 0 ? (requested - 1) / sh.epoch * sh.epoch : 0, requested);
         if (sums && ok) {
             // lanes of the same plane
 #pragma unroll
