@@ -461,17 +461,19 @@ __global__ void __launch_bounds__(kSlabThreads) conv3_slab_kernel(const __grid_c
 // three MMAs with accumulators of their own.  So every voxel of X and dZ is brought once per CTA, and 27
 // taps cost three MMAs per 16 positions.
 //
-// Eight warps bring the tiles (two stages), sum dZ for the bias and add the results to dw with atomics;
-// the ninth issues the MMAs.  The tensor core's accumulation truncates, and its error grows by about
-// 1.4e-8 of the result per K step, so the accumulators are added to dw (and start again) after at most
-// `epoch` tiles.  A CTA computes 32 (or 16) x 32 (or 16) channels of dW for its
-// share of the tiles.
+// Eight warps bring the tiles (two stages), sum dZ for the bias, take each tile's accumulators into registers
+// and add the sums to dw with atomics; the ninth issues the MMAs.  The tensor core's accumulation truncates,
+// and its error grows by about 1e-8 of the result per K step: with accumulators of at least 96 steps the
+// error was up to 1.7 times that of shorter ones on small grids and deep layers.  A tile takes at most a few
+// tens, and reading it costs nothing, since the next tile arrives meanwhile.  A CTA computes 32 (or 16) x 32
+// (or 16) channels of dW for its share of the tiles.
 //
-// One pass, in us (the kernel that gathered each tap's rows by threads, 128 rows of dW a CTA, in
-// brackets): 200x200x32, 16 to 16 channels 80 (394), 32 to 16 upsampled 128 (643); 100x100x16, 32 to
-// 32 57 (160) with the bias sums (8) in it; 50x50x8, 64 to 64 22 (56); 25x25x4, 128 to 128 16 (18).
-// All layers of the 200x200x32 network 0.79 ms (3.23, and 0.22 for the bias sums).  The bytes brought
-// bound it: halos double X, and dZ is read with two more slices per run.
+// One pass, in us (in brackets with accumulators of 96 steps or more, then the kernel that gathered each
+// tap's rows by threads, 128 rows of dW a CTA): 200x200x32, 16 to 16 channels 52 (70, 394), 32 to 16 82
+// (120); 100x100x16, 32 to 32 24 (37, 160 with its bias sums), 64 to 32 35 (48); 50x50x8, 64 to 64 18 (18, 56),
+// 128 to 64 22 (28); 25x25x4, 128 to 128 15 (15, 18); 32 to 128 at 50x50x8 21 (18).  All layers of the
+// 200x200x32 network 0.68 ms (0.77; 3.23, and 0.22 for the bias sums).  The bytes brought bound it: halos
+// double X, and dZ is read with two more slices per run.
 struct ConvWgradArgs {
     const bf16* in;  // forward input, [nz>>up][ny>>up][nx>>up][cin]
     int cin, up;
@@ -487,7 +489,6 @@ struct WgradShape {
     int W, positions, steps;  // patch width, positions of an X plane (4 pitch), K steps of 16
     int tiles_x, tiles_y, zt; // patches, slices of a run
     int tiles, ctas;          // patches x runs, CTAs per channel tile
-    int epoch;                // tiles of a CTA between two additions of the accumulators to dw
     int ci_tiles, co_tiles, co;  // channel tiles, output channels of a tile
     int x_plane, x_slice, z_plane, z_slice, stage, smem;  // bytes
     unsigned columns;
@@ -496,19 +497,19 @@ struct WgradShape {
 constexpr int kWgradLoaders = 256;
 constexpr int kWgradThreads = kWgradLoaders + 32;
 
-// The elements `which` (bits: output channels from co on) of a CTA's tiles [from, to), summed from memory and
+// The elements `which` (bits: output channels from co on) of a CTA's tiles, summed from memory and
 // added to dw: those whose accumulator is not finite.  The zeros of dZ between a patch's rows meet
 // values of X there, and an infinity or a NaN among these would reach taps that never see it.  The
 // check for it costs 1 us of 70 a call at 100x100x16, 32 to 32 channels, and none at 200x200x32.
 template <bool kPair>
-__device__ __forceinline__ void wgrad_direct(const ConvWgradArgs& p, const WgradShape& sh, int from, int to, unsigned which,
+__device__ __forceinline__ void wgrad_direct(const ConvWgradArgs& p, const WgradShape& sh, int tiles, unsigned which,
                                           int half, int dz, int dy, int dx, int ci, int co)
 {
     const int patches = sh.tiles_x * sh.tiles_y, sx = p.nx >> p.up, sy = p.ny >> p.up;
     for (; which; which &= which - 1) {
         const int c = co + __ffs(which) - 1;
         float sum = 0.f;
-        for (int k = from; k < to && !isnan(sum); ++k) {
+        for (int k = 0; k < tiles && !isnan(sum); ++k) {
             const int tile = blockIdx.x + k * sh.ctas, run = tile / patches, patch = tile - run * patches;
             const int py = patch / sh.tiles_x, x0 = (patch - py * sh.tiles_x) * sh.W, y0 = py * 2, z0 = run * sh.zt;
             for (int zi = z0 + half; zi < min(z0 + sh.zt, p.nz); zi += kPair ? 2 : 1) {
@@ -529,8 +530,8 @@ __device__ __forceinline__ void wgrad_direct(const ConvWgradArgs& p, const Wgrad
     }
 }
 
-template <bool kPair>
-__global__ void __launch_bounds__(kWgradThreads, 2) conv3_wgrad_slab_kernel(const __grid_constant__ ConvWgradArgs p,
+template <bool kPair, int kCo>
+__global__ void __launch_bounds__(kWgradThreads, 1) conv3_wgrad_slab_kernel(const __grid_constant__ ConvWgradArgs p,
                                                                          const __grid_constant__ WgradShape sh)
 {
     constexpr int kXPlanes = kPair ? 2 : 4, kXLog = kPair ? 1 : 2;  // 8-channel planes of an input tile
@@ -538,16 +539,15 @@ __global__ void __launch_bounds__(kWgradThreads, 2) conv3_wgrad_slab_kernel(cons
     extern __shared__ uint8_t smem_raw[];
     __shared__ __align__(8) uint64_t full[2];
     __shared__ __align__(8) uint64_t empty[2];
-    __shared__ __align__(8) uint64_t done;     // an epoch's MMAs
-    __shared__ __align__(8) uint64_t flushed;  // an epoch's accumulators read
+    __shared__ __align__(8) uint64_t taken;  // a tile's accumulators read
     __shared__ uint32_t tmem_slot;
     __shared__ int failed;
     __shared__ uint32_t corner[272];  // row << 16 | column of a position
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     const uint32_t base = (tc::smem_addr(smem_raw) + 127u) & ~127u;
     const int pitch = sh.W + 2;
-    const int ci0 = blockIdx.y % sh.ci_tiles * 32, co0 = blockIdx.y / sh.ci_tiles * sh.co;
-    const int zc = sh.co >> 3, zcl = zc == 2 ? 1 : 2;  // 8-channel planes of dZ
+    const int ci0 = blockIdx.y % sh.ci_tiles * 32, co0 = blockIdx.y / sh.ci_tiles * kCo;
+    constexpr int zc = kCo >> 3, zcl = zc == 2 ? 1 : 2;  // 8-channel planes of dZ
     const int patches = sh.tiles_x * sh.tiles_y;
 
     if (warp == 8) tc::tmem_alloc(tc::smem_addr(&tmem_slot), sh.columns);
@@ -555,9 +555,8 @@ __global__ void __launch_bounds__(kWgradThreads, 2) conv3_wgrad_slab_kernel(cons
         tc::mbar_init(tc::smem_addr(&full[tid]), kWgradLoaders / 32);
         tc::mbar_init(tc::smem_addr(&empty[tid]), 1);
     }
-    if (tid == 2) tc::mbar_init(tc::smem_addr(&done), 1);
-    if (tid == 3) tc::mbar_init(tc::smem_addr(&flushed), kWgradLoaders / 32);
-    if (tid < 4) tc::mbar_init_fence();
+    if (tid == 2) tc::mbar_init(tc::smem_addr(&taken), kWgradLoaders / 32);
+    if (tid < 3) tc::mbar_init_fence();
     if (tid == 0) failed = 0;
     for (int q = tid; q < sh.positions; q += kWgradThreads) {
         const int row = q / pitch;
@@ -573,85 +572,31 @@ __global__ void __launch_bounds__(kWgradThreads, 2) conv3_wgrad_slab_kernel(cons
         const int x_units = sh.positions << kXLog, z_units = (sh.steps * 16) << zcl;
         const bool sums = p.db != nullptr && ci0 == 0;
         float bias[8] = {0, 0, 0, 0, 0, 0, 0, 0};  // of dZ plane tid % zc
-        bool ok = true;
-        int pending = 0, told = 0, requested = 0;
-        // Announces all but the newest `keep` requested tiles; this thread adds up the dZ units it brought.
-        auto announce = [&](int keep) {
-            if (keep == 0) cp_async_wait<0>();
-            else cp_async_wait<1>();
-            tc::fence_proxy_async();
-            __syncwarp();
-            for (; pending > keep; --pending) {
-                if ((tid & 31) == 0) tc::mbar_arrive(tc::smem_addr(&full[told & 1]));
-                if (sums) {
-                    const uint32_t from = base + (told & 1) * sh.stage + sh.zt * sh.x_slice + (tid & (zc - 1)) * sh.z_plane;
-                    for (int s = 1; s <= sh.zt; ++s)  // the run's own slices
-                        for (int u = tid; u < z_units; u += kWgradLoaders) {
-                            uint4 raw;
-                            asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
-                                         : "=r"(raw.x), "=r"(raw.y), "=r"(raw.z), "=r"(raw.w)
-                                         : "r"(from + s * sh.z_slice + (u >> zcl) * 16) : "memory");
-                            float f[8];
-                            unpack8(raw, f);
-#pragma unroll
-                            for (int i = 0; i < 8; ++i) bias[i] += f[i];
-                        }
-                }
-                ++told;
-            }
-        };
         // TMEM lane (row) m of the M side: plane, row shift and channel; upper half: the next slice
         const int m = (warp & 3) * 32 + (tid & 31);
         const int half = kPair ? m >> 6 : 0, dy = (m >> 3) & 3;
         const int ci = ci0 + (kPair ? (m & 63) >> 5 : m >> 5) * 8 + (m & 7);
-        int epochs = 0;
-        auto flush = [&](int from, int to) {  // waits for the MMAs of tiles [from, to) and adds their accumulators to dw
-            if (!__all_sync(0xffffffffu, tc::mbar_wait(tc::smem_addr(&done), epochs++ & 1))) return false;
+        const uint32_t lane = tmem + (static_cast<uint32_t>(warp & 3) * 32u << 16);
+        // The tiles' sums wait in registers, and go back to TMEM before they are added to dw, so that the code
+        // for that is there once (unrolled it cost 3 us of instruction fetches).
+        constexpr int n = kWindow * kCo, kBlocks = 3 * n / 16, kHeld = (kBlocks + 1) / 2;  // 16 columns each; of this warp
+        const int first = warp >> 2;
+        float sum[kHeld][16];
+#pragma unroll
+        for (int h = 0; h < kHeld; ++h)
+#pragma unroll
+            for (int i = 0; i < 16; ++i) sum[h][i] = 0.f;
+        bool ok = true;
+        int tiles = 0;  // requested so far
+        auto multiplied = [&](int k) {  // waits for the MMAs of tile k
+            const bool in_time = __all_sync(0xffffffffu, tc::mbar_wait(tc::smem_addr(&empty[k & 1]), (k >> 1) & 1));
             tc::fence_after_sync();
-            const uint32_t lane = tmem + (static_cast<uint32_t>(warp & 3) * 32u << 16);
-            const int n = kWindow * sh.co;
-            for (int b = warp >> 2; b < 3 * n / 16; b += 2) {  // 16 columns: one tap in x, dZ slice, output channels
-                float acc[16];
-                tc::tmem_load16(lane + b * 16, acc);
-                const int dx = b * 16 / n, column = b * 16 - dx * n;
-                const int w = column / sh.co, co = co0 + column - w * sh.co;
-                const int dz = half + 2 - w;
-                if (dy < 3 && dz >= 0 && dz < 3) {
-                    float finite = 0.f;
-#pragma unroll
-                    for (int i = 0; i < 16; ++i) finite = fmaf(acc[i], 0.f, finite);
-                    float* dw = p.dw + (static_cast<size_t>(co) * 27 + dz * 9 + dy * 3 + dx) * p.cin + ci;
-                    if (finite == 0.f) {
-#pragma unroll
-                        for (int i = 0; i < 16; ++i) atomicAdd(dw + static_cast<size_t>(i) * 27 * p.cin, acc[i]);
-                    } else {
-                        unsigned direct = 0;
-#pragma unroll
-                        for (int i = 0; i < 16; ++i)
-                            if (isfinite(acc[i])) atomicAdd(dw + static_cast<size_t>(i) * 27 * p.cin, acc[i]);
-                            else direct |= 1u << i;
-                        wgrad_direct<kPair>(p, sh, from, to, direct, half, dz, dy, dx, ci, co);
-                    }
-                }
-                __syncwarp();
-            }
-            tc::fence_before_sync();
-            __syncwarp();
-            if ((tid & 31) == 0) tc::mbar_arrive(tc::smem_addr(&flushed));
-            return true;
+            return in_time;
         };
-        for (int tile = blockIdx.x; tile < sh.tiles && ok; tile += sh.ctas, ++requested) {
+        for (int tile = blockIdx.x; tile < sh.tiles && ok; tile += sh.ctas, ++tiles) {
             const int run = tile / patches, patch = tile - run * patches, py = patch / sh.tiles_x;
             const int x0 = (patch - py * sh.tiles_x) * sh.W, y0 = py * 2, z0 = run * sh.zt;
-            const int stage = requested & 1;
-            if (requested >= 2) {
-                const uint32_t parity = (requested / 2 - 1) & 1;
-                if (!__all_sync(0xffffffffu, tc::mbar_test(tc::smem_addr(&empty[stage]), parity))) {
-                    if (pending > 0) announce(0);
-                    ok = __all_sync(0xffffffffu, tc::mbar_wait(tc::smem_addr(&empty[stage]), parity));
-                    if (!ok) break;
-                }
-            }
+            const int stage = tiles & 1;  // free: the MMAs of tile tiles - 2 have been waited for
             const uint32_t dst = base + stage * sh.stage, dst_z = dst + sh.zt * sh.x_slice;
             for (int u = tid; u < x_units; u += kWgradLoaders) {
                 const int q = u >> kXLog, c = u & (kXPlanes - 1);
@@ -682,11 +627,79 @@ __global__ void __launch_bounds__(kWgradThreads, 2) conv3_wgrad_slab_kernel(cons
                 }
             }
             cp_async_commit();
-            if (++pending > 1) announce(1);
-            if (requested > 0 && requested % sh.epoch == 0) ok = flush(requested - sh.epoch, requested);
+            cp_async_wait<0>();
+            tc::fence_proxy_async();
+            __syncwarp();
+            if ((tid & 31) == 0) tc::mbar_arrive(tc::smem_addr(&full[stage]));
+            if (sums) {  // this thread adds up the dZ units it brought
+                const uint32_t from = dst_z + (tid & (zc - 1)) * sh.z_plane;
+                for (int s = 1; s <= sh.zt; ++s)  // the run's own slices
+                    for (int u = tid; u < z_units; u += kWgradLoaders) {
+                        uint4 raw;
+                        asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
+                                     : "=r"(raw.x), "=r"(raw.y), "=r"(raw.z), "=r"(raw.w)
+                                     : "r"(from + s * sh.z_slice + (u >> zcl) * 16) : "memory");
+                        float f[8];
+                        unpack8(raw, f);
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) bias[i] += f[i];
+                    }
+            }
+            if (tiles == 0) continue;
+            ok = multiplied(tiles - 1);
+            if (!ok) break;
+#pragma unroll
+            for (int h = 0; h < kHeld; ++h)
+                if (2 * h + first < kBlocks) {
+                    float acc[16];
+                    tc::tmem_load16(lane + (2 * h + first) * 16, acc);
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) sum[h][i] += acc[i];
+                }
+            tc::fence_before_sync();
+            __syncwarp();
+            if ((tid & 31) == 0) tc::mbar_arrive(tc::smem_addr(&taken));
         }
-        announce(0);
-        if (ok) ok = flush(requested > 0 ? (requested - 1) / sh.epoch * sh.epoch : 0, requested);
+        ok = ok && tiles > 0 && multiplied(tiles - 1);
+        if (ok) {
+            if (tiles > 1) {
+#pragma unroll
+                for (int h = 0; h < kHeld; ++h)
+                    if (2 * h + first < kBlocks) {
+                        float acc[16];
+                        tc::tmem_load16(lane + (2 * h + first) * 16, acc);
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) acc[i] += sum[h][i];
+                        tc::tmem_store16(lane + (2 * h + first) * 16, acc);
+                    }
+                tc::tmem_store_wait();
+            }
+            for (int b = first; b < kBlocks; b += 2) {  // one tap in x, dZ slice, output channels
+                float acc[16];
+                tc::tmem_load16(lane + b * 16, acc);
+                const int dx = b * 16 / n, column = b * 16 - dx * n;
+                const int w = column / kCo, co = co0 + column - w * kCo;
+                const int dz = half + 2 - w;
+                if (dy < 3 && dz >= 0 && dz < 3) {
+                    float finite = 0.f;
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) finite = fmaf(acc[i], 0.f, finite);
+                    float* dw = p.dw + (static_cast<size_t>(co) * 27 + dz * 9 + dy * 3 + dx) * p.cin + ci;
+                    if (finite == 0.f) {
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) atomicAdd(dw + static_cast<size_t>(i) * 27 * p.cin, acc[i]);
+                    } else {
+                        unsigned direct = 0;
+#pragma unroll
+                        for (int i = 0; i < 16; ++i)
+                            if (isfinite(acc[i])) atomicAdd(dw + static_cast<size_t>(i) * 27 * p.cin, acc[i]);
+                            else direct |= 1u << i;
+                        wgrad_direct<kPair>(p, sh, tiles, direct, half, dz, dy, dx, ci, co);
+                    }
+                }
+                __syncwarp();
+            }
+        }
         if (sums && ok) {
             // lanes of the same plane
 #pragma unroll
@@ -701,25 +714,20 @@ __global__ void __launch_bounds__(kWgradThreads, 2) conv3_wgrad_slab_kernel(cons
         if (!ok) failed = 1;
     } else {
         const uint32_t leader = tc::elect_one();
-        const uint32_t n = kWindow * sh.co, idesc = tc::idesc_bf16_f32(static_cast<int>(n), true);
+        constexpr uint32_t n = kWindow * kCo;
+        const uint32_t idesc = tc::idesc_bf16_f32(static_cast<int>(n), true);
         const uint64_t a_base = tc::smem_desc(base, 128, pitch * 16), b_base = tc::smem_desc(base + sh.zt * sh.x_slice, 128, sh.z_plane);
         const uint32_t a_hi = static_cast<uint32_t>(a_base >> 32), b_hi = static_cast<uint32_t>(b_base >> 32);
         bool ok = true;
-        uint32_t started = 0;
         int k = 0;
         for (int tile = blockIdx.x; tile < sh.tiles && ok; tile += sh.ctas, ++k) {
             const int z0 = tile / patches * sh.zt, stage = k & 1;
-            if (k > 0 && k % sh.epoch == 0) {
-                tc::mma_commit_warp(tc::smem_addr(&done), leader);
-                ok = __all_sync(0xffffffffu, tc::mbar_wait(tc::smem_addr(&flushed), (k / sh.epoch - 1) & 1));
-                if (!ok) break;
-                tc::fence_after_sync();
-                started = 0;
-            }
-            ok = __all_sync(0xffffffffu, tc::mbar_wait(tc::smem_addr(&full[stage]), (k >> 1) & 1));
+            ok = __all_sync(0xffffffffu, tc::mbar_wait(tc::smem_addr(&full[stage]), (k >> 1) & 1)) &&
+                 (k == 0 || __all_sync(0xffffffffu, tc::mbar_wait(tc::smem_addr(&taken), (k - 1) & 1)));
             if (!ok) break;
             tc::fence_after_sync();
             const int slices = z0 + sh.zt < p.nz ? sh.zt : p.nz - z0;
+            uint32_t started = 0;
             for (int s = 0; s < slices; s += kPair ? 2 : 1) {
                 // the descriptors' address fields count 16 bytes: one position
                 uint32_t a = static_cast<uint32_t>(a_base) + ((stage * sh.stage + s * sh.x_slice) >> 4);
@@ -733,7 +741,6 @@ __global__ void __launch_bounds__(kWgradThreads, 2) conv3_wgrad_slab_kernel(cons
             }
             tc::mma_commit_warp(tc::smem_addr(&empty[stage]), leader);
         }
-        tc::mma_commit_warp(tc::smem_addr(&done), leader);
         if (!ok) failed = 1;
     }
     tc::fence_before_sync();
@@ -946,7 +953,7 @@ cudaError_t set_smem_limits()
     if (dev >= 0 && dev < 64 && done[dev]) return cudaSuccess;
     for (auto kernel : {conv3_slab_kernel<16>, conv3_slab_kernel<32>, conv3_slab_kernel<64>, conv3_slab_kernel<128>})
         if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSlabSmemLimit);
-    for (auto kernel : {conv3_wgrad_slab_kernel<false>, conv3_wgrad_slab_kernel<true>})
+    for (auto kernel : {conv3_wgrad_slab_kernel<false, 16>, conv3_wgrad_slab_kernel<false, 32>, conv3_wgrad_slab_kernel<true, 16>, conv3_wgrad_slab_kernel<true, 32>})
         if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSlabSmemLimit);
     if (e == cudaSuccess && dev >= 0 && dev < 64) done[dev] = true;
     return e;
@@ -1060,61 +1067,70 @@ cudaError_t launch_conv_fwd(const ConvFwdArgs& a, cudaStream_t s)
     }
 }
 
-// The weight gradient's shape: the patch width with the fewest K steps over the grid, and the run length
-// with the least estimated time (MMAs at 32 + N/4 cycles or bytes at 40 a cycle, whichever is more, the
-// first tile's bytes, which nothing overlaps, and the additions to dw).
+// The weight gradient's shape: patch width, run length and CTAs with the least estimated time among those whose
+// estimated error is at most that of a split of the voxels in chunks of 64 over 888 CTAs of 128 rows of
+// dW.  That was a kernel of one accumulation per CTA, whose errors are the bar.
+//  * Error, relative, fitted to those of both from 24x24x4 to 200x200x32 (within 10%): 1e-8 for each K step of
+//    an accumulator, its truncation, and 1.8e-8 times the root of the additions to an element of dw.
+//  * Time, cycles, fitted to 250 shapes of 18 layers (12% rms; the shape it picks is the fastest of those
+//    tried or within 10% of it): per tile its MMAs at 1.27 (32 + N/4) or its bytes at 16.4 a cycle,
+//    whichever is more, and 2600 for the rest; and the first tile's bytes, which nothing overlaps.
 WgradShape wgrad_shape(int cin, int cout, int nx, int ny, int nz)
 {
     const bool pair = cin == 16;
-    WgradShape best{};
-    int fewest = 0;
-    for (int W = 7; W <= 63; W += 8) {
-        const int cost = (nx + W - 1) / W * (2 * W + 2 + 16);
-        if (fewest == 0 || cost <= fewest) {
-            fewest = cost;
-            best.W = W;
-        }
-    }
     const int planes = pair ? 2 : 4;
-    best.positions = 4 * (best.W + 2);
-    best.steps = (2 * best.W + 2) / 16;
-    best.tiles_x = (nx + best.W - 1) / best.W;
-    best.tiles_y = (ny + 1) / 2;
+    WgradShape best{};
     best.ci_tiles = pair ? 1 : cin / 32;
     best.co = cout == 16 ? 16 : 32;
     best.co_tiles = cout / best.co;
-    best.x_plane = best.positions * 16;
-    best.x_slice = best.x_plane * planes;
-    best.z_plane = best.steps * 256;
-    best.z_slice = best.z_plane * (best.co / 8);
+    best.tiles_y = (ny + 1) / 2;
     const int n = (pair ? 4 : 3) * best.co;
     best.columns = 3 * n <= 256 ? 256 : 512;
     const int groups = best.ci_tiles * best.co_tiles;
-    // K steps of an accumulator: at most 96 (an error near 1.3e-6), or on larger grids what 888 CTAs of 128
-    // rows of dW would take
-    const long long share = (static_cast<long long>(nx) * ny * nz * ((27 * cin + 127) / 128)) / (16 * 888);
-    const int chain = static_cast<int>(share > 96 ? share : 96);
+    auto error = [](double steps, double additions) { return 1e-16 * steps * steps + 3.24e-16 * additions; };  // squared
+    const long long chunks = (static_cast<long long>(nx) * ny * nz + 63) / 64, rows = (27 * cin + 127) / 128;
+    const long long splits = (888 + rows - 1) / rows < chunks ? (888 + rows - 1) / rows : chunks;
+    const long long share = (chunks + splits - 1) / splits;
+    const long long parts = (chunks + share - 1) / share, halves = pair ? 2 : 1;  // halves: additions of a CTA to an element
+    const double allowed = error(4.0 * share, static_cast<double>(parts));
+    auto patch_cost = [&](int W) { return (nx + W - 1) / W * (2 * W + 2 + 16); };
+    int fewest = patch_cost(7);
+    for (int W = 15; W <= 63; W += 8)
+        if (patch_cost(W) < fewest) fewest = patch_cost(W);
     WgradShape chosen = best;
-    double least = 0.0;
-    for (int zt = pair ? 2 : 1; zt <= (pair ? nz + 1 : nz) && zt <= 32; zt += pair ? 2 : 1) {
-        WgradShape t = best;
-        t.zt = zt;
-        t.stage = (zt * t.x_slice + (zt + 2) * t.z_slice + 127) & ~127;
-        // rows that are not used read up to a pitch and a step past the last plane
-        t.smem = 2 * t.stage + (t.W + 24) * 16 + 128;
-        const int per_tile = (pair ? (zt + 1) / 2 : zt) * t.steps;
-        if (t.smem > kSlabSmemLimit || (per_tile > chain && chosen.smem != 0)) break;
-        t.epoch = chain / per_tile > 1 ? chain / per_tile : 1;
-        t.tiles = t.tiles_x * t.tiles_y * ((nz + zt - 1) / zt);
-        const int ctas = 148 / groups > 1 ? 148 / groups : 1;
-        t.ctas = ctas < t.tiles ? ctas : t.tiles;
-        const double laps = ceil(static_cast<double>(t.tiles) / t.ctas);
-        const double mma = (pair ? (zt + 1) / 2 : zt) * t.steps * 3.0 * (32 + n / 4.0);
-        const double load = (zt * t.x_slice + (zt + 2.0) * t.z_slice) / 40.0;
-        const double time = laps * ((mma > load ? mma : load) + 300.0) + load + ceil(laps / t.epoch) * (1000.0 + 10.0 * n);
-        if (least == 0.0 || time < least) {
-            least = time;
-            chosen = t;
+    double least = 0.0, nearest = 0.0;  // the nearest error, until one is allowed
+    for (int W = 7; W <= 63; W += 8) {
+        if (patch_cost(W) > fewest * 5 / 4) continue;
+        best.W = W;
+        best.positions = 4 * (W + 2);
+        best.steps = (2 * W + 2) / 16;
+        best.tiles_x = (nx + W - 1) / W;
+        best.x_plane = best.positions * 16;
+        best.x_slice = best.x_plane * planes;
+        best.z_plane = best.steps * 256;
+        best.z_slice = best.z_plane * (best.co / 8);
+        for (int zt = pair ? 2 : 1; zt <= (pair ? nz + 1 : nz) && zt <= 32; zt += pair ? 2 : 1) {
+            WgradShape t = best;
+            t.zt = zt;
+            t.stage = (zt * t.x_slice + (zt + 2) * t.z_slice + 127) & ~127;
+            // rows that are not used read up to a pitch and a step past the last plane
+            t.smem = 2 * t.stage + (t.W + 24) * 16 + 128;
+            const int per_tile = (pair ? zt / 2 : zt) * t.steps;
+            if (t.smem > kSlabSmemLimit || (per_tile > 4 * share && nearest != 0.0)) break;
+            t.tiles = t.tiles_x * t.tiles_y * ((nz + zt - 1) / zt);
+            const double mma = per_tile * 3.8 * (32 + n / 4.0), load = (zt * t.x_slice + (zt + 2.0) * t.z_slice) / 16.4;
+            for (const long long most : {148LL, groups * (parts / halves)}) {  // CTAs: all, or for as many additions
+                const long long ctas = (most < 148 ? most : 148) / groups;
+                t.ctas = static_cast<int>(ctas < 1 ? 1 : ctas < t.tiles ? ctas : t.tiles);
+                const int laps = (t.tiles + t.ctas - 1) / t.ctas;
+                const double time = laps * ((mma > load ? mma : load) + 2600.0) + load;
+                const double e = error(per_tile, static_cast<double>(t.ctas) * halves);
+                if (e <= allowed ? least == 0.0 || time < least : least == 0.0 && (nearest == 0.0 || e < nearest)) {
+                    if (e <= allowed) least = time;
+                    nearest = e;
+                    chosen = t;
+                }
+            }
         }
     }
     return chosen;
@@ -1127,8 +1143,9 @@ cudaError_t launch_conv_wgrad(const ConvWgradArgs& a, cudaStream_t s)
     const WgradShape sh = wgrad_shape(a.cin, a.cout, a.nx, a.ny, a.nz);
     if (sh.smem == 0) return cudaErrorInvalidConfiguration;
     const dim3 grid(sh.ctas, sh.ci_tiles * sh.co_tiles);
-    if (a.cin == 16) conv3_wgrad_slab_kernel<true><<<grid, kWgradThreads, sh.smem, s>>>(a, sh);
-    else conv3_wgrad_slab_kernel<false><<<grid, kWgradThreads, sh.smem, s>>>(a, sh);
+    const auto kernel = a.cin == 16 ? (a.cout == 16 ? conv3_wgrad_slab_kernel<true, 16> : conv3_wgrad_slab_kernel<true, 32>)
+                                    : (a.cout == 16 ? conv3_wgrad_slab_kernel<false, 16> : conv3_wgrad_slab_kernel<false, 32>);
+    kernel<<<grid, kWgradThreads, sh.smem, s>>>(a, sh);
     return cudaGetLastError();
 }
 
