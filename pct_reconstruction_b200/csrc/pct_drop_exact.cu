@@ -375,8 +375,10 @@ __device__ __forceinline__ float two_sum(float a, float b, float& e)
     return s;
 }
 
+// x is read as ordinary memory: the image update before this kernel writes it while this kernel's CTAs are
+// already there (they wait), and the read-only path wants data that no one writes while the kernel lives.
 template <int kAlgo, bool kDet, int kMixed, bool kSCurve = false, bool kMany = false>
-__global__ void __launch_bounds__(256, kSCurve ? 6 : kMany && kMixed ? 8 : 0) drop_phase2_kernel(Geometry g, const float* __restrict__ x, float2* __restrict__ acc,
+__global__ void __launch_bounds__(256, kSCurve ? 6 : kMany && kMixed ? 8 : 0) drop_phase2_kernel(Geometry g, const float* x, float2* __restrict__ acc,
                                                           float* __restrict__ normA, FixedAcc fx,
                                                           const float* __restrict__ WEPL,
                                                           const long long* __restrict__ offsets, long long offset_base,
@@ -406,13 +408,13 @@ __global__ void __launch_bounds__(256, kSCurve ? 6 : kMany && kMixed ? 8 : 0) dr
 #pragma unroll
         for (int m = 0; m < kRegEntries; m++)
             if (v[m] < npad) {
-                hi = two_sum(hi, __ldg(x + v[m]), e);
+                hi = two_sum(hi, x[v[m]], e);
                 lo = __fadd_rn(lo, e);
             }
         for (int j = lane + 32 * kRegEntries; j < n; j += 32) {
             const uint32_t u = __ldg(p + j);
             if (u < npad) {
-                hi = two_sum(hi, __ldg(x + u), e);
+                hi = two_sum(hi, x[u], e);
                 lo = __fadd_rn(lo, e);
             }
         }
@@ -456,10 +458,10 @@ __global__ void __launch_bounds__(256, kSCurve ? 6 : kMany && kMixed ? 8 : 0) dr
     double sum = 0.0;
 #pragma unroll
     for (int m = 0; m < kRegEntries; m++)
-        if (v[m] < npad) sum += (double)__ldg(x + v[m]);
+        if (v[m] < npad) sum += (double)x[v[m]];
     for (int j = lane + 32 * kRegEntries; j < n; j += 32) {
         const uint32_t u = __ldg(p + j);
-        if (u < npad) sum += (double)__ldg(x + u);
+        if (u < npad) sum += (double)x[u];
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
@@ -505,7 +507,7 @@ __global__ void __launch_bounds__(256, kSCurve ? 6 : kMany && kMixed ? 8 : 0) dr
         const double a_i_dot_a_i = L * L * n;
         const double residual = (double)__ldg(WEPL + id) - sum * L;
         auto add = [&](uint32_t u) {
-            const double psi = ((1.0 - (double)__ldg(x + u)) * g.eta) * g.psi_sign;
+            const double psi = ((1.0 - (double)x[u]) * g.eta) * g.psi_sign;
             put(u, (float)(g.lambda * (residual / (a_i_dot_a_i + psi))));
         };
 #pragma unroll

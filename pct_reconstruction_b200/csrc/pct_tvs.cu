@@ -89,8 +89,12 @@ __device__ __forceinline__ float eta_at(const TvsTable& t, int L)
     return (e >= 0 && e < t.len) ? t.eta[e] : 0.0f;
 }
 
+// The kernels of a repetition overlap (each lets the next one start), and x, G and the state are written by one
+// and read by the next after its wait: they are read as ordinary memory, without __restrict__, since the
+// read-only path wants data that no one writes while the kernel lives.
+
 // Forward differences at voxel v: gx = x[v+1]-x[v], gy = x[v+C]-x[v].
-__device__ __forceinline__ void forward_diff(const float* __restrict__ x, int v, int C, float& gx, float& gy)
+__device__ __forceinline__ void forward_diff(const float* x, int v, int C, float& gx, float& gy)
 {
     const float x0 = x[v];
     gx = __fsub_rn(x[v + 1], x0);
@@ -189,7 +193,7 @@ __device__ bool grid_sum(double (&v)[N], double* __restrict__ partials, unsigned
 }
 
 // generate_perturbation_array (B.cu:10246-10324) in gather form, ||G||^2 and TV(x).
-__global__ void __launch_bounds__(kTvsThreads) tvs_gradient_kernel(const float* __restrict__ x, float* __restrict__ G,
+__global__ void __launch_bounds__(kTvsThreads) tvs_gradient_kernel(const float* x, float* G,
                                                                  TvsDims d, TvsTable tab, TvsStep step,
                                                                  double* __restrict__ partials, unsigned nblocks,
                                                                  TvsState* st)
@@ -240,7 +244,7 @@ __global__ void __launch_bounds__(kTvsThreads) tvs_gradient_kernel(const float* 
 }
 
 // The perturbation direction v = G/||G|| (0 when ||G|| = 0), B.cu:10309-10316.
-__device__ __forceinline__ float direction(const float* __restrict__ G, int v, float norm)
+__device__ __forceinline__ float direction(const float* G, int v, float norm)
 {
     return norm != 0.0f ? over(G[v], norm) : 0.0f;
 }
@@ -254,8 +258,7 @@ __device__ __forceinline__ float perturbed(float x, bool in_hull, float beta, fl
 // B.cu:10499).  Every launch sums in the gradient kernel's order, so that a beta that changes nothing
 // gives TV(x) itself.
 template <int kTrials>
-__global__ void __launch_bounds__(kTvsThreads) tvs_trials_kernel(const float* __restrict__ x,
-                                                               const float* __restrict__ G,
+__global__ void __launch_bounds__(kTvsThreads) tvs_trials_kernel(const float* x, const float* G,
                                                                const uint8_t* __restrict__ hull, TvsDims d,
                                                                TvsTable tab, int base, int passes, double threshold,
                                                                double* __restrict__ partials, unsigned nblocks,
@@ -321,8 +324,8 @@ __global__ void __launch_bounds__(kTvsThreads) tvs_trials_kernel(const float* __
 }
 
 // image = x_TVS - beta v on hull voxels (apply_TVS_perturbation B.cu:10413).
-__global__ void tvs_apply_kernel(float* __restrict__ x, const float* __restrict__ G, const uint8_t* __restrict__ hull,
-                                 int nv, const TvsState* __restrict__ st, unsigned long long* counters)
+__global__ void tvs_apply_kernel(float* x, const float* G, const uint8_t* __restrict__ hull,
+                                 int nv, const TvsState* st, unsigned long long* counters)
 {
     allow_dependent_launch();
     grid_dependency_wait();
