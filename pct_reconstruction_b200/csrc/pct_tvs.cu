@@ -243,10 +243,11 @@ __global__ void __launch_bounds__(kTvsThreads) tvs_gradient_kernel(const float* 
     }
 }
 
-// The perturbation direction v = G/||G|| (0 when ||G|| = 0), B.cu:10309-10316.
+// The perturbation direction v = G/||G|| (0 when ||G|| = 0, NaN everywhere when ||G|| is NaN, as 0/NaN is),
+// B.cu:10309-10316.
 __device__ __forceinline__ float direction(const float* G, int v, float norm)
 {
-    return norm != 0.0f ? over(G[v], norm) : 0.0f;
+    return norm > 0.0f ? over(G[v], norm) : norm;
 }
 
 __device__ __forceinline__ float perturbed(float x, bool in_hull, float beta, float w)
