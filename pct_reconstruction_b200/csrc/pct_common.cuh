@@ -50,6 +50,7 @@ struct Geometry {
     double air_threshold;           // X_N_AIR_THRESHOLD with IDENTIFY_X_N_AIR, else -infinity
     const float* s_curve;           // S_CURVE_ON: s(k) for k < kSCurveEntries (device), else nullptr
     int dual_sided_s_curve;         // DUAL_SIDED_S_CURVE
+    int carveout;                   // shared-memory carve-out of an iteration's kernels (iteration_carveout)
 };
 
 // Entries of the S-curve table: one per index of a path of at most PCT_MLP_PATH_CAP entries.
@@ -109,22 +110,35 @@ struct HistorySoA {
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void allow_dependent_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
-// Launch `kernel`, with programmatic stream serialization when `pdl` is set.
+// Launch `kernel`, with programmatic stream serialization when `pdl` is set, and with a preferred shared-memory
+// carve-out (percent) unless it is negative.
 template <typename... KArgs, typename... Args>
-cudaError_t launch_kernel(bool pdl, void (*kernel)(KArgs...), unsigned grid, unsigned block, cudaStream_t stream,
-                          Args... args)
+cudaError_t launch_carved_kernel(bool pdl, int carveout, void (*kernel)(KArgs...), unsigned grid, unsigned block,
+                                 cudaStream_t stream, Args... args)
 {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(block);
     cfg.dynamicSmemBytes = 0;
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchAttribute attr[2];
     cfg.attrs = attr;
-    cfg.numAttrs = pdl ? 1 : 0;
+    if (pdl) {
+        attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (carveout >= 0) {
+        attr[cfg.numAttrs].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+        attr[cfg.numAttrs++].val.sharedMemCarveout = (unsigned)carveout;
+    }
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+
+template <typename... KArgs, typename... Args>
+cudaError_t launch_kernel(bool pdl, void (*kernel)(KArgs...), unsigned grid, unsigned block, cudaStream_t stream,
+                          Args... args)
+{
+    return launch_carved_kernel(pdl, -1, kernel, grid, block, stream, args...);
 }
 
 // Reference constants (B.h:741-754, 818).

@@ -75,6 +75,7 @@ Geometry make_geometry(const pct_config& c)
     g.air_threshold = c.IDENTIFY_X_N_AIR ? c.X_N_AIR_THRESHOLD : -INFINITY;
     g.s_curve = nullptr;  // set by pct_create once the table exists
     g.dual_sided_s_curve = c.DUAL_SIDED_S_CURVE;
+    g.carveout = -1;  // set with the path kernel
     return g;
 }
 
@@ -239,8 +240,6 @@ extern "C" pct_status pct_create(const pct_config* cfg_in, int device, pct_ctx**
             ctx->launches += 1;
             ctx->geo.s_curve = table;
         }
-        e = pct::set_iteration_carveout();
-        if (e != cudaSuccess) { st = ctx_fail(ctx, PCT_ERR_CUDA, "shared-memory carve-out", e); break; }
         e = cudaMalloc(&ctx->d_steps, (size_t)(ctx->kmax + 1) * sizeof(pct::StepConst));
         if (e != cudaSuccess) { st = ctx_fail(ctx, PCT_ERR_NOMEM, "cudaMalloc(steps)", e); break; }
         e = pct::launch_build_step_table(ctx->tables, ctx->geo.sigma_index_step, ctx->geo.poly_index_step, ctx->kmax,
@@ -260,6 +259,7 @@ extern "C" pct_status pct_create(const pct_config* cfg_in, int device, pct_ctx**
             ctx->launches += 1;
             ctx->mlp_table = pct::MlpTable{rows, buckets, shape.buckets, shape.frac_bits, shape.t_max, 1.0 / shape.width};
         }
+        ctx->geo.carveout = pct::iteration_carveout(ctx->geo, ctx->mlp_table.buckets > 0);
 
         // Image and accumulator, padded by one slice (z index SLICES is reachable, B.cu:11091).
         const size_t npad = (size_t)ctx->geo.padded_voxels;

@@ -776,27 +776,24 @@ cudaError_t launch_mlp_phase1_exact(const Geometry& g, const Tables& tab, const 
                                     double* chord, unsigned long long* counters, cudaStream_t stream)
 {
     if (count <= 0) return cudaSuccess;
+    cudaError_t e = cudaSuccess;
 #define PCT_PHASE1(T)                                                                                             \
     do {                                                                                                          \
         const unsigned blocks = (unsigned)((count + (T) - 1) / (T));                                              \
-        if (tb.buckets > 0)                                                                                       \
-            mlp_phase1_table_kernel<T><<<blocks, T, 0, stream>>>(g, tab, tb, steps, kmax, h, perm, count, offsets, \
-                                                                 offset_base, bounds, paths, path_n, chord, counters); \
-        else if (g.mixed_precision)                                                                               \
-            mlp_phase1_mixed_kernel<T><<<blocks, T, 0, stream>>>(g, tab, steps, kmax, h, perm, count, offsets,    \
-                                                                 offset_base, bounds, paths, path_n, chord, counters); \
-        else if (g.exact_fast_points)                                                                             \
-            mlp_phase1_exact_kernel<T, true><<<blocks, T, 0, stream>>>(                                           \
-                g, tab, steps, kmax, h, perm, count, offsets, offset_base, bounds, paths, path_n, chord, counters); \
-        else                                                                                                      \
-            mlp_phase1_exact_kernel<T, false><<<blocks, T, 0, stream>>>(                                          \
-                g, tab, steps, kmax, h, perm, count, offsets, offset_base, bounds, paths, path_n, chord, counters); \
+        auto launch = [&](auto kernel, auto... first) {                                                           \
+            e = launch_carved_kernel(false, g.carveout, kernel, blocks, T, stream, first..., steps, kmax, h, perm, count, \
+                                     offsets, offset_base, bounds, paths, path_n, chord, counters);               \
+        };                                                                                                        \
+        if (tb.buckets > 0) launch(mlp_phase1_table_kernel<T>, g, tab, tb);                                       \
+        else if (g.mixed_precision) launch(mlp_phase1_mixed_kernel<T>, g, tab);                                   \
+        else if (g.exact_fast_points) launch(mlp_phase1_exact_kernel<T, true>, g, tab);                           \
+        else launch(mlp_phase1_exact_kernel<T, false>, g, tab);                                                   \
     } while (0)
     if (g.path_cta_threads == 64) PCT_PHASE1(64);
     else if (g.path_cta_threads == 256) PCT_PHASE1(256);
     else PCT_PHASE1(128);
 #undef PCT_PHASE1
-    return cudaGetLastError();
+    return e;
 }
 
 cudaError_t launch_drop_phase2(const Geometry& g, const float* x, float2* acc, float* normA, const FixedAcc& fx,
@@ -809,8 +806,8 @@ cudaError_t launch_drop_phase2(const Geometry& g, const float* x, float2* acc, f
     const unsigned blocks = (unsigned)((count * 32 + threads - 1) / threads);
     cudaError_t e = cudaSuccess;
 #define PCT_PHASE2(ALGO, DET, MIXED, SC, MANY)                                                              \
-    e = launch_kernel(pdl, drop_phase2_kernel<ALGO, DET, MIXED, SC, MANY>, blocks, threads, stream, g, x, acc,  \
-                      normA, fx, WEPL, offsets, offset_base, paths, path_n, chord, begin, count)
+    e = launch_carved_kernel(pdl, g.carveout, drop_phase2_kernel<ALGO, DET, MIXED, SC, MANY>, blocks, threads, stream, \
+                             g, x, acc, normA, fx, WEPL, offsets, offset_base, paths, path_n, chord, begin, count)
     const bool many = count >= (long long)sm_count() * (g.mixed_precision ? kManyFloat : kManyDouble);
     if (g.projection_algorithm == PCT_ROBUSTA) {
         if (g.deterministic) PCT_PHASE2(PCT_ROBUSTA, true, 0, false, false);
@@ -834,41 +831,16 @@ cudaError_t launch_drop_phase2(const Geometry& g, const float* x, float2* acc, f
     return e;
 }
 
-// The carve-out, in percent of the largest shared memory an SM offers (228 KB on B200), for every kernel
-// of an iteration: 7 path CTAs keep 10 KB of list staging each, the rest is L1 for the table rows and
-// the gathers.  Measured on B200 (ms per iteration; 4M head / 600k small / 2M head mixed): 25% 6.94 /
-// 1.467 / 3.82 (6 path CTAs), 35% 6.59 / 1.471 / 3.46, 45% 6.64 / 1.466 / 3.47, 58% 6.69 / 1.482 /
-// 3.49, 75% 6.82 / 1.509 / 3.49, each kernel's own 6.85 / 2.172 / 3.47.
-#ifndef PCT_ITERATION_CARVEOUT
-#define PCT_ITERATION_CARVEOUT 40
-#endif
-
-cudaError_t set_iteration_carveout()
-{
-    const int percent = PCT_ITERATION_CARVEOUT;
-    if (percent < 0) return cudaSuccess;
-    const void* kernels[] = {
-        (const void*)mlp_phase1_exact_kernel<64, false>, (const void*)mlp_phase1_exact_kernel<128, false>,
-        (const void*)mlp_phase1_exact_kernel<256, false>, (const void*)mlp_phase1_exact_kernel<64, true>,
-        (const void*)mlp_phase1_exact_kernel<128, true>, (const void*)mlp_phase1_exact_kernel<256, true>,
-        (const void*)mlp_phase1_table_kernel<64>,
-        (const void*)mlp_phase1_table_kernel<128>, (const void*)mlp_phase1_table_kernel<256>,
-        (const void*)mlp_phase1_mixed_kernel<64>, (const void*)mlp_phase1_mixed_kernel<128>,
-        (const void*)mlp_phase1_mixed_kernel<256>,
-        (const void*)drop_phase2_kernel<PCT_DROP, false, 0>, (const void*)drop_phase2_kernel<PCT_DROP, true, 0>,
-        (const void*)drop_phase2_kernel<PCT_DROP, false, 1>, (const void*)drop_phase2_kernel<PCT_DROP, true, 1>,
-        (const void*)drop_phase2_kernel<PCT_DROP, false, 2>,
-        (const void*)drop_phase2_kernel<PCT_ROBUSTA, false, 0>, (const void*)drop_phase2_kernel<PCT_ROBUSTA, true, 0>,
-        (const void*)drop_phase2_kernel<PCT_ROBUSTB, false, 0>,
-        (const void*)drop_phase2_kernel<PCT_DROP, false, 0, true>, (const void*)drop_phase2_kernel<PCT_DROP, true, 0, true>,
-        (const void*)drop_phase2_kernel<PCT_DROP, false, 0, false, true>,
-        (const void*)drop_phase2_kernel<PCT_DROP, false, 1, false, true>};
-    for (const void* k : kernels) {
-        const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, percent);
-        if (e != cudaSuccess) return e;
-    }
-    return set_image_update_carveout(percent);
-}
+// The carve-out, in percent of the largest shared memory an SM offers (228 KB on B200).  An SM runs CTAs of
+// kernels with different carve-outs only after it has drained and been reconfigured, so the block chain's small
+// kernels, interleaved with path-kernel chunks, would wait for whole SMs to empty: all have the same.
+//  * With the table 7 path CTAs keep 10 KB of list staging each, the rest is L1 for the table rows and the
+//    gathers.  Measured on B200 (ms per iteration; 4M head / 600k small / 2M head mixed): 25% (6 path CTAs)
+//    6.68 / 1.450 / 3.36, 35% 6.38 / 1.461 / 3.16, 40% 6.39 / 1.459 / 3.15, 45% 6.43 / 1.468 / 3.17, 58%
+//    6.50 / 1.477 / 3.19, 75% 6.64 / 1.513 / 3.26, each kernel's own 6.73 / 2.261 / 3.37.
+//  * FP32 points (mixed precision without the table) keep no shared memory: the driver's choice, all of it L1
+//    for their table gathers.  2M head: 4.91 so, 25% 4.97, 40% 5.04, 58% 5.26.
+int iteration_carveout(const Geometry& g, bool table) { return g.mixed_precision && !table ? -1 : 40; }
 
 cudaError_t launch_drop_block_exact(const Geometry& g, const Tables& tab, const StepConst* steps, int kmax,
                                     const float* x, float2* acc, const HistorySoA& h, long long begin,

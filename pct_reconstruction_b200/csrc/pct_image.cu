@@ -125,17 +125,6 @@ __global__ void __launch_bounds__(256) image_update_robustb_kernel(float* __rest
 
 }  // namespace
 
-cudaError_t set_image_update_carveout(int percent)
-{
-    const void* kernels[] = {(const void*)image_update_kernel, (const void*)image_update_fixed_kernel,
-                             (const void*)image_update_comp_kernel, (const void*)image_update_robustb_kernel};
-    for (const void* k : kernels) {
-        const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, percent);
-        if (e != cudaSuccess) return e;
-    }
-    return cudaSuccess;
-}
-
 int sm_count()
 {
     static int n = 0;
@@ -158,24 +147,24 @@ cudaError_t launch_image_update(const Geometry& g, float* x, float2* acc, float*
     if (g.deterministic) {
         const long long want = ((long long)(num_voxels >> 1) + threads - 1) / threads;
         const int blocks = (int)(want < 1 ? 1 : (want < cap ? want : cap));
-        return launch_kernel(pdl, image_update_fixed_kernel, blocks, threads, stream, x, fx, num_voxels,
+        return launch_carved_kernel(pdl, g.carveout, image_update_fixed_kernel, blocks, threads, stream, x, fx, num_voxels,
                              g.air_threshold);
     }
     if (g.projection_algorithm == PCT_ROBUSTB) {
         const long long want = ((long long)num_voxels + threads - 1) / threads;
         const int blocks = (int)(want < 1 ? 1 : (want < cap ? want : cap));
-        return launch_kernel(pdl, image_update_robustb_kernel, blocks, threads, stream, x, acc, normA, num_voxels,
+        return launch_carved_kernel(pdl, g.carveout, image_update_robustb_kernel, blocks, threads, stream, x, acc, normA, num_voxels,
                              g.psi_sign, g.eta, g.air_threshold);
     }
     if (g.compensated && normA) {  // compensated FP32 accumulation: normA holds the errors
         const long long want = ((long long)num_voxels + threads - 1) / threads;
         const int blocks = (int)(want < 1 ? 1 : (want < cap ? want : cap));
-        return launch_kernel(pdl, image_update_comp_kernel, blocks, threads, stream, x, acc, normA, num_voxels,
+        return launch_carved_kernel(pdl, g.carveout, image_update_comp_kernel, blocks, threads, stream, x, acc, normA, num_voxels,
                              g.air_threshold);
     }
     const long long want = ((long long)(num_voxels >> 1) + threads - 1) / threads;
     const int blocks = (int)(want < 1 ? 1 : (want < cap ? want : cap));
-    return launch_kernel(pdl, image_update_kernel, blocks, threads, stream, x, acc, num_voxels, g.air_threshold);
+    return launch_carved_kernel(pdl, g.carveout, image_update_kernel, blocks, threads, stream, x, acc, num_voxels, g.air_threshold);
 }
 
 }  // namespace pct

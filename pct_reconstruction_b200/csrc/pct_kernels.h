@@ -9,13 +9,10 @@ namespace pct {
 // Streaming-multiprocessor count of the current device (cached after the first call).
 int sm_count();
 
-// One shared-memory carve-out for every kernel a captured DROP iteration runs concurrently (path
-// kernels, DROP block kernels, image updates), set on the current device.  An SM runs CTAs of
-// kernels with different carve-outs only after it has drained and been reconfigured, so the block
-// chain's small kernels, interleaved with path-kernel chunks that keep 10 KB of shared memory per
-// CTA, would otherwise wait for whole SMs to empty.
-cudaError_t set_iteration_carveout();
-cudaError_t set_image_update_carveout(int percent);
+// The shared-memory carve-out, in percent, of every kernel that a DROP iteration runs concurrently (path
+// kernels, DROP block kernels, image updates); -1: the driver's choice.  It goes with each launch, so that
+// contexts with other kernels on the same device keep theirs.
+int iteration_carveout(const Geometry& g, bool table);
 
 // Per-step MLP table entries 0..kmax on the device (entry 0 zero).
 // The S-curve table s(k), k < kSCurveEntries, of configuration c (pct_scurve.cu).
