@@ -258,15 +258,21 @@ __global__ void __launch_bounds__(kThreads, PCT_PHASE1_MIN_BLOCKS * 128 / kThrea
     path_n[perm[i]] = n;
 }
 
-// Without a table: reference-order points, or (kTryFast) a grid too large for the fixed-point positions.
-// Without the certain points' code in it, reference-order points take 10.11 ms for 3M head histories (11.04
-// with it, chosen at run time; 10.46 with 6 CTAs per SM, 10.22 with 8).
+// Without a table: reference-order points.  Without the certain points' code in it, they take 10.11 ms for 3M head
+// histories (11.04 with it, chosen at run time; 10.46 with 6 CTAs per SM, 10.22 with 8).
+// kTryFast: a grid too large for the fixed-point positions.  The certain points need more registers than 7 CTAs
+// have: the history's constants and its chord wait in shared memory, and the list leaves it in sectors of 8
+// entries.  500k histories on 1100x1100x8 voxels: 1.83 ms; with the constants in registers and each entry stored
+// by itself 2.22 (2.14 with 6 CTAs per SM, 2.23 with 5, 2.39 with 4).
 template <int kThreads, bool kTryFast>
 __global__ void __launch_bounds__(kThreads, 7 * 128 / kThreads) mlp_phase1_exact_kernel(
     Geometry g, Tables tab, const StepConst* __restrict__ steps, int kmax, HistorySoA h, const int* __restrict__ perm,
     long long count, const long long* __restrict__ offsets, long long offset_base, const int* __restrict__ bounds,
     uint32_t* __restrict__ paths, int* __restrict__ path_n, double* __restrict__ chord, unsigned long long* counters)
 {
+    constexpr int kPark = kTryFast ? kThreads * (int)sizeof(double) : 0;
+    __shared__ double park[kTryFast ? (kHistoryFields + 1) * kThreads : 1];
+    __shared__ uint32_t stage[kTryFast ? kThreads * (kPathChunk + 1) : 1];  // odd stride in words: no bank conflicts
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= count) return;
     const long long id = perm[i];
@@ -276,20 +282,33 @@ __global__ void __launch_bounds__(kThreads, 7 * 128 / kThreads) mlp_phase1_exact
         chord[id] = 0.0;
         return;
     }
-    uint32_t* out = paths + (offsets[i] - offset_base);
-    const WalkResult r = mlp_walk_exact<false, kTryFast>(
+    uint32_t* out = paths + (offsets[i] - offset_base);  // 32-byte aligned, cap a multiple of 8
+    uint32_t* mine = stage + (kTryFast ? threadIdx.x * (kPathChunk + 1) : 0);
+    auto send = [&](int j0) {
+        uint4* to = reinterpret_cast<uint4*>(out + j0);
+        to[0] = make_uint4(mine[0], mine[1], mine[2], mine[3]);
+        to[1] = make_uint4(mine[4], mine[5], mine[6], mine[7]);
+    };
+    const WalkResult r = mlp_walk_exact<false, kTryFast, kPark>(
         g, tab, steps, kmax, nullptr, __ldg(h.first_MLP_voxel + i), __ldg(h.x_entry + i), __ldg(h.y_entry + i),
         __ldg(h.z_entry + i), __ldg(h.x_exit + i), __ldg(h.y_exit + i), __ldg(h.z_exit + i),
         __ldg(h.xy_entry_angle + i), __ldg(h.xz_entry_angle + i), __ldg(h.xy_exit_angle + i),
         __ldg(h.xz_exit_angle + i), [&](int j, uint32_t v) {
-            if (j < cap) out[j] = v;
-        });
+            if (j >= cap) return;
+            if (!kTryFast) {
+                out[j] = v;
+                return;
+            }
+            mine[j % kPathChunk] = v;
+            if (j % kPathChunk == kPathChunk - 1) send(j - (kPathChunk - 1));
+        }, (uint32_t)__cvta_generic_to_shared(park + (kTryFast ? threadIdx.x : 0)));
     unsigned flags = r.flags;
     int n = r.n;
     if (n > cap) {
         flags |= kFlagPathOverflow;
         n = cap;
     }
+    if (kTryFast && n % kPathChunk) send(n - n % kPathChunk);  // the last sector, padded
     if (flags) count_flags(flags, counters);
     path_n[id] = n;
     chord[id] = r.chord;
@@ -840,7 +859,13 @@ cudaError_t launch_drop_phase2(const Geometry& g, const float* x, float2* acc, f
 //    6.50 / 1.477 / 3.19, 75% 6.64 / 1.513 / 3.26, each kernel's own 6.73 / 2.261 / 3.37.
 //  * FP32 points (mixed precision without the table) keep no shared memory: the driver's choice, all of it L1
 //    for their table gathers.  2M head: 4.91 so, 25% 4.97, 40% 5.04, 58% 5.26.
-int iteration_carveout(const Geometry& g, bool table) { return g.mixed_precision && !table ? -1 : 40; }
+//  * Certain points without the table keep 20.5 KB for each of 7 CTAs, which 58% holds (57% gives 6 CTAs).
+int iteration_carveout(const Geometry& g, bool table)
+{
+    if (table) return 40;
+    if (g.mixed_precision) return -1;
+    return g.exact_fast_points ? 58 : 40;
+}
 
 cudaError_t launch_drop_block_exact(const Geometry& g, const Tables& tab, const StepConst* steps, int kmax,
                                     const float* x, float2* acc, const HistorySoA& h, long long begin,

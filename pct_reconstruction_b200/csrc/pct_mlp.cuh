@@ -146,6 +146,58 @@ struct MlpHistory {
     double mag_tv;  // max(|t_in| + |t_out| + |T_2_1|, |z_in| + |z_out| + |V_2_1|): the guarded fast point's bound
 };
 
+// The same in shared memory, field f of this thread at byte address at + f * kStride, each loaded where it is
+// used: the loads are volatile, so that they stay inside the loop trip and the constants are not held in
+// registers across trips.
+constexpr int kHistoryFields = 15;
+static_assert(sizeof(MlpHistory) == kHistoryFields * sizeof(double), "MlpHistory is 15 doubles");
+template <int kStride>
+struct ParkedHistory {
+    template <int F>
+    struct Field {
+        uint32_t at;
+        __device__ __forceinline__ operator double() const
+        {
+            double v;
+            asm volatile("ld.shared.f64 %0, [%1 + %2];" : "=d"(v) : "r"(at), "n"(F * kStride));
+            return v;
+        }
+    };
+    Field<0> sin_term;
+    Field<1> cos_term;
+    Field<2> t_in;
+    Field<3> t_out;
+    Field<4> z_in;
+    Field<5> z_out;
+    Field<6> T_2_1;
+    Field<7> V_2_1;
+    Field<8> u_2;
+    Field<9> u_2_sq;
+    Field<10> two_u_2;
+    Field<11> u_2_poly_3_12;
+    Field<12> u_2_poly_2_6;
+    Field<13> u_2_poly_1_2;
+    Field<14> mag_tv;
+    Field<15> chord;  // the walk's, while it loops
+    __device__ __forceinline__ explicit ParkedHistory(uint32_t a)
+        : sin_term{a}, cos_term{a}, t_in{a}, t_out{a}, z_in{a}, z_out{a}, T_2_1{a}, V_2_1{a}, u_2{a}, u_2_sq{a}, two_u_2{a},
+          u_2_poly_3_12{a}, u_2_poly_2_6{a}, u_2_poly_1_2{a}, mag_tv{a}, chord{a}
+    {
+    }
+    __device__ __forceinline__ void park(const MlpHistory& h, double chord_length) const
+    {
+        const double* f = reinterpret_cast<const double*>(&h);
+#pragma unroll
+        for (int i = 0; i <= kHistoryFields; i++)
+            asm volatile("st.shared.f64 [%0], %1;" ::"r"(chord.at + i * kStride), "d"(i < kHistoryFields ? f[i] : chord_length) : "memory");
+    }
+    __device__ __forceinline__ MlpHistory all() const
+    {
+        return MlpHistory{sin_term, cos_term, t_in, t_out, z_in, z_out, T_2_1, V_2_1, u_2, u_2_sq, two_u_2, u_2_poly_3_12,
+                          u_2_poly_2_6, u_2_poly_1_2, mag_tv};
+    }
+};
+
 // MLP point (t_1, v_1) of one loop iteration (B.cu:9180-9226): Sigma_2 from the tables, its
 // inverse, the 2x2 solve for t and v.  Same operations, same order as the reference.
 struct Sigma2 {
@@ -154,7 +206,8 @@ struct Sigma2 {
 
 // The Sigma_2 moments of one point and their determinant (B.cu:9180-9186), in the reference's
 // operations and order.
-__device__ __forceinline__ Sigma2 sigma2_moments(const MlpHistory& h, const StepConst& st,
+template <class History>
+__device__ __forceinline__ Sigma2 sigma2_moments(const History& h, const StepConst& st,
                                                  const double* __restrict__ scattering, unsigned sigma_2_index)
 {
     Sigma2 m;
@@ -256,7 +309,8 @@ __device__ __forceinline__ bool guarded_indices(const Geometry& g, double x, dou
 
 // The fast point and its voxel (see above); false when the bound cannot prove the voxel.
 // h.mag_tv is |t_in| + |t_out| + |T_2_1| and the same for v, the larger of the two.
-__device__ __forceinline__ bool mlp_point_fast(const Geometry& g, const MlpHistory& h, const StepConst& st, double sigma_t2,
+template <class History>
+__device__ __forceinline__ bool mlp_point_fast(const Geometry& g, const History& h, const StepConst& st, double sigma_t2,
                                                double sigma_t2_theta2, double sigma_theta2, double det2, double d,
                                                double u_shifted, uint32_t& voxel)
 {
@@ -427,15 +481,17 @@ struct PathWriter {
 // One history's MLP.  emit(j, voxel) is called for every path entry j in order.  With kSumX the
 // walk also sums the padded image x over the path (reads beyond it are reported and count as 0);
 // without it x is not touched (the voxel list does not depend on the image).  kTryFast: with
-// EXACT_FAST_POINTS, points whose voxel is certain skip the reference's order of operations.
-template <bool kSumX, bool kTryFast = true, class Emit>
+// EXACT_FAST_POINTS, points whose voxel is certain skip the reference's order of operations.  kPark > 0 keeps the
+// history's constants and the chord in shared memory at `parked`, kPark bytes apart.
+template <bool kSumX, bool kTryFast = true, int kPark = 0, class Emit>
 __device__ __forceinline__ WalkResult mlp_walk_exact(const Geometry& g, const Tables& tab,
                                                      const StepConst* __restrict__ steps, int kmax,
                                                      const float* __restrict__ x, uint32_t first_MLP_voxel,
                                                      double x_in_object, double y_in_object, double z_in_object,
                                                      double x_out_object, double y_out_object, double z_out_object,
                                                      double xy_entry_angle, double xz_entry_angle,
-                                                     double xy_exit_angle, double xz_exit_angle, Emit emit)
+                                                     double xy_exit_angle, double xz_exit_angle, Emit emit,
+                                                     uint32_t parked = 0)
 {
     const double s = g.mlp_u_step;
     WalkResult r;
@@ -449,6 +505,8 @@ __device__ __forceinline__ WalkResult mlp_walk_exact(const Geometry& g, const Ta
     w.first(first_MLP_voxel);
     r.chord = effective_chord_length(g, (xy_entry_angle + xy_exit_angle) / 2.0, (xz_entry_angle + xz_exit_angle) / 2.0);
     r.aia = powf_square(r.chord);
+    const ParkedHistory<kPark> ph(parked);
+    if (kPark > 0) ph.park(m.h, r.chord);
 
     int k = 1;
     while (m.tables_ok && depth_2_go > s) {
@@ -457,22 +515,30 @@ __device__ __forceinline__ WalkResult mlp_walk_exact(const Geometry& g, const Ta
             break;
         }
         const StepConst& st = steps[k];
-        const Sigma2 m2 = sigma2_moments(m.h, st, tab.scattering_table, sigma_2_index);
         u_shifted += s;
         uint32_t voxel;
-        if (!(kTryFast && g.exact_fast_points &&
-              mlp_point_fast(g, m.h, st, m2.sigma_t2, m2.sigma_t2_theta2, m2.sigma_theta2,
-                             m2.determinant, depth_2_go, u_shifted, voxel))) {
+        auto point = [&](const auto& h) {
+            const Sigma2 m2 = sigma2_moments(h, st, tab.scattering_table, sigma_2_index);
+            if (kTryFast && g.exact_fast_points &&
+                mlp_point_fast(g, h, st, m2.sigma_t2, m2.sigma_t2_theta2, m2.sigma_theta2, m2.determinant, depth_2_go,
+                               u_shifted, voxel))
+                return;
+            MlpHistory all;
+            if constexpr (kPark > 0) all = h.all();
+            else all = h;
             double t_1, v_1;
-            mlp_point_rest(m.h, st, m2, depth_2_go, t_1, v_1);
-            voxel = mlp_voxel(g, m.h, u_shifted, t_1, v_1);
-        }
+            mlp_point_rest(all, st, m2, depth_2_go, t_1, v_1);
+            voxel = mlp_voxel(g, all, u_shifted, t_1, v_1);
+        };
+        if constexpr (kPark > 0) point(ph);
+        else point(m.h);
         w.visit(voxel);
         depth_2_go -= s;
         sigma_2_index -= g.sigma_index_step;
         k++;
     }
     r.n = w.n < kPathCap ? w.n : kPathCap;
+    if (kPark > 0) r.chord = ph.chord;
     return r;
 }
 
