@@ -246,20 +246,6 @@ extern "C" pct_status pct_create(const pct_config* cfg_in, int device, pct_ctx**
                                          ctx->d_steps, ctx->own_stream);
         if (e != cudaSuccess) { st = ctx_fail(ctx, PCT_ERR_CUDA, "step table kernel", e); break; }
         ctx->launches += 1;
-        const pct::MlpTableShape shape = pct::mlp_table_shape(ctx->geo, ctx->kmax);
-        ctx->path_key_scale = shape.buckets > 0 ? 1.0 / shape.width : 0.0;
-        if (shape.buckets > 0) {
-            const size_t row_bytes = align256((size_t)shape.rows * 2 * sizeof(float4));
-            e = cudaMalloc(&ctx->d_mlp_table, row_bytes + (size_t)shape.buckets * sizeof(pct::MlpBucket));
-            if (e != cudaSuccess) { st = ctx_fail(ctx, PCT_ERR_NOMEM, "cudaMalloc(MLP weights)", e); break; }
-            float4* rows = static_cast<float4*>(ctx->d_mlp_table);
-            pct::MlpBucket* buckets = reinterpret_cast<pct::MlpBucket*>(static_cast<char*>(ctx->d_mlp_table) + row_bytes);
-            e = pct::launch_build_mlp_table(ctx->tables, ctx->d_steps, ctx->geo, shape, rows, buckets, ctx->own_stream);
-            if (e != cudaSuccess) { st = ctx_fail(ctx, PCT_ERR_CUDA, "MLP weight table kernel", e); break; }
-            ctx->launches += 1;
-            ctx->mlp_table = pct::MlpTable{rows, buckets, shape.buckets, shape.frac_bits, shape.t_max, 1.0 / shape.width};
-        }
-        ctx->geo.carveout = pct::iteration_carveout(ctx->geo, ctx->mlp_table.buckets > 0);
 
         // Image and accumulator, padded by one slice (z index SLICES is reachable, B.cu:11091).
         const size_t npad = (size_t)ctx->geo.padded_voxels;
@@ -316,7 +302,51 @@ extern "C" pct_status pct_synchronize(pct_ctx* ctx)
     return PCT_OK;
 }
 
+namespace {
+
+// Whether the context's path kernel has, or will have, the table of MLP weights.
+bool has_mlp_table(const pct_ctx* ctx)
+{
+    return ctx->mlp_table_tried ? ctx->mlp_table.buckets > 0 : pct::mlp_table_shape(ctx->geo, ctx->kmax).buckets > 0;
+}
+
+// Builds the table of MLP weights when histories are loaded for the first time, or with the first path layout
+// (histories of the preprocessing): contexts that never run a path kernel do without the 2 ms and the memory.
+// Where memory is short the context goes on without it, for good.
+pct_status ensure_mlp_table(pct_ctx* ctx)
+{
+    if (ctx->mlp_table_tried) return PCT_OK;
+    const pct::MlpTableShape shape = pct::mlp_table_shape(ctx->geo, ctx->kmax);
+    if (shape.buckets > 0) {
+        const size_t row_bytes = align256((size_t)shape.rows * 2 * sizeof(float4));
+        cudaError_t e = cudaMalloc(&ctx->d_mlp_table, row_bytes + (size_t)shape.buckets * sizeof(pct::MlpBucket));
+        if (e == cudaSuccess) {
+            float4* rows = static_cast<float4*>(ctx->d_mlp_table);
+            pct::MlpBucket* buckets = reinterpret_cast<pct::MlpBucket*>(static_cast<char*>(ctx->d_mlp_table) + row_bytes);
+            e = pct::launch_build_mlp_table(ctx->tables, ctx->d_steps, ctx->geo, shape, rows, buckets, ctx->stream);
+            if (e != cudaSuccess) return ctx_fail(ctx, PCT_ERR_CUDA, "MLP weight table kernel", e);
+            ctx->launches += 1;
+            ctx->mlp_table = pct::MlpTable{rows, buckets, shape.buckets, shape.frac_bits, shape.t_max, 1.0 / shape.width};
+            ctx->path_key_scale = 1.0 / shape.width;
+        } else {
+            ctx->d_mlp_table = nullptr;
+            cudaGetLastError();
+        }
+    }
+    ctx->mlp_table_tried = true;
+    ctx->geo.carveout = pct::iteration_carveout(ctx->geo, ctx->mlp_table.buckets > 0);
+    return PCT_OK;
+}
+
+}  // namespace
+
 extern "C" pct_status pct_set_reconstruction_histories(pct_ctx* ctx, const pct_histories* h, int64_t n, pct_memory where)
+{
+    const pct_status st = pct::load_histories(ctx, h, n, where);
+    return st == PCT_OK && n > 0 && ctx->path_limit_bytes >= 0 ? ensure_mlp_table(ctx) : st;
+}
+
+pct_status pct::load_histories(pct_ctx* ctx, const pct_histories* h, long long n, pct_memory where)
 {
     if (!ctx || !h || n < 0 || n > 0x7fffffffLL) return PCT_ERR_ARG;
     const void* src[12] = {h->x_entry, h->y_entry, h->z_entry, h->x_exit, h->y_exit, h->z_exit,
@@ -502,6 +532,8 @@ pct_status prepare_layout(pct_ctx* ctx)
     ctx->sbs.clear();
     ctx->two_phase = false;
     if (ctx->path_limit_bytes >= 0 && n > 0) {
+        const pct_status st = ensure_mlp_table(ctx);
+        if (st != PCT_OK) return st;
         long long cap = ctx->layout_cap;
         if (n > cap) {
             long long c1 = 0, c2 = 0, c3 = 0, c4 = 0, c5 = 0, c6 = 0, c7 = 0;
@@ -1235,7 +1267,7 @@ extern "C" pct_status pct_mlp_paths(pct_ctx* ctx, int64_t start, int64_t n, int3
     cudaError_t e = pct::launch_mlp_paths_exact(ctx->geo, ctx->tables, ctx->d_steps, ctx->kmax, ctx->d_x, ctx->hist,
                                                 start, n, stride, dc, dv, dl, da, ctx->d_counters,
                                                 // the lists an iteration uses: see launch_mlp_phase1_exact
-                                                ctx->geo.mixed_precision && ctx->mlp_table.buckets == 0, ctx->stream);
+                                                ctx->geo.mixed_precision && !has_mlp_table(ctx), ctx->stream);
     if (e != cudaSuccess) {
         cudaFree(tmp);
         return ctx_fail(ctx, PCT_ERR_CUDA, "mlp_paths kernel", e);

@@ -23,6 +23,8 @@ void tvs_release(pct_tvs* t);
 const uint8_t* preproc_hull(pct_ctx* ctx);
 // Reserve device tracker arrays for n histories and return them (pct_preprocess.cu).
 pct_status preproc_reserve_tracker(pct_ctx* ctx, long long n, float* dst[kTrackerSlots]);
+// pct_set_reconstruction_histories but for the table of MLP weights, which is then left to the first layout.
+pct_status load_histories(pct_ctx* ctx, const pct_histories* h, long long n, pct_memory where);
 // Lay out path storage for the loaded histories (pct_context.cu); no-op when up to date.
 pct_status layout_prepare(pct_ctx* ctx);
 // The path kernel's gathered inputs (processing order) from position p on.
@@ -48,8 +50,10 @@ struct pct_ctx {
     pct::Tables tables{};
     pct::StepConst* d_steps = nullptr;
     int kmax = 0;
-    // table of MLP weights (EXACT_FAST_POINTS): rows and buckets in one allocation
+    // table of MLP weights (EXACT_FAST_POINTS): rows and buckets in one allocation, built with the first
+    // histories
     void* d_mlp_table = nullptr;
+    bool mlp_table_tried = false;
     pct::MlpTable mlp_table{};
     double path_key_scale = 0.0;  // path-order keys per cm of u_2 (the table's buckets)
     // image and accumulator, padded by one slice; one allocation (d_acc follows d_x) so that a

@@ -2197,7 +2197,7 @@ extern "C" pct_status pct_reconstruction_cuts(pct_ctx* ctx)
     h.xz_exit_angle = p->vec_geom[pct::kXZO];
     h.WEPL = p->vec_wepl;
     h.first_MLP_voxel = p->vec_first_voxel;
-    pct_status st = pct_set_reconstruction_histories(ctx, &h, total, PCT_DEVICE);
+    pct_status st = pct::load_histories(ctx, &h, total, PCT_DEVICE);
     // apply_history_sequence (B.cu:8691): the reconstruction order of the histories
     if (st == PCT_OK && ctx->cfg.RECON_HISTORY_ORDERING == PCT_PRIME_PERMUTATION)
         st = pct_apply_history_sequence(ctx, ctx->cfg.PRIME_OFFSET);
