@@ -63,17 +63,7 @@ __host__ __device__ constexpr uint32_t idesc_bf16_f32(int n, bool mn_major)
          | (static_cast<uint32_t>(kTileM >> 4) << 24);  // M / 16
 }
 
-__device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint64_t a, uint64_t b, uint32_t idesc,
-                                         uint32_t accumulate)
-{
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n"
-        :: "r"(tmem_d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate));
-}
-
-// The same for a warp that runs the issuing code with all its lanes: only the lane with leader != 0
+// D (+)= A B, for a warp that runs the issuing code with all its lanes: only the lane with leader != 0
 // issues.  Control flow and descriptors stay warp-uniform, so they live in uniform registers; issued
 // from a branch of one thread, an MMA of 128 x 48 x 16 took twice as long to issue as to execute.  A
 // descriptor is its high word and a low word whose address field counts 16 bytes.
@@ -101,12 +91,6 @@ __device__ __forceinline__ uint32_t elect_one()
     uint32_t is;
     asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.b32 %0, 1, 0, p;\n\t}\n" : "=r"(is));
     return is;
-}
-
-__device__ __forceinline__ void mma_commit(uint32_t mbar)
-{
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
-                 :: "r"(mbar) : "memory");
 }
 
 __device__ __forceinline__ void fence_before_sync() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
@@ -184,12 +168,6 @@ __device__ __forceinline__ void tmem_store16(uint32_t taddr, const float (&v)[16
            "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(taddr) : "memory");
 }
 __device__ __forceinline__ void tmem_store_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-
-// TMEM columns to allocate for an N-column accumulator: a power of two, at least 32.
-__host__ __device__ constexpr uint32_t tmem_columns(int n)
-{
-    return n <= 32 ? 32u : n <= 64 ? 64u : n <= 128 ? 128u : 256u;
-}
 
 }  // namespace tc
 }  // namespace pct
