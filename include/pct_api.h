@@ -521,6 +521,9 @@ pct_status pct_selftest_powf_square(int64_t n, uint64_t seed, int64_t* mismatche
  * every float f of magnitude in [2^-60, 2^60) and zero (the CPU oracle squares with f*f, so this
  * bounds each square behind an engine-vs-oracle tie). */
 pct_status pct_selftest_powf_square_max_ulp(int64_t* max_ulp);
+/* The backprojection's quotient by a reciprocal against the division, on n pairs of its ranges;
+ * *mismatches receives the number of pairs that differ (FBP images rely on it being 0). */
+pct_status pct_selftest_quotient(int64_t n, uint64_t seed, int64_t* mismatches);
 
 /* Measurement support (no reference counterpart).  pct_fp64_fma_rate: the FP64 fused-multiply-add
  * issue rate of `device` (FMA instructions per second, all SMs, timed with CUDA events), the peak

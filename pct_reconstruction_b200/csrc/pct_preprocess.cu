@@ -532,12 +532,43 @@ constexpr int kBackSlices = 2;
 
 // a / b from b's correctly rounded reciprocal r: two steps of q + (a - q b) r from q = a r.  The first
 // leaves q within one unit in the last place, and from such a q the second gives the correctly rounded
-// quotient (Markstein, IBM J. Res. Dev. 34, 1990).  For a zero or well inside the range of double.
+// quotient (Markstein, IBM J. Res. Dev. 34, 1990).  For a zero or well inside the range of double; the sign of
+// a zero is lost.  pct_selftest_quotient compares it with the division.
 __device__ __forceinline__ double quotient(double a, double b, double r)
 {
     double q = a * r;
     q = __fma_rn(__fma_rn(-q, b, a), r, q);
     return __fma_rn(__fma_rn(-q, b, a), r, q);
+}
+
+// quotient(a, b, 1/b) against a / b over n pairs of the backprojection's ranges: a heights, distances and positions
+// up to 2^8 with exponents down to 2^-40, whole eighths, and zero; b ranges, bin sizes, and mantissas of all ones
+// and near ones.
+__global__ void quotient_check_kernel(long long n, unsigned long long seed, unsigned long long* mismatches)
+{
+    const long long stride = (long long)gridDim.x * blockDim.x;
+    unsigned long long local = 0, state = seed;
+    auto next = [&](unsigned long long counter) {  // splitmix64
+        unsigned long long z = state + counter * 0x9e3779b97f4a7c15ull;
+        z = (z ^ (z >> 30)) * 0xbf58476d1ce4e5b9ull;
+        z = (z ^ (z >> 27)) * 0x94d049bb133111ebull;
+        return z ^ (z >> 31);
+    };
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
+        const unsigned long long ra = next(2 * i + 1), rb = next(2 * i + 2), mantissa = 0xfffffffffffffull;
+        double a = __longlong_as_double((long long)((983 + (ra >> 52) % 48) << 52 | (ra & mantissa)));
+        double b = __longlong_as_double((long long)((1013 + (rb >> 52) % 20) << 52 | (rb & mantissa)));  // 2^-10 to 2^10
+        const int kind = (int)(i & 7);
+        if (kind == 1) b = __longlong_as_double(__double_as_longlong(b) | (long long)mantissa);
+        if (kind == 2) b = __longlong_as_double((__double_as_longlong(b) & ~(long long)mantissa) | (long long)(rb >> 40 & 15));
+        if (kind == 3) b = __longlong_as_double(__double_as_longlong(b) | (long long)(mantissa & ~15ull));
+        if (kind == 4) a = (double)((long long)(ra & 4095) - 2048) * 0.125;
+        if (kind == 5) b = (double)(1 + (rb & 1023)) * 0.05;
+        if (kind == 6) a = b * (double)(1 + (ra & 255));  // whole and nearly whole quotients
+        if (i & 8) a = -a;
+        if (quotient(a, b, __drcp_rn(b)) != a / b) local++;
+    }
+    if (local) atomicAdd(mismatches, local);
 }
 
 template <bool kRegular>
@@ -2421,5 +2452,20 @@ extern "C" pct_status pct_set_array(pct_ctx* ctx, const char* name, const void* 
                                 ctx->stream), "pct_set_array copy");
     PRE_TRY(cudaStreamSynchronize(ctx->stream), "pct_set_array sync");
     if (std::string(name) == "hull") ctx->pre->hull_ready = true;
+    return PCT_OK;
+}
+
+extern "C" pct_status pct_selftest_quotient(int64_t n, uint64_t seed, int64_t* mismatches)
+{
+    if (n < 0 || !mismatches) return PCT_ERR_ARG;
+    unsigned long long *d = nullptr, h = 0;
+    if (cudaMalloc(&d, sizeof(*d)) != cudaSuccess) return PCT_ERR_NOMEM;
+    cudaError_t e = cudaMemset(d, 0, sizeof(*d));
+    pct::quotient_check_kernel<<<148 * 4, 256>>>(n, seed, d);
+    if (e == cudaSuccess) e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaMemcpy(&h, d, sizeof(h), cudaMemcpyDeviceToHost);
+    cudaFree(d);
+    if (e != cudaSuccess) return PCT_ERR_CUDA;
+    *mismatches = (int64_t)h;
     return PCT_OK;
 }
