@@ -333,32 +333,38 @@ def secondary_measurements(cfg, ctx, hist, x0, stream, args):
     for i in range(2):
         ctx.DROP_full_tx_iteration(i + 1)
     x_exact = ctx.x_GPU_2_host().astype(np.float64)
-    m = Context(Config(**dict(workload_params(args.workload), PRECISION="MIXED")))
-    try:
-        m.set_stream(stream.cuda_stream)
-        m.set_reconstruction_histories(hist)
-        m.x_host_2_GPU(x0)
-        for i in range(2):
-            m.DROP_full_tx_iteration(i + 1)
-        x_mixed = m.x_GPU_2_host().astype(np.float64)
-        rmse = float(np.sqrt(np.mean((x_mixed - x_exact) ** 2)) / np.sqrt(np.mean(x_exact ** 2)))
-        ms_m = timed(m)
-        k = min(n, 1_000_000)
-        dt, dv, mism, ill = m.mlp_precision(0, k)
-        dev_mm = np.maximum(dt, dv) * 10.0
-        prof = m.profile_drop_iteration()
-        out["mixed_precision"] = {
-            "ms_per_iteration": ms_m, "histories_per_s": n / (ms_m / 1000.0),
-            "path_kernel_ms": prof["path"]["ms"],
-            "image_rel_rmse_vs_exact_2_iterations": rmse,
-            "sample_histories": k,
-            "histories_with_differing_voxel_steps": float(np.mean(mism > 0)),
-            "point_deviation_mm": {"p99": float(np.quantile(dev_mm, 0.99)), "p99.9": float(np.quantile(dev_mm, 0.999)),
-                                   "max": float(dev_mm.max())},
-            "histories_with_ill_conditioned_reference_steps": float(np.mean(ill > 0)),
-            "note": "deviation over steps where the reference's Sigma_2 is well conditioned"}
-    finally:
-        m.close()
+    # FP32 updates on the exact mode's path points (the table's), and on FP32 points, whose deviation is
+    # reported with them
+    for key, fast in (("mixed_precision", 1), ("mixed_precision_fp32_points", 0)):
+        m = Context(Config(**dict(workload_params(args.workload), PRECISION="MIXED", EXACT_FAST_POINTS=fast)))
+        try:
+            m.set_stream(stream.cuda_stream)
+            m.set_reconstruction_histories(hist)
+            m.x_host_2_GPU(x0)
+            for i in range(2):
+                m.DROP_full_tx_iteration(i + 1)
+            x_mixed = m.x_GPU_2_host().astype(np.float64)
+            rmse = float(np.sqrt(np.mean((x_mixed - x_exact) ** 2)) / np.sqrt(np.mean(x_exact ** 2)))
+            ms_m = timed(m)
+            out[key] = {"ms_per_iteration": ms_m, "histories_per_s": n / (ms_m / 1000.0),
+                        "path_kernel_ms": m.profile_drop_iteration()["path"]["ms"],
+                        "image_rel_rmse_vs_exact_2_iterations": rmse}
+            if fast:
+                out[key]["note"] = "FP32 updates; the voxel lists are the exact mode's"
+                continue
+            k = min(n, 1_000_000)
+            dt, dv, mism, ill = m.mlp_precision(0, k)
+            dev_mm = np.maximum(dt, dv) * 10.0
+            out[key].update({
+                "sample_histories": k,
+                "histories_with_differing_voxel_steps": float(np.mean(mism > 0)),
+                "point_deviation_mm": {"p99": float(np.quantile(dev_mm, 0.99)), "p99.9": float(np.quantile(dev_mm, 0.999)),
+                                       "max": float(dev_mm.max())},
+                "histories_with_ill_conditioned_reference_steps": float(np.mean(ill > 0)),
+                "note": "EXACT_FAST_POINTS = 0: FP32 path points too; deviation over steps where the reference's "
+                        "Sigma_2 is well conditioned"})
+        finally:
+            m.close()
     # the mixed mode with the compensated per-voxel accumulation (a returning atomic and a second
     # reduction per path entry)
     mc = Context(Config(**dict(workload_params(args.workload), PRECISION="MIXED_COMPENSATED")))
@@ -630,10 +636,11 @@ def precision_main(args):
     """--workload precision: the precision study on the small configuration's inputs (128x128x16,
     water cylinder with four inserts, 1 mm MLP step, blocks of 3200, 6 iterations) at 10M
     histories.  The FP64 reference is the exact mode (bit-identical voxel lists to the reference's
-    FP64 device code); against it: the mixed-precision MLP's point deviation (mm, over the steps
-    where the reference's Sigma_2 is well conditioned), histories whose voxel lists differ, and the
-    relative RSP RMSE after 6 iterations for mixed/exact x atomic/deterministic scatter, with the
-    atomic mode's own run-to-run RMSE as the floor."""
+    FP64 device code); against it: the FP32 path points' deviation (EXACT_FAST_POINTS = 0; mm, over the
+    steps where the reference's Sigma_2 is well conditioned), histories whose voxel lists then differ,
+    and the relative RSP RMSE after 6 iterations for mixed/exact x atomic/deterministic scatter, with the
+    atomic mode's own run-to-run RMSE as the floor.  Mixed precision with EXACT_FAST_POINTS = 1 walks the
+    exact mode's points."""
     import torch
     from pct_reconstruction_b200 import Config, Context
     from pct_reconstruction_b200 import replicas
@@ -649,8 +656,8 @@ def precision_main(args):
     iters = cfg0.ITERATIONS
     images, times, kernel_ms = {}, {}, {}
 
-    def run(precision, scatter, key):
-        c = Config(**dict(base, PRECISION=precision, SCATTER_MODE=scatter))
+    def run(precision, scatter, key, fast=1):
+        c = Config(**dict(base, PRECISION=precision, SCATTER_MODE=scatter, EXACT_FAST_POINTS=fast))
         with Context(c) as ctx:
             ctx.set_reconstruction_histories(hist)
             ctx.x_host_2_GPU(x0)
@@ -668,7 +675,7 @@ def precision_main(args):
             prof = ctx.profile_drop_iteration()
             kernel_ms[key] = {"path": prof["path"]["ms"], "drop_blocks": prof["block"]["ms"],
                               "image_updates": prof["update"]["ms"]}
-            if precision == "MIXED" and scatter == "ATOMIC":
+            if not fast:
                 dmax, mism_h, ill_h, steps_dev = 0.0, 0, 0, []
                 for s0 in range(0, n, 2_000_000):
                     k = min(2_000_000, n - s0)
@@ -690,7 +697,8 @@ def precision_main(args):
         run("EXACT", "DETERMINISTIC", "exact_det_again")
         run("EXACT", "ATOMIC", "exact_atomic")
         run("EXACT", "ATOMIC", "exact_atomic_again")
-        mlp = run("MIXED", "ATOMIC", "mixed_atomic")
+        run("MIXED", "ATOMIC", "mixed_atomic")
+        mlp = run("MIXED", "ATOMIC", "mixed_fp32_points_atomic", fast=0)
         run("MIXED_COMPENSATED", "ATOMIC", "mixed_compensated_atomic")
         run("MIXED", "DETERMINISTIC", "mixed_det")
     ref = images["exact_det"]
@@ -701,13 +709,14 @@ def precision_main(args):
             "scaling": "weak", "vs_baseline": None, "dtype": "f64/f32", "data": "synthetic",
             "config": {"workload": f"small plain pipeline inputs: 128x128x16 voxels, water cylinder with 4 inserts, "
                                    f"{n} reconstruction histories, 1 mm MLP step, blocks of 3200, {iters} iterations"},
-            "mlp": mlp,
+            "fp32_points": mlp,
             "rel_rmse_vs_exact_deterministic": {
                 "exact_deterministic_rerun": rel(images["exact_det_again"]),
                 "exact_atomic": rel(images["exact_atomic"]),
                 "exact_atomic_rerun_vs_exact_atomic": float(
                     np.sqrt(np.mean((images["exact_atomic_again"] - images["exact_atomic"]) ** 2)) / np.sqrt(np.mean(ref ** 2))),
                 "mixed_atomic": rel(images["mixed_atomic"]),
+                "mixed_fp32_points_atomic": rel(images["mixed_fp32_points_atomic"]),
                 "mixed_compensated_atomic": rel(images["mixed_compensated_atomic"]),
                 "mixed_deterministic": rel(images["mixed_det"])},
             "ms_per_iteration": times, "kernel_ms_per_iteration": kernel_ms, "clocks": clocks.summary()}

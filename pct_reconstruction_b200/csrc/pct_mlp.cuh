@@ -660,8 +660,7 @@ __device__ __forceinline__ TableWalk table_walk_start(const Geometry& g, const M
     // from the start 0.93 / 0.93.  (Not for lines along a voxel face: of 4M head histories 25 to 40 have eight points
     // that are not proven, and walking on without the table from the eighth made an iteration 150 us longer, the
     // time that one such walk takes on its own.)
-    if (fmin(fmin(fmin(px, px + reach * sx), fmin(py, py + reach * sy)), fmin(pz, pz - dz * g.inv_voxel_thickness)) < -2.0)
-        t.klast = t.early = 0;
+    if (fmin(fmin(px, px + reach * sx), fmin(py, py + reach * sy)) < -2.0) t.klast = t.early = 0;
     const float dt_max = tb.t_max, dz_max = kMaxOffset;
     if (fabsf(t.dt) * bk.max_b + fabsf(t.T) * bk.max_c >= dt_max || fabsf(t.dz) * bk.max_b + fabsf(t.V) * bk.max_c >= dz_max)
         while (t.klast > 0) {
@@ -688,9 +687,10 @@ __device__ __forceinline__ bool table_point(const Geometry& g, const MlpTable& t
     const int frac_bits = tb.frac_bits, left = 32 - frac_bits;
     const unsigned band = t.tol << 1;
     const bool proven = ((px << left) + t.tol >= band) & ((py << left) + t.tol >= band) & ((pz << left) + t.tol >= band) &
-                        ((int)(px | py | pz) >= 0) & (fabsf(lateral) < tb.t_max) & (fabsf(vertical) < kMaxOffset);
+                        ((int)(px | py) >= 0) & (fabsf(lateral) < tb.t_max) & (fabsf(vertical) < kMaxOffset);
+    // above the grid's top the index is mirrored (calculate_voxel_GPU takes |z - zero|); faces mirror with it
     voxel = (px >> frac_bits) + (py >> frac_bits) * (unsigned)g.columns +
-            (pz >> frac_bits) * (unsigned)(g.columns * g.rows);
+            ((unsigned)abs((int)pz) >> frac_bits) * (unsigned)(g.columns * g.rows);
     return proven;
 }
 
