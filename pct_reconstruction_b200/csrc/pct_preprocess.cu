@@ -958,6 +958,7 @@ struct CrossingTimes {
     unsigned stop;         // from here on a crossing may leave the grid
     unsigned lead;         // by which a crossing decides
     int exit_axis;         // the crossing that leaves the grid (kAxisNone: through its top)
+    bool above;            // more than half of the way lies beyond the grid's top, where every step is the reference's
 };
 
 // w: the walk's initial state; |dx|, |dy|, |dz|: the line's direction.  `error`: how far the reference's
@@ -998,6 +999,7 @@ __device__ __forceinline__ bool crossing_times(const PreGeom& g, const WalkLine&
     if (c.lead > min(min(c.bx, c.by), c.bz) / 8) return false;  // also tells the last crossing from the one before
     const double leave = 1073741824.0 - 2.0 * c.lead;
     c.stop = leave > 0.0 ? (unsigned)leave : 0u;
+    c.above = l.zd > 0 && end < 0.5 * fmin(ex, ey);
     c.exit_axis = ex == end ? kAxisX : ey == end ? kAxisY : l.zd > 0 ? kAxisNone : kAxisZ;
     return true;
 }
@@ -1009,15 +1011,33 @@ __device__ __forceinline__ bool crossing_times(const PreGeom& g, const WalkLine&
 // voxel.  `slopes` gives the line's slopes, only where a step needs them.
 // visit(voxel, step, timed) is also called without a step (step = false), with any voxel of the grid, and
 // returns false then; timed tells the steps by crossing times, which never enter a voxel twice.
-template <class Slopes, class Visit>
+enum WalkMode { kReferenceWalk, kTimedWalk, kMixedWalk };
+// kMode: every step the reference's, lane by lane (kReferenceWalk); by crossing times in the lanes that can
+// (kMixedWalk); kTimedWalk: by crossing times in the warps all of whose lanes can, and stay below the grid's top
+// for half of their way or more.  A lane without crossing times walks alone while the rest of its warp waits,
+// and then waits itself, where with all lanes in step the reference's steps take twice the time of the others.
+template <WalkMode kMode, class Slopes, class Visit>
 __device__ __forceinline__ int walk_3D(const PreGeom& g, const WalkLine& l, const CrossingTimes& times, bool fast, bool done,
                                        const Slopes& slopes, const Visit& visit, int max_steps, WalkState& w, bool& limit)
 {
+    limit = false;
+    if (kMode == kReferenceWalk || (kMode == kTimedWalk && __any_sync(0xffffffffu, !done && (!fast || times.above)))) {
+        if (done) return kAxisNone;
+        const WalkSlopes m = slopes();
+        for (int steps = 0; !done;) {
+            take_3D_step(g, l.xd, l.yd, l.zd, m.dy_dx, m.dz_dx, m.dz_dy, m.dx_dy, m.dx_dz, m.dy_dz, l.x0, l.y0, l.z0, w);
+            done = walk_outside(g, w) || visit(w.voxel, true, false);
+            if (!done && ++steps > max_steps) {
+                limit = true;
+                done = true;
+            }
+        }
+        return kAxisNone;
+    }
     CrossingTimes c = times;
     const int vx0 = w.vx, vy0 = w.vy, vz0 = w.vz;
     int voxel = w.voxel, before = voxel, extra = 0;  // before: the last step; extra: steps that did not move one index
     bool left = false;
-    limit = false;
     const bool walked = !done;
     if (done) voxel = before = 0;  // any index that may be looked at
     // a step that is not certain leaves its lane as it is, and so does every step after it, until the
@@ -1166,7 +1186,7 @@ __device__ __forceinline__ void hull_mark(const HullImages& im, int mask, int vo
 
 // The walk of history i, by all lanes of a warp (have = false: without one); count(voxel, timed) is called
 // for every voxel but the last.
-template <class Count>
+template <WalkMode kMode, class Count>
 __device__ __forceinline__ void hull_walk(const PreGeom& g, bool have, long long i, const GeomPtrs& G, const Count& count,
                                           unsigned long long* counters)
 {
@@ -1208,10 +1228,10 @@ __device__ __forceinline__ void hull_walk(const PreGeom& g, bool have, long long
     // the slopes are float quotients of dx, dy and dz, 2^-24 off each; a comparison involves up to four
     CrossingTimes times{};
     const bool flat = l.zd == 0;
-    const bool fast = !done && !flat && crossing_times(g, l, w, fabs((double)dx), fabs((double)dy), fabs((double)dz), 5.0e-7,
-                                                       times);
+    const bool fast = kMode != kReferenceWalk && !done && !flat && crossing_times(g, l, w, fabs((double)dx), fabs((double)dy), fabs((double)dz),
+                                                                 5.0e-7, times);
     bool limit;
-    walk_3D(g, l, times, fast, done || flat, slopes, mark, max_steps, w, limit);
+    walk_3D<kMode>(g, l, times, fast, done || flat, slopes, mark, max_steps, w, limit);
     if (flat && !done) {
         const WalkSlopes m = slopes();
         int steps = 0;
@@ -1229,6 +1249,7 @@ __device__ __forceinline__ void hull_walk(const PreGeom& g, bool have, long long
 }
 
 // One thread per history, every mark an atomic on its image: bound by the L2's atomics, 155 G/s.
+template <WalkMode kMode>
 __global__ void __launch_bounds__(128) hull_walks_kernel(PreGeom g, long long n, const int* __restrict__ order, GeomPtrs G,
                                                          const float* __restrict__ WEPL, const uint8_t* __restrict__ missed,
                                                          HullImages im, unsigned long long* counters)
@@ -1236,7 +1257,7 @@ __global__ void __launch_bounds__(128) hull_walks_kernel(PreGeom g, long long n,
     const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const long long i = k < n ? order[k] : 0;
     const int mask = k < n && !missed[i] ? hull_mask(g, im, WEPL[i]) : 0;
-    hull_walk(g, mask != 0, i, G, [&](int voxel, bool) { hull_mark(im, mask, voxel, 1); }, counters);
+    hull_walk<kMode>(g, mask != 0, i, G, [&](int voxel, bool) { hull_mark(im, mask, voxel, 1); }, counters);
 }
 
 // The same with the marks counted in shared memory.  All histories of one mask mark the same voxels in
@@ -1370,7 +1391,7 @@ __global__ void __launch_bounds__(kHullThreads, 1)
             first = __shfl_sync(0xffffffffu, first, 0);
             if (first >= last) break;
             const bool have = first + lane < last;
-            hull_walk(g, have, have ? order[first + lane] : 0, G,
+            hull_walk<kMixedWalk>(g, have, have ? order[first + lane] : 0, G,
                       [&](int voxel, bool timed) {
                           const unsigned local = (unsigned)(voxel - base);
                           if (timed && local < (unsigned)voxels) atomicAdd(window + (local >> 1), (local & 1) ? 0x10000u : 1u);
@@ -1513,6 +1534,7 @@ __global__ void hull_bits_kernel(long long words, long long n, const uint8_t* __
 // find_MLP_endpoints_GPU (B.cu:7581-7773): walk from the cylinder point along the straight line
 // (angle + PI when leaving) until the first hull voxel or the image edge.  All lanes of a warp call it;
 // lanes without a history (have = false) walk nothing.
+template <WalkMode kMode>
 __device__ __forceinline__ bool find_endpoint(const PreGeom& g, const uint32_t* __restrict__ bits, bool have, double x_start,
                                               double y_start, double z_start, double xy_angle, double xz_angle,
                                               double& x_object, double& y_object, double& z_object, int& voxel_x,
@@ -1557,10 +1579,10 @@ __device__ __forceinline__ bool find_endpoint(const PreGeom& g, const uint32_t* 
     const double turn = 1.2e-7 * fabs(xy_angle) + 1.0e-7;
     // an elevation beyond a right angle moves z against its own direction: left to the reference's steps
     const bool forward = (tan_xy > 0) == (l.xd * l.yd > 0) && (tan_xz > 0) == (l.xd * l.zd > 0);
-    const bool fast = !done && !flat && forward && crossing_times(g, l, w, scale, a_xy * scale, a_xz * scale,
+    const bool fast = kMode != kReferenceWalk && !done && !flat && forward && crossing_times(g, l, w, scale, a_xy * scale, a_xz * scale,
                                                        2.4e-6 + turn * (a_xy + 1.0 / a_xy), times);
     bool limit;
-    int axis = walk_3D(g, l, times, fast, done || flat, slopes, visit, max_steps - 1, w, limit);
+    int axis = walk_3D<kMode>(g, l, times, fast, done || flat, slopes, visit, max_steps - 1, w, limit);
     if (flat && !done) {
         // the reference's 2D loop of this walk (B.cu:7718-7752) keeps its slice index and its start height
         const double delta_yx = fabs(tan_xy);
@@ -1611,6 +1633,7 @@ __device__ __forceinline__ bool find_endpoint(const PreGeom& g, const uint32_t* 
 
 // collect_MLP_endpoints_GPU_nobool (B.cu:7819-7854).  Six CTAs per SM: 2.53 ms for 3.3M histories, five
 // 2.63 ms (before the steps were shortened: six 3.20 ms, four 4.26, eight, which spill, 3.34).
+template <WalkMode kMode>
 __global__ void __launch_bounds__(128, 6) endpoints_kernel(PreGeom g, long long n, const int* __restrict__ order,
                                                            const uint32_t* __restrict__ hull_bits, GeomPtrs G,
                                                            uint32_t* __restrict__ first_voxel, int* __restrict__ keep)
@@ -1624,8 +1647,8 @@ __global__ void __launch_bounds__(128, 6) endpoints_kernel(PreGeom g, long long 
     int vx = 0, vy = 0, vz = 0, vx2 = 0, vy2 = 0, vz2 = 0;
     double xin = 0, yin = 0, zin = 0, xout = 0, yout = 0, zout = 0;
     const bool entered =
-        find_endpoint(g, hull_bits, have, p[kXE], p[kYE], p[kZE], p[kXYE], p[kXZE], xin, yin, zin, vx, vy, vz, true);
-    const bool exited = find_endpoint(g, hull_bits, have && entered, p[kXO], p[kYO], p[kZO], p[kXYO], p[kXZO], xout, yout,
+        find_endpoint<kMode>(g, hull_bits, have, p[kXE], p[kYE], p[kZE], p[kXYE], p[kXZE], xin, yin, zin, vx, vy, vz, true);
+    const bool exited = find_endpoint<kMode>(g, hull_bits, have && entered, p[kXO], p[kYO], p[kZO], p[kXYO], p[kXZO], xout, yout,
                                       zout, vx2, vy2, vz2, false);
     if (!have) return;
     if (entered && exited) {
@@ -1986,8 +2009,8 @@ extern "C" pct_status pct_hull_detection(pct_ctx* ctx)
             } else {
                 int* order = walk_order(ctx, p, n, p->raw_geom, 1);
                 if (!order) return fail(ctx, PCT_ERR_CUDA, "walk order", cudaGetLastError());
-                pct::hull_walks_kernel<<<pct::grid_for(n, 128), 128, 0, s>>>(g, n, order, G, p->raw_wepl, p->missed, im,
-                                                                             ctx->d_counters);
+                const auto kernel = g.fast_walks ? pct::hull_walks_kernel<pct::kMixedWalk> : pct::hull_walks_kernel<pct::kReferenceWalk>;
+                kernel<<<pct::grid_for(n, 128), 128, 0, s>>>(g, n, order, G, p->raw_wepl, p->missed, im, ctx->d_counters);
                 ctx->launches += 1;
             }
         }
@@ -2184,8 +2207,14 @@ extern "C" pct_status pct_reconstruction_cuts(pct_ctx* ctx)
         const long long words = (ctx->cfg.NUM_VOXELS + 31LL) / 32;
         pct::hull_bits_kernel<<<pct::grid_for(words * 32, 256), 256, 0, s>>>(words, ctx->cfg.NUM_VOXELS, p->hull, p->hull_bits);
         ctx->launches += 1;
-        pct::endpoints_kernel<<<pct::grid_for(n, 128), 128, 0, s>>>(g, n, order, p->hull_bits, geom_ptrs(p->vec_geom),
-                                                                    p->vec_first_voxel, p->flags);
+        // grids lower than a fifth of their width: most lines leave through the top or the bottom.  500k histories,
+        // timed / mixed / reference steps, us: 200x200 voxels of 1 slice 424 / 777 / 424, 2 353 / 608 / 415, 4 520 / 648 /
+        // 637, 8 350 / 392 / 508; 128x128x16 188 / 182 / 278, 48x48x32 88 / 81 / 106, 200x200x32 41 / 37 / 29
+        const auto kernel = !g.fast_walks     ? pct::endpoints_kernel<pct::kReferenceWalk>
+                            : 10 * g.H <= 4 * g.R ? pct::endpoints_kernel<pct::kTimedWalk>
+                                                  : pct::endpoints_kernel<pct::kMixedWalk>;
+        kernel<<<pct::grid_for(n, 128), 128, 0, s>>>(g, n, order, p->hull_bits, geom_ptrs(p->vec_geom), p->vec_first_voxel,
+                                                     p->flags);
     }
     PRE_TRY(cudaGetLastError(), "endpoints kernel");
     ctx->launches += 1;
