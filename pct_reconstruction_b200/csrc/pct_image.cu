@@ -52,6 +52,11 @@ __global__ void __launch_bounds__(256) image_update_kernel(float* __restrict__ x
     }
 }
 
+// kPairs: two voxels per thread, all loads at once; one voxel where pairs leave SMs with little or no work.  A
+// block of DROP with kept paths and its update, singles / pairs, us: 64x64x16 voxels 4.09 / 4.72, 96x96x16 5.54 /
+// 5.64, 128x128x16 8.70 / 8.51, 200x200x32 22.6 / 22.0.
+constexpr int kPairedUpdate = 3 << 16;
+template <bool kPairs>
 __global__ void __launch_bounds__(256) image_update_fixed_kernel(float* __restrict__ x, FixedAcc fx, int num_voxels,
                                                                  double air)
 {
@@ -61,12 +66,26 @@ __global__ void __launch_bounds__(256) image_update_fixed_kernel(float* __restri
         const float xu = (float)((double)(long long)sum * (1.0 / kFixedScale));
         return air_cut(xv + __fdiv_rn(xu, (float)c), air);
     };
-    // two voxels per thread, all loads at once
-    const int stride = gridDim.x * blockDim.x, pairs = num_voxels >> 1;
+    const int stride = gridDim.x * blockDim.x, first = blockIdx.x * blockDim.x + threadIdx.x;
+    auto single = [&](int v) {
+        const unsigned c = fx.cnt[v];
+        const unsigned long long sum = fx.sum[v];
+        const float xv = x[v];
+        if (c > 0) {
+            x[v] = updated(xv, sum, c);
+            fx.sum[v] = 0ull;
+            fx.cnt[v] = 0u;
+        }
+    };
+    if (!kPairs) {
+        for (int v = first; v < num_voxels; v += stride) single(v);
+        return;
+    }
+    const int pairs = num_voxels >> 1;
     float2* __restrict__ x2 = reinterpret_cast<float2*>(x);
     ulonglong2* __restrict__ sum2 = reinterpret_cast<ulonglong2*>(fx.sum);
     uint2* __restrict__ cnt2 = reinterpret_cast<uint2*>(fx.cnt);
-    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < pairs; q += stride) {
+    for (int q = first; q < pairs; q += stride) {
         const uint2 c = cnt2[q];
         const ulonglong2 sum = sum2[q];
         float2 xv = x2[q];
@@ -78,14 +97,7 @@ __global__ void __launch_bounds__(256) image_update_fixed_kernel(float* __restri
             cnt2[q] = make_uint2(0u, 0u);
         }
     }
-    if ((num_voxels & 1) && blockIdx.x == 0 && threadIdx.x == 0) {
-        const int v = num_voxels - 1;
-        if (fx.cnt[v] > 0) {
-            x[v] = updated(x[v], fx.sum[v], fx.cnt[v]);
-            fx.sum[v] = 0ull;
-            fx.cnt[v] = 0u;
-        }
-    }
+    if ((num_voxels & 1) && first == 0) single(num_voxels - 1);
 }
 
 __global__ void __launch_bounds__(256) image_update_comp_kernel(float* __restrict__ x, float2* __restrict__ acc,
@@ -145,10 +157,11 @@ cudaError_t launch_image_update(const Geometry& g, float* x, float2* acc, float*
     const int threads = 256;
     const long long cap = (long long)sm_count() * 8;  // 8 resident 256-thread CTAs per SM
     if (g.deterministic) {
-        const long long want = ((long long)(num_voxels >> 1) + threads - 1) / threads;
+        const bool in_pairs = num_voxels >= kPairedUpdate;
+        const long long want = ((long long)(in_pairs ? num_voxels >> 1 : num_voxels) + threads - 1) / threads;
         const int blocks = (int)(want < 1 ? 1 : (want < cap ? want : cap));
-        return launch_carved_kernel(pdl, g.carveout, image_update_fixed_kernel, blocks, threads, stream, x, fx, num_voxels,
-                             g.air_threshold);
+        return launch_carved_kernel(pdl, g.carveout, in_pairs ? image_update_fixed_kernel<true> : image_update_fixed_kernel<false>,
+                                    blocks, threads, stream, x, fx, num_voxels, g.air_threshold);
     }
     if (g.projection_algorithm == PCT_ROBUSTB) {
         const long long want = ((long long)num_voxels + threads - 1) / threads;
