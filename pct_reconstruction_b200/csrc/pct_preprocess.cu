@@ -1268,11 +1268,13 @@ __global__ void __launch_bounds__(128) hull_walks_kernel(PreGeom g, long long n,
 // outside the window, and those of the reference's own steps, go to the images directly.
 // On the head scan (4M histories, 650M marks, windows of two slices) 1.61 ms against 4.21 ms with every
 // mark in L2, bound by the walks' instructions; before the steps were shortened 768 threads took 1.75 ms,
-// 512 1.97 and 1024 (which spill) 1.74.  The
-// sort by more keys and the ranges take 65 us where the other walk's order takes 30, so few histories
-// stay with that (300,000 with few marks: 71 us against 45).  Above the line the whole stage of 600,000
-// histories takes 338 us on 200x200x32 voxels (697 with the reference's steps and every mark in L2), 213 with
-// few marks (571), and 573 where a window holds one slice of 316x316 (773).
+// 512 1.97 and 1024 (which spill) 1.74.
+// The line lies where the windows win with any number of marks.  Order and walks of 300k / 600k / 1.2M histories,
+// us, windows and (every mark in L2): 200x200x32 voxels with all histories marked 362 / 455 / 753 (498 / 966 / 1877),
+// a third of them 132 / 174 / 250 (213 / 394 / 768), almost none 29 / 32 / 40 (24 / 36 / 60); 128x128x16 227 / 309 / 489
+// (467 / 873 / 1741), 121 / 164 / 219 (221 / 446 / 803), 27 / 29 / 37 (24 / 36 / 60); 316x316x8, a window of one slice, 512 /
+// 825 / 1574 (817 / 1565 / 2998), 246 / 326 / 468 (406 / 683 / 1370), 27 / 29 / 37 (25 / 37 / 60).  From 262,144 on, the
+// preprocessing of a 300,000-proton scan of a cylinder that fills the grid takes 1066 us where it takes 1037.
 constexpr long long kHullWindowMin = 1 << 19;
 constexpr int kHullKeys = 4096, kHullThreads = 768, kHullWindow = 200 * 1024;
 // histories between two additions of the window: a timed step enters a voxel once, so counts stay below 2^16
