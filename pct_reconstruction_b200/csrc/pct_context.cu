@@ -246,6 +246,22 @@ extern "C" pct_status pct_create(const pct_config* cfg_in, int device, pct_ctx**
                                          ctx->d_steps, ctx->own_stream);
         if (e != cudaSuccess) { st = ctx_fail(ctx, PCT_ERR_CUDA, "step table kernel", e); break; }
         ctx->launches += 1;
+        // memory of the table of MLP weights (built by ensure_mlp_table); where it cannot be had, the context goes
+        // on with the path kernel without a table
+        const pct::MlpTableShape shape = pct::mlp_table_shape(ctx->geo, ctx->kmax);
+        if (shape.buckets > 0) {
+            const size_t row_bytes = align256((size_t)shape.rows * 2 * sizeof(float4));
+            if (cudaMalloc(&ctx->d_mlp_table, row_bytes + (size_t)shape.buckets * sizeof(pct::MlpBucket)) == cudaSuccess) {
+                ctx->mlp_table = pct::MlpTable{static_cast<float4*>(ctx->d_mlp_table),
+                                               reinterpret_cast<pct::MlpBucket*>(static_cast<char*>(ctx->d_mlp_table) + row_bytes),
+                                               shape.buckets, shape.frac_bits, shape.t_max, 1.0 / shape.width};
+                ctx->path_key_scale = 1.0 / shape.width;
+            } else {
+                ctx->d_mlp_table = nullptr;
+                cudaGetLastError();
+            }
+        }
+        ctx->geo.carveout = pct::iteration_carveout(ctx->geo, ctx->mlp_table.buckets > 0);
 
         // Image and accumulator, padded by one slice (z index SLICES is reachable, B.cu:11091).
         const size_t npad = (size_t)ctx->geo.padded_voxels;
@@ -304,37 +320,19 @@ extern "C" pct_status pct_synchronize(pct_ctx* ctx)
 
 namespace {
 
-// Whether the context's path kernel has, or will have, the table of MLP weights.
-bool has_mlp_table(const pct_ctx* ctx)
-{
-    return ctx->mlp_table_tried ? ctx->mlp_table.buckets > 0 : pct::mlp_table_shape(ctx->geo, ctx->kmax).buckets > 0;
-}
-
 // Builds the table of MLP weights when histories are loaded for the first time, or with the first path layout
-// (histories of the preprocessing): contexts that never run a path kernel do without the 2 ms and the memory.
-// Where memory is short the context goes on without it, for good.
+// (histories of the preprocessing): contexts that never run a path kernel do without the 2 ms.
 pct_status ensure_mlp_table(pct_ctx* ctx)
 {
-    if (ctx->mlp_table_tried) return PCT_OK;
-    const pct::MlpTableShape shape = pct::mlp_table_shape(ctx->geo, ctx->kmax);
-    if (shape.buckets > 0) {
-        const size_t row_bytes = align256((size_t)shape.rows * 2 * sizeof(float4));
-        cudaError_t e = cudaMalloc(&ctx->d_mlp_table, row_bytes + (size_t)shape.buckets * sizeof(pct::MlpBucket));
-        if (e == cudaSuccess) {
-            float4* rows = static_cast<float4*>(ctx->d_mlp_table);
-            pct::MlpBucket* buckets = reinterpret_cast<pct::MlpBucket*>(static_cast<char*>(ctx->d_mlp_table) + row_bytes);
-            e = pct::launch_build_mlp_table(ctx->tables, ctx->d_steps, ctx->geo, shape, rows, buckets, ctx->stream);
-            if (e != cudaSuccess) return ctx_fail(ctx, PCT_ERR_CUDA, "MLP weight table kernel", e);
-            ctx->launches += 1;
-            ctx->mlp_table = pct::MlpTable{rows, buckets, shape.buckets, shape.frac_bits, shape.t_max, 1.0 / shape.width};
-            ctx->path_key_scale = 1.0 / shape.width;
-        } else {
-            ctx->d_mlp_table = nullptr;
-            cudaGetLastError();
-        }
+    if (ctx->mlp_table_built) return PCT_OK;
+    if (ctx->mlp_table.buckets > 0) {
+        const cudaError_t e = pct::launch_build_mlp_table(ctx->tables, ctx->d_steps, ctx->geo, pct::mlp_table_shape(ctx->geo, ctx->kmax),
+                                                          const_cast<float4*>(ctx->mlp_table.rows),
+                                                          const_cast<pct::MlpBucket*>(ctx->mlp_table.bucket), ctx->stream);
+        if (e != cudaSuccess) return ctx_fail(ctx, PCT_ERR_CUDA, "MLP weight table kernel", e);
+        ctx->launches += 1;
     }
-    ctx->mlp_table_tried = true;
-    ctx->geo.carveout = pct::iteration_carveout(ctx->geo, ctx->mlp_table.buckets > 0);
+    ctx->mlp_table_built = true;
     return PCT_OK;
 }
 
@@ -1267,7 +1265,7 @@ extern "C" pct_status pct_mlp_paths(pct_ctx* ctx, int64_t start, int64_t n, int3
     cudaError_t e = pct::launch_mlp_paths_exact(ctx->geo, ctx->tables, ctx->d_steps, ctx->kmax, ctx->d_x, ctx->hist,
                                                 start, n, stride, dc, dv, dl, da, ctx->d_counters,
                                                 // the lists an iteration uses: see launch_mlp_phase1_exact
-                                                ctx->geo.mixed_precision && !has_mlp_table(ctx), ctx->stream);
+                                                ctx->geo.mixed_precision && ctx->mlp_table.buckets == 0, ctx->stream);
     if (e != cudaSuccess) {
         cudaFree(tmp);
         return ctx_fail(ctx, PCT_ERR_CUDA, "mlp_paths kernel", e);

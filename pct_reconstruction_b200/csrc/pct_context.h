@@ -50,10 +50,10 @@ struct pct_ctx {
     pct::Tables tables{};
     pct::StepConst* d_steps = nullptr;
     int kmax = 0;
-    // table of MLP weights (EXACT_FAST_POINTS): rows and buckets in one allocation, built with the first
-    // histories
+    // table of MLP weights (EXACT_FAST_POINTS): rows and buckets in one allocation (null: none), built
+    // with the first histories
     void* d_mlp_table = nullptr;
-    bool mlp_table_tried = false;
+    bool mlp_table_built = false;
     pct::MlpTable mlp_table{};
     double path_key_scale = 0.0;  // path-order keys per cm of u_2 (the table's buckets)
     // image and accumulator, padded by one slice; one allocation (d_acc follows d_x) so that a
