@@ -676,7 +676,7 @@ __global__ void __launch_bounds__(128) build_mlp_table_kernel(Tables tab, const 
                                       (float)(0.5 * ((na.C - at(qc, za)) - (nb.C - at(qc, zb)))));
         rows[2 * (first + k - 1)] = rb;
         rows[2 * (first + k - 1) + 1] = rc;
-        double err_b = 0.0, err_c = 0.0;
+        double err_b = 0.0, err_c = 0.0, finite = 0.0;  // finite: NaN once a value is not
         for (int i = 0; i < 81; i++) {
             const double delta = (i / 9 % 3 - 1) * kSigmaUnit, eps = (i / 27 - 1) * eps_max;
             double zeta;
@@ -684,11 +684,18 @@ __global__ void __launch_bounds__(128) build_mlp_table_kernel(Tables tab, const 
             const float z = (float)zeta, sigma = (float)((delta + k * kappa * eps) * kInvSigmaUnit);
             err_b = fmax(err_b, fabs((double)table_weight(rb, z, sigma) - w.B));
             err_c = fmax(err_c, fabs((double)table_weight(rc, z, sigma) - w.C));
+            finite += 0.0 * (w.B + w.C + w.mag_num + w.mag_det);
         }
-        double ze;
-        const double eta = 4.0e-7 * n0.ratio + 6.0e-6 / (center - k * s);
-        const WeightNode ne = node(0.0, 0.0, 0.0, eta, ze);
-        const float eb = (float)(2.0 * err_b + 2.0 * fabs(ne.B - n0.B)), ec = (float)(2.0 * err_c + 2.0 * fabs(ne.C - n0.C));
+        double det_b = 0.0, det_c = 0.0;
+        for (int i = -1; i <= 1; i++) {
+            double ze;
+            const WeightNode w = node(i, 0.0, 0.0, 0.0, ze);
+            const WeightNode we = node(i, 0.0, 0.0, 4.0e-7 * w.ratio + 6.0e-6 / (center + 0.5 * i * width - k * s), ze);
+            det_b = fmax(det_b, fabs(we.B - w.B));
+            det_c = fmax(det_c, fabs(we.C - w.C));
+            finite += 0.0 * (we.B + we.C);
+        }
+        const float eb = (float)(2.0 * (err_b + det_b) + finite), ec = (float)(2.0 * (err_c + det_c));
         const float er = (float)(kBoundK * (n0.mag_num + 2.0 * n0.mag_det) * 2.0);
         e_b[k - 1] = eb;
         e_c[k - 1] = ec;

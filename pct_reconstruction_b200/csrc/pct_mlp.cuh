@@ -553,17 +553,21 @@ __device__ __forceinline__ WalkResult mlp_walk_exact(const Geometry& g, const Ta
 // poly_1_2(u_1) is nearly proportional to k.  So B and C are tabulated once per context
 // (build_mlp_table_kernel): for every bucket of u_2 (MLP_U_STEP wide, at most 0.05 cm) and every step
 // k, a quadratic in u_2 plus a linear term in sigma = delta + k kappa epsilon, as 8 floats, and per
-// bucket a bound on how far the tabulated weights can be from the ones the reference's operations
-// give.  The bound adds
+// bucket an estimate of how far the tabulated weights can be from the ones the reference's operations
+// give.  It adds
 //   * twice the largest difference between the float evaluation and the double-precision formula
 //     over a 9 x 3 x 3 grid of (u_2, delta, epsilon),
-//   * the change of B and C when Sigma_2 is scaled by the largest relative error of its determinant
-//     (powf's rounding and a scattering-table index one entry off), and
-//   * the forward rounding error bound of the guarded fast point (kBoundK) on the history's scale.
-// A point's voxel is accepted when its position is farther than that (plus the fixed-point and float
-// roundings below) from every voxel face, which leaves a few points in 10^5; those, and steps without
-// a usable row, are computed by the guarded fast point or in the reference's order.  The voxel list is
-// the reference's either way.
+//   * twice the largest change of B and C, over the bucket's ends and centre, when Sigma_2 is scaled by
+//     the largest relative error of its determinant (powf's rounding and a scattering-table index one
+//     entry off), and
+//   * twice the forward rounding error bound of the guarded fast point (kBoundK, some 8000 units in the last
+//     place where the evaluations differ by a few) at the bucket's centre, on the history's scale; its largest
+//     value over the grid instead made a head iteration 2% longer.
+// Sampled, not derived: the weights are smooth over a bucket (0.05 cm of u_2), and the factors of two stand
+// for what lies between the samples.  A point's voxel is accepted when its position is farther than that
+// (plus the fixed-point and float roundings below) from every voxel face, which leaves a few points in 10^5;
+// those, and steps without a usable row, are computed by the guarded fast point or in the reference's order.
+// In the tests' tens of millions of points every list is the reference's.
 //
 // The position is fixed point, in voxels from the grid's corner with frac_bits fraction bits: the
 // straight line u -> (u cos - t_in sin, u sin + t_in cos) advances in a 64-bit accumulator per axis,
@@ -674,7 +678,7 @@ __device__ __forceinline__ TableWalk table_walk_start(const Geometry& g, const M
     return t;
 }
 
-// The tabulated point of the step whose row is r0, r1: its voxel, and whether the bound proves it.
+// The tabulated point of the step whose row is r0, r1: its voxel, and whether the estimated error clears the faces.
 __device__ __forceinline__ bool table_point(const Geometry& g, const MlpTable& tb, const TableWalk& t, const float4& r0,
                                             const float4& r1, uint32_t& voxel)
 {
